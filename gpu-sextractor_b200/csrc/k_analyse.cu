@@ -9,6 +9,7 @@
 // a fixed lane order.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "pixmom.cuh"
 
 namespace sx {
 
@@ -95,14 +96,6 @@ __device__ unsigned warp_select(const unsigned *opix, int n, const float *cd, in
     return prefix;
 }
 
-// what the pixel pass of the robust preanalysis hands to its finishing
-// kernel (one thread per object)
-struct RobustRaw {
-    double mx, my, mx2, my2, mxy;
-    float rv, peak, cpeak;
-    int dnpix, area2, xmin, xmax, ymin, ymax, flags;
-};
-
 // what the pixel pass of examineiso hands to its finishing kernel
 struct ExamRaw {
     XSum stv, svar;
@@ -112,7 +105,8 @@ struct ExamRaw {
 };
 
 struct AnaArgs {
-    RobustRaw *raw;     // per-object scratch between the two robust kernels
+    MomentRaw *raw;     // per-object scratch between the robust kernels
+    int *biglist, *counts;  // objects summed by a whole block (list 5)
     ExamRaw *xraw;      // per-object scratch between the two examineiso kernels
     const float *cd, *sub, *back;
     const unsigned *opix;
@@ -130,130 +124,44 @@ struct AnaArgs {
 
 // Robust preanalysis of a deblended object over its final pixels
 // (src/cuda/cudaanalyse.cu:1906-2124); objects of level 0 kept the values of
-// the first preanalysis.  One warp per object sums over the pixels; the
-// moments, ellipse and area correction are finished by k_robust_finish, one
-// thread per object, so that the double-precision tail does not run on one
-// lane of a warp.
-__global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_analyse_robust(AnaArgs A) {
+// the first preanalysis.  One warp per object sums over the pixels (a block
+// over those of more than DA_WARP_MAX); the moments, ellipse and area
+// correction are finished by k_robust_finish, one thread per object, so that
+// the double-precision tail does not run on one lane of a warp.
+__global__ void __launch_bounds__(AN_WARPS * 32, 3) k_analyse_robust(AnaArgs A) {
     const int lane = threadIdx.x & 31;
     const int o = blockIdx.x * AN_WARPS + (threadIdx.x >> 5);
     if (o >= sx_count(A.nobj, A.nobj_dev) || A.O.level[o] == 0) return;
-    const int n = A.O.n[o], off = A.O.off[o], w = A.w, h = A.h;
-    const unsigned *pix = A.opix + off;
-    const float dthresh = A.O.dthr[o];
-    int flags = A.O.flags[o];
+    const int n = A.O.n[o];
+    if (n > DA_WARP_MAX) {
+        if (lane == 0) A.biglist[atomicAdd(A.counts + 5, 1)] = o;
+        return;
+    }
+    const unsigned *pix = A.opix + A.O.off[o];
+    PixBox b = pix_box(A.cd, A.sub, pix, lane, n, 32, A.wdiv, A.w);
+    pixbox_warp(b);
+    PixMoments M;
+    pix_moments(A.cd, A.sub, pix, 0, n, A.wdiv, A.w, b, A.O.dthr[o], M);
+    pix_moments_store(M, b, A.raw + o);
+}
 
-    // exact sums in double bins (hint: the object's filtered peak), or with
-    // XSum when a term falls outside them or the object is too large
-    const bool binned = n <= BS_MAX_TERMS;
-    BinSum brv;
-    bs_init(brv);
-    bool ok = binned;
-    const int top_c = bs_order(A.O.fdpeak[o]);
-    unsigned pk = 0u, cpk = 0u;
-    int xmin = 0x7fffffff, xmax = -1, ymin = 0x7fffffff, ymax = -1;
-    for (int i = lane; i < n; i += 32) {
-        unsigned p = __ldg(pix + i);
-        int y = (int)fdiv(p, A.wdiv), x = (int)p - y * w;
-        pk = max(pk, f2ord(__ldg(A.sub + p)));
-        float c = __ldg(A.cd + p);
-        cpk = max(cpk, f2ord(c));
-        if (binned) ok &= bs_add(brv, c, top_c);
-        xmin = min(xmin, x);
-        xmax = max(xmax, x);
-        ymin = min(ymin, y);
-        ymax = max(ymax, y);
+__global__ void __launch_bounds__(AN_WARPS * 32, 2) k_analyse_robust_big(AnaArgs A) {
+    __shared__ PixBlock sh;
+    const int nb = A.counts[5];
+    for (int i = blockIdx.x; i < nb; i += gridDim.x) {
+        const int o = A.biglist[i];
+        pix_moments_block(A.cd, A.sub, A.opix + A.O.off[o], A.O.n[o], A.wdiv, A.w, A.O.dthr[o], sh, A.raw + o);
     }
-    XSum srv;
-    if (__all_sync(0xffffffffu, ok)) {
-        srv = bs_to_xsum(bs_warp_sum(brv));
-    } else {
-        xs_init(srv);
-        for (int i = lane; i < n; i += 32) xs_add(srv, __ldg(A.cd + __ldg(pix + i)));
-        srv = xs_warp_sum(srv);
-    }
-    float peak = ord2f(warp_max_u(pk)), cpeak = ord2f(warp_max_u(cpk));
-    xmin = warp_min_i(xmin);
-    xmax = warp_max_i(xmax);
-    ymin = warp_min_i(ymin);
-    ymax = warp_max_i(ymax);
-    if (xmin == 0 || xmax == w - 1 || ymin == 0 || ymax == h - 1) flags |= SX_OBJ_TRUNC;
-    float rv = xs_float(srv);
-    double dth = dthresh, dthresh2 = (dth + peak) / 2.0;
-    // second pass: the moments' terms are below cpeak times the box sides
-    const int bx = 32 - __clz(xmax - xmin), by = 32 - __clz(ymax - ymin), tc = bs_order(cpeak) + 1;
-    BinSum bmx, bmy, bmx2, bmy2, bmxy, btv;
-    bs_init(bmx);
-    bs_init(bmy);
-    bs_init(bmx2);
-    bs_init(bmy2);
-    bs_init(bmxy);
-    bs_init(btv);
-    ok = binned;
-    const int tv_top = bs_order(peak);
-    int dnpix = 0, area2 = 0;
-    for (int i = lane; i < n; i += 32) {
-        unsigned p = __ldg(pix + i);
-        int yy = (int)fdiv(p, A.wdiv), x = (int)p - yy * w - xmin, y = yy - ymin;
-        float cval = __ldg(A.cd + p), val = __ldg(A.sub + p);
-        dnpix += val > dth;
-        area2 += val > dthresh2;
-        if (binned) {
-            ok &= bs_add(btv, val, tv_top);
-            ok &= bs_add(bmx, cval * x, tc + bx);
-            ok &= bs_add(bmy, cval * y, tc + by);
-            ok &= bs_add(bmx2, cval * x * x, tc + 2 * bx);
-            ok &= bs_add(bmy2, cval * y * y, tc + 2 * by);
-            ok &= bs_add(bmxy, cval * x * y, tc + bx + by);
-        }
-    }
-    dnpix = warp_sum_i(dnpix);
-    area2 = warp_sum_i(area2);
-    XSum stv, smx, smy, smx2, smy2, smxy;
-    if (__all_sync(0xffffffffu, ok)) {
-        stv = bs_to_xsum(bs_warp_sum(btv));
-        smx = bs_to_xsum(bs_warp_sum(bmx));
-        smy = bs_to_xsum(bs_warp_sum(bmy));
-        smx2 = bs_to_xsum(bs_warp_sum(bmx2));
-        smy2 = bs_to_xsum(bs_warp_sum(bmy2));
-        smxy = bs_to_xsum(bs_warp_sum(bmxy));
-    } else {
-        Moments6 m;
-        moments_xsum(A.cd, A.sub, pix, nullptr, 0, n, A.wdiv, w, xmin, ymin, &m);
-        stv = m.tv;
-        smx = m.mx;
-        smy = m.my;
-        smx2 = m.mx2;
-        smy2 = m.my2;
-        smxy = m.mxy;
-    }
-    if (lane != 0) return;
-    if (srv.ovf | stv.ovf | smx.ovf | smy.ovf | smx2.ovf | smy2.ovf | smxy.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
-    RobustRaw R;
-    R.mx = xs_double(smx);
-    R.my = xs_double(smy);
-    R.mx2 = xs_double(smx2);
-    R.my2 = xs_double(smy2);
-    R.mxy = xs_double(smxy);
-    R.rv = rv;
-    R.peak = peak;
-    R.cpeak = cpeak;
-    R.dnpix = dnpix;
-    R.area2 = area2;
-    R.xmin = xmin;
-    R.xmax = xmax;
-    R.ymin = ymin;
-    R.ymax = ymax;
-    R.flags = flags;
-    A.raw[o] = R;
-    A.O.dflux[o] = xs_float(stv);
 }
 
 __global__ void k_robust_finish(AnaArgs A) {
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(A.nobj, A.nobj_dev) || A.O.level[o] == 0) return;
-    const RobustRaw R = A.raw[o];
-    const int xmin = R.xmin, ymin = R.ymin, flags = R.flags, dnpix = R.dnpix, area2 = R.area2;
+    const MomentRaw R = A.raw[o];
+    if (R.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
+    const int xmin = R.xmin, ymin = R.ymin, dnpix = R.dnpix, area2 = R.area2;
+    int flags = A.O.flags[o];
+    if (xmin == 0 || R.xmax == A.w - 1 || ymin == 0 || R.ymax == A.h - 1) flags |= SX_OBJ_TRUNC;
     const float rv = R.rv, peak = R.peak, cpeak = R.cpeak;
     const double dth = A.O.dthr[o], dthresh2 = (dth + peak) / 2.0;
     double mxo = A.O.mx[o], myo = A.O.my[o];
@@ -304,6 +212,7 @@ __global__ void k_robust_finish(AnaArgs A) {
     A.O.ymin[o] = ymin;
     A.O.ymax[o] = R.ymax;
     A.O.fdflux[o] = rv;
+    A.O.dflux[o] = R.tv;
     A.O.fdpeak[o] = cpeak;
     A.O.dpeak[o] = peak;
     A.O.dnpix[o] = dnpix;
@@ -638,6 +547,7 @@ void launch_analyse(const AnaArgs &A, cudaStream_t st) {
     if (A.nobj <= 0) return;
     const unsigned grid = (A.nobj + AN_WARPS - 1) / AN_WARPS;
     k_analyse_robust<<<grid, AN_WARPS * 32, 0, st>>>(A);
+    k_analyse_robust_big<<<dt_grid(A.nobj, 2), AN_WARPS * 32, 0, st>>>(A);
     k_robust_finish<<<(unsigned)((A.nobj + 127) / 128), 128, 0, st>>>(A);
     if (A.O.dbkg) {
         k_local_stat<<<(unsigned)((A.nobj + 127) / 128), 128, 0, st>>>(A.sub, A.w, A.h, A.bp_thick, A.O.xmin,

@@ -22,25 +22,49 @@ struct BackBufs {
 struct RootBufs {
     int *size, *off, *first;            // pixels, offset in the root pixel list, first pixel
     int *ymax, *lastx;                  // completion-order keys
-    float *fdpeak, *fdflux;
     int *nkept, *objbase;
     float *dthresh, *thresh;            // smallest detection / analysis threshold of its pixels
+    unsigned *peak;                     // f2ord of its largest filtered value
+    int *npk, *nbkt, *nown;             // peaks, buckets, pixels of kept branches (deblending)
 };
 
-// per-element scratch of the deblending (index = position in the root pixel list)
+// deblending scratch (k_deblend.cu).  "Element" is a position in the root
+// pixel list; the arrays "per raw object, from its offset" hold one entry per
+// peak, bucket or kept branch, of which a raw object has no more than pixels.
 struct DebBufs {
-    int *par, *lev, *sz, *order, *rl0, *rl1, *nid0, *nid1;
-    unsigned long long *acc;            // 4 limbs per element
-    int *nd_root0, *nd_root1, *nd_flag0, *nd_flag1, *nd_nson0, *nd_nson1, *nd_okc0, *nd_okc1;
-    int *nd_oka0, *nd_oka1;
-    unsigned long long *kept;           // packed (level << 32) | element, per root at its offset
-    int *own, *kl, *kidx;
-    int *pint;                          // xmin, xmax, ymin, ymax, peak(ord), cpeak(ord), dnpix, area2
-    unsigned char *arena;               // 48 B per element: the compact per-object state of k_dl_*
-    int *rec;                           // merge record per element (k_dl_sweep -> k_dl_assign)
+    // per element
+    int *up;                            // towards its peak, then its peak, then its first representative
+    unsigned char *lev;                 // level
+    // per peak, at its element
+    unsigned long long *rec, *evm;      // join record; levels of the joins it stands for
+    int *boff, *pidx;                   // first bucket; index among its raw object's peaks
+    int2 *kown;                         // kept branch it stands for: level + 1 (0: none), rank
+    int *peaks;                         // every peak of the frame
+    // per raw object, from its offset
+    int *plist;                         // peaks
+    int *bsz, *bmin;                    // buckets: pixels, smallest index,
+    unsigned long long *acc;            // flux limbs
+    int *olev;                          // kept branches in order: level
+    unsigned *ownpix;                   // the branches' own pixels
+    // the same, for the raw objects whose joins are taken in global memory
+    unsigned long long *kept, *g_evm;
+    int *krep, *g_b0, *g_par, *g_nson, *g_label, *g_flags, *g_dlist, *g_elist;
+    signed char *g_m;
+    float *thr;                         // nthresh thresholds per raw object
+    int *lists, *counts;                // raw objects by class of peaks (stride nroots); list lengths
+    int *biglist;                       // objects whose pixels a whole block sums
 };
+// raw objects of at most this many peaks: joins taken by one warp, a block of
+// 256 threads, a block of 512 (state in shared memory); more: a block of 1024
+// on global memory
+constexpr int DT_WARP_PEAKS = 32;
+constexpr int DT_MID_PEAKS = 320;
+constexpr int DT_BIG_PEAKS = 1536;
+constexpr int DT_NCOUNTS = 8;
+// objects of more pixels than this are summed by a block, not a warp
+constexpr int DA_WARP_MAX = 1024;
 
-// Persistent grids (deblending classes, subtract/filter tiles) are sized to
+// Persistent grids (deblending joins, subtract/filter tiles) are sized to
 // the resident capacity divided by this (set per host thread; 1 by default,
 // the batch workers take the "batch_grid_div" parameter of their context:
 // measured on the 64-frame batch, whole-GPU grids with 8 workers were the
@@ -137,33 +161,30 @@ bool launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const 
 void launch_ccl(int *lab, int *cnt, const FrameParams &P, FrameScalars *d_sc, cudaStream_t st, int &launches,
                 bool tiled);
 
+struct MomentRaw;
 struct DebArgs {
     const float *cd, *sub;
     const int *pos2idx;
     const unsigned *rpix;       // root pixel lists (raster order per root)
+    const unsigned *rid;        // raw object of every element
     RootBufs R;
     DebBufs D;
     ObjBufs O;
+    MomentRaw *raw;             // per-object scratch of the preanalysis
     FrameScalars *sc;
     int *alloc;                 // W*H object id map (-1 elsewhere)
     unsigned *objkey;           // object id per root-list element
+    int nroots, nrootpix, nobj; // counts, or the capacities of the launches when the device counts are given
+    const int *nroots_dev, *nrootpix_dev, *nobj_dev;
     int w, h, N, debminarea;
     FastDiv wdiv;
     double mincont;
-    int loop_cap;               // > 0: cap on union-find walks (failure tests); 0: the object's size
+    int loop_cap;               // > 0: cap on join walks and retries (failure tests); 0: the object's size
 };
 
-// the main stream, the side streams and the events that fork and join them
-constexpr int DL_SIDE = 3;
-struct DebStreams {
-    cudaStream_t main, side[DL_SIDE];
-    cudaEvent_t fork, join[DL_SIDE];
-};
-
-void launch_deblend_split(const int *size, int nroots, const int *nroots_dev, int *lists, int *counts,
-                          unsigned *keys, unsigned *vals, unsigned *kalt, unsigned *valt, int *tmp, cudaStream_t st);
-int deblend_split_launches(int nroots);
-void launch_deblend_sweep(const DebArgs &A, const int *lists, int *counts, int nroots, const DebStreams &S);
-void launch_deblend_assign(const DebArgs &A, const int *lists, int *counts, int nroots, const DebStreams &S);
+// merge trees and kept branches (R.nkept), then the objects; both return the
+// number of kernels launched
+int launch_deblend_tree(const DebArgs &A, cudaStream_t st);
+int launch_deblend_assign(const DebArgs &A, cudaStream_t st);
 
 }  // namespace sx

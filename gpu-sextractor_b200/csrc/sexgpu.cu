@@ -5,7 +5,7 @@
 // background (makeback), filter + threshold, connected components, deblending
 // (init_deblend/parcel_out), analysis (analyse_gpu), CLEAN (run_clean),
 // photometry/FLAGS (endobject_gpu), catalogue.  All stages run on one CUDA
-// stream (the deblending forks two more).  In the plain form the host reads
+// stream.  In the plain form the host reads
 // back the counts between stages to size the launches; in the capacity form
 // the launches are sized by capacities learned from an earlier frame, the
 // counts stay on the device, and the whole frame is one CUDA graph.
@@ -31,7 +31,6 @@
 #include "k_detect.cu"
 #include "k_roots.cu"
 #include "k_deblend.cu"
-#include "k_deblend_local.cu"
 #include "k_analyse.cu"
 #include "k_post.cu"
 #include "k_fits.cu"
@@ -134,8 +133,6 @@ struct sexgpu_ctx {
     cudaEvent_t ev_block = nullptr;
     PipeState ps;
     cudaStream_t stream = nullptr;
-    cudaStream_t side[DL_SIDE] = {};  // fork/join helpers of the deblending
-    cudaEvent_t ev_fork = nullptr, ev_join[DL_SIDE] = {};
     bool own_stream = false;
     std::vector<DevBuf *> bufs;
     std::string err;
@@ -153,15 +150,18 @@ struct sexgpu_ctx {
     // background
     DevBuf ms, back, sigma, back2, back3, sigma3, dback, bu, rownode, rowdnode, rowu, colk, coldx;
     // roots
-    DevBuf rsize, roff, rfirst, rymax, rlastx, rfdpeak, rfdflux, rnkept, robjbase, rdthr, rathr, rlists, rcounts;
+    DevBuf rsize, roff, rfirst, rymax, rlastx, rnkept, robjbase, rdthr, rathr, rzero, rlists, rthr;
     // deblend scratch
-    DevBuf dpar, dlev, dsz, dorder, drl0, drl1, dnid0, dnid1, dacc, nr0, nr1, nf0, nf1, ns0, ns1, nc0, nc1, na0, na1,
-        dkept, down, dkl, dkidx, dpint, objkey, rpix, darena, drec;
+    DevBuf objkey, rpix;
+    enum { D_UP, D_LEV, D_REC, D_EVM, D_BOFF, D_PIDX, D_KOWN, D_PEAKS, D_PLIST, D_BSZ, D_BMIN, D_ACC, D_OLEV, D_OWNPIX,
+           D_KEPT, D_GEVM, D_KREP, D_GB0, D_GPAR, D_GNSON, D_GLABEL, D_GFLAGS, D_GDLIST, D_GELIST, D_GM, D_COUNT };
+    DevBuf deb;  // all of them
     // objects
     DevBuf o_i[20], o_f[32], o_d[10], o_iso, o_sortkey, amp, alpha, cellhead, cellnext, vkey, vval, vkalt, vvalt,
         skeys, svals, skalt, svalt, rows;
     DevBuf kitem[2], kchunk[2], kpart[2];  // queued Kron boxes
     DevBuf o_sprob;                        // CLASS_STAR per object
+    DevBuf o_big;                          // objects summed by whole blocks
     DevBuf o_raw, o_xraw, o_eraw;          // robust preanalysis / examineiso / photometry scratch per object
     DevBuf o_dbkg, o_lstat;                // BACKPHOTO_TYPE LOCAL: annulus mode, annulus statistics
     DevBuf o_aper, aperrows;               // every aperture per object; per catalogue row
@@ -389,17 +389,15 @@ __global__ void k_init_scalars(FrameScalars *sc) {
 // Capacity form: the checks the plain form makes on the host between stages.
 // An error so far, a zero or negative threshold (check_thr) or a count beyond
 // the capacity the launches were sized for sets the counts the later stages
-// read to 0, and the nl deblending list lengths at lists, so that the rest of
-// the frame does nothing; the status tells the host afterwards.
-__global__ void k_gate(FrameScalars *sc, int check_thr, int cap_roots, int cap_rootpix, int cap_obj, int *lists,
-                       int nl) {
+// read to 0, so that the rest of the frame does nothing; the status tells the
+// host afterwards.
+__global__ void k_gate(FrameScalars *sc, int check_thr, int cap_roots, int cap_rootpix, int cap_obj) {
     int st = sc->status;
     if (check_thr && (sc->dthresh <= 0.0f || sc->thresh <= 0.0f)) st |= SX_ST_THRESH;
     if (sc->nroots > cap_roots || sc->nrootpix > cap_rootpix || sc->nobj > cap_obj) st |= SX_ST_CAPACITY;
     sc->status = st;
     if (st & SX_ST_STOP) {
         sc->nroots = sc->nrootpix = sc->nobj = sc->nsurv = 0;
-        for (int k = 0; k < nl; k++) lists[k] = 0;
     }
 }
 
@@ -716,7 +714,7 @@ int pipe_detect(sexgpu_ctx *ctx) {
     if (ps.capf) {
         nroots = ps.cap_roots;
         rlen = (int)(N / std::max(Pm.minarea, 1));
-        k_gate<<<1, 1, 0, st>>>(d_sc, 1, ps.cap_roots, ps.cap_rootpix, ps.cap_obj, nullptr, 0);
+        k_gate<<<1, 1, 0, st>>>(d_sc, 1, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
     } else {
         rc = read_scalars(ctx);
         if (rc) return rc;
@@ -733,8 +731,6 @@ int pipe_detect(sexgpu_ctx *ctx) {
     EN(rfirst, ((size_t)rlen + 1) * 4);
     EN(rymax, ((size_t)rlen + 1) * 4);
     EN(rlastx, ((size_t)rlen + 1) * 4);
-    EN(rfdpeak, ((size_t)rlen + 1) * 4);
-    EN(rfdflux, ((size_t)rlen + 1) * 4);
     EN(rnkept, ((size_t)rlen + 1) * 4);
     EN(robjbase, ((size_t)rlen + 1) * 4);
     EN(rdthr, ((size_t)rlen + 1) * 4);
@@ -745,8 +741,6 @@ int pipe_detect(sexgpu_ctx *ctx) {
     R.first = P<int>(ctx->rfirst);
     R.ymax = P<int>(ctx->rymax);
     R.lastx = P<int>(ctx->rlastx);
-    R.fdpeak = P<float>(ctx->rfdpeak);
-    R.fdflux = P<float>(ctx->rfdflux);
     R.nkept = P<int>(ctx->rnkept);
     R.objbase = P<int>(ctx->robjbase);
     R.dthresh = P<float>(ctx->rdthr);
@@ -770,7 +764,7 @@ int pipe_detect(sexgpu_ctx *ctx) {
     int nrootpix;
     if (ps.capf) {
         nrootpix = ps.cap_rootpix;
-        k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj, nullptr, 0);
+        k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
     } else {
         rc = read_scalars(ctx);
         if (rc) return rc;
@@ -798,73 +792,73 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     RootBufs &R = ps.R;
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int *tmp = P<int>(ctx->scan_tmp);
-    int *pos2idx = P<int>(ctx->pos2idx);
     unsigned *rpix = P<unsigned>(ctx->rpix);
     int rc = SEXGPU_OK;
     // ---- deblending
-    size_t M = (size_t)nrootpix + 1;
-    EN(dpar, M * 4);
-    EN(dlev, M * 4);
-    EN(dsz, M * 4);
-    EN(dorder, M * 4);
-    EN(drl0, M * 4);
-    EN(drl1, M * 4);
-    EN(dnid0, M * 4);
-    EN(dnid1, M * 4);
-    EN(dacc, M * 32);
-    EN(nr0, M * 4);
-    EN(nr1, M * 4);
-    EN(nf0, M * 4);
-    EN(nf1, M * 4);
-    EN(ns0, M * 4);
-    EN(ns1, M * 4);
-    EN(nc0, M * 4);
-    EN(nc1, M * 4);
-    EN(na0, M * 4);
-    EN(na1, M * 4);
-    EN(dkept, M * 8);
-    EN(down, M * 4);
-    EN(dkl, M * 4);
-    EN(dkidx, M * 4);
-    EN(dpint, M * 8 * 4);
-    EN(darena, M * DL_ARENA_BYTES);
-    EN(drec, M * 4);
+    static const size_t elem[sexgpu_ctx::D_COUNT] = {
+        4, 1, 8, 8, 4, 4, 8, 4, 4, 4, 4, 8 * DT_LIMBS, 4, 4, 8, 8, 4, 4, 4, 4, 4, 4, 4, 4, 1};
+    const size_t M = (size_t)nrootpix + 1, NR = (size_t)nroots + 1;
+    size_t at[sexgpu_ctx::D_COUNT], bytes = 0;
+    for (int k = 0; k < sexgpu_ctx::D_COUNT; k++) {
+        at[k] = bytes;
+        bytes += (M * elem[k] + 255) & ~(size_t)255;
+    }
+    EN(deb, bytes);
+    unsigned char *const deb = P<unsigned char>(ctx->deb);
+    // per raw object, zeroed: peak, counts of peaks, buckets and own pixels;
+    // then the list lengths
+    EN(rzero, (4 * NR + DT_NCOUNTS) * 4);
+    EN(rlists, 4 * NR * 4);
+    EN(rthr, NR * Pm.nthresh * 4);
+    CK(cudaMemsetAsync(ctx->rzero.p, 0, (4 * NR + DT_NCOUNTS) * 4, st));
+    R.peak = P<unsigned>(ctx->rzero);
+    R.npk = P<int>(ctx->rzero) + NR;
+    R.nbkt = R.npk + NR;
+    R.nown = R.nbkt + NR;
     DebArgs &A = ps.A;
     A.cd = P<float>(ctx->cd);
     A.sub = P<float>(ctx->sub);
-    A.pos2idx = pos2idx;
+    A.pos2idx = P<int>(ctx->pos2idx);
     A.rpix = rpix;
+    A.rid = P<unsigned>(ctx->keys);
     A.R = R;
     DebBufs &D = A.D;
-    D.par = P<int>(ctx->dpar);
-    D.lev = P<int>(ctx->dlev);
-    D.sz = P<int>(ctx->dsz);
-    D.order = P<int>(ctx->dorder);
-    D.rl0 = P<int>(ctx->drl0);
-    D.rl1 = P<int>(ctx->drl1);
-    D.nid0 = P<int>(ctx->dnid0);
-    D.nid1 = P<int>(ctx->dnid1);
-    D.acc = P<unsigned long long>(ctx->dacc);
-    D.nd_root0 = P<int>(ctx->nr0);
-    D.nd_root1 = P<int>(ctx->nr1);
-    D.nd_flag0 = P<int>(ctx->nf0);
-    D.nd_flag1 = P<int>(ctx->nf1);
-    D.nd_nson0 = P<int>(ctx->ns0);
-    D.nd_nson1 = P<int>(ctx->ns1);
-    D.nd_okc0 = P<int>(ctx->nc0);
-    D.nd_okc1 = P<int>(ctx->nc1);
-    D.nd_oka0 = P<int>(ctx->na0);
-    D.nd_oka1 = P<int>(ctx->na1);
-    D.kept = P<unsigned long long>(ctx->dkept);
-    D.own = P<int>(ctx->down);
-    D.kl = P<int>(ctx->dkl);
-    D.kidx = P<int>(ctx->dkidx);
-    D.pint = P<int>(ctx->dpint);
-    D.arena = P<unsigned char>(ctx->darena);
-    D.rec = P<int>(ctx->drec);
+    D.up = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_UP]);
+    D.lev = reinterpret_cast<unsigned char *>(deb + at[sexgpu_ctx::D_LEV]);
+    D.rec = reinterpret_cast<unsigned long long *>(deb + at[sexgpu_ctx::D_REC]);
+    D.evm = reinterpret_cast<unsigned long long *>(deb + at[sexgpu_ctx::D_EVM]);
+    D.boff = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_BOFF]);
+    D.pidx = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_PIDX]);
+    D.kown = reinterpret_cast<int2 *>(deb + at[sexgpu_ctx::D_KOWN]);
+    D.peaks = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_PEAKS]);
+    D.plist = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_PLIST]);
+    D.bsz = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_BSZ]);
+    D.bmin = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_BMIN]);
+    D.acc = reinterpret_cast<unsigned long long *>(deb + at[sexgpu_ctx::D_ACC]);
+    D.olev = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_OLEV]);
+    D.ownpix = reinterpret_cast<unsigned *>(deb + at[sexgpu_ctx::D_OWNPIX]);
+    D.kept = reinterpret_cast<unsigned long long *>(deb + at[sexgpu_ctx::D_KEPT]);
+    D.g_evm = reinterpret_cast<unsigned long long *>(deb + at[sexgpu_ctx::D_GEVM]);
+    D.krep = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_KREP]);
+    D.g_b0 = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_GB0]);
+    D.g_par = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_GPAR]);
+    D.g_nson = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_GNSON]);
+    D.g_label = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_GLABEL]);
+    D.g_flags = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_GFLAGS]);
+    D.g_dlist = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_GDLIST]);
+    D.g_elist = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_GELIST]);
+    D.g_m = reinterpret_cast<signed char *>(deb + at[sexgpu_ctx::D_GM]);
+    D.thr = P<float>(ctx->rthr);
+    D.lists = P<int>(ctx->rlists);
+    D.counts = R.nown + NR;
     A.sc = d_sc;
     A.alloc = P<int>(ctx->alloc);
     A.objkey = P<unsigned>(ctx->objkey);
+    A.nroots = nroots;
+    A.nrootpix = nrootpix;
+    const int *nroots_dev = ps.capf ? &d_sc->nroots : nullptr;
+    A.nroots_dev = nroots_dev;
+    A.nrootpix_dev = ps.capf ? &d_sc->nrootpix : nullptr;
     A.w = w;
     A.h = h;
     A.N = Pm.nthresh;
@@ -872,25 +866,12 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     A.mincont = Pm.mincont;
     A.loop_cap = Pm.loop_cap;
     A.wdiv = make_fastdiv((unsigned)w);
-    EN(rlists, (size_t)(DL_NLISTS * (nroots + 1)) * 4);
-    EN(rcounts, 5 * DL_NLISTS * 4);
-    DebStreams S;
-    S.main = st;
-    for (int i = 0; i < DL_SIDE; i++) {
-        S.side[i] = ctx->side[i];
-        S.join[i] = ctx->ev_join[i];
-    }
-    S.fork = ctx->ev_fork;
-    const int *nroots_dev = ps.capf ? &d_sc->nroots : nullptr;
-    launch_deblend_split(R.size, nroots, nroots_dev, P<int>(ctx->rlists), P<int>(ctx->rcounts), P<unsigned>(ctx->keys),
-                         P<unsigned>(ctx->vals), P<unsigned>(ctx->kalt), P<unsigned>(ctx->valt), tmp, st);
-    launch_deblend_sweep(A, P<int>(ctx->rlists), P<int>(ctx->rcounts), nroots, S);
+    int nl = launch_deblend_tree(A, st);
     exclusive_scan(R.nkept, R.objbase, nroots, &d_sc->nobj, tmp, st, nroots_dev);
     int nobj;
     if (ps.capf) {
-        // a stop also empties the size-class lists, so that no branch is assigned
         nobj = ps.cap_obj;
-        k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj, P<int>(ctx->rcounts), DL_NLISTS);
+        k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
     } else {
         rc = read_scalars(ctx);
         if (rc) return rc;
@@ -900,9 +881,15 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     ctx->cfg_local = Pm.bp_local != 0;
     rc = alloc_objects(ctx, nobj);
     if (rc) return rc;
+    EN(o_raw, (size_t)(nobj + 1) * sizeof(MomentRaw));
+    EN(o_big, (size_t)(nobj + 1) * 4);
     A.O = ctx->O;
-    launch_deblend_assign(A, P<int>(ctx->rlists), P<int>(ctx->rcounts), nroots, S);
-    stage_mark(ctx, "deblend", 16 + deblend_split_launches(nroots) + scan_launches(nroots));
+    A.raw = P<MomentRaw>(ctx->o_raw);
+    A.nobj = nobj;
+    A.nobj_dev = ps.capf ? &d_sc->nobj : nullptr;
+    D.biglist = P<int>(ctx->o_big);
+    nl += launch_deblend_assign(A, st);
+    stage_mark(ctx, "deblend", nl + scan_launches(nroots));
     ps.stage = 3;
     return SEXGPU_OK;
 }
@@ -928,8 +915,9 @@ int pipe_analyse(sexgpu_ctx *ctx) {
     launch_obj_partition(rpix, A.objkey, ps.R, O.off, ps.nroots, ps.capf ? &d_sc->nroots : nullptr, vals,
                          P<int>(ctx->kalt), &d_sc->nbig, P<int>(ctx->rlists), st);
     AnaArgs AA;
-    EN(o_raw, (size_t)(nobj + 1) * sizeof(RobustRaw));
-    AA.raw = P<RobustRaw>(ctx->o_raw);
+    AA.raw = A.raw;
+    AA.biglist = A.D.biglist;
+    AA.counts = A.D.counts;
     EN(o_xraw, (size_t)(nobj + 1) * sizeof(ExamRaw));
     AA.xraw = P<ExamRaw>(ctx->o_xraw);
     AA.cd = A.cd;
@@ -956,7 +944,7 @@ int pipe_analyse(sexgpu_ctx *ctx) {
     AA.afac = Pm.analysis_thresh;
     AA.bp_thick = Pm.bp_thick;
     launch_analyse(AA, st);
-    stage_mark(ctx, "analyse", 6 + (Pm.bp_local ? 2 : 0) + scan_launches(nobj));
+    stage_mark(ctx, "analyse", 7 + (Pm.bp_local ? 2 : 0) + scan_launches(nobj));
     ps.stage = 4;
     return SEXGPU_OK;
 }
@@ -1003,7 +991,7 @@ int pipe_clean(sexgpu_ctx *ctx) {
             // the victim count stays on the device: the one-block sort takes
             // short lists, the radix sorts (counted by nvbig) long ones
             unsigned *vkey = P<unsigned>(ctx->vkey), *vval = P<unsigned>(ctx->vval);
-            k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj, nullptr, 0);
+            k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
             k_victim_sort<<<1, 1024, 0, st>>>(vkey, vval, nobj, &d_sc->nsurv, &d_sc->nvbig);
             radix_sort_pairs(vval, vkey, P<unsigned>(ctx->vkalt), P<unsigned>(ctx->vvalt), nobj, bits_for(nobj), tmp,
                              st, &d_sc->nvbig);
@@ -1108,7 +1096,7 @@ int pipe_end(sexgpu_ctx *ctx) {
     int ns;
     if (ps.capf) {
         ns = nobj;
-        k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj, nullptr, 0);
+        k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
     } else {
         rc = read_scalars(ctx);
         if (rc) return rc;
@@ -1484,14 +1472,6 @@ int sexgpu_create(sexgpu_ctx **out, int device) {
         return SEXGPU_ERR_CUDA;
     }
     ctx->own_stream = true;
-    bool ok = true;
-    for (int i = 0; i < DL_SIDE; i++)
-        ok = ok && cudaStreamCreateWithFlags(&ctx->side[i], cudaStreamNonBlocking) == cudaSuccess &&
-             cudaEventCreateWithFlags(&ctx->ev_join[i], cudaEventDisableTiming) == cudaSuccess;
-    if (!ok || cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess) {
-        sexgpu_destroy(ctx);
-        return SEXGPU_ERR_CUDA;
-    }
     *out = ctx;
     return SEXGPU_OK;
 }
@@ -1510,15 +1490,14 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
                      &ctx->seg, &ctx->pos2idx, &ctx->var, &ctx->scan_tmp, &ctx->keys, &ctx->vals, &ctx->kalt,
                      &ctx->valt, &ctx->ms, &ctx->back, &ctx->sigma, &ctx->back2, &ctx->back3, &ctx->sigma3,
                      &ctx->dback, &ctx->bu, &ctx->rownode, &ctx->rowdnode, &ctx->rowu, &ctx->colk, &ctx->coldx,
-                     &ctx->rsize, &ctx->roff, &ctx->rfirst, &ctx->rymax, &ctx->rlastx, &ctx->rfdpeak,
-                     &ctx->rfdflux, &ctx->rnkept, &ctx->robjbase, &ctx->rdthr, &ctx->rathr, &ctx->imgm, &ctx->wvar, &ctx->wratio, &ctx->rlists, &ctx->rcounts, &ctx->dpar, &ctx->dlev, &ctx->dsz, &ctx->dorder,
-                     &ctx->drl0, &ctx->drl1, &ctx->dnid0, &ctx->dnid1, &ctx->dacc, &ctx->nr0, &ctx->nr1,
-                     &ctx->nf0, &ctx->nf1, &ctx->ns0, &ctx->ns1, &ctx->nc0, &ctx->nc1, &ctx->na0, &ctx->na1,
-                     &ctx->dkept, &ctx->down, &ctx->dkl, &ctx->dkidx, &ctx->dpint, &ctx->objkey,
-                     &ctx->rpix, &ctx->darena, &ctx->drec, &ctx->o_iso, &ctx->o_sortkey, &ctx->amp, &ctx->alpha, &ctx->cellhead,
+                     &ctx->rsize, &ctx->roff, &ctx->rfirst, &ctx->rymax, &ctx->rlastx, &ctx->rnkept, &ctx->robjbase,
+                     &ctx->rdthr, &ctx->rathr, &ctx->rzero, &ctx->rlists, &ctx->rthr, &ctx->imgm, &ctx->wvar,
+                     &ctx->wratio, &ctx->objkey, &ctx->rpix, &ctx->o_big,
+                     &ctx->o_iso, &ctx->o_sortkey, &ctx->amp, &ctx->alpha, &ctx->cellhead,
                      &ctx->cellnext, &ctx->vkey, &ctx->vval, &ctx->vkalt, &ctx->vvalt, &ctx->skeys, &ctx->svals,
                      &ctx->skalt, &ctx->svalt, &ctx->rows, &ctx->sc};
     for (DevBuf *b : all) free_buf(*b);
+    free_buf(ctx->deb);
     for (auto &b : ctx->o_i) free_buf(b);
     for (auto &b : ctx->o_f) free_buf(b);
     for (auto &b : ctx->o_d) free_buf(b);
@@ -1545,11 +1524,6 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
     free_buf(ctx->dmask);
     for (auto &s : ctx->stages) cudaEventDestroy(s.ev);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
-    for (int i = 0; i < DL_SIDE; i++) {
-        if (ctx->side[i]) cudaStreamDestroy(ctx->side[i]);
-        if (ctx->ev_join[i]) cudaEventDestroy(ctx->ev_join[i]);
-    }
-    if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_block) cudaEventDestroy(ctx->ev_block);
     free_batch_graph(ctx);
     for (GraphEntry &e : ctx->graphs) drop_graph(ctx, e);

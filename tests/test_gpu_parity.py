@@ -330,3 +330,29 @@ def test_several_apertures(gpu_ctx, masks, mask_type, gain):
     assert np.array_equal(ga[:, 0, 0], g["flux_aper"])
     # a wider aperture holds more flux on average
     assert (np.median(ga[:, 4, 0]) > np.median(ga[:, 1, 0]))
+
+
+@pytest.mark.parametrize("peaks", [2, 31, 32, 33, 319, 320, 321, 1535, 1536, 1537, 5000])
+@pytest.mark.parametrize("nthresh,mincont,minarea", [(32, 0.005, 5), (64, 0.0, 1), (2, 1e-4, 3)])
+def test_deblending_by_number_of_peaks(gpu_ctx, peaks, nthresh, mincont, minarea):
+    """One raw object with a given number of local maxima on either side of
+    the sizes at which its merge tree goes to a warp, a block in shared memory
+    or a block on global memory: bumps of random heights, three pixels apart, on
+    a plateau of random saddles, beside a single bump and a flat-topped one."""
+    rng = np.random.default_rng(peaks)
+    nx = max(2, int(np.sqrt(peaks)))
+    ny = -(-peaks // nx)
+    img = np.zeros((3 * ny + 20, 3 * nx + 40), np.float32)
+    img[2:3 * ny + 3, 2:3 * nx + 3] = rng.uniform(10.0, 12.0, (3 * ny + 1, 3 * nx + 1))
+    tops = np.exp(rng.uniform(np.log(13.0), np.log(2e4), nx * ny)).astype(np.float32)
+    for k in range(peaks):
+        y, x = 4 + 3 * (k // nx), 4 + 3 * (k % nx)
+        img[y - 1:y + 2, x - 1:x + 2] += tops[k] * rng.uniform(0.05, 0.9, (3, 3)).astype(np.float32)
+        img[y, x] = 13.0 + 2.0 * tops[k]
+    img[3 * ny + 8:3 * ny + 13, 5:10] = 50.0
+    img[3 * ny + 10, 7] = 90.0
+    img[3 * ny + 8:3 * ny + 14, 20:27] = 40.0
+    g = run_both(gpu_ctx, img, filter_flag=0, back_type=1, back_value=0.0, thresh_type=1, detect_thresh=5.0,
+                 analysis_thresh=5.0, deblend_nthresh=nthresh, deblend_mincont=mincont, detect_minarea=minarea,
+                 clean_flag=0)
+    assert len(g) >= 3
