@@ -550,9 +550,9 @@ void launch_analyse(const AnaArgs &A, cudaStream_t st) {
     k_analyse_robust_big<<<dt_grid(A.nobj, 2), AN_WARPS * 32, 0, st>>>(A);
     k_robust_finish<<<(unsigned)((A.nobj + 127) / 128), 128, 0, st>>>(A);
     if (A.O.dbkg) {
-        k_local_stat<<<(unsigned)((A.nobj + 127) / 128), 128, 0, st>>>(A.sub, A.w, A.h, A.bp_thick, A.O.xmin,
-                                                                         A.O.xmax, A.O.ymin, A.O.ymax, A.nobj,
-                                                                         A.nobj_dev, A.O.lstat);
+        k_local_stat<<<(unsigned)((A.nobj + GW_WARPS - 1) / GW_WARPS), 32 * GW_WARPS, 0, st>>>(
+            A.sub, A.w, A.h, A.bp_thick, A.O.xmin, A.O.xmax, A.O.ymin, A.O.ymax, A.nobj, A.nobj_dev, A.O.lstat,
+            A.O.dbkg);
         k_local_guess<<<(unsigned)A.nobj, GUESS_THREADS, 0, st>>>(A.sub, A.w, A.h, A.bp_thick, A.O.xmin, A.O.xmax,
                                                                    A.O.ymin, A.O.ymax, A.nobj, A.nobj_dev, A.O.lstat,
                                                                    A.O.dbkg);

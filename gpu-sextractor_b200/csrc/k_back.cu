@@ -3,8 +3,8 @@
 // the CUDA driver src/cuda/cudaback.cu:1212).
 //
 // Results are bit-identical to the reference's CPU functions:
-//  * the per-mesh mean/sigma are the reference's sequential double sums, run
-//    one thread per mesh in the same pixel order;
+//  * the per-mesh mean/sigma are the reference's sequential double sums with
+//    its roundings, composed from stretches of the sequence (seq_sums);
 //  * histogram sums are exact integers, so they are reduced in parallel;
 //  * the two-pointer median walk of backguess is replaced by a binary search
 //    on the merge path of the two cumulative sums, which lands on the same
@@ -15,63 +15,265 @@
 
 namespace sx {
 
-// src/back.c:214-279 for one mesh: the reference's two sequential double
-// passes, in its pixel order.  `row0` points at the mesh's first pixel, rows
-// `stride` floats apart.  A pixel left out adds +0.0 instead of skipping the
-// addition: the sums start at +0.0 and so are never -0.0, hence s + 0.0 == s
-// exactly, and the select stays off the dependent chain of additions (the
-// chain is the cost of these loops: two passes over 64 x 64 meshes take about
-// 33 cycles per pixel and pass on B200).
-__device__ __forceinline__ void mesh_stat_seq(const float *row0, int stride, int mw, int mh, MeshStat &o) {
-    double pix, sig, mean = 0.0, sigma = 0.0;
+// ---------------------------------------------------------------------------
+// The two sequential double sums of backstat (src/back.c:214-279), sum of
+// the pixels and sum of their squares in pixel order, by one warp.
+//
+// A sequential sum is a chain of roundings, but in the one binade [2^k,
+// 2^(k+1)) that the partial sum stays in for long it can be cut into pieces:
+// there S + t is rounded to a multiple of q = 2^(k-52), and how depends on t
+// and on whether S / q is even or odd (ties), on nothing else of S.  So each
+// lane adds its stretch of the sequence to 2^k and, in a second chain, to
+// 2^k + q; the two increments and final parities describe what the stretch
+// does to any sum of that binade.  A scan over the lanes composes them in
+// order.  Where the sum reaches 2^(k+1) in a lane's stretch, that stretch is
+// added pixel by pixel and the lanes after it start again in the new binade:
+// a handful of times, since the sum has to double each time.  The squares of
+// floats are exact in double, so fma(p, p, s) is s + p * p rounded once.
+//
+// The sum of the pixels themselves is exact whatever the order when the sum
+// of the magnitudes is below 2^53 units of the smallest exponent present
+// (checked; pixel by pixel otherwise).
+//
+// One lane per mesh adding pixel by pixel took 33 cycles a pixel and pass:
+// 138 us for the 64 x 64 meshes of any frame, 0.55 ms for 128 x 128.  Composed
+// and followed by the mode in the same warp, the background stage went from
+// 0.165 to 0.083 ms (160 x 160), 0.375 to 0.249 (4096 x 4096, 64 x 64
+// meshes), 0.67 to 0.215 (128 x 128), 4.6 to 4.1 (16384 x 16384); it is bound
+// by issue there (about 45 warp instructions per 32 pixels and pass).
+// ---------------------------------------------------------------------------
+constexpr int SEQ_G = 16;                          // pixels of a lane's stretch
+constexpr int SEQ_CHUNK = 32 * SEQ_G;              // pixels taken at a time
+constexpr int SEQ_PITCH = SEQ_G + 4;               // staged stretches: 16-byte reads on distinct banks
+
+struct SeqSums {
+    double sum, sq;
+    int n;
+    bool exact;     // the sum of the pixels is the sequential one
+    unsigned amin;  // smallest nonzero magnitude's bits - 1 (0xffffffff: none)
+};
+
+// the test of a pixel: pass 0 valid (above -BIG), pass 1 inside the cuts
+// (and, for an annulus, valid).  It is made on the float: a float compares
+// with the float cuts as its double does, and f > (float)-BIG as (double)f >
+// -BIG (the float nearest -1e30 lies below it, the next one up above it).
+template <int PASS, bool VALID>
+__device__ __forceinline__ bool seq_in(float f, float lcut, float hcut) {
+    if (PASS == 0) return f > (float)-SX_BIG;
+    return (!VALID || f > (float)-SX_BIG) && f <= hcut && f >= lcut;
+}
+
+// LOAD: chunk(v) loads the sequence's next SEQ_CHUNK pixels, SEQ_G per lane
+// (NaN beyond the end), store(stage, v) puts them at their places of the
+// staged stretches; stage: 32 * SEQ_PITCH floats of this warp, 16-byte
+// aligned.  amin: for pass 1, what pass 0 found (its pixels are among them).
+template <int PASS, bool VALID, class LOAD>
+__device__ __forceinline__ SeqSums seq_sums(LOAD load, int n, float lcut, float hcut, unsigned amin, float *stage) {
+    const int lane = threadIdx.x & 31;
+    double S = 0.0, m = 0.0;
+    int cnt = 0;
+    for (int c0 = 0; c0 < n; c0 += SEQ_CHUNK) {
+        float v[SEQ_G];
+        load.chunk(v);
+#pragma unroll
+        for (int g = 0; g < SEQ_G; g++) {
+            const bool in = seq_in<PASS, VALID>(v[g], lcut, hcut);
+            v[g] = in ? v[g] : 0.0f;
+            cnt += in;
+            if (PASS == 0) amin = min(amin, (__float_as_uint(v[g]) & 0x7fffffffu) - 1u);
+        }
+        LOAD::store(stage, v);
+        __syncwarp();
+        const float4 *mine = reinterpret_cast<const float4 *>(stage + lane * SEQ_PITCH);
+        double d[SEQ_G];
+#pragma unroll
+        for (int g = 0; g < SEQ_G / 4; g++) {
+            const float4 f = mine[g];
+            d[4 * g] = (double)f.x;
+            d[4 * g + 1] = (double)f.y;
+            d[4 * g + 2] = (double)f.z;
+            d[4 * g + 3] = (double)f.w;
+            m += d[4 * g];
+            m += d[4 * g + 1];
+            m += d[4 * g + 2];
+            m += d[4 * g + 3];
+        }
+        for (int first = 0; first < 32;) {
+            // S in [2^k, 2 * 2^k)
+            const long long bits = __double_as_longlong(S);
+            const double lo = __longlong_as_double(bits & 0x7ff0000000000000ll),
+                         lo1 = __longlong_as_double((bits & 0x7ff0000000000000ll) | 1ll), hi = lo + lo;
+            int stop = first;  // the lane whose stretch is added pixel by pixel
+            if (S > 1e-290 && hi < 1e300) {
+                double s0 = lo, s1 = lo1;
+                if (lane >= first) {
+#pragma unroll
+                    for (int g = 0; g < SEQ_G; g++) {
+                        s0 = fma(d[g], d[g], s0);
+                        s1 = fma(d[g], d[g], s1);
+                    }
+                }
+                // the parity each lane's stretch begins with: parity in ->
+                // parity out of a stretch is one of two constants, or keeps
+                // or flips it; so the last constant below the lane (or the
+                // sum's own parity), flipped as often as lanes after it flip
+                const unsigned b0 = __ballot_sync(0xffffffffu, (int)(__double_as_longlong(s0) & 1ll)),
+                               b1 = __ballot_sync(0xffffffffu, (int)(__double_as_longlong(s1) & 1ll));
+                const unsigned below = (1u << lane) - 1u, flips = b0 & ~b1, consts = ~(b0 ^ b1) & below;
+                const int c = 31 - __clz(consts);  // -1: none
+                const unsigned since = c < 0 ? below : below & ~((2u << c) - 1u);
+                const unsigned par = ((c < 0 ? (unsigned)(bits & 1ll) : b0 >> c) + __popc(flips & since)) & 1u;
+                // (a stretch that leaves the binade takes the sum with it)
+                const double se = par ? s1 : s0;
+                double f = s0 < hi && s1 < hi ? se - (par ? lo1 : lo) : hi;
+                // inclusive scan (multiples of 2^(k-52) below 2^(k+1): exact)
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const double e = __shfl_up_sync(0xffffffffu, f, o);
+                    if (lane >= o) f += e;
+                }
+                const double after = S + f;
+                const unsigned bal = __ballot_sync(0xffffffffu, !(after < hi));
+                stop = bal ? __ffs(bal) - 1 : 32;
+                if (stop > 0) S = __shfl_sync(0xffffffffu, after, stop - 1);
+            }
+            if (stop < 32) {
+                const float *st = stage + stop * SEQ_PITCH;
+#pragma unroll
+                for (int g = 0; g < SEQ_G; g++) {
+                    const double x = (double)st[g];
+                    S = fma(x, x, S);
+                }
+            }
+            first = stop + 1;
+        }
+        __syncwarp();
+    }
+    SeqSums r;
+    r.sq = S;
+    r.n = (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
+    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+    r.sum = m;
+    r.amin = PASS == 0 ? __reduce_min_sync(0xffffffffu, amin) : amin;
+    // every partial sum is a multiple of 2^(e - 23), e the smallest exponent,
+    // and at most the sum of the magnitudes, itself at most sqrt(n S); exact
+    // in any order when that is below 2^53 units
+    const int e = (int)((r.amin + 1u) >> 23) - 127;
+    r.exact = r.amin == 0xffffffffu || (e > -127 && sqrt((double)r.n * S) < scalbn(1.0, e - 23 + 52));
+    return r;
+}
+
+// the sum of the pixels one by one, for data whose sums round
+template <int PASS, bool VALID, class LOAD>
+__device__ __noinline__ double seq_sum_slow(LOAD load, int n, float lcut, float hcut, float *stage) {
+    double m = 0.0;
+    for (int c0 = 0; c0 < n; c0 += SEQ_CHUNK) {
+        float v[SEQ_G];
+        load.chunk(v);
+        for (int g = 0; g < SEQ_G; g++) v[g] = seq_in<PASS, VALID>(v[g], lcut, hcut) ? v[g] : 0.0f;
+        __syncwarp();
+        LOAD::store(stage, v);
+        __syncwarp();
+        for (int l = 0; l < 32; l++)
+#pragma unroll
+            for (int k = 0; k < SEQ_G; k++) m += (double)stage[l * SEQ_PITCH + k];
+    }
+    return m;
+}
+
+// backstat of one sequence of pixels by one warp (all lanes get the result).
+// minpix: valid pixels below which the mesh is bad (mean = sigma = -BIG)
+template <bool VALID, class LOAD>
+__device__ __forceinline__ void seq_stat(const LOAD &load, int n, float minpix, float *stage, MeshStat &o, int &nvalid) {
     const double step = sqrt(2 / SX_PI) * SX_QUANTIF_NSIGMA / SX_QUANTIF_AMIN;
-    int npix = 0;
     o.mean = o.sigma = o.lcut = o.hcut = o.qzero = o.qscale = 0.f;
     o.nlevels = o.npix = 0;
-    for (int y = 0; y < mh; y++) {
-        const float *row = row0 + (size_t)y * stride;
-        // unrolled so that loads and conversions run ahead of the two
-        // accumulation chains; the additions stay in pixel order
-#pragma unroll 8
-        for (int x = 0; x < mw; x++) {
-            pix = row[x];
-            const bool in = pix > -SX_BIG;
-            mean += in ? pix : 0.0;
-            sigma += in ? pix * pix : 0.0;
-            npix += in;
-        }
-    }
-    if ((float)npix < (float)(mw * mh * SX_BACK_MINGOODFRAC)) {
+    SeqSums a = seq_sums<0, VALID>(load, n, 0.0f, 0.0f, 0xffffffffu, stage);
+    nvalid = a.n;
+    if ((float)a.n < minpix) {
         o.mean = o.sigma = -SX_BIG;
         return;
     }
-    mean /= (double)npix;
-    sigma = (sig = sigma / npix - mean * mean) > 0.0 ? sqrt(sig) : 0.0;
+    if (!a.exact) a.sum = seq_sum_slow<0, VALID>(load, n, 0.0f, 0.0f, stage);
+    double sig, mean = a.sum, sigma = a.sq;
+    mean /= (double)a.n;
+    sigma = (sig = sigma / a.n - mean * mean) > 0.0 ? sqrt(sig) : 0.0;
     const float lcut = o.lcut = (float)(mean - 2.0 * sigma);
     const float hcut = o.hcut = (float)(mean + 2.0 * sigma);
-    mean = sigma = 0.0;
-    npix = 0;
-    for (int y = 0; y < mh; y++) {
-        const float *row = row0 + (size_t)y * stride;
-#pragma unroll 8
-        for (int x = 0; x < mw; x++) {
-            pix = row[x];
-            const bool in = pix <= hcut && pix >= lcut;
-            mean += in ? pix : 0.0;
-            sigma += in ? pix * pix : 0.0;
-            npix += in;
-        }
-    }
-    o.npix = npix;
-    mean /= (double)npix;
-    sig = sigma / npix - mean * mean;
+    a = seq_sums<1, VALID>(load, n, lcut, hcut, a.amin, stage);
+    if (!a.exact) a.sum = seq_sum_slow<1, VALID>(load, n, lcut, hcut, stage);
+    mean = a.sum;
+    sigma = a.sq;
+    o.npix = a.n;
+    mean /= (double)a.n;
+    sig = sigma / a.n - mean * mean;
     sigma = sig > 0.0 ? sqrt(sig) : 0.0;
     o.mean = mean;
     o.sigma = sigma;
-    if ((o.nlevels = (int)(step * npix + 1)) > SX_QUANTIF_NMAXLEVELS) o.nlevels = SX_QUANTIF_NMAXLEVELS;
+    if ((o.nlevels = (int)(step * a.n + 1)) > SX_QUANTIF_NMAXLEVELS) o.nlevels = SX_QUANTIF_NMAXLEVELS;
     o.qscale = sigma > 0.0 ? 2 * SX_QUANTIF_NSIGMA * sigma / o.nlevels : 1.0;
     o.qzero = mean - SX_QUANTIF_NSIGMA * sigma;
 }
+
+// staged place of chunk pixel i
+__device__ __forceinline__ int seq_slot(int i) { return (i / SEQ_G) * SEQ_PITCH + i % SEQ_G; }
+
+// the pixels of a mw x mh mesh in row-major order, SEQ_CHUNK at a time: lane
+// l loads words l, l + 32, ... of a chunk, of four pixels (VEC: frame and mesh
+// width multiples of 4, frame 16-byte aligned) or one
+template <bool VEC>
+struct MeshLoad {
+    static constexpr int V = VEC ? 4 : 1;
+    const float *origin;
+    int off, left, col, mw, step, wrap, dcol;
+    __device__ __forceinline__ MeshLoad(const float *origin_, int w, int mw_, int mh) {
+        const int lane = threadIdx.x & 31;
+        origin = origin_;
+        mw = mw_;
+        const int drow = 32 * V / mw, row = V * lane / mw;
+        dcol = 32 * V - drow * mw;
+        col = V * lane - row * mw;
+        off = row * w + col;
+        step = drow * w + dcol;
+        wrap = w - mw;
+        left = mw * mh - V * lane;
+    }
+    __device__ __forceinline__ void chunk(float *v) {
+        // beyond the mesh: NaN, which every test rejects as it does a NaN pixel
+        const float nan = __int_as_float(0x7fffffff);
+#pragma unroll
+        for (int g = 0; g < SEQ_G / V; g++) {
+            if (VEC) {
+                const float4 f = left > 0 ? __ldg(reinterpret_cast<const float4 *>(origin + off))
+                                          : make_float4(nan, nan, nan, nan);
+                v[4 * g] = f.x;
+                v[4 * g + 1] = f.y;
+                v[4 * g + 2] = f.z;
+                v[4 * g + 3] = f.w;
+            } else {
+                v[g] = left > 0 ? __ldg(origin + off) : nan;
+            }
+            left -= 32 * V;
+            col += dcol;
+            off += step;
+            if (col >= mw) {
+                col -= mw;
+                off += wrap;
+            }
+        }
+    }
+    static __device__ __forceinline__ void store(float *stage, const float *v) {
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int g = 0; g < SEQ_G / V; g++) {
+            if (VEC)
+                *reinterpret_cast<float4 *>(stage + seq_slot(4 * (lane + 32 * g))) =
+                    make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+            else
+                stage[seq_slot(lane + 32 * g)] = v[g];
+        }
+    }
+};
 
 __device__ __forceinline__ void mesh_geometry(int m, int w, int h, int bw, int bh, int nbx, int nby, int &x0, int &y0,
                                               int &mw, int &mh) {
@@ -82,187 +284,18 @@ __device__ __forceinline__ void mesh_geometry(int m, int w, int h, int bw, int b
     mh = (my == nby - 1 && h % bh) ? h % bh : bh;
 }
 
-// one thread per mesh, straight from the frame (meshes too large to stage)
-__global__ void k_mesh_stat(const float *__restrict__ img, int w, int h, int bw, int bh, int nbx, int nby,
-                            MeshStat *__restrict__ ms) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= nbx * nby) return;
-    int x0, y0, mw, mh;
+// backstat of every mesh, one warp each (meshes whose histogram takes a block)
+template <bool VEC>
+__global__ void __launch_bounds__(32) k_mesh_stat(const float *__restrict__ img, int w, int h, int bw, int bh, int nbx,
+                                                  int nby, MeshStat *__restrict__ ms) {
+    __shared__ __align__(16) float stage[32 * SEQ_PITCH];
+    const int m = blockIdx.x;
+    int x0, y0, mw, mh, nv;
     mesh_geometry(m, w, h, bw, bh, nbx, nby, x0, y0, mw, mh);
     MeshStat o;
-    mesh_stat_seq(img + (size_t)y0 * w + x0, w, mw, mh, o);
-    ms[m] = o;
-}
-
-// One warp per row band of 32 meshes, one lane per mesh.  The band's pixel
-// rows are staged in shared memory by cp.async (coalesced across the band) in
-// a ring of BAND_STAGES rows, so that the loads of the next rows are in
-// flight while the lanes add the current one; every lane then adds its mesh's
-// part of the row to its own sums, so each lane performs the reference's
-// sequential double sums in the reference's pixel order.  Mesh j of the band
-// sits at j * stride in a row buffer.  VEC (frame width and mesh width
-// multiples of 4): 16-byte copies, float4 reads, stride = 4 (mod 8) so that
-// the eight lanes of a float4 read phase hit distinct banks; otherwise 4-byte
-// copies and an odd stride.
-constexpr int BAND_STAGES = 4;
-
-// Copy c of a row (c = lane, lane + 32, ...; float4s when VEC, else floats)
-// is element r of mesh j, c = j q + r with q the copies per mesh row; (j0, r0)
-// is the lane's first and (dj, dr) the step of 32 copies, so no division is
-// needed per copy.
-struct BandCopy {
-    int q, j0, r0, dj, dr;
-};
-
-template <bool VEC>
-__device__ __forceinline__ void band_row_async(float *dst, const float *img, int w, int gy, int x0, int tw,
-                                               int stride, const BandCopy &bc) {
-    const int lane = threadIdx.x & 31;
-    const float *src = img + (size_t)gy * w + x0;
-    int j = bc.j0, r = bc.r0;
-    if (VEC) {
-        for (int c = lane; 4 * c < tw; c += 32) {
-            const unsigned d = (unsigned)__cvta_generic_to_shared(dst + j * stride + 4 * r);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + 4 * c) : "memory");
-            r += bc.dr;
-            j += bc.dj;
-            if (r >= bc.q) {
-                r -= bc.q;
-                j++;
-            }
-        }
-    } else {
-        for (int c = lane; c < tw; c += 32) {
-            const unsigned d = (unsigned)__cvta_generic_to_shared(dst + j * stride + r);
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src + c) : "memory");
-            r += bc.dr;
-            j += bc.dj;
-            if (r >= bc.q) {
-                r -= bc.q;
-                j++;
-            }
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-// the two accumulation loops of one row (pass 0: valid pixels; pass 1:
-// pixels inside [lcut, hcut]).  The tests are made on the float: a float
-// compares with the float cuts as its double does, and f > (float)-BIG as
-// (double)f > -BIG (the float nearest -1e30 lies below it, the next one up
-// above it).  The square of a float is exact in double, so fma(p, p, s) is
-// s + p * p rounded once, as the reference adds it.
-template <int PASS>
-__device__ __forceinline__ void band_add(float f, float lcut, float hcut, double &mean, double &sigma, int &npix) {
-    const bool in = PASS == 0 ? f > (float)-SX_BIG : (f <= hcut && f >= lcut);
-    const double pix = (double)(in ? f : 0.0f);
-    mean += pix;
-    sigma = fma(pix, pix, sigma);
-    npix += in;
-}
-
-template <int PASS, bool VEC>
-__device__ __forceinline__ void band_row_add(const float *row, int mw, float lcut, float hcut, double &mean,
-                                             double &sigma, int &npix) {
-    if (VEC) {
-        const float4 *r4 = reinterpret_cast<const float4 *>(row);
-#pragma unroll 4
-        for (int q = 0; q < (mw >> 2); q++) {
-            const float4 v = r4[q];
-            band_add<PASS>(v.x, lcut, hcut, mean, sigma, npix);
-            band_add<PASS>(v.y, lcut, hcut, mean, sigma, npix);
-            band_add<PASS>(v.z, lcut, hcut, mean, sigma, npix);
-            band_add<PASS>(v.w, lcut, hcut, mean, sigma, npix);
-        }
-    } else {
-#pragma unroll 8
-        for (int x = 0; x < mw; x++) band_add<PASS>(row[x], lcut, hcut, mean, sigma, npix);
-    }
-}
-
-template <bool VEC>
-__global__ void __launch_bounds__(32) k_mesh_stat_band(const float *__restrict__ img, int w, int h, int bw, int bh,
-                                                       int nbx, int nby, int stride, MeshStat *__restrict__ ms) {
-    extern __shared__ __align__(16) float band_smem[];
-    const int lane = threadIdx.x;
-    const int mx0 = blockIdx.x * 32, my = blockIdx.y;
-    const int nmesh = min(32, nbx - mx0);
-    const int x0 = mx0 * bw, y0 = my * bh;
-    const int mh = (my == nby - 1 && h % bh) ? h % bh : bh;
-    const int mw_last = (mx0 + nmesh == nbx && w % bw) ? w % bw : bw;
-    const int tw = (nmesh - 1) * bw + mw_last;  // band width in pixels
-    const bool active = lane < nmesh;
-    const int mw = lane == nmesh - 1 ? mw_last : bw;
-    const int rowf = 32 * stride;  // floats per staged row
-    BandCopy bc;
-    bc.q = VEC ? bw >> 2 : bw;
-    bc.j0 = lane / bc.q;
-    bc.r0 = lane - bc.j0 * bc.q;
-    bc.dj = 32 / bc.q;
-    bc.dr = 32 - bc.dj * bc.q;
-    double sig, mean = 0.0, sigma = 0.0;
-    const double step = sqrt(2 / SX_PI) * SX_QUANTIF_NSIGMA / SX_QUANTIF_AMIN;
-    int npix = 0;
-    float lcut = 0.0f, hcut = 0.0f;
-    bool bad = false;
-    for (int pass = 0; pass < 2; pass++) {
-        for (int y = 0; y < BAND_STAGES - 1; y++) {
-            if (y < mh)
-                band_row_async<VEC>(band_smem + y * rowf, img, w, y0 + y, x0, tw, stride, bc);
-            else
-                asm volatile("cp.async.commit_group;" ::: "memory");
-        }
-        for (int y = 0; y < mh; y++) {
-            const int ya = y + BAND_STAGES - 1;
-            if (ya < mh)
-                band_row_async<VEC>(band_smem + (ya % BAND_STAGES) * rowf, img, w, y0 + ya, x0, tw, stride, bc);
-            else
-                asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("cp.async.wait_group %0;" ::"n"(BAND_STAGES - 1) : "memory");
-            __syncwarp();
-            if (active) {
-                const float *row = band_smem + (y % BAND_STAGES) * rowf + lane * stride;
-                if (pass == 0)
-                    band_row_add<0, VEC>(row, mw, lcut, hcut, mean, sigma, npix);
-                else
-                    band_row_add<1, VEC>(row, mw, lcut, hcut, mean, sigma, npix);
-            }
-            __syncwarp();
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncwarp();
-        if (pass == 0) {
-            // src/back.c:249: too few valid pixels: a bad mesh
-            if ((float)npix < (float)(mw * mh * SX_BACK_MINGOODFRAC)) bad = true;
-            mean /= (double)npix;
-            sigma = (sig = sigma / npix - mean * mean) > 0.0 ? sqrt(sig) : 0.0;
-            lcut = (float)(mean - 2.0 * sigma);
-            hcut = (float)(mean + 2.0 * sigma);
-            mean = sigma = 0.0;
-            npix = 0;
-            if (__all_sync(0xffffffffu, bad || !active)) break;
-        }
-    }
-    if (!active) return;
-    MeshStat o;
-    o.mean = o.sigma = o.lcut = o.hcut = o.qzero = o.qscale = 0.f;
-    o.nlevels = o.npix = 0;
-    if (bad) {
-        o.mean = o.sigma = -SX_BIG;
-    } else {
-        o.lcut = lcut;
-        o.hcut = hcut;
-        o.npix = npix;
-        mean /= (double)npix;
-        sig = sigma / npix - mean * mean;
-        sigma = sig > 0.0 ? sqrt(sig) : 0.0;
-        o.mean = mean;
-        o.sigma = sigma;
-        if ((o.nlevels = (int)(step * npix + 1)) > SX_QUANTIF_NMAXLEVELS) o.nlevels = SX_QUANTIF_NMAXLEVELS;
-        o.qscale = sigma > 0.0 ? 2 * SX_QUANTIF_NSIGMA * sigma / o.nlevels : 1.0;
-        o.qzero = mean - SX_QUANTIF_NSIGMA * sigma;
-    }
-    ms[my * nbx + mx0 + lane] = o;
+    seq_stat<false>(MeshLoad<VEC>(img + (size_t)y0 * w + x0, w, mw, mh), mw * mh,
+                    (float)(mw * mh * SX_BACK_MINGOODFRAC), stage, o, nv);
+    if (threadIdx.x == 0) ms[m] = o;
 }
 
 constexpr int GUESS_THREADS = 256;
@@ -412,7 +445,7 @@ __global__ void __launch_bounds__(GUESS_THREADS) k_mesh_guess(const float *__res
 }
 
 // ---------------------------------------------------------------------------
-// backhisto + backguess with one warp per mesh, for meshes of fewer than
+// backhisto + backguess with one warp per mesh (or annulus), for fewer than
 // 65536 pixels (no bin count reaches 2^16).  The histogram is kept as 16-bit
 // counts, two per word, and summarised per chunk of 32 bins: the counts
 // below each chunk (cp) and each chunk's first and second moments (c1, c2).
@@ -425,11 +458,11 @@ constexpr int GW_WARPS = 4;                        // meshes (warps) per CTA
 constexpr int GW_CH = (SX_QUANTIF_NMAXLEVELS + 2 + 31) / 32;  // 32-bin chunks
 constexpr int GW_WORDS = GW_CH * 16;              // 16-bit counts of GW_CH * 32 bins
 
-struct GuessWarpSmem {
+struct __align__(16) GuessWarpSmem {
+    unsigned hw[GW_WORDS];  // bin b: bits 16 (b & 1) .. of word b >> 1
     long long c2[GW_CH];    // sum over the chunk of bin^2 * count
     int c1[GW_CH];          // sum over the chunk of bin * count (< 2^28)
     int cp[GW_CH + 1];      // counts of the bins below chunk c
-    unsigned hw[GW_WORDS];  // bin b: bits 16 (b & 1) .. of word b >> 1
 };
 
 __device__ __forceinline__ int gw_hist(const GuessWarpSmem &S, int b) {
@@ -443,61 +476,17 @@ __device__ __forceinline__ int gw_pfx(const GuessWarpSmem &S, int i, int lane) {
     return S.cp[c] + (int)__reduce_add_sync(0xffffffffu, (unsigned)v);
 }
 
-__global__ void __launch_bounds__(32 * GW_WARPS) k_mesh_guess_warp(const float *__restrict__ img, int w, int h, int bw,
-                                                                    int bh, int nbx, int nby,
-                                                                    const MeshStat *__restrict__ ms,
-                                                                    float *__restrict__ back,
-                                                                    float *__restrict__ sig) {
-    __shared__ GuessWarpSmem smem[GW_WARPS];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int m = blockIdx.x * GW_WARPS + wid;
-    if (m >= nbx * nby) return;  // whole warp
-    GuessWarpSmem &S = smem[wid];
-    const MeshStat bm = ms[m];
-    if (bm.mean <= -SX_BIG) {
-        if (lane == 0) back[m] = sig[m] = -SX_BIG;
-        return;
-    }
-    const int mx = m % nbx, my = m / nbx;
-    const int x0 = mx * bw, y0 = my * bh;
-    const int mw = (mx == nbx - 1 && w % bw) ? w % bw : bw;
-    const int mh = (my == nby - 1 && h % bh) ? h % bh : bh;
-    for (int i = lane; i < GW_WORDS; i += 32) S.hw[i] = 0u;
-    __syncwarp();
-    const int nlevels = bm.nlevels;
-    const float qscale = bm.qscale;
-    const float cste = 0.499999 - bm.qzero / qscale;
-    // the mesh's pixels k = lane, lane + 32, ... in row-major order, GW_LOADS
-    // loads in flight per lane; (row, col) of k advance by (drow, dcol) per 32
-    {
-        constexpr int GW_LOADS = 16;
-        const int npx = mw * mh;
-        const int drow = 32 / mw, dcol = 32 - drow * mw;
-        int row = lane / mw, col = lane - row * mw;
-        for (int k0 = 0; k0 < npx; k0 += 32 * GW_LOADS) {
-            float v[GW_LOADS];
-#pragma unroll
-            for (int g = 0; g < GW_LOADS; g++) {
-                // beyond the mesh: NaN, which the histogram skips as it does a NaN pixel
-                v[g] = k0 + 32 * g + lane < npx ? __ldg(img + (size_t)(y0 + row) * w + x0 + col)
-                                                : __int_as_float(0x7fffffff);
-                row += drow;
-                col += dcol;
-                if (col >= mw) {
-                    col -= mw;
-                    row++;
-                }
-            }
-#pragma unroll
-            for (int g = 0; g < GW_LOADS; g++) {
-                const float b = v[g] / qscale + cste;
-                if (b != b) continue;  // NaN: the host conversion yields INT_MIN
-                const int bin = (int)b;
-                if (bin >= 0 && bin < nlevels) atomicAdd(&S.hw[bin >> 1], 1u << ((bin & 1) << 4));
-            }
-        }
-    }
-    __syncwarp();
+// one pixel into the histogram
+__device__ __forceinline__ void gw_count(GuessWarpSmem &S, float v, float qscale, float cste, int nlevels) {
+    const float b = v / qscale + cste;
+    if (b != b) return;  // NaN: the host conversion yields INT_MIN
+    const int bin = (int)b;
+    if (bin >= 0 && bin < nlevels) atomicAdd(&S.hw[bin >> 1], 1u << ((bin & 1) << 4));
+}
+
+// backguess on the warp's histogram; every lane gets the mode and sigma
+__device__ __forceinline__ void gw_guess(GuessWarpSmem &S, const MeshStat &bm, float &mode, float &sg) {
+    const int lane = threadIdx.x & 31, nlevels = bm.nlevels;
     // chunk sums: lane owns chunks lane, lane + 32, ...; words read in an
     // order rotated by the lane (at most two lanes on a bank)
     int carry = 0;
@@ -612,18 +601,61 @@ __global__ void __launch_bounds__(32 * GW_WARPS) k_mesh_guess_warp(const float *
         lcut = (ftemp = med - 3.0 * sig_) > 0.0 ? (int)(ftemp > 0.0 ? ftemp + 0.5 : ftemp - 0.5) : 0;
         hcut = (ftemp = med + 3.0 * sig_) < nlevelsm1 ? (int)(ftemp > 0.0 ? ftemp + 0.5 : ftemp - 0.5) : nlevelsm1;
     }
+    // src/back.c:408: the C library abs(int) applied to the double sig
+    if (abs((int)sig_) > 0.0) {
+        if (fabs((mea - med) / sig_) < 0.3)
+            mode = bm.qzero + (2.5 * med - 1.5 * mea) * bm.qscale;
+        else
+            mode = bm.qzero + med * bm.qscale;
+    } else
+        mode = bm.qzero + mea * bm.qscale;
+    sg = sig_ * bm.qscale;
+}
+
+// the histogram of the n pixels of a sequence and its mode, by one warp
+template <bool VALID, class LOAD>
+__device__ __forceinline__ void gw_mode(LOAD load, int n, GuessWarpSmem &S, const MeshStat &bm, float &mode, float &sg) {
+    const int lane = threadIdx.x & 31;
+    for (int i = lane; i < GW_WORDS; i += 32) S.hw[i] = 0u;
+    __syncwarp();
+    const int nlevels = bm.nlevels;
+    const float qscale = bm.qscale;
+    const float cste = 0.499999 - bm.qzero / qscale;
+    for (int k0 = 0; k0 < n; k0 += SEQ_CHUNK) {
+        float v[SEQ_G];
+        load.chunk(v);
+#pragma unroll
+        for (int g = 0; g < SEQ_G; g++)
+            if (!VALID || v[g] > (float)-SX_BIG) gw_count(S, v[g], qscale, cste, nlevels);
+    }
+    __syncwarp();
+    gw_guess(S, bm, mode, sg);
+}
+
+// backstat, backhisto and backguess of every mesh, one warp each
+template <bool VEC>
+__global__ void __launch_bounds__(32 * GW_WARPS) k_mesh_mode(const float *__restrict__ img, int w, int h, int bw, int bh,
+                                                             int nbx, int nby, float *__restrict__ back,
+                                                             float *__restrict__ sig) {
+    __shared__ GuessWarpSmem smem[GW_WARPS];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int m = blockIdx.x * GW_WARPS + wid;
+    if (m >= nbx * nby) return;  // whole warp
+    int x0, y0, mw, mh, nv;
+    mesh_geometry(m, w, h, bw, bh, nbx, nby, x0, y0, mw, mh);
+    const MeshLoad<VEC> load(img + (size_t)y0 * w + x0, w, mw, mh);
+    MeshStat bm;
+    // (the histogram's words hold the staged stretches first)
+    seq_stat<false>(load, mw * mh, (float)(mw * mh * SX_BACK_MINGOODFRAC), reinterpret_cast<float *>(smem[wid].hw), bm,
+                    nv);
+    float mode = -SX_BIG, sg = -SX_BIG;
+    if (bm.mean > -SX_BIG) {
+        __syncwarp();
+        gw_mode<false>(load, mw * mh, smem[wid], bm, mode, sg);
+    }
     if (lane == 0) {
-        float mean;
-        // src/back.c:408: the C library abs(int) applied to the double sig
-        if (abs((int)sig_) > 0.0) {
-            if (fabs((mea - med) / sig_) < 0.3)
-                mean = bm.qzero + (2.5 * med - 1.5 * mea) * bm.qscale;
-            else
-                mean = bm.qzero + med * bm.qscale;
-        } else
-            mean = bm.qzero + mea * bm.qscale;
-        back[m] = mean;
-        sig[m] = sig_ * bm.qscale;
+        back[m] = mode;
+        sig[m] = sg;
     }
 }
 
@@ -656,79 +688,97 @@ __device__ __forceinline__ LocalBox local_box(int xmin, int xmax, int ymin, int 
     return B;
 }
 
-// the annulus pixels in the reference's collection order
-template <class F>
-__device__ __forceinline__ void local_visit(const float *__restrict__ sub, int w, const LocalBox &B, int pbs, F f) {
-    for (int y = B.bymin; y < B.bymax; y++) {
-        const float *row = sub + (size_t)y * w;
-        for (int x = B.bxmin; x < B.bxmin + pbs; x++) f(row[x]);
-        for (int x = B.ixmax; x < B.ixmax + pbs; x++) f(row[x]);
-    }
-    for (int y = B.bymin; y < B.iymin; y++)
-        for (int x = B.ixmin; x < B.ixmax; x++) f(sub[(size_t)y * w + x]);
-    for (int y = B.iymax; y < B.bymax; y++)
-        for (int x = B.ixmin; x < B.ixmax; x++) f(sub[(size_t)y * w + x]);
+__device__ __forceinline__ int local_npix(const LocalBox &B, int pbs) {
+    return (B.bymax - B.bymin) * 2 * pbs + ((B.iymin - B.bymin) + (B.bymax - B.iymax)) * (B.ixmax - B.ixmin);
 }
 
-// one thread per object: backstat over the valid annulus pixels (one mesh of
-// one column); nlevels = -1 marks "no local background" (annulus outside the
-// frame, or no valid pixel)
-__global__ void k_local_stat(const float *__restrict__ sub, int w, int h, int pbs, const int *__restrict__ xmin,
-                             const int *__restrict__ xmax, const int *__restrict__ ymin,
-                             const int *__restrict__ ymax, int n, const int *n_dev, MeshStat *__restrict__ ls) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+// the annulus pixels lane, lane + 32, ... in the reference's collection order
+struct LocalLoad {
+    const float *sub;
+    int w, i, n, ns, pbs, iw, bxmin, bymin, ixmin, ixmax, iymin, iymax;
+    FastDiv dsw, diw;
+    __device__ __forceinline__ LocalLoad(const float *sub_, int w_, const LocalBox &B, int pbs_) {
+        sub = sub_;
+        w = w_;
+        pbs = pbs_;
+        i = threadIdx.x & 31;
+        n = local_npix(B, pbs);
+        ns = (B.bymax - B.bymin) * 2 * pbs;
+        iw = B.ixmax - B.ixmin;
+        bxmin = B.bxmin;
+        bymin = B.bymin;
+        ixmin = B.ixmin;
+        ixmax = B.ixmax;
+        iymin = B.iymin;
+        iymax = B.iymax;
+        dsw = make_fastdiv_dev((unsigned)(2 * pbs));
+        diw = make_fastdiv_dev((unsigned)iw);
+    }
+    __device__ __forceinline__ void chunk(float *v) {
+#pragma unroll
+        for (int g = 0; g < SEQ_G; g++, i += 32) {
+            v[g] = __int_as_float(0x7fffffff);
+            if (i < n) {
+                int x, y;
+                if (i < ns) {
+                    const int r = (int)fdiv((unsigned)i, dsw), c = i - r * 2 * pbs;
+                    y = bymin + r;
+                    x = c < pbs ? bxmin + c : ixmax + c - pbs;
+                } else {
+                    const int k = i - ns, r = (int)fdiv((unsigned)k, diw);
+                    x = ixmin + k - r * iw;
+                    y = r < iymin - bymin ? bymin + r : iymax + r - (iymin - bymin);
+                }
+                v[g] = __ldg(sub + (size_t)y * w + x);
+            }
+        }
+    }
+    static __device__ __forceinline__ void store(float *stage, const float *v) {
+#pragma unroll
+        for (int g = 0; g < SEQ_G; g++) stage[seq_slot((threadIdx.x & 31) + 32 * g)] = v[g];
+    }
+};
+
+// one warp per object: backstat over the valid annulus pixels (one mesh of
+// one column) and, for annuli of fewer than 65536 pixels, the mode; nlevels =
+// -1 marks "no local background" (annulus outside the frame, or no valid
+// pixel)
+__global__ void __launch_bounds__(32 * GW_WARPS) k_local_stat(const float *__restrict__ sub, int w, int h, int pbs,
+                                                              const int *__restrict__ xmin,
+                                                              const int *__restrict__ xmax,
+                                                              const int *__restrict__ ymin,
+                                                              const int *__restrict__ ymax, int n, const int *n_dev,
+                                                              MeshStat *__restrict__ ls, float *__restrict__ dbkg) {
+    __shared__ GuessWarpSmem smem[GW_WARPS];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int o = blockIdx.x * GW_WARPS + wid;
     if (o >= sx_count(n, n_dev)) return;
     MeshStat s;
     s.mean = s.sigma = s.lcut = s.hcut = s.qzero = s.qscale = 0.f;
     s.nlevels = -1;
     s.npix = 0;
+    float mode = 0.0f;
     const LocalBox B = local_box(xmin[o], xmax[o], ymin[o], ymax[o], w, h, pbs);
-    if (!B.ok) {
-        ls[o] = s;
-        return;
+    if (B.ok) {
+        const LocalLoad load(sub, w, B, pbs);
+        MeshStat t;
+        int nv;
+        seq_stat<true>(load, load.n, 1.0f, reinterpret_cast<float *>(smem[wid].hw), t, nv);
+        if (nv) {
+            s = t;
+            float sg;
+            __syncwarp();
+            if (load.n < 65536) gw_mode<true>(load, load.n, smem[wid], s, mode, sg);
+        }
     }
-    const double step = sqrt(2 / SX_PI) * SX_QUANTIF_NSIGMA / SX_QUANTIF_AMIN;
-    double mean = 0.0, sigma = 0.0, sig;
-    int npix = 0;
-    // a pixel left out adds +0.0 (the sums are never -0.0), see mesh_stat_seq
-    local_visit(sub, w, B, pbs, [&](float p) {
-        const double pix = p;
-        const bool in = pix > -SX_BIG;
-        mean += in ? pix : 0.0;
-        sigma += in ? pix * pix : 0.0;
-        npix += in;
-    });
-    if (!npix) {
+    if (lane == 0) {
         ls[o] = s;
-        return;
+        dbkg[o] = mode;
     }
-    mean /= (double)npix;
-    sigma = (sig = sigma / npix - mean * mean) > 0.0 ? sqrt(sig) : 0.0;
-    const float lcut = s.lcut = (float)(mean - 2.0 * sigma);
-    const float hcut = s.hcut = (float)(mean + 2.0 * sigma);
-    mean = sigma = 0.0;
-    int npix2 = 0;
-    local_visit(sub, w, B, pbs, [&](float p) {
-        const double pix = p;
-        const bool in = pix > -SX_BIG && pix <= hcut && pix >= lcut;
-        mean += in ? pix : 0.0;
-        sigma += in ? pix * pix : 0.0;
-        npix2 += in;
-    });
-    s.npix = npix2;
-    mean /= (double)npix2;
-    sig = sigma / npix2 - mean * mean;
-    sigma = sig > 0.0 ? sqrt(sig) : 0.0;
-    s.mean = mean;
-    s.sigma = sigma;
-    if ((s.nlevels = (int)(step * npix2 + 1)) > SX_QUANTIF_NMAXLEVELS) s.nlevels = SX_QUANTIF_NMAXLEVELS;
-    s.qscale = sigma > 0.0 ? 2 * SX_QUANTIF_NSIGMA * sigma / s.nlevels : 1.0;
-    s.qzero = mean - SX_QUANTIF_NSIGMA * sigma;
-    ls[o] = s;
 }
 
-// one CTA per object: the annulus histogram (integer counts, any order) and
-// backguess; dbkg = its mode, 0 without a local background
+// annuli of 65536 pixels or more, one CTA per object: the histogram (integer
+// counts, any order) and backguess
 __global__ void __launch_bounds__(GUESS_THREADS) k_local_guess(const float *__restrict__ sub, int w, int h, int pbs,
                                                                  const int *__restrict__ xmin,
                                                                  const int *__restrict__ xmax,
@@ -741,11 +791,9 @@ __global__ void __launch_bounds__(GUESS_THREADS) k_local_guess(const float *__re
     const int o = blockIdx.x;
     if (o >= sx_count(n, n_dev)) return;
     const MeshStat bm = ls[o];
-    if (bm.nlevels < 0) {
-        if (threadIdx.x == 0) dbkg[o] = 0.0f;
-        return;
-    }
+    if (bm.nlevels < 0) return;
     const LocalBox B = local_box(xmin[o], xmax[o], ymin[o], ymax[o], w, h, pbs);
+    if (local_npix(B, pbs) < 65536) return;
     for (int i = threadIdx.x; i < SX_QUANTIF_NMAXLEVELS + 2; i += GUESS_THREADS) hist[i] = 0;
     __syncthreads();
     const int nlevels = bm.nlevels;
@@ -856,7 +904,11 @@ __device__ unsigned select_kth(const float *v, int n, int k, unsigned lowkey, un
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
             unsigned key = f2ord(v[i]);
             if (key < lowkey) continue;
-            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255], 1u);
+            if ((key & mask) == prefix) {
+                // (mesh values are close together: most of a warp on one bin)
+                const unsigned d = (key >> shift) & 255, same = __match_any_sync(__activemask(), d);
+                if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&hist[d], (unsigned)__popc(same));
+            }
         }
         __syncthreads();
         __shared__ unsigned s_digit, s_k;
@@ -895,24 +947,53 @@ __device__ unsigned select_kth(const float *v, int n, int k, unsigned lowkey, un
     return prefix;
 }
 
-// global medians of the filtered maps (src/back.c:536-557), one CTA
+// median of the n values with key >= lowkey out of v[0..m), by one CTA: the
+// element of rank n / 2, or for even n the mean with the one below it (the
+// next rank is the same value again or the smallest above it)
+__device__ float median_of(const float *v, int m, int n, unsigned lowkey, unsigned *hist) {
+    __shared__ unsigned s_le, s_above;
+    const int k = n & 1 ? n / 2 : n / 2 - 1;
+    const unsigned ka = select_kth(v, m, k, lowkey, hist);
+    if (n & 1) return ord2f(ka);
+    if (threadIdx.x == 0) {
+        s_le = 0u;
+        s_above = 0xffffffffu;
+    }
+    __syncthreads();
+    unsigned le = 0, above = 0xffffffffu;
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const unsigned key = f2ord(v[i]);
+        if (key < lowkey) continue;
+        if (key <= ka)
+            le++;
+        else
+            above = min(above, key);
+    }
+    le = __reduce_add_sync(0xffffffffu, le);
+    above = __reduce_min_sync(0xffffffffu, above);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&s_le, le);
+        atomicMin(&s_above, above);
+    }
+    __syncthreads();
+    const float a = ord2f(ka), b = s_le > (unsigned)k + 1u ? a : ord2f(s_above);
+    __syncthreads();
+    return (float)((a + b) / 2.0);
+}
+
+// global medians of the filtered maps (src/back.c:536-557), one CTA for the
+// background and one for the rms and the thresholds that follow from it
 __global__ void k_back_medians(const float *__restrict__ back3, const float *__restrict__ sigma3, int nb,
                                FrameScalars *sc, int back_type, float back_value, int thresh_type,
                                double dthr, double athr) {
     __shared__ unsigned hist[256];
     __shared__ unsigned s_npos;
-    float med[2];
-    for (int q = 0; q < 2; q++) {
-        const float *v = q ? sigma3 : back3;
-        if (nb & 1) {
-            med[q] = ord2f(select_kth(v, nb, nb / 2, 0u, hist));
-        } else {
-            float a = ord2f(select_kth(v, nb, nb / 2 - 1, 0u, hist));
-            float b = ord2f(select_kth(v, nb, nb / 2, 0u, hist));
-            med[q] = (float)((a + b) / 2.0);
-        }
+    if (blockIdx.x == 0) {
+        const float med = median_of(back3, nb, nb, 0u, hist);
+        if (threadIdx.x == 0) sc->backmean = back_type == 1 ? back_value : med;
+        return;
     }
-    float backsig = med[1];
+    float backsig = median_of(sigma3, nb, nb, 0u, hist);
     if (backsig <= 0.0) {
         // median of the strictly positive sigmas, else 1.0
         if (threadIdx.x == 0) s_npos = 0;
@@ -921,21 +1002,14 @@ __global__ void k_back_medians(const float *__restrict__ back3, const float *__r
         for (int i = threadIdx.x; i < nb; i += blockDim.x) c += sigma3[i] > 0.0f;
         atomicAdd(&s_npos, c);
         __syncthreads();
-        int npos = (int)s_npos;
-        unsigned low = f2ord(__uint_as_float(1u));  // smallest positive float
-        if (npos > 0 && npos < nb) {
-            if (npos & 1)
-                backsig = ord2f(select_kth(sigma3, nb, npos / 2, low, hist));
-            else {
-                float a = ord2f(select_kth(sigma3, nb, npos / 2 - 1, low, hist));
-                float b = ord2f(select_kth(sigma3, nb, npos / 2, low, hist));
-                backsig = (float)((a + b) / 2.0);
-            }
-        } else
+        const int npos = (int)s_npos;
+        const unsigned low = f2ord(__uint_as_float(1u));  // smallest positive float
+        if (npos > 0 && npos < nb)
+            backsig = median_of(sigma3, nb, npos, low, hist);
+        else
             backsig = 1.0;
     }
     if (threadIdx.x == 0) {
-        sc->backmean = back_type == 1 ? back_value : med[0];
         sc->backsig = backsig;
         if (thresh_type == 1) {
             sc->dthresh = (float)dthr;
@@ -948,31 +1022,52 @@ __global__ void k_back_medians(const float *__restrict__ back3, const float *__r
     }
 }
 
-// src/back.c:739-773 (makebackspline), one thread per mesh column
-__global__ void k_back_spline(const float *__restrict__ map, float *__restrict__ dmap, float *__restrict__ u,
-                              int nbx, int nby) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
+// Splines.  The forward recurrences of src/back.c divide by values that do not
+// depend on the data, and end in (float) / 6.0, a double division rounded to
+// float.  A float divided by 6 never lies near the middle of two floats (6 m
+// would need 25 bits or more for a midpoint m, and a float is at least 2^-28
+// of it away), or is that middle exactly, so the float division gives the same
+// value and is a third of the latency.
+//
+// One thread walks a line; what it reads again on the way back is kept in
+// shared memory (the walks waited about 600 cycles a step on their own stores:
+// 40 us and 37 us under ncu for the 64 x 64 meshes of a 4096 x 4096 frame, 28
+// and 13 so).
+constexpr int SPL_MAX = 768;   // longest line kept there; longer ones use the global arrays
+
+// src/back.c:739-773 (makebackspline), one thread per mesh column; u: scratch
+// of the columns longer than SPL_MAX
+__global__ void __launch_bounds__(32) k_back_spline(const float *__restrict__ map, float *__restrict__ dmap,
+                                                    float *__restrict__ u, int nbx, int nby) {
+    extern __shared__ float spl[];
+    const int x = blockIdx.x * 32 + threadIdx.x;
     if (x >= nbx) return;
-    float temp;
-    if (nby > 1) {
-        // the previous step's values are carried in registers, not read back
-        // from the arrays just written (same operations, same order)
-        float *ux = u + (size_t)x * nby;
-        float dprev = 0.0f, uprev = 0.0f;
-        dmap[x] = ux[0] = 0.0;
-        for (int y = 1; y < nby - 1; y++) {
-            temp = -1 / (dprev + 4);
-            dmap[(size_t)y * nbx + x] = dprev = temp;
-            temp *= uprev - 6 * (map[(size_t)(y + 1) * nbx + x] + map[(size_t)(y - 1) * nbx + x]
-                                 - 2 * map[(size_t)y * nbx + x]);
-            ux[y] = uprev = temp;
-        }
-        dmap[(size_t)(nby - 1) * nbx + x] = 0.0;
-        float dnext = 0.0f;
-        for (int y = nby - 2; y >= 1; y--)
-            dmap[(size_t)y * nbx + x] = dnext = (dmap[(size_t)y * nbx + x] * dnext + ux[y]) / 6.0;
-    } else
+    if (nby <= 1) {
         dmap[x] = 0.0;
+        return;
+    }
+    const bool in_smem = nby <= SPL_MAX;
+    float *ux = in_smem ? spl + threadIdx.x : u + (size_t)x * nby;
+    float *dx = in_smem ? spl + (size_t)32 * nby + threadIdx.x : dmap + x;
+    const int us = in_smem ? 32 : 1, ds = in_smem ? 32 : nbx;
+    float temp, dprev = 0.0f, uprev = 0.0f;
+    dmap[x] = 0.0;
+    float m0 = map[x], m1 = map[nbx + x];
+#pragma unroll 8
+    for (int y = 1; y < nby - 1; y++) {
+        const float m2 = map[(size_t)(y + 1) * nbx + x];
+        temp = -1 / (dprev + 4);
+        dx[(size_t)y * ds] = dprev = temp;
+        temp *= uprev - 6 * (m2 + m0 - 2 * m1);
+        ux[(size_t)y * us] = uprev = temp;
+        m0 = m1;
+        m1 = m2;
+    }
+    dmap[(size_t)(nby - 1) * nbx + x] = 0.0;
+    float dnext = 0.0f;
+#pragma unroll 4
+    for (int y = nby - 2; y >= 1; y--)
+        dmap[(size_t)y * nbx + x] = dnext = (dx[(size_t)y * ds] * dnext + ux[(size_t)y * us]) / 6.0f;
 }
 
 // src/back.c:938-1040 (backrmsline): the rms map of every pixel from the
@@ -997,16 +1092,16 @@ __global__ void k_rms_map(const float *__restrict__ node, const float *__restric
 }
 
 // src/back.c:790-862: y-interpolated nodes of every image row and their
-// x-direction second derivatives (one thread per row)
-__global__ void k_row_nodes(const float *__restrict__ back, const float *__restrict__ dback, int nbx, int nby,
-                            int backh, int h, float *__restrict__ node, float *__restrict__ dnode,
-                            float *__restrict__ u) {
-    int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= h) return;
-    float *nd = node + (size_t)y * nbx, *dnd = dnode + (size_t)y * nbx, *uu = u + (size_t)y * nbx;
-    if (nby > 1) {
+// x-direction second derivatives; one block takes SPL_ROWS rows, all its
+// threads the nodes, then one thread per row the recurrence
+constexpr int SPL_ROWS = 32;
+constexpr int SPL_THREADS = 256;
+
+struct RowNode {
+    const float *blo, *bhi, *dblo, *dbhi;
+    float dy, cdy, dy3, cdy3;
+    __device__ __forceinline__ RowNode(const float *back, const float *dback, int nbx, int nby, int backh, int y) {
         int yl;
-        float dy, dy3, cdy, cdy3, temp;
         dy = (float)y / backh - 0.5;
         dy -= (yl = (int)dy);
         if (yl < 0) {
@@ -1019,39 +1114,114 @@ __global__ void k_row_nodes(const float *__restrict__ back, const float *__restr
         cdy = 1 - dy;
         dy3 = (dy * dy * dy - dy);
         cdy3 = (cdy * cdy * cdy - cdy);
-        const float *blo = back + (size_t)nbx * yl, *bhi = blo + nbx;
-        const float *dblo = dback + (size_t)nbx * yl, *dbhi = dblo + nbx;
-        for (int x = 0; x < nbx; x++) nd[x] = cdy * blo[x] + dy * bhi[x] + cdy3 * dblo[x] + dy3 * dbhi[x];
-        if (nbx > 1) {
-            // node values recomputed and the previous step carried in
-            // registers instead of read back from this thread's own stores
-            // (the same operations in the same order, so the same values)
-            auto node_at = [&](int x) { return cdy * blo[x] + dy * bhi[x] + cdy3 * dblo[x] + dy3 * dbhi[x]; };
-            float dprev = 0.0f, uprev = 0.0f, nm = node_at(0), n0 = node_at(1);
-            dnd[0] = uu[0] = 0.0;
-            for (int x = 1; x < nbx - 1; x++) {
-                const float np = node_at(x + 1);
-                temp = -1 / (dprev + 4);
-                dnd[x] = dprev = temp;
-                temp *= uprev - 6 * (np + nm - 2 * n0);
-                uu[x] = uprev = temp;
-                nm = n0;
-                n0 = np;
+        blo = back + (size_t)nbx * yl;
+        bhi = blo + nbx;
+        dblo = dback + (size_t)nbx * yl;
+        dbhi = dblo + nbx;
+    }
+    __device__ __forceinline__ float at(int x) const {
+        return cdy * __ldg(blo + x) + dy * __ldg(bhi + x) + cdy3 * __ldg(dblo + x) + dy3 * __ldg(dbhi + x);
+    }
+};
+
+__global__ void __launch_bounds__(SPL_THREADS) k_row_nodes(const float *__restrict__ back,
+                                                           const float *__restrict__ dback, int nbx, int nby,
+                                                           int backh, int h, float *__restrict__ node,
+                                                           float *__restrict__ dnode) {
+    extern __shared__ float spl[];  // SPL_ROWS x (nbx | 1) nodes, as many u, the d of every column
+    const int y0 = blockIdx.x * SPL_ROWS, rows = min(SPL_ROWS, h - y0), pitch = nbx | 1;
+    float *su = spl + SPL_ROWS * pitch, *sd = su + SPL_ROWS * pitch;
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < rows; r += SPL_THREADS / 32) {
+        const size_t at = (size_t)(y0 + r) * nbx;
+        if (nby > 1) {
+            const RowNode N(back, dback, nbx, nby, backh, y0 + r);
+            for (int x = lane; x < nbx; x += 32) node[at + x] = spl[r * pitch + x] = N.at(x);
+        } else {
+            for (int x = lane; x < nbx; x += 32) {
+                node[at + x] = __ldg(back + x);
+                dnode[at + x] = __ldg(dback + x);
             }
-            dnd[nbx - 1] = 0.0;
-            float dnext = 0.0f;
-            for (int x = nbx - 2; x >= 1; x--) dnd[x] = dnext = (dnd[x] * dnext + uu[x]) / 6.0;
-        } else
-            dnd[0] = 0.0;
-    } else {
+        }
+    }
+    if (nby <= 1) return;
+    __syncthreads();
+    if (threadIdx.x < rows) {
+        const float *n = spl + threadIdx.x * pitch;
+        float *u = su + threadIdx.x * pitch;
+        float temp, dprev = 0.0f, uprev = 0.0f;
+        // (every row's d is the same: written alike by all)
+#pragma unroll 4
+        for (int x = 1; x < nbx - 1; x++) {
+            temp = -1 / (dprev + 4);
+            sd[x] = dprev = temp;
+            temp *= uprev - 6 * (n[x + 1] + n[x - 1] - 2 * n[x]);
+            u[x] = uprev = temp;
+        }
+        u[0] = u[nbx - 1] = 0.0;
+        float dnext = 0.0f;
+        __syncwarp(__activemask());
+#pragma unroll 4
+        for (int x = nbx - 2; x >= 1; x--) u[x] = dnext = (sd[x] * dnext + u[x]) / 6.0f;
+    }
+    __syncthreads();
+    for (int r = threadIdx.x >> 5; r < rows; r += SPL_THREADS / 32)
+        for (int x = lane; x < nbx; x += 32) dnode[(size_t)(y0 + r) * nbx + x] = su[r * pitch + x];
+}
+
+// the same for rows of more than SPL_MAX nodes, one thread per row, what it
+// reads again in global memory (u: h x nbx)
+__global__ void k_row_nodes_long(const float *__restrict__ back, const float *__restrict__ dback, int nbx, int nby,
+                                 int backh, int h, float *__restrict__ node, float *__restrict__ dnode,
+                                 float *__restrict__ u) {
+    const int y = blockIdx.x * blockDim.x + threadIdx.x;
+    if (y >= h) return;
+    float *nd = node + (size_t)y * nbx, *dnd = dnode + (size_t)y * nbx, *uu = u + (size_t)y * nbx;
+    if (nby <= 1) {
         for (int x = 0; x < nbx; x++) {
             nd[x] = back[x];
             dnd[x] = dback[x];
         }
+        return;
     }
+    const RowNode N(back, dback, nbx, nby, backh, y);
+    for (int x = 0; x < nbx; x++) nd[x] = N.at(x);
+    float temp, dprev = 0.0f, uprev = 0.0f, nm = N.at(0), n0 = N.at(1);
+    dnd[0] = uu[0] = 0.0;
+    for (int x = 1; x < nbx - 1; x++) {
+        const float np = N.at(x + 1);
+        temp = -1 / (dprev + 4);
+        dnd[x] = dprev = temp;
+        temp *= uprev - 6 * (np + nm - 2 * n0);
+        uu[x] = uprev = temp;
+        nm = n0;
+        n0 = np;
+    }
+    dnd[nbx - 1] = 0.0;
+    float dnext = 0.0f;
+    for (int x = nbx - 2; x >= 1; x--) dnd[x] = dnext = (dnd[x] * dnext + uu[x]) / 6.0f;
 }
 
-// ---------------------------------------------------------------------------
+// the splines of a mesh map along y (dmap), then the nodes of every image row
+// and their second derivatives along x; u: max(nbx * nby, h * nbx) floats
+void launch_map_nodes(const float *map, float *dmap, float *u, int nbx, int nby, int bh, int h, float *node,
+                      float *dnode, float *rowu, cudaStream_t st) {
+    static DevCache attr;
+    attr.get([](int) {
+        cudaFuncSetAttribute(k_back_spline, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * SPL_MAX * 4);
+        cudaFuncSetAttribute(k_row_nodes, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             ((2 * SPL_ROWS + 1) * (SPL_MAX + 1)) * 4);
+        return 1;
+    });
+    const size_t sb = nby <= SPL_MAX ? (size_t)64 * nby * 4 : 0;
+    k_back_spline<<<(nbx + 31) / 32, 32, sb, st>>>(map, dmap, u, nbx, nby);
+    if (nbx <= SPL_MAX)
+        k_row_nodes<<<(h + SPL_ROWS - 1) / SPL_ROWS, SPL_THREADS, (size_t)(2 * SPL_ROWS + 1) * (nbx | 1) * 4, st>>>(
+            map, dmap, nbx, nby, bh, h, node, dnode);
+    else
+        k_row_nodes_long<<<(h + 127) / 128, 128, 0, st>>>(map, dmap, nbx, nby, bh, h, node, dnode, rowu);
+}
+
 // ---------------------------------------------------------------------------
 // weight maps: blank the unusable pixels, then (after the background) the
 // scale factor sigfac and the calibrated variance map
@@ -1109,13 +1279,7 @@ __global__ void k_weight_sigfac(const float *__restrict__ ratio, int nb, FrameSc
     const int npos = (int)s_npos;
     const unsigned low = f2ord(__uint_as_float(1u));  // smallest positive float
     float f = 1.0f;
-    if (npos & 1) {
-        f = ord2f(select_kth(ratio, nb, npos / 2, low, hist));
-    } else if (npos) {
-        const float a = ord2f(select_kth(ratio, nb, npos / 2 - 1, low, hist));
-        const float b = ord2f(select_kth(ratio, nb, npos / 2, low, hist));
-        f = (float)((a + b) / 2.0);
-    }
+    if (npos) f = median_of(ratio, nb, npos, low, hist);
     if (threadIdx.x == 0) sc->sigfac = f;
 }
 
@@ -1147,50 +1311,29 @@ void launch_weight_var(const BackBufs &B, const float *wmap, const FrameParams &
 void launch_background(BackBufs &B, const float *img, const FrameParams &P, FrameScalars *d_sc,
                        cudaStream_t st, int &launches) {
     int nb = P.nbx * P.nby;
-    // row-band kernel when BAND_STAGES rows of 32 meshes fit in 200 KB of
-    // shared memory
-    const bool vec = (P.w % 4) == 0 && (P.bw % 4) == 0 && ((uintptr_t)img & 15) == 0;
-    int stride;
-    if (vec) {
-        stride = (P.bw + 3) & ~3;
-        if (((stride >> 2) & 1) == 0) stride += 4;  // stride / 4 odd
-    } else {
-        stride = P.bw | 1;  // odd
-    }
-    const size_t band_bytes = (size_t)BAND_STAGES * 32 * stride * sizeof(float);
-    constexpr int BAND_SMEM_MAX = 200 * 1024;
-    if (band_bytes <= BAND_SMEM_MAX) {
-        // the shared memory limit of both instances, once per device (host
-        // threads of a batch may get here at the same time)
-        static DevCache attr_set;
-        attr_set.get([](int) {
-            cudaFuncSetAttribute(k_mesh_stat_band<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, BAND_SMEM_MAX);
-            cudaFuncSetAttribute(k_mesh_stat_band<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, BAND_SMEM_MAX);
-            return 1;
-        });
-        dim3 grid((P.nbx + 31) / 32, P.nby);
+    // 16-byte loads where every mesh row begins on and is a multiple of 16 bytes
+    const bool vec = P.w % 4 == 0 && P.bw % 4 == 0 && ((uintptr_t)img & 15) == 0;
+    if ((long long)P.bw * P.bh < 65536) {
+        const unsigned g = (unsigned)((nb + GW_WARPS - 1) / GW_WARPS);
         if (vec)
-            k_mesh_stat_band<true><<<grid, 32, band_bytes, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, stride, B.ms);
+            k_mesh_mode<true><<<g, 32 * GW_WARPS, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.back, B.sigma);
         else
-            k_mesh_stat_band<false><<<grid, 32, band_bytes, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, stride,
-                                                                   B.ms);
+            k_mesh_mode<false><<<g, 32 * GW_WARPS, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.back, B.sigma);
     } else {
-        k_mesh_stat<<<(nb + 127) / 128, 128, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms);
-    }
-    if ((long long)P.bw * P.bh < 65536)
-        k_mesh_guess_warp<<<(nb + GW_WARPS - 1) / GW_WARPS, 32 * GW_WARPS, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx,
-                                                                                   P.nby, B.ms, B.back, B.sigma);
-    else
+        if (vec)
+            k_mesh_stat<true><<<nb, 32, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms);
+        else
+            k_mesh_stat<false><<<nb, 32, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms);
         k_mesh_guess<<<nb, GUESS_THREADS, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms, B.back, B.sigma);
+        launches += 1;
+    }
     k_mesh_badfill<<<(nb + 127) / 128, 128, 0, st>>>(B.back, B.sigma, B.back2, P.nbx, P.nby);
     k_mesh_median<<<(nb + 127) / 128, 128, 0, st>>>(B.back2, B.sigma, B.back3, B.sigma3, P.nbx, P.nby, P.nfx / 2,
                                                    P.nfy / 2, P.fthresh);
-    k_back_medians<<<1, 1024, 0, st>>>(B.back3, B.sigma3, nb, d_sc, P.back_type, P.back_value, P.thresh_type,
+    k_back_medians<<<2, 1024, 0, st>>>(B.back3, B.sigma3, nb, d_sc, P.back_type, P.back_value, P.thresh_type,
                                        P.detect_thresh, P.analysis_thresh);
-    k_back_spline<<<(P.nbx + 127) / 128, 128, 0, st>>>(B.back3, B.dback, B.u, P.nbx, P.nby);
-    k_row_nodes<<<(P.h + 127) / 128, 128, 0, st>>>(B.back3, B.dback, P.nbx, P.nby, P.bh, P.h, B.rownode,
-                                                  B.rowdnode, B.rowu);
-    launches += 7;
+    launch_map_nodes(B.back3, B.dback, B.u, P.nbx, P.nby, P.bh, P.h, B.rownode, B.rowdnode, B.rowu, st);
+    launches += 6;
 }
 
 }  // namespace sx

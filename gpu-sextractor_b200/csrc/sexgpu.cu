@@ -662,11 +662,8 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
         EN(rmsu, std::max((size_t)nbm * 4 + 64, (size_t)h * Pm.nbx * 4));
         EN(rmsnode, (size_t)h * Pm.nbx * 4);
         EN(rmsdnode, (size_t)h * Pm.nbx * 4);
-        k_back_spline<<<(Pm.nbx + 127) / 128, 128, 0, st>>>(B.sigma3, P<float>(ctx->rmsd), P<float>(ctx->rmsu), Pm.nbx,
-                                                            Pm.nby);
-        k_row_nodes<<<(h + 127) / 128, 128, 0, st>>>(B.sigma3, P<float>(ctx->rmsd), Pm.nbx, Pm.nby, Pm.bh, h,
-                                                     P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode),
-                                                     P<float>(ctx->rmsu));
+        launch_map_nodes(B.sigma3, P<float>(ctx->rmsd), P<float>(ctx->rmsu), Pm.nbx, Pm.nby, Pm.bh, h,
+                         P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), P<float>(ctx->rmsu), st);
         k_rms_map<<<grid1(N, 256), 256, 0, st>>>(P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), B.colk, B.coldx,
                                                 Pm.nbx, w, N, P<float>(ctx->wvar), 1);
         ps.wvar = P<float>(ctx->wvar);
@@ -1736,11 +1733,8 @@ int sexgpu_background_rms(sexgpu_ctx *ctx, float *rms) {
     EN(rmsnode, (size_t)h * Pm.nbx * 4);
     EN(rmsdnode, (size_t)h * Pm.nbx * 4);
     EN(rmsmap, (size_t)N * 4);
-    k_back_spline<<<(Pm.nbx + 127) / 128, 128, 0, st>>>(ps.B.sigma3, P<float>(ctx->rmsd), P<float>(ctx->rmsu), Pm.nbx,
-                                                        Pm.nby);
-    k_row_nodes<<<(h + 127) / 128, 128, 0, st>>>(ps.B.sigma3, P<float>(ctx->rmsd), Pm.nbx, Pm.nby, Pm.bh, h,
-                                                 P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode),
-                                                 P<float>(ctx->rmsu));
+    launch_map_nodes(ps.B.sigma3, P<float>(ctx->rmsd), P<float>(ctx->rmsu), Pm.nbx, Pm.nby, Pm.bh, h,
+                     P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), P<float>(ctx->rmsu), st);
     k_rms_map<<<grid1(N, 256), 256, 0, st>>>(P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), ps.B.colk, ps.B.coldx,
                                             Pm.nbx, w, N, P<float>(ctx->rmsmap), 0);
     CK(cudaMemcpyAsync(rms, ctx->rmsmap.p, (size_t)N * 4, cudaMemcpyDeviceToHost, st));

@@ -356,3 +356,54 @@ def test_deblending_by_number_of_peaks(gpu_ctx, peaks, nthresh, mincont, minarea
                  analysis_thresh=5.0, deblend_nthresh=nthresh, deblend_mincont=mincont, detect_minarea=minarea,
                  clean_flag=0)
     assert len(g) >= 3
+
+
+@pytest.mark.parametrize("kind", ["halves", "eighths", "zero_mean", "wide", "growing", "tiny", "inf", "mostly_blank",
+                                  "integers"])
+@pytest.mark.parametrize("shape,bs", [((200, 333), 37), ((300, 516), 128), ((64, 64), 64), ((640, 700), 300),
+                                      ((9, 2000), 1024)])
+def test_background_sums_round_like_the_sequence(gpu_ctx, kind, shape, bs):
+    """The mesh sums are cut into stretches and composed; every rounding of the
+    reference's pixel-by-pixel sums has to come out: squares that tie half way
+    between two doubles (values with few bits), sums that jump over binades
+    inside a stretch, sums of both signs, pixels whose sum is not exact,
+    infinities, blanks.  Bit for bit, with ragged meshes and meshes above 65535
+    pixels."""
+    rng = np.random.default_rng(len(kind) * 1000 + bs)
+    n = rng.normal(0.0, 1.0, shape)
+    if kind == "halves":
+        img = np.round(2 * (1000.5 + 40 * n)) / 2 + 2.0 ** -13
+    elif kind == "eighths":
+        img = np.round(8 * (90000.0 + 3000 * n)) / 8
+    elif kind == "zero_mean":
+        img = 8.0 * n
+    elif kind == "wide":
+        img = np.exp(rng.uniform(-25, 25, shape))
+    elif kind == "growing":
+        img = np.exp(np.linspace(-20, 40, n.size)).reshape(shape) * (1 + 0.01 * n)
+    elif kind == "tiny":
+        img = 1e-42 * (1.0 + n * n) + np.where(n > 2, 1e-20, 0.0)
+    elif kind == "inf":
+        img = 100.0 + n
+        img[shape[0] // 2, ::71] = np.inf
+    elif kind == "mostly_blank":
+        img = np.where(rng.random(shape) < 0.47, -1e30, 500.0 + 20 * n)
+    else:
+        img = np.rint(30000.0 + 200 * n)
+    img = img.astype(np.float32)
+    with np.errstate(all="ignore"):
+        sub_o, back_o, sig_o, so = O.background(img, back_size=bs)
+    sub_g, back_g, sig_g, sg = gpu_ctx.background(img, back_size=bs)
+    assert np.array_equal(back_g, back_o, equal_nan=True)
+    assert np.array_equal(sig_g, sig_o, equal_nan=True)
+    assert np.array_equal([sg.backmean, sg.backsig], [so.backmean, so.backsig], equal_nan=True)
+
+
+@pytest.mark.parametrize("w,h,bs", [(70, 1600, 2), (1600, 70, 2), (1536, 40, 2), (33, 1540, 2), (64, 64, 64), (3, 90, 2)])
+def test_background_splines_long_and_short(gpu_ctx, w, h, bs):
+    """Mesh grids on either side of the longest line whose spline is kept on
+    chip (768 meshes), one mesh, two meshes: background and rms maps."""
+    img = synth.frame_c0(seed=31, w=w, h=h, nsrc=20)
+    gpu_ctx.extract(img, back_size=bs)
+    assert gpu_ctx.background_map(img.shape).tobytes() == O.background_map(img, back_size=bs).tobytes()
+    assert gpu_ctx.background_rms(img.shape).tobytes() == O.background_rms(img, back_size=bs).tobytes()
