@@ -110,6 +110,7 @@ struct AnaArgs {
     ExamRaw *xraw;      // per-object scratch between the two examineiso kernels
     const float *cd, *sub, *back;
     const unsigned *opix;
+    unsigned long long *last;   // completion key of every raw object
     ObjBufs O;
     FrameScalars *sc;
     int w, h, nbx, nby, bw, bh, nobj, minarea, clean_flag;
@@ -413,6 +414,22 @@ __global__ void k_examine_finish(AnaArgs A) {
             if (fwhm > 0.0) fwhm -= 1 / (4 * fwhm);
         }
     }
+    // completion order of the raw object: its last row and the first column on
+    // it, over its objects' lists (a list's pixels on its last row come last)
+    if (n > 0) {
+        const unsigned *pix = A.opix + A.O.off[o];
+        const int ymax = (int)fdiv(pix[n - 1], A.wdiv);
+        int lo = 0, hi = n - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if ((int)pix[mid] >= ymax * w)
+                hi = mid;
+            else
+                lo = mid + 1;
+        }
+        atomicMax(A.last + A.O.root[o],
+                  ((unsigned long long)(unsigned)ymax << 32) | (0xffffffffu - (pix[lo] - (unsigned)ymax * w)));
+    }
     int py = (int)fdiv((unsigned)peakpix, A.wdiv);
     // the mode is added only where it was measured (src/back.c:659)
     A.O.bkg[o] = A.O.dbkg && A.O.lstat[o].nlevels >= 0 ? bkg + dbkg : bkg;
@@ -431,116 +448,157 @@ __global__ void k_examine_finish(AnaArgs A) {
     if (stv.ovf | svar.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
 }
 
-// Object pixel lists: the objects of one raw object are consecutive and
-// share out exactly its pixels, so ordering all pixels by object (raster
-// order inside each object) is a stable partition of every raw object's
-// pixel range by object.  One warp per raw object walks its pixels in order,
-// 32 at a time; lanes holding the same object take consecutive slots from
-// that object's cursor in shared memory.  A raw object that is one object is
-// copied; raw objects of more than OP_KMAX objects are left to
-// k_obj_partition_big (their cursors in dynamic shared memory).
-constexpr int OP_WARPS = 8;
-constexpr int OP_KMAX = 256;
-constexpr int OP_BIG_KMAX = 12288;  // cursors of k_obj_partition_big in shared memory (48 KB)
-constexpr int OP_BIG_GRID = 148;
+// Object pixel lists, in raster order inside each object: an object's pixels
+// are those of its box that the allocation map gives to it, read row by row.
+// One warp reads a box of up to OL_WARP_MAX pixels; larger ones are cut into
+// bands of rows for whole blocks (a branch that gathers a crowded core's
+// outskirts can span the frame), counted first, then written.
+constexpr int OL_THREADS = 256;
+constexpr int OL_WARP_MAX = 4096;
+constexpr int OL_CHUNK = 16384;      // box pixels per band (at least one row)
+constexpr int OL_ITEMS = 1 << 17;    // bands per frame; objects beyond are left to their warps
 
-// one warp: the raw object's pixels in order, 32 at a time, each lane's
-// pixel to the next slot of its object (cursors c[0..K), any memory space)
-__device__ __forceinline__ void obj_partition_walk(const unsigned *__restrict__ rpix,
-                                                   const unsigned *__restrict__ objkey, int off, int P, int K, int ob,
-                                                   const int *__restrict__ ooff, unsigned *__restrict__ opix, int *c) {
-    const int lane = threadIdx.x & 31;
-    for (int k = lane; k < K; k += 32) c[k] = ooff[ob + k];
-    __syncwarp();
-    // OP_AHEAD chunks of 32 pixels per step: their loads are issued together,
-    // then the chunks take their slots in order
-    constexpr int OP_AHEAD = 4;
-    for (int i0 = 0; i0 < P; i0 += 32 * OP_AHEAD) {
-        int key[OP_AHEAD];
-        unsigned px[OP_AHEAD];
+struct ListItem {
+    int o, y0, rows, first;  // object, first row, rows, the object's first band
+};
+
+// (row, column) of box pixel `start` and its step of `step` pixels
+struct BoxWalk {
+    int x, y, dx, dy, bw;
+    __device__ __forceinline__ BoxWalk(int bw_, int start, int step) {
+        bw = bw_;
+        y = start / bw;
+        x = start - y * bw;
+        dy = step / bw;
+        dx = step - dy * bw;
+    }
+    __device__ __forceinline__ void next() {
+        x += dx;
+        y += dy;
+        if (x >= bw) {
+            x -= bw;
+            y++;
+        }
+    }
+};
+
+struct ListArgs {
+    const int *alloc;
+    ObjBufs O;
+    int w, nobj;
+    const int *nobj_dev;
+    unsigned *opix;
+    ListItem *items;
+    int *icount;        // pixels of every band
+    int *nitems;        // zero on entry
+};
+
+__global__ void __launch_bounds__(OL_THREADS) k_obj_lists(const ListArgs A) {
+    const int lane = threadIdx.x & 31, o = (blockIdx.x * OL_THREADS + threadIdx.x) >> 5;
+    if (o >= sx_count(A.nobj, A.nobj_dev)) return;
+    const int x0 = A.O.xmin[o], y0 = A.O.ymin[o], bw = A.O.xmax[o] - x0 + 1, bh = A.O.ymax[o] - y0 + 1;
+    if (bw <= 0 || bh <= 0) return;
+    const long long area = (long long)bw * bh;
+    if (area > OL_WARP_MAX) {
+        const int rows = max(1, OL_CHUNK / bw), nit = (bh + rows - 1) / rows;
+        int c0 = 0;
+        if (lane == 0) c0 = atomicAdd(A.nitems, nit);
+        c0 = __shfl_sync(0xffffffffu, c0, 0);
+        const bool fits = c0 >= 0 && c0 <= OL_ITEMS - nit;
+        const int cend = c0 < 0 ? c0 : min(c0 + nit, OL_ITEMS);
+        for (int c = c0 + lane; c < cend; c += 32) {
+            ListItem it;
+            it.o = fits ? o : -1;
+            it.y0 = y0 + (c - c0) * rows;
+            it.rows = min(rows, y0 + bh - it.y0);
+            it.first = c0;
+            A.items[c] = it;
+        }
+        if (fits) return;
+    }
+    unsigned *out = A.opix + A.O.off[o];
+    BoxWalk q(bw, lane, 32);
+    constexpr int AHEAD = 4;  // rows of 32 box pixels whose loads are in flight
+    for (long long i0 = 0; i0 < area; i0 += 32 * AHEAD) {
+        int a[AHEAD], p[AHEAD];
 #pragma unroll
-        for (int a = 0; a < OP_AHEAD; a++) {
-            const int i = i0 + a * 32 + lane;
-            key[a] = i < P ? (int)objkey[off + i] - ob : -1;
-            px[a] = i < P ? rpix[off + i] : 0u;
+        for (int k = 0; k < AHEAD; k++) {
+            p[k] = (y0 + q.y) * A.w + x0 + q.x;
+            a[k] = q.y < bh ? __ldg(A.alloc + p[k]) : -1;
+            q.next();
         }
 #pragma unroll
-        for (int a = 0; a < OP_AHEAD; a++) {
-            const unsigned grp = __match_any_sync(0xffffffffu, key[a]);
-            const int leader = __ffs(grp) - 1;
-            const int rank = __popc(grp & ((1u << lane) - 1u));
-            int base = 0;
-            if (key[a] >= 0 && lane == leader) {
-                base = c[key[a]];
-                c[key[a]] = base + __popc(grp);
-            }
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (key[a] >= 0) opix[base + rank] = px[a];
-            __syncwarp();
+        for (int k = 0; k < AHEAD; k++) {
+            const unsigned m = __ballot_sync(0xffffffffu, a[k] == o);
+            if (a[k] == o) out[__popc(m & ((1u << lane) - 1u))] = (unsigned)p[k];
+            out += __popc(m);
         }
     }
 }
 
-__global__ void __launch_bounds__(OP_WARPS * 32) k_obj_partition(const unsigned *__restrict__ rpix,
-                                                                 const unsigned *__restrict__ objkey,
-                                                                 const int *__restrict__ roff,
-                                                                 const int *__restrict__ rsize,
-                                                                 const int *__restrict__ rnkept,
-                                                                 const int *__restrict__ objbase,
-                                                                 const int *__restrict__ ooff, int nroots,
-                                                                 const int *nroots_dev, unsigned *__restrict__ opix,
-                                                                 int *nbig, int *biglist) {
-    __shared__ int cur[OP_WARPS][OP_KMAX];
+__global__ void __launch_bounds__(OL_THREADS) k_obj_list_count(const ListArgs A) {
+    __shared__ int s_n;
+    const int n = min(*A.nitems, OL_ITEMS);
+    for (int c = blockIdx.x; c < n; c += gridDim.x) {
+        const ListItem it = A.items[c];
+        if (it.o < 0) continue;
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        const int x0 = A.O.xmin[it.o], bw = A.O.xmax[it.o] - x0 + 1;
+        BoxWalk q(bw, threadIdx.x, OL_THREADS);
+        int k = 0;
+        for (; q.y < it.rows; q.next()) k += __ldg(A.alloc + (size_t)(it.y0 + q.y) * A.w + x0 + q.x) == it.o;
+        k = __reduce_add_sync(0xffffffffu, k);
+        if ((threadIdx.x & 31) == 0 && k) atomicAdd(&s_n, k);
+        __syncthreads();
+        if (threadIdx.x == 0) A.icount[c] = s_n;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(OL_THREADS) k_obj_list_write(const ListArgs A) {
+    __shared__ int s_base, s_warp[2][OL_THREADS / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int r = blockIdx.x * OP_WARPS + wid;
-    if (r >= sx_count(nroots, nroots_dev)) return;
-    const int off = roff[r], P = rsize[r], K = rnkept[r], ob = objbase[r];
-    if (K <= 1) {
-#pragma unroll 4
-        for (int i = lane; i < P; i += 32) opix[off + i] = rpix[off + i];
-        return;
-    }
-    if (K > OP_KMAX) {  // left to k_obj_partition_big
-        if (lane == 0) biglist[atomicAdd(nbig, 1)] = r;
-        return;
-    }
-    obj_partition_walk(rpix, objkey, off, P, K, ob, ooff, opix, cur[wid]);
-}
-
-// raw objects of more than OP_KMAX objects (the list k_obj_partition made, in
-// any order: each writes its own range): one warp each, cursors in dynamic
-// shared memory up to OP_BIG_KMAX objects, else in gcur (global)
-__global__ void __launch_bounds__(32) k_obj_partition_big(const unsigned *__restrict__ rpix,
-                                                          const unsigned *__restrict__ objkey,
-                                                          const int *__restrict__ roff, const int *__restrict__ rsize,
-                                                          const int *__restrict__ rnkept,
-                                                          const int *__restrict__ objbase,
-                                                          const int *__restrict__ ooff, const int *nbig,
-                                                          const int *__restrict__ biglist,
-                                                          unsigned *__restrict__ opix, int *gcur) {
-    extern __shared__ int bigcur[];
-    const int nb = *nbig;
-    for (int i = blockIdx.x; i < nb; i += gridDim.x) {
-        const int r = biglist[i], K = rnkept[r];
-        const int ob = objbase[r];
-        obj_partition_walk(rpix, objkey, roff[r], rsize[r], K, ob, ooff, opix,
-                           K <= OP_BIG_KMAX ? bigcur : gcur + ob);
-        __syncwarp();
+    const int n = min(*A.nitems, OL_ITEMS);
+    for (int c = blockIdx.x; c < n; c += gridDim.x) {
+        const ListItem it = A.items[c];
+        if (it.o < 0) continue;
+        if (threadIdx.x == 0) s_base = A.O.off[it.o];
+        __syncthreads();
+        int before = 0;
+        for (int k = it.first + threadIdx.x; k < c; k += OL_THREADS) before += A.icount[k];
+        before = __reduce_add_sync(0xffffffffu, before);
+        if (lane == 0 && before) atomicAdd(&s_base, before);
+        __syncthreads();
+        int base = s_base;
+        const int x0 = A.O.xmin[it.o], bw = A.O.xmax[it.o] - x0 + 1, npix = bw * it.rows;
+        BoxWalk q(bw, threadIdx.x, OL_THREADS);
+        for (int i0 = 0, turn = 0; i0 < npix; i0 += OL_THREADS, turn ^= 1, q.next()) {
+            const int p = (it.y0 + q.y) * A.w + x0 + q.x;
+            const bool in = q.y < it.rows && __ldg(A.alloc + p) == it.o;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (lane == 0) s_warp[turn][wid] = __popc(m);
+            __syncthreads();
+            int pre = 0, tot = 0;
+#pragma unroll
+            for (int k = 0; k < OL_THREADS / 32; k++) {
+                if (k < wid) pre += s_warp[turn][k];
+                tot += s_warp[turn][k];
+            }
+            if (in) A.opix[base + pre + __popc(m & ((1u << lane) - 1u))] = (unsigned)p;
+            base += tot;
+        }
+        __syncthreads();
     }
 }
 
-// gcur: scratch of one int per object; nbig (zero on entry) and biglist
-// (nroots ints): the raw objects k_obj_partition leaves to the big kernel.
-// nroots_dev (device, or null): the number of roots when only the device
-// knows it; nroots is then the capacity.
-void launch_obj_partition(const unsigned *rpix, const unsigned *objkey, const RootBufs &R, const int *ooff,
-                          int nroots, const int *nroots_dev, unsigned *opix, int *gcur, int *nbig, int *biglist,
-                          cudaStream_t st) {
-    if (nroots <= 0) return;
-    k_obj_partition<<<(unsigned)((nroots + OP_WARPS - 1) / OP_WARPS), OP_WARPS * 32, 0, st>>>(
-        rpix, objkey, R.off, R.size, R.nkept, R.objbase, ooff, nroots, nroots_dev, opix, nbig, biglist);
-    k_obj_partition_big<<<(unsigned)std::min(nroots, OP_BIG_GRID), 32, OP_BIG_KMAX * sizeof(int), st>>>(
-        rpix, objkey, R.off, R.size, R.nkept, R.objbase, ooff, nbig, biglist, opix, gcur);
+int launch_obj_lists(const ListArgs &A, cudaStream_t st) {
+    if (A.nobj <= 0) return 0;
+    const unsigned per = OL_THREADS / 32;
+    k_obj_lists<<<(A.nobj + per - 1) / per, OL_THREADS, 0, st>>>(A);
+    k_obj_list_count<<<dt_grid(A.nobj, 4), OL_THREADS, 0, st>>>(A);
+    k_obj_list_write<<<dt_grid(A.nobj, 4), OL_THREADS, 0, st>>>(A);
+    return 3;
 }
 
 void launch_analyse(const AnaArgs &A, cudaStream_t st) {

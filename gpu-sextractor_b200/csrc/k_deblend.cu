@@ -186,8 +186,8 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_up(const __grid_constant__ De
 
 // Thresholds of every raw object (d0, then N-1 above it, src/cuda/
 // cudadeblend.cu:199-217), one thread each; the first of a raw object also
-// reads off its completion keys and puts it on the list of its class:
-// one peak (done here), up to 32 peaks (one warp), more (blocks).
+// puts it on the list of its class: one peak (done here), up to 32 peaks (one
+// warp), more (blocks).
 __global__ void __launch_bounds__(DT_THREADS) k_dt_thresholds(const __grid_constant__ DebArgs A) {
     const long long t = (long long)blockIdx.x * DT_THREADS + threadIdx.x;
     const int r = (int)(t / A.N), i = (int)(t - (long long)r * A.N);
@@ -200,19 +200,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_thresholds(const __grid_const
         return;
     }
     thr[0] = d0;
-    const int off = A.R.off[r], P = A.R.size[r];
-    // completion keys: the last row and the first column of the object on it
-    const int ymax = (int)fdiv(A.rpix[off + P - 1], A.wdiv);
-    int lo = 0, hi = P - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if ((int)A.rpix[off + mid] >= ymax * A.w)
-            hi = mid;
-        else
-            lo = mid + 1;
-    }
-    A.R.ymax[r] = ymax;
-    A.R.lastx[r] = (int)A.rpix[off + lo] - ymax * A.w;
+    const int off = A.R.off[r];
     // a term the fixed-scale sums cannot hold
     if (fexpo(fdpeak) - A.sc->e0cd > 100) atomicOr(&A.sc->status, SX_ST_RANGE);
     const int B = A.R.npk[r];
@@ -346,7 +334,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_fill(const __grid_constant__ 
             const int q = dt_rep(A.D.rec, A.D.up[j], l, dt_cap(A), &A.sc->status);
             A.D.up[j] = q;
             bkt = A.D.boff[q] + __popcll(A.D.evm[q] >> l);
-            e = j - A.R.off[r];
+            e = j;
             // (a term of exponent below e0cd cannot occur: every pixel is at
             // or above the smallest threshold; one more than 100 above it
             // has set SX_ST_RANGE)
@@ -366,7 +354,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_fill(const __grid_constant__ 
     const unsigned grp = __match_any_sync(0xffffffffu, key);
     if (bkt < 0) return;
     const int lane = threadIdx.x & 31, lead = __ffs(grp) - 1;
-    // (list indices rise with the lane: the first lane has the smallest)
+    // (elements rise with the lane: the first lane has the smallest)
     if (lane == lead) {
         atomicAdd(A.D.bsz + bkt, __popc(grp));
         atomicMin(A.D.bmin + bkt, e);
@@ -760,9 +748,9 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_whole(const __grid_constant__
 // 5. ownership of the kept branches, preanalysis, gatherup
 // ---------------------------------------------------------------------------
 // objects of every raw object, one warp each.  O.n counts the pixels (all of
-// them where the raw object is one branch at level 0), O.off the place of
-// the branch's own pixels and O.npix the fill of that list until later
-// stages set them.
+// them where the raw object is one branch at level 0), O.off is the place of
+// the branch's own pixels and O.npix the fill of that list until later stages
+// set them.
 __global__ void __launch_bounds__(DT_THREADS) k_da_objects(const __grid_constant__ DebArgs A) {
     const int lane = threadIdx.x & 31, r = (blockIdx.x * DT_THREADS + threadIdx.x) >> 5;
     if (r >= sx_count(A.nroots, A.nroots_dev)) return;
@@ -838,11 +826,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_scatter(const __grid_constant
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     const int n = sx_count(A.nrootpix, A.nrootpix_dev);
     if (blockIdx.x * DT_THREADS >= n) return;
-    int o = -1;
-    if (j < n) {
-        const int r = (int)A.rid[j];
-        if (!da_whole(A, r, A.R.nkept[r])) o = (int)A.objkey[j];
-    }
+    const int o = j < n ? (int)A.objkey[j] : -1;
     const unsigned grp = __match_any_sync(0xffffffffu, o);
     if (o < 0) return;
     const int lane = threadIdx.x & 31, lead = __ffs(grp) - 1;
@@ -856,11 +840,6 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_scatter(const __grid_constant
 // 1686-1903): one warp per branch, one block for those of more than
 // DA_WARP_MAX pixels; the ellipse is finished by k_da_finish, one thread per
 // object
-__device__ __forceinline__ const unsigned *da_pixels(const DebArgs &A, int o) {
-    const int r = A.O.root[o];
-    return (da_whole(A, r, A.R.nkept[r]) ? A.rpix : A.D.ownpix) + A.O.off[o];
-}
-
 __global__ void __launch_bounds__(DT_THREADS, 3) k_da_moments(const __grid_constant__ DebArgs A) {
     const int o = (blockIdx.x * DT_THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (o >= sx_count(A.nobj, A.nobj_dev)) return;
@@ -869,7 +848,7 @@ __global__ void __launch_bounds__(DT_THREADS, 3) k_da_moments(const __grid_const
         if (lane == 0) A.D.biglist[atomicAdd(A.D.counts + 4, 1)] = o;
         return;
     }
-    const unsigned *pix = da_pixels(A, o);
+    const unsigned *pix = A.D.ownpix + A.O.off[o];
     PixBox b = pix_box(A.cd, A.sub, pix, lane, n, 32, A.wdiv, A.w);
     pixbox_warp(b);
     PixMoments M;
@@ -882,7 +861,7 @@ __global__ void __launch_bounds__(DT_THREADS, 2) k_da_moments_big(const __grid_c
     const int nb = A.D.counts[4];
     for (int i = blockIdx.x; i < nb; i += gridDim.x) {
         const int o = A.D.biglist[i];
-        pix_moments_block(A.cd, A.sub, da_pixels(A, o), A.O.n[o], A.wdiv, A.w, A.O.node_dthresh[o], sh, A.raw + o);
+        pix_moments_block(A.cd, A.sub, A.D.ownpix + A.O.off[o], A.O.n[o], A.wdiv, A.w, A.O.node_dthresh[o], sh, A.raw + o);
     }
 }
 
@@ -959,10 +938,12 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_gather(const __grid_constant_
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     const int n = sx_count(A.nrootpix, A.nrootpix_dev);
     if (blockIdx.x * DT_THREADS >= n) return;
-    int o = -1;
+    int o = -1, x = 0, y = 0;
     if (j < n && (int)A.objkey[j] < 0) {
         const int r = (int)A.rid[j], K = A.R.nkept[r], ob = A.R.objbase[r];
-        const int p = (int)A.rpix[j], y = (int)fdiv((unsigned)p, A.wdiv), x = p - y * A.w;
+        const int p = (int)A.rpix[j];
+        y = (int)fdiv((unsigned)p, A.wdiv);
+        x = p - y * A.w;
         int iclst = 0;
         float distmin = 1e+31f;
         for (int i = 0; i < K; i++) {
@@ -979,10 +960,19 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_gather(const __grid_constant_
         }
         o = ob + iclst;
         A.alloc[p] = o;
-        A.objkey[j] = (unsigned)o;
     }
+    // the objects grow by them: their pixel counts and boxes
     const unsigned grp = __match_any_sync(0xffffffffu, o);
-    if (o >= 0 && (int)(threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(A.O.n + o, __popc(grp));
+    if (o < 0) return;
+    const int x0 = __reduce_min_sync(grp, x), x1 = __reduce_max_sync(grp, x);
+    const int y0 = __reduce_min_sync(grp, y), y1 = __reduce_max_sync(grp, y);
+    if ((int)(threadIdx.x & 31) == __ffs(grp) - 1) {
+        atomicAdd(A.O.n + o, __popc(grp));
+        if (x0 < A.O.xmin[o]) atomicMin(A.O.xmin + o, x0);
+        if (x1 > A.O.xmax[o]) atomicMax(A.O.xmax + o, x1);
+        if (y0 < A.O.ymin[o]) atomicMin(A.O.ymin + o, y0);
+        if (y1 > A.O.ymax[o]) atomicMax(A.O.ymax + o, y1);
+    }
 }
 
 // resident blocks of a grid-stride kernel over a device-side count, at most n

@@ -120,12 +120,11 @@ __global__ void __launch_bounds__(CL_PAIR_WARPS * 32) k_clean_pairs(const CleanO
     }
 }
 
-// end of the master chain; victims with a master get sort keys for merging
-// the chain of masters of a victim ends at a survivor after fewer than n
-// steps (masters have smaller indices); cap: a smaller bound set for a
-// failure test (0: n); running out sets SX_ST_LOOP
-__global__ void k_clean_chain(ObjBufs O, int n, const int *n_dev, unsigned *vkey, unsigned *vval, int *nvict,
-                              int *status, int cap) {
+// end of the master chain.  The chain of masters of a victim ends at a survivor
+// after fewer than n steps (masters have smaller indices); cap: a smaller
+// bound set for a failure test (0: n); running out sets SX_ST_LOOP.  Every
+// survivor counts its victims (vcnt, zeroed before).
+__global__ void k_clean_chain(ObjBufs O, int n, const int *n_dev, int *vcnt, int *status, int cap) {
     n = sx_count(n, n_dev);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -139,58 +138,39 @@ __global__ void k_clean_chain(ObjBufs O, int n, const int *n_dev, unsigned *vkey
     for (; it < lim && O.master[m] != 0x7fffffff; it++) m = O.master[m];
     if (O.master[m] != 0x7fffffff) atomicOr(status, SX_ST_LOOP);
     O.fmaster[i] = m;
-    int k = atomicAdd(nvict, 1);
-    vkey[k] = (unsigned)m;
-    vval[k] = (unsigned)i;
+    atomicAdd(vcnt + m, 1);
 }
 
-// victims in (master, index) order: one block sorts the (master << 32 |
-// index) keys, all distinct, in shared memory (bitonic network); larger
-// victim lists go through two stable radix sorts instead.  With the count on
-// the device (nv_dev), a list too long for the block is left alone and its
-// length written to *big (0 otherwise): the count of the radix sorts.
-constexpr int CL_SORT_MAX = 4096;
-
-__global__ void __launch_bounds__(1024) k_victim_sort(unsigned *vkey, unsigned *vval, int nv, const int *nv_dev,
-                                                      int *big) {
-    __shared__ unsigned long long s[CL_SORT_MAX];
-    nv = sx_count(nv, nv_dev);
-    if (big && threadIdx.x == 0) *big = nv > CL_SORT_MAX ? nv : 0;
-    if (nv > CL_SORT_MAX) return;
-    int n2 = 1;
-    while (n2 < nv) n2 <<= 1;
-    for (int i = threadIdx.x; i < n2; i += blockDim.x)
-        s[i] = i < nv ? ((unsigned long long)vkey[i] << 32) | vval[i] : ~0ull;
-    __syncthreads();
-    for (int k = 2; k <= n2; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const unsigned long long a = s[i], b = s[l];
-                    if ((a > b) == ((i & k) == 0)) {
-                        s[i] = b;
-                        s[l] = a;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-        vkey[i] = (unsigned)(s[i] >> 32);
-        vval[i] = (unsigned)s[i];
-    }
+// The victims of every survivor, in index order: put into its range of vlist
+// in any order (voff: exclusive sums of vcnt; vfill zeroed before), then each
+// to its rank among them in vsort.  A victim compares itself with the others
+// of its survivor only, usually a handful.
+__global__ void k_victim_scatter(ObjBufs O, int n, const int *n_dev, const int *voff, int *vfill, int *vlist) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= sx_count(n, n_dev)) return;
+    const int m = O.fmaster[i];
+    if (m >= 0) vlist[voff[m] + atomicAdd(vfill + m, 1)] = i;
 }
 
-// victims sorted by (master, index): each segment head merges its segment
-__global__ void k_clean_merge(ObjBufs O, const unsigned *vkey, const unsigned *vval, int nv, const int *nv_dev) {
-    nv = sx_count(nv, nv_dev);
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nv) return;
-    if (k > 0 && vkey[k - 1] == vkey[k]) return;
-    int m = (int)vkey[k];
-    for (int j = k; j < nv && (int)vkey[j] == m; j++) {
-        int s = (int)vval[j];
+__global__ void k_victim_rank(ObjBufs O, int n, const int *n_dev, const int *voff, const int *vcnt, const int *vlist,
+                              int *vsort) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= sx_count(n, n_dev)) return;
+    const int m = O.fmaster[i];
+    if (m < 0) return;
+    const int v0 = voff[m], v1 = v0 + vcnt[m];
+    int rank = 0;
+    for (int k = v0; k < v1; k++) rank += vlist[k] < i;
+    vsort[v0 + rank] = i;
+}
+
+// each survivor merges its victims in index order (src/clean.c:234-287)
+__global__ void k_clean_merge(ObjBufs O, int n, const int *n_dev, const int *voff, const int *vcnt, const int *vsort) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= sx_count(n, n_dev)) return;
+    const int v0 = voff[m], v1 = v0 + vcnt[m];
+    for (int j = v0; j < v1; j++) {
+        const int s = vsort[j];
         O.fdnpix[m] += O.fdnpix[s];
         O.dnpix[m] += O.dnpix[s];
         O.fdflux[m] += O.fdflux[s];
@@ -212,14 +192,15 @@ __global__ void k_clean_merge(ObjBufs O, const unsigned *vkey, const unsigned *v
     }
 }
 
-// pixels of cleaned objects belong to their master in the allocation map
+// pixels of cleaned objects belong to their master in the allocation map (one
+// warp per object)
 __global__ void k_alloc_victims(ObjBufs O, const unsigned *opix, int *alloc, int n, const int *n_dev) {
-    int o = blockIdx.x;
+    const int o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (o >= sx_count(n, n_dev)) return;
-    int m = O.fmaster[o];
+    const int m = O.fmaster[o];
     if (m < 0) return;
-    int off = O.off[o], cnt = O.n[o];
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x) alloc[opix[off + i]] = m;
+    const int off = O.off[o], cnt = O.n[o];
+    for (int i = threadIdx.x & 31; i < cnt; i += 32) alloc[opix[off + i]] = m;
 }
 
 // ---------------------------------------------------------------------------
@@ -836,24 +817,60 @@ void launch_endobject(const EndArgs &E, int nobj, cudaStream_t st, int &launches
 // ---------------------------------------------------------------------------
 // catalogue order and output
 // ---------------------------------------------------------------------------
-// survivors compacted in index order (scan of the survivor flags)
+// Completion order: raw objects by the position of the first pixel on their
+// last row, the survivors of one raw object in index order.  Raw objects have
+// distinct such pixels, and their elements (raster order) come in the same
+// order, so the place of a raw object's survivors is a count: those of the
+// element tiles before its own, and those of the raw objects of its tile whose
+// element is smaller (a linked list of a few).
+constexpr int NO_TILE = 1024;  // elements; 3 to 20 raw objects of a crowded frame
+
 __global__ void k_surv_flags(ObjBufs O, int n, const int *n_dev, int *flag) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < sx_count(n, n_dev)) flag[i] = O.fmaster[i] < 0 ? 1 : 0;
 }
 
-__global__ void k_surv_compact(ObjBufs O, const int *rymax, const int *rlastx, const int *pos, int n,
-                               const int *n_dev, int w, int numbering, unsigned *keys, unsigned *vals) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= sx_count(n, n_dev) || O.fmaster[i] >= 0) return;
-    int r = O.root[i], j = pos[i];
-    keys[j] = numbering == 0 ? (unsigned)rymax[r] * (unsigned)w + (unsigned)rlastx[r] : 0u;
-    vals[j] = (unsigned)i;
+struct OrderBufs {
+    const int *pos;         // exclusive sums of the survivor flags
+    int *tcnt, *thead;      // per tile: survivors (then their exclusive sums), list head + 1 (zeroed before)
+    int *next, *elem, *ns;  // per raw object: list, its element, survivors
+};
+
+__global__ void k_order_roots(ObjBufs O, RootBufs R, const int *pos2idx, int w, int nroots, const int *nroots_dev,
+                              OrderBufs Q) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= sx_count(nroots, nroots_dev)) return;
+    const int K = R.nkept[r], ob = R.objbase[r];
+    if (K <= 0) return;
+    const int last = ob + K - 1, ns = Q.pos[last] + (O.fmaster[last] < 0) - Q.pos[ob];
+    if (ns == 0) return;
+    const unsigned long long key = R.last[r];
+    const int e = pos2idx[(size_t)(key >> 32) * w + (0xffffffffu - (unsigned)key)], t = e / NO_TILE;
+    Q.elem[r] = e;
+    Q.ns[r] = ns;
+    atomicAdd(Q.tcnt + t, ns);
+    Q.next[r] = atomicExch(Q.thead + t, r + 1);
 }
 
-__global__ void k_number(ObjBufs O, const unsigned *vals, int ns, const int *ns_dev) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < sx_count(ns, ns_dev)) O.number[vals[k]] = k + 1;
+// NUMBER of every survivor and the objects in catalogue order (numbering 1:
+// index order)
+__global__ void k_order_objs(ObjBufs O, RootBufs R, int n, const int *n_dev, int numbering, OrderBufs Q,
+                             unsigned *order) {
+    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= sx_count(n, n_dev)) return;
+    if (O.fmaster[o] >= 0) {
+        O.number[o] = 0;
+        return;
+    }
+    int k = Q.pos[o];
+    if (numbering == 0) {
+        const int r = O.root[o], e = Q.elem[r], t = e / NO_TILE;
+        k += Q.tcnt[t] - Q.pos[R.objbase[r]];
+        for (int q = Q.thead[t]; q; q = Q.next[q - 1])
+            if (Q.elem[q - 1] < e) k += Q.ns[q - 1];
+    }
+    O.number[o] = k + 1;
+    order[k] = (unsigned)o;
 }
 
 __global__ void k_write_rows(ObjBufs O, const unsigned *vals, int ns, const int *ns_dev, sexgpu_object *rows) {

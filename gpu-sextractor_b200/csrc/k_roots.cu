@@ -1,6 +1,8 @@
 // k_roots.cu -- raw objects ("roots"): connected components of at least
-// DETECT_MINAREA pixels, numbered in order of their first pixel, with their
-// pixel lists contiguous and in raster order.
+// DETECT_MINAREA pixels, numbered in order of their first pixel, and their
+// pixels compacted in raster order of the frame.  (The pixels are not grouped
+// by raw object: the deblending works on all of them at once, and only the
+// objects it ends with get pixel lists, k_analyse.cu.)
 //
 // Reference: src/cuda/cudadetection.cu:677-897 (compact_and_sort: sort by
 // label, segment counts, minarea prune, consecutive relabel) and :899-1105
@@ -109,11 +111,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_tile_counts(const int *__
     if (threadIdx.x == 0) tkept[blockIdx.x] = tot;
 }
 
-// roots numbered in raster order: rid at the root pixel, size and first pixel
+// roots numbered in raster order: rid at the root pixel, and size
 __global__ void __launch_bounds__(SCAN_THREADS) k_root_number(const int *__restrict__ lab, const int *__restrict__ cnt,
                                                              long long n, int minarea, const int *__restrict__ toff,
-                                                             int *__restrict__ rid, int *__restrict__ rsize,
-                                                             int *__restrict__ rfirst) {
+                                                             int *__restrict__ rid, int *__restrict__ rsize) {
     __shared__ int sh[32];
     const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
     int fr[SCAN_ITEMS], kp[SCAN_ITEMS], l[SCAN_ITEMS], c = 0;
@@ -128,18 +129,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_number(const int *__restr
             const long long p = base + k;
             rid[p] = id;
             rsize[id] = cnt[p];
-            rfirst[id] = (int)p;
             id++;
         }
 }
 
-// kept pixels compacted in raster order with their root id as sort key; the
-// allocation map starts as "unassigned object pixel" / background and the
-// pixel -> list index map as -1
+// kept pixels compacted in raster order: their positions, raw objects and the
+// pixel -> element map (-1 elsewhere); the allocation map starts as "unassigned
+// object pixel" / background
 __global__ void __launch_bounds__(SCAN_THREADS) k_root_compact(const int *__restrict__ lab, const int *__restrict__ cnt,
                                                               long long n, int minarea, const int *__restrict__ toff,
-                                                              const int *__restrict__ rid, unsigned *__restrict__ keys,
-                                                              unsigned *__restrict__ vals, int *__restrict__ alloc,
+                                                              const int *__restrict__ rid, unsigned *__restrict__ erid,
+                                                              unsigned *__restrict__ epix, int *__restrict__ alloc,
                                                               int *__restrict__ pos2idx) {
     __shared__ int sh[32];
     const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
@@ -154,7 +154,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_compact(const int *__rest
         *reinterpret_cast<int4 *>(alloc + base) =
             make_int4(lb[0] >= 0 ? SX_ALLOC_OTHER : -1, lb[1] >= 0 ? SX_ALLOC_OTHER : -1,
                       lb[2] >= 0 ? SX_ALLOC_OTHER : -1, lb[3] >= 0 ? SX_ALLOC_OTHER : -1);
-        *reinterpret_cast<int4 *>(pos2idx + base) = make_int4(-1, -1, -1, -1);
+        int e[4], i = j;
+#pragma unroll
+        for (int k = 0; k < 4; k++) e[k] = fk[k] ? i++ : -1;
+        *reinterpret_cast<int4 *>(pos2idx + base) = make_int4(e[0], e[1], e[2], e[3]);
     }
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; k++) {
@@ -162,20 +165,14 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_compact(const int *__rest
         if (p >= n) break;
         if (!vec) {
             alloc[p] = lb[k] >= 0 ? SX_ALLOC_OTHER : -1;
-            pos2idx[p] = -1;
+            pos2idx[p] = fk[k] ? j : -1;
         }
         if (fk[k]) {
-            keys[j] = (unsigned)rid[lb[k]];
-            vals[j] = (unsigned)p;
+            erid[j] = (unsigned)rid[lb[k]];
+            epix[j] = (unsigned)p;
             j++;
         }
     }
-}
-
-int bits_for(long long v) {
-    int b = 1;
-    while ((1ll << b) <= v) b++;
-    return b;
 }
 
 }  // namespace sx

@@ -20,17 +20,18 @@ struct BackBufs {
 
 // per-root data (index = root id, first-pixel order)
 struct RootBufs {
-    int *size, *off, *first;            // pixels, offset in the root pixel list, first pixel
-    int *ymax, *lastx;                  // completion-order keys
+    int *size, *off;                    // pixels, their exclusive sums
+    unsigned long long *last;           // completion order: last row << 32 | ~(first column on it), over its objects
     int *nkept, *objbase;
     float *dthresh, *thresh;            // smallest detection / analysis threshold of its pixels
     unsigned *peak;                     // f2ord of its largest filtered value
     int *npk, *nbkt, *nown;             // peaks, buckets, pixels of kept branches (deblending)
 };
 
-// deblending scratch (k_deblend.cu).  "Element" is a position in the root
-// pixel list; the arrays "per raw object, from its offset" hold one entry per
-// peak, bucket or kept branch, of which a raw object has no more than pixels.
+// deblending scratch (k_deblend.cu).  "Element" is a position in the list of
+// all raw objects' pixels (raster order); the arrays "per raw object, from its
+// offset" hold one entry per peak, bucket, kept branch or branch pixel, of
+// which a raw object has no more than pixels.
 struct DebBufs {
     // per element
     int *up;                            // towards its peak, then its peak, then its first representative
@@ -165,7 +166,7 @@ struct MomentRaw;
 struct DebArgs {
     const float *cd, *sub;
     const int *pos2idx;
-    const unsigned *rpix;       // root pixel lists (raster order per root)
+    const unsigned *rpix;       // pixel of every element
     const unsigned *rid;        // raw object of every element
     RootBufs R;
     DebBufs D;
@@ -173,7 +174,7 @@ struct DebArgs {
     MomentRaw *raw;             // per-object scratch of the preanalysis
     FrameScalars *sc;
     int *alloc;                 // W*H object id map (-1 elsewhere)
-    unsigned *objkey;           // object id per root-list element
+    unsigned *objkey;           // object of every element (~0: not a branch's own pixel)
     int nroots, nrootpix, nobj; // counts, or the capacities of the launches when the device counts are given
     const int *nroots_dev, *nrootpix_dev, *nobj_dev;
     int w, h, N, debminarea;

@@ -146,19 +146,19 @@ struct sexgpu_ctx {
     cudaStream_t qstream = nullptr;
     cudaEvent_t qev[2] = {nullptr, nullptr};
     // scan / sort scratch
-    DevBuf scan_tmp, keys, vals, kalt, valt;
+    DevBuf scan_tmp, keys, vals;  // scan scratch; raw object of every element; object pixel lists
     // background
     DevBuf ms, back, sigma, back2, back3, sigma3, dback, bu, rownode, rowdnode, rowu, colk, coldx;
     // roots
-    DevBuf rsize, roff, rfirst, rymax, rlastx, rnkept, robjbase, rdthr, rathr, rzero, rlists, rthr;
+    DevBuf rsize, roff, rnkept, robjbase, rdthr, rathr, rzero, rlists, rthr;
     // deblend scratch
     DevBuf objkey, rpix;
     enum { D_UP, D_LEV, D_REC, D_EVM, D_BOFF, D_PIDX, D_KOWN, D_PEAKS, D_PLIST, D_BSZ, D_BMIN, D_ACC, D_OLEV, D_OWNPIX,
            D_KEPT, D_GEVM, D_KREP, D_GB0, D_GPAR, D_GNSON, D_GLABEL, D_GFLAGS, D_GDLIST, D_GELIST, D_GM, D_COUNT };
     DevBuf deb;  // all of them
     // objects
-    DevBuf o_i[20], o_f[32], o_d[10], o_iso, o_sortkey, amp, alpha, cellhead, cellnext, vkey, vval, vkalt, vvalt,
-        skeys, svals, skalt, svalt, rows;
+    DevBuf o_i[20], o_f[32], o_d[10], o_iso, o_sortkey, amp, alpha, cellhead, vict, svals, order, rows;
+    DevBuf oitems;                         // bands of large objects' boxes (pixel lists)
     DevBuf kitem[2], kchunk[2], kpart[2];  // queued Kron boxes
     DevBuf o_sprob;                        // CLASS_STAR per object
     DevBuf o_big;                          // objects summed by whole blocks
@@ -587,11 +587,9 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
     EN(pos2idx, N * 4);
     EN(keys, N * 4);
     EN(vals, N * 4);
-    EN(kalt, N * 4);
-    EN(valt, N * 4);
     EN(rpix, N * 4);
     EN(objkey, N * 4);
-    EN(scan_tmp, (std::max(scan_temp_ints(N), radix_temp_ints(N)) + 64) * 4);
+    EN(scan_tmp, (scan_temp_ints(N) + 64) * 4);
     EN(ms, nb * sizeof(MeshStat));
     EN(back, nb * 4);
     EN(sigma, nb * 4);
@@ -702,14 +700,14 @@ int pipe_detect(sexgpu_ctx *ctx) {
     const int ntile = (int)((N + SCAN_TILE - 1) / SCAN_TILE);
     int *troots = pos, *tkept = pos + ntile, *troff = pos + 2 * ntile, *tkoff = pos + 3 * ntile;
     k_root_tile_counts<<<ntile, SCAN_THREADS, 0, st>>>(lab, cnt, N, Pm.minarea, troots, tkept);
-    exclusive_scan(troots, troff, ntile, &d_sc->nroots, tmp, st);
-    exclusive_scan(tkept, tkoff, ntile, nullptr, tmp, st);
+    nl = 1 + exclusive_scan2(troots, troff, &d_sc->nroots, tkept, tkoff, &d_sc->nrootpix, ntile, tmp, st);
     // roots (the capacity in the capacity form) and the length of the root
     // arrays: in the capacity form, the most roots the frame can hold (each
-    // has minarea pixels), since they are numbered before the gate checks
-    int nroots, rlen;
+    // has minarea pixels), since they are numbered whatever the gate says
+    int nroots, rlen, nrootpix;
     if (ps.capf) {
         nroots = ps.cap_roots;
+        nrootpix = ps.cap_rootpix;
         rlen = (int)(N / std::max(Pm.minarea, 1));
         k_gate<<<1, 1, 0, st>>>(d_sc, 1, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
     } else {
@@ -720,14 +718,13 @@ int pipe_detect(sexgpu_ctx *ctx) {
             return SEXGPU_ERR_THRESH;
         }
         nroots = rlen = ctx->hsc.nroots;
+        nrootpix = ctx->hsc.nrootpix;
     }
     ps.nroots = nroots;
+    ps.nrootpix = nrootpix;
     const int *nroots_dev = ps.capf ? &d_sc->nroots : nullptr;
     EN(rsize, ((size_t)rlen + 1) * 4);
     EN(roff, ((size_t)rlen + 1) * 4);
-    EN(rfirst, ((size_t)rlen + 1) * 4);
-    EN(rymax, ((size_t)rlen + 1) * 4);
-    EN(rlastx, ((size_t)rlen + 1) * 4);
     EN(rnkept, ((size_t)rlen + 1) * 4);
     EN(robjbase, ((size_t)rlen + 1) * 4);
     EN(rdthr, ((size_t)rlen + 1) * 4);
@@ -735,19 +732,14 @@ int pipe_detect(sexgpu_ctx *ctx) {
     RootBufs &R = ps.R;
     R.size = P<int>(ctx->rsize);
     R.off = P<int>(ctx->roff);
-    R.first = P<int>(ctx->rfirst);
-    R.ymax = P<int>(ctx->rymax);
-    R.lastx = P<int>(ctx->rlastx);
     R.nkept = P<int>(ctx->rnkept);
     R.objbase = P<int>(ctx->robjbase);
     R.dthresh = P<float>(ctx->rdthr);
     R.thresh = P<float>(ctx->rathr);
-    k_root_number<<<ntile, SCAN_THREADS, 0, st>>>(lab, cnt, N, Pm.minarea, troff, flag, R.size, R.first);
-    exclusive_scan(R.size, R.off, nroots, &d_sc->nrootpix, tmp, st, nroots_dev);
-    unsigned *keys = P<unsigned>(ctx->keys), *vals = P<unsigned>(ctx->vals);
-    int *pos2idx = P<int>(ctx->pos2idx);
-    k_root_compact<<<ntile, SCAN_THREADS, 0, st>>>(lab, cnt, N, Pm.minarea, tkoff, flag, keys, vals,
-                                                   P<int>(ctx->alloc), pos2idx);
+    k_root_number<<<ntile, SCAN_THREADS, 0, st>>>(lab, cnt, N, Pm.minarea, troff, flag, R.size);
+    nl += 3 + exclusive_scan(R.size, R.off, nroots, nullptr, tmp, st, nroots_dev);
+    k_root_compact<<<ntile, SCAN_THREADS, 0, st>>>(lab, cnt, N, Pm.minarea, tkoff, flag, P<unsigned>(ctx->keys),
+                                                   P<unsigned>(ctx->rpix), P<int>(ctx->alloc), P<int>(ctx->pos2idx));
     if (ps.wvar) {
         CK(cudaMemsetAsync(R.dthresh, 0x7f, (size_t)(nroots + 1) * 4, st));
         CK(cudaMemsetAsync(R.thresh, 0x7f, (size_t)(nroots + 1) * 4, st));
@@ -758,24 +750,7 @@ int pipe_detect(sexgpu_ctx *ctx) {
         k_root_thresholds_global<<<grid1(nroots, 256), 256, 0, st>>>(nroots, nroots_dev, d_sc, R.dthresh,
                                                                        R.thresh);
     }
-    int nrootpix;
-    if (ps.capf) {
-        nrootpix = ps.cap_rootpix;
-        k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
-    } else {
-        rc = read_scalars(ctx);
-        if (rc) return rc;
-        nrootpix = ctx->hsc.nrootpix;
-    }
-    ps.nrootpix = nrootpix;
-    const int *nrootpix_dev = ps.capf ? &d_sc->nrootpix : nullptr;
-    // the sort's last pass writes the pixel lists (rpix) and each root
-    // pixel's list index (pos2idx) directly
-    unsigned *rpix = P<unsigned>(ctx->rpix);
-    radix_sort_pairs(keys, vals, P<unsigned>(ctx->kalt), P<unsigned>(ctx->valt), nrootpix, bits_for(nroots), tmp, st,
-                     nrootpix_dev, rpix, pos2idx);
-    stage_mark(ctx, "roots", 4 + 2 * scan_launches(ntile) + scan_launches(nroots) +
-                                 radix_launches(bits_for(nroots), nrootpix) + (nrootpix == 1 ? 1 : 0));
+    stage_mark(ctx, "roots", nl);
     ps.stage = 2;
     return SEXGPU_OK;
 }
@@ -802,14 +777,15 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     }
     EN(deb, bytes);
     unsigned char *const deb = P<unsigned char>(ctx->deb);
-    // per raw object, zeroed: peak, counts of peaks, buckets and own pixels;
-    // then the list lengths
-    EN(rzero, (4 * NR + DT_NCOUNTS) * 4);
+    // per raw object, zeroed: completion key, peak, counts of peaks, buckets
+    // and own pixels; then the list lengths
+    EN(rzero, (6 * NR + DT_NCOUNTS) * 4);
     EN(rlists, 4 * NR * 4);
     EN(rthr, NR * Pm.nthresh * 4);
-    CK(cudaMemsetAsync(ctx->rzero.p, 0, (4 * NR + DT_NCOUNTS) * 4, st));
-    R.peak = P<unsigned>(ctx->rzero);
-    R.npk = P<int>(ctx->rzero) + NR;
+    CK(cudaMemsetAsync(ctx->rzero.p, 0, (6 * NR + DT_NCOUNTS) * 4, st));
+    R.last = P<unsigned long long>(ctx->rzero);
+    R.peak = P<unsigned>(ctx->rzero) + 2 * NR;
+    R.npk = P<int>(ctx->rzero) + 3 * NR;
     R.nbkt = R.npk + NR;
     R.nown = R.nbkt + NR;
     DebArgs &A = ps.A;
@@ -864,7 +840,7 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     A.loop_cap = Pm.loop_cap;
     A.wdiv = make_fastdiv((unsigned)w);
     int nl = launch_deblend_tree(A, st);
-    exclusive_scan(R.nkept, R.objbase, nroots, &d_sc->nobj, tmp, st, nroots_dev);
+    nl += exclusive_scan(R.nkept, R.objbase, nroots, &d_sc->nobj, tmp, st, nroots_dev);
     int nobj;
     if (ps.capf) {
         nobj = ps.cap_obj;
@@ -886,7 +862,7 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     A.nobj_dev = ps.capf ? &d_sc->nobj : nullptr;
     D.biglist = P<int>(ctx->o_big);
     nl += launch_deblend_assign(A, st);
-    stage_mark(ctx, "deblend", nl + scan_launches(nroots));
+    stage_mark(ctx, "deblend", nl);
     ps.stage = 3;
     return SEXGPU_OK;
 }
@@ -902,15 +878,22 @@ int pipe_analyse(sexgpu_ctx *ctx) {
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int *tmp = P<int>(ctx->scan_tmp);
     unsigned *vals = P<unsigned>(ctx->vals);
-    unsigned *rpix = P<unsigned>(ctx->rpix);
-    // ---- object pixel lists (stable by object id: raster order inside)
+    // ---- object pixel lists (raster order inside each object)
     ObjBufs &O = ctx->O;
     const int *nobj_dev = ps.capf ? &d_sc->nobj : nullptr;
-    exclusive_scan(O.n, O.off, nobj, nullptr, tmp, st, nobj_dev);
-    // the deblending's size-class lists are free now: the list of the raw
-    // objects too large for the one-warp partition goes there
-    launch_obj_partition(rpix, A.objkey, ps.R, O.off, ps.nroots, ps.capf ? &d_sc->nroots : nullptr, vals,
-                         P<int>(ctx->kalt), &d_sc->nbig, P<int>(ctx->rlists), st);
+    int nl = exclusive_scan(O.n, O.off, nobj, nullptr, tmp, st, nobj_dev);
+    EN(oitems, (size_t)OL_ITEMS * (sizeof(ListItem) + 4));
+    ListArgs LA;
+    LA.alloc = A.alloc;
+    LA.O = O;
+    LA.w = w;
+    LA.nobj = nobj;
+    LA.nobj_dev = nobj_dev;
+    LA.opix = vals;
+    LA.items = P<ListItem>(ctx->oitems);
+    LA.icount = reinterpret_cast<int *>(LA.items + OL_ITEMS);
+    LA.nitems = A.D.counts + 6;
+    nl += launch_obj_lists(LA, st);
     AnaArgs AA;
     AA.raw = A.raw;
     AA.biglist = A.D.biglist;
@@ -921,6 +904,7 @@ int pipe_analyse(sexgpu_ctx *ctx) {
     AA.sub = A.sub;
     AA.back = B.back3;
     AA.opix = vals;
+    AA.last = ps.R.last;
     AA.O = O;
     AA.sc = d_sc;
     AA.w = w;
@@ -941,7 +925,7 @@ int pipe_analyse(sexgpu_ctx *ctx) {
     AA.afac = Pm.analysis_thresh;
     AA.bp_thick = Pm.bp_thick;
     launch_analyse(AA, st);
-    stage_mark(ctx, "analyse", 7 + (Pm.bp_local ? 2 : 0) + scan_launches(nobj));
+    stage_mark(ctx, "analyse", nl + 5 + (Pm.bp_local ? 2 : 0));
     ps.stage = 4;
     return SEXGPU_OK;
 }
@@ -957,73 +941,38 @@ int pipe_clean(sexgpu_ctx *ctx) {
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int *tmp = P<int>(ctx->scan_tmp);
     unsigned *vals = P<unsigned>(ctx->vals);
-    int rc = SEXGPU_OK;
     // ---- CLEAN
-    int nv = 0;
-    int cl_launch = 0;
+    int nl = 0;
     if (Pm.clean_flag && nobj > 0) {
-        int gx = (int)(w / CL_CELL) + 2, gy = (int)(h / CL_CELL) + 2, ncell = gx * gy;
-        EN(cellhead, (size_t)(ncell + 1) * 4);   // cell counts, then starts
-        EN(cellnext, (size_t)(ncell + 1) * 4);   // fill cursors
-        EN(amp, (size_t)(nobj + 1) * sizeof(CleanObj));
-        EN(vkey, (size_t)(nobj + 1) * 4);
-        EN(vval, (size_t)(nobj + 1) * 4);
-        EN(vkalt, (size_t)(nobj + 1) * 4);
-        EN(vvalt, (size_t)(nobj + 1) * 4);
-        int *cellcnt = P<int>(ctx->cellhead), *cellcur = P<int>(ctx->cellnext);
-        CK(cudaMemsetAsync(cellcnt, 0, (size_t)(ncell + 1) * 4, st));
-        CK(cudaMemsetAsync(cellcur, 0, (size_t)(ncell + 1) * 4, st));
+        const int gx = (int)(w / CL_CELL) + 2, gy = (int)(h / CL_CELL) + 2, ncell = gx * gy;
+        const size_t n1 = (size_t)nobj + 1;
+        // zeroed: cell counts (then starts) and fills, victim counts and fills
+        EN(cellhead, (2 * (size_t)(ncell + 1) + 2 * n1) * 4);
+        EN(vict, 3 * n1 * 4);
+        EN(amp, n1 * sizeof(CleanObj));
+        int *cellcnt = P<int>(ctx->cellhead), *cellcur = cellcnt + ncell + 1, *vcnt = cellcur + ncell + 1,
+            *vfill = vcnt + n1;
+        int *voff = P<int>(ctx->vict), *vlist = voff + n1, *vsort = vlist + n1;
+        CK(cudaMemsetAsync(cellcnt, 0, (2 * (size_t)(ncell + 1) + 2 * n1) * 4, st));
         const int *nobj_dev = ps.capf ? &d_sc->nobj : nullptr;
-        k_clean_count<<<grid1(nobj, 128), 128, 0, st>>>(O, nobj, nobj_dev, cellcnt, gx, gy);
-        exclusive_scan(cellcnt, cellcnt, ncell + 1, nullptr, tmp, st);
-        k_clean_pack<<<grid1(nobj, 128), 128, 0, st>>>(O, nobj, nobj_dev, Pm.clean_param, cellcnt, cellcur,
-                                                       P<CleanObj>(ctx->amp), gx, gy);
+        const unsigned g = grid1(nobj, 128);
+        k_clean_count<<<g, 128, 0, st>>>(O, nobj, nobj_dev, cellcnt, gx, gy);
+        nl += exclusive_scan(cellcnt, cellcnt, ncell + 1, nullptr, tmp, st);
+        k_clean_pack<<<g, 128, 0, st>>>(O, nobj, nobj_dev, Pm.clean_param, cellcnt, cellcur, P<CleanObj>(ctx->amp), gx,
+                                        gy);
         k_clean_pairs<<<(unsigned)nobj, CL_PAIR_WARPS * 32, 0, st>>>(P<CleanObj>(ctx->amp), nobj, nobj_dev,
                                                                       Pm.clean_param, cellcnt, O.master, gx, gy);
-        CK(cudaMemsetAsync(&d_sc->nsurv, 0, 4, st));
-        k_clean_chain<<<grid1(nobj, 256), 256, 0, st>>>(O, nobj, nobj_dev, P<unsigned>(ctx->vkey),
-                                                        P<unsigned>(ctx->vval), &d_sc->nsurv, &d_sc->status,
-                                                        Pm.loop_cap);
-        if (ps.capf) {
-            // the victim count stays on the device: the one-block sort takes
-            // short lists, the radix sorts (counted by nvbig) long ones
-            unsigned *vkey = P<unsigned>(ctx->vkey), *vval = P<unsigned>(ctx->vval);
-            k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
-            k_victim_sort<<<1, 1024, 0, st>>>(vkey, vval, nobj, &d_sc->nsurv, &d_sc->nvbig);
-            radix_sort_pairs(vval, vkey, P<unsigned>(ctx->vkalt), P<unsigned>(ctx->vvalt), nobj, bits_for(nobj), tmp,
-                             st, &d_sc->nvbig);
-            radix_sort_pairs(vkey, vval, P<unsigned>(ctx->vkalt), P<unsigned>(ctx->vvalt), nobj, bits_for(nobj), tmp,
-                             st, &d_sc->nvbig);
-            k_clean_merge<<<grid1(nobj, 128), 128, 0, st>>>(O, vkey, vval, nobj, &d_sc->nsurv);
-            k_alloc_victims<<<nobj, 128, 0, st>>>(O, vals, A.alloc, nobj, nobj_dev);
-            stage_mark(ctx, "clean", 0);
-            ps.stage = 5;
-            return SEXGPU_OK;
-        }
-        rc = read_scalars(ctx);
-        if (rc) return rc;
-        nv = ctx->hsc.nsurv;
-        int sort_launches = 0;
-        if (nv > 0 && nv <= CL_SORT_MAX) {
-            k_victim_sort<<<1, 1024, 0, st>>>(P<unsigned>(ctx->vkey), P<unsigned>(ctx->vval), nv, nullptr, nullptr);
-            sort_launches = 1;
-        } else if (nv > 0) {
-            radix_sort_pairs(P<unsigned>(ctx->vval), P<unsigned>(ctx->vkey), P<unsigned>(ctx->vkalt),
-                             P<unsigned>(ctx->vvalt), nv, bits_for(nobj), tmp, st);  // victims by index
-            radix_sort_pairs(P<unsigned>(ctx->vkey), P<unsigned>(ctx->vval), P<unsigned>(ctx->vkalt),
-                             P<unsigned>(ctx->vvalt), nv, bits_for(nobj), tmp, st);  // then by master
-            sort_launches = 2 * radix_launches(bits_for(nobj), nv);
-        }
-        if (nv > 0) {
-            k_clean_merge<<<grid1(nv, 128), 128, 0, st>>>(O, P<unsigned>(ctx->vkey), P<unsigned>(ctx->vval), nv,
-                                                          nullptr);
-            k_alloc_victims<<<nobj, 128, 0, st>>>(O, vals, A.alloc, nobj, nullptr);
-        }
-        cl_launch = 6 + scan_launches(ncell + 1) + sort_launches;
+        k_clean_chain<<<g, 128, 0, st>>>(O, nobj, nobj_dev, vcnt, &d_sc->status, Pm.loop_cap);
+        nl += exclusive_scan(vcnt, voff, nobj, nullptr, tmp, st, nobj_dev);
+        k_victim_scatter<<<g, 128, 0, st>>>(O, nobj, nobj_dev, voff, vfill, vlist);
+        k_victim_rank<<<g, 128, 0, st>>>(O, nobj, nobj_dev, voff, vcnt, vlist, vsort);
+        k_clean_merge<<<g, 128, 0, st>>>(O, nobj, nobj_dev, voff, vcnt, vsort);
+        k_alloc_victims<<<grid1((long long)nobj * 32, 256), 256, 0, st>>>(O, vals, A.alloc, nobj, nobj_dev);
+        nl += 8;
     } else if (nobj > 0) {
         CK(cudaMemsetAsync(O.fmaster, 0xff, (size_t)nobj * 4, st));
     }
-    stage_mark(ctx, "clean", cl_launch);
+    stage_mark(ctx, "clean", nl);
     ps.stage = 5;
     return SEXGPU_OK;
 }
@@ -1039,7 +988,10 @@ int pipe_end(sexgpu_ctx *ctx) {
     ObjBufs &O = ctx->O;
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int *tmp = P<int>(ctx->scan_tmp);
-    int rc = SEXGPU_OK;
+    // an error so far empties the frame (the host reads the status at its end)
+    constexpr int NOCAP = 0x7fffffff;
+    k_gate<<<1, 1, 0, st>>>(d_sc, 0, NOCAP, NOCAP, NOCAP);
+    const int *nobj_dev = &d_sc->nobj;
     // ---- photometry / FLAGS
     EndArgs E;
     EN(o_eraw, (size_t)(nobj + 1) * sizeof(EndRaw));
@@ -1051,7 +1003,6 @@ int pipe_end(sexgpu_ctx *ctx) {
     E.w = w;
     E.h = h;
     E.n = nobj;
-    const int *nobj_dev = ps.capf ? &d_sc->nobj : nullptr;
     E.n_dev = nobj_dev;
     E.mask_type = Pm.mask_type;
     E.aperture = Pm.aperture;
@@ -1077,41 +1028,40 @@ int pipe_end(sexgpu_ctx *ctx) {
     E.nnw = ctx->nnw_dev;
     E.seeing = Pm.seeing;
     E.pixscale = Pm.pixscale;
-    int nl = 0;
+    int nl = 1;
     launch_endobject(E, nobj, st, nl);
     stage_mark(ctx, "endobject", nl);
 
     // ---- catalogue order
-    EN(skeys, (size_t)(nobj + 1) * 4);
-    EN(svals, (size_t)(nobj + 1) * 4);
-    EN(skalt, (size_t)(nobj + 1) * 4);
-    EN(svalt, (size_t)(nobj + 1) * 4);
-    int *sflag = P<int>(ctx->cnt);  // free now
-    CK(cudaMemsetAsync(O.number, 0, (size_t)(nobj + 1) * 4, st));
-    k_surv_flags<<<grid1(nobj + 1, 256), 256, 0, st>>>(O, nobj, nobj_dev, sflag);
-    exclusive_scan(sflag, sflag, nobj, &d_sc->nsurv, tmp, st, nobj_dev);
-    int ns;
-    if (ps.capf) {
-        ns = nobj;
-        k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
-    } else {
-        rc = read_scalars(ctx);
-        if (rc) return rc;
-        ns = ctx->hsc.nsurv;
+    const size_t n1 = (size_t)nobj + 1, nr1 = (size_t)ps.nroots + 1;
+    const int nt = ps.nrootpix / NO_TILE + 1;
+    EN(svals, n1 * 4);
+    EN(order, (2 * (size_t)nt + 3 * nr1 + n1) * 4);
+    OrderBufs Q;
+    Q.tcnt = P<int>(ctx->order);
+    Q.thead = Q.tcnt + nt;
+    Q.next = Q.thead + nt;
+    Q.elem = Q.next + nr1;
+    Q.ns = Q.elem + nr1;
+    int *const pos = Q.ns + nr1;
+    Q.pos = pos;
+    CK(cudaMemsetAsync(Q.tcnt, 0, 2 * (size_t)nt * 4, st));
+    k_surv_flags<<<grid1(nobj, 256), 256, 0, st>>>(O, nobj, nobj_dev, pos);
+    nl = 3 + exclusive_scan(pos, pos, nobj, &d_sc->nsurv, tmp, st, nobj_dev);
+    if (Pm.numbering == 0) {
+        k_order_roots<<<grid1(ps.nroots, 128), 128, 0, st>>>(O, R, P<int>(ctx->pos2idx), w, ps.nroots,
+                                                             &d_sc->nroots, Q);
+        nl += 1 + exclusive_scan(Q.tcnt, Q.tcnt, nt, nullptr, tmp, st);
     }
-    const int *ns_dev = ps.capf ? &d_sc->nsurv : nullptr;
-    k_surv_compact<<<grid1(nobj + 1, 256), 256, 0, st>>>(O, R.ymax, R.lastx, sflag, nobj, nobj_dev, w, Pm.numbering,
-                                                         P<unsigned>(ctx->skeys), P<unsigned>(ctx->svals));
-    // completion keys are below w*h; first-pixel numbering has all keys 0
-    // (the survivors are already in index order)
-    const int cbits = Pm.numbering == 0 ? bits_for((long long)w * h - 1) : 0;
-    radix_sort_pairs(P<unsigned>(ctx->skeys), P<unsigned>(ctx->svals), P<unsigned>(ctx->skalt),
-                     P<unsigned>(ctx->svalt), ns, cbits, tmp, st, ns_dev);
-    k_number<<<grid1(ns + 1, 256), 256, 0, st>>>(O, P<unsigned>(ctx->svals), ns, ns_dev);
+    k_order_objs<<<grid1(nobj, 128), 128, 0, st>>>(O, R, nobj, nobj_dev, Pm.numbering, Q, P<unsigned>(ctx->svals));
+    // rows for every object: the survivors' count stays on the device until
+    // the end of the frame
+    const int ns = nobj;
+    const int *ns_dev = &d_sc->nsurv;
     EN(rows, (size_t)(ns + 1) * sizeof(sexgpu_object));
     k_write_rows<<<grid1(ns + 1, 128), 128, 0, st>>>(O, P<unsigned>(ctx->svals), ns, ns_dev,
                                                      P<sexgpu_object>(ctx->rows));
-    stage_mark(ctx, "catalog", 4 + scan_launches(nobj) + radix_launches(cbits, ns));
+    stage_mark(ctx, "catalog", nl);
     CK(cudaGetLastError());
     if (ps.capf) {
         // the scalars come back with the frame; the host reads them after the
@@ -1121,14 +1071,13 @@ int pipe_end(sexgpu_ctx *ctx) {
         ps.stage = 6;
         return SEXGPU_OK;
     }
-    rc = read_scalars(ctx);
+    const int rc = read_scalars(ctx);
     if (rc) return rc;
     stage_collect(ctx);
     ctx->last_w = w;
     ctx->last_h = h;
     ctx->last_nobj = nobj;
-    ctx->last_ns = ns;
-    ps.ns = ns;
+    ctx->last_ns = ps.ns = ctx->hsc.nsurv;
     ps.stage = 6;
     return SEXGPU_OK;
 }
@@ -1484,15 +1433,13 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     DevBuf *all[] = {&ctx->img, &ctx->sub, &ctx->cd, &ctx->lab, &ctx->cnt, &ctx->flag, &ctx->pos, &ctx->alloc,
-                     &ctx->seg, &ctx->pos2idx, &ctx->var, &ctx->scan_tmp, &ctx->keys, &ctx->vals, &ctx->kalt,
-                     &ctx->valt, &ctx->ms, &ctx->back, &ctx->sigma, &ctx->back2, &ctx->back3, &ctx->sigma3,
+                     &ctx->seg, &ctx->pos2idx, &ctx->var, &ctx->scan_tmp, &ctx->keys, &ctx->vals, &ctx->ms, &ctx->back, &ctx->sigma, &ctx->back2, &ctx->back3, &ctx->sigma3,
                      &ctx->dback, &ctx->bu, &ctx->rownode, &ctx->rowdnode, &ctx->rowu, &ctx->colk, &ctx->coldx,
-                     &ctx->rsize, &ctx->roff, &ctx->rfirst, &ctx->rymax, &ctx->rlastx, &ctx->rnkept, &ctx->robjbase,
+                     &ctx->rsize, &ctx->roff, &ctx->rnkept, &ctx->robjbase,
                      &ctx->rdthr, &ctx->rathr, &ctx->rzero, &ctx->rlists, &ctx->rthr, &ctx->imgm, &ctx->wvar,
                      &ctx->wratio, &ctx->objkey, &ctx->rpix, &ctx->o_big,
                      &ctx->o_iso, &ctx->o_sortkey, &ctx->amp, &ctx->alpha, &ctx->cellhead,
-                     &ctx->cellnext, &ctx->vkey, &ctx->vval, &ctx->vkalt, &ctx->vvalt, &ctx->skeys, &ctx->svals,
-                     &ctx->skalt, &ctx->svalt, &ctx->rows, &ctx->sc};
+                     &ctx->vict, &ctx->svals, &ctx->order, &ctx->oitems, &ctx->rows, &ctx->sc};
     for (DevBuf *b : all) free_buf(*b);
     free_buf(ctx->deb);
     for (auto &b : ctx->o_i) free_buf(b);

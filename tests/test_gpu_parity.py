@@ -407,3 +407,25 @@ def test_background_splines_long_and_short(gpu_ctx, w, h, bs):
     gpu_ctx.extract(img, back_size=bs)
     assert gpu_ctx.background_map(img.shape).tobytes() == O.background_map(img, back_size=bs).tobytes()
     assert gpu_ctx.background_rms(img.shape).tobytes() == O.background_rms(img, back_size=bs).tobytes()
+
+
+@pytest.mark.parametrize("w,h,minarea", [(1031, 517, 1), (64, 3000, 5), (3000, 64, 5), (2048, 2048, 5)])
+def test_lists_and_catalogue_order(gpu_ctx, w, h, minarea):
+    """Object pixel lists read from boxes of one pixel up to boxes cut into
+    bands of rows (a frame-wide object with a deblended chain of knots, objects
+    inside its box), and the completion order over many raw objects of one row:
+    completion and first-pixel numbering against the oracle, CLEAN on."""
+    rng = np.random.default_rng(w + h)
+    img = rng.normal(0.0, 1.0, (h, w)).astype(np.float32)
+    t = np.arange(max(w, h) * 2)
+    x = np.clip((w - 1) * t / (t.size - 1), 0, w - 1).astype(int)
+    y = np.clip((h - 1) * (0.5 + 0.45 * np.sin(9.0 * t / t.size)), 0, h - 1).astype(int)
+    for d in range(-2, 3):
+        img[np.clip(y + d, 0, h - 1), x] = np.maximum(img[np.clip(y + d, 0, h - 1), x], 30.0 - 4 * abs(d))
+    for k in range(0, t.size, max(1, t.size // 40)):
+        _blob(img, float(x[k]), float(y[k]), 1.5, float(rng.uniform(300, 9000)))
+    img[h // 3, 1::7] += 40.0
+    for numbering in (0, 1):
+        g = run_both(gpu_ctx, img, filter_flag=0, back_type=1, back_value=0.0, thresh_type=1, detect_thresh=3.2,
+                     analysis_thresh=3.2, detect_minarea=minarea, numbering=numbering, deblend_mincont=0.001)
+        assert len(g) > 10
