@@ -243,9 +243,10 @@ __device__ __forceinline__ bool bs_add(BinSum &s, float f, int top) {
     if (ef == 0) return true;
     const int k = (top + 127 - ef) >> 4;
     const double d = (double)f;
-    s.b0 += k == 0 ? d : 0.0;
-    s.b1 += k == 1 ? d : 0.0;
-    s.b2 += k == 2 ? d : 0.0;
+    // (predicated additions: neither a branch nor an addition of 0.0 a bin)
+    asm("{ .reg .pred p; setp.eq.s32 p, %1, 0; @p add.rn.f64 %0, %0, %2; }" : "+d"(s.b0) : "r"(k), "d"(d));
+    asm("{ .reg .pred p; setp.eq.s32 p, %1, 1; @p add.rn.f64 %0, %0, %2; }" : "+d"(s.b1) : "r"(k), "d"(d));
+    asm("{ .reg .pred p; setp.eq.s32 p, %1, 2; @p add.rn.f64 %0, %0, %2; }" : "+d"(s.b2) : "r"(k), "d"(d));
     return (unsigned)k < 3u;
 }
 

@@ -9,6 +9,7 @@
 // a fixed lane order.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "kron.cuh"
 #include "pixmom.cuh"
 
 namespace sx {
@@ -121,6 +122,7 @@ struct AnaArgs {
     int wthr;           // analysis threshold follows the local rms
     double afac;        // ANALYSIS_THRESH
     int bp_thick;       // BACKPHOTO_THICK (used when O.dbkg is set)
+    KronGeo *geo;       // the photometry's first ellipse and box
 };
 
 // Robust preanalysis of a deblended object over its final pixels
@@ -430,6 +432,9 @@ __global__ void k_examine_finish(AnaArgs A) {
         atomicMax(A.last + A.O.root[o],
                   ((unsigned long long)(unsigned)ymax << 32) | (0xffffffffu - (pix[lo] - (unsigned)ymax * w)));
     }
+    // the 6-sigma ellipse and box of the Kron radius (cudaanalyse.cu:318-357)
+    kron_geo(A.w, A.h, mxo, myo, a, b, A.O.cxx[o], A.O.cyy[o], A.O.cxy[o], SX_KRON_NSIG, SX_KRON_NSIG * SX_KRON_NSIG,
+             A.geo[o]);
     int py = (int)fdiv((unsigned)peakpix, A.wdiv);
     // the mode is added only where it was measured (src/back.c:659)
     A.O.bkg[o] = A.O.dbkg && A.O.lstat[o].nlevels >= 0 ? bkg + dbkg : bkg;

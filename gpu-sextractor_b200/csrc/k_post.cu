@@ -7,6 +7,8 @@
 // OBJ_APERT_PB), :2874 (OBJ_SATUR); catalogue numbering src/scan.c:148-157.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "kron.cuh"
+#include "pixmom.cuh"
 #include "sexgpu.h"
 
 namespace sx {
@@ -209,15 +211,17 @@ __global__ void k_alloc_victims(ObjBufs O, const unsigned *opix, int *alloc, int
 struct EndRaw;
 
 struct EndArgs {
-    EndRaw *raw;    // per-object scratch between the photometry warps and k_end_finish
+    EndRaw *raw;    // per-object state between the photometry kernels
+    KronGeo *geo;   // per object: the next pass's ellipse and box (pass 1's from k_examine_finish)
+    double2 *aper;  // per object and aperture: flux, variance
     const float *sub;
     const int *alloc;
     ObjBufs O;
     FrameScalars *sc;
     int w, h, n, mask_type;
     const int *n_dev;   // the object count on the device (n is then the capacity), or null
-    double aperture, autoparam0, autoparam1, gain, zp, satur;
-    int naper;                          // apertures (>= 1); the first is `aperture`
+    double autoparam0, autoparam1, gain, zp, satur;
+    int naper;                          // apertures (>= 1)
     double apertures[SEXGPU_MAXAPER];
     const float *wvar;  // calibrated variance map, or null
     KronBufs K;         // queued Kron boxes
@@ -225,13 +229,18 @@ struct EndArgs {
     double seeing, pixscale;
 };
 
-// src/cuda/cudaanalyse.cu:104-287 (computeaperflux, aperture k of diameter
+// src/cuda/cudaanalyse.cu:104-287 (computeaperflux, one aperture of diameter
 // `diameter`).  The lanes of the warp evaluate 32 aperture pixels at a time
-// (sub-pixel area, masked value); the three double sums then take the terms
-// one by one in the raster order of the sequential loop, so the rounding is
-// that loop's.  The first aperture fills the catalogue columns; with several,
-// every one goes to O.aper.
-__device__ void aper_warp(const EndArgs &A, int o, double mx, double my, int &flags, double diameter, int k) {
+// (sub-pixel area, masked value) and put the terms of the three double sums in
+// raster order in shared memory; one lane per sum then adds them one by one, so
+// the rounding is the sequential loop's.  Lane 1 gets the variance, lane 2 the
+// flux.
+struct AperTerms {
+    double t[3][32];  // area, variance, flux
+};
+
+__device__ __forceinline__ double aper_warp(const EndArgs &A, int o, double mx, double my, int &flags, double diameter,
+                                            AperTerms &T) {
     const int lane = threadIdx.x & 31, w = A.w, h = A.h;
     const int corrflag = (A.mask_type == 2);
     const float backsig = A.sc->backsig;
@@ -264,30 +273,37 @@ __device__ void aper_warp(const EndArgs &A, int o, double mx, double my, int &fl
         ymax = h;
         flags |= SX_OBJ_APERT_PB;
     }
-    double tv = 0.0, sigtv = 0.0, area = 0.0;
-    const int bw = xmax - xmin, nn = bw * (ymax - ymin);
+    double acc = 0.0;
+    const int bw = xmax - xmin, bh = ymax - ymin, nn = bw * bh;
+    if (bw <= 0 || bh <= 0) return 0.0;
+    int yo = lane / bw, xo = lane - yo * bw;
+    const int dyo = 32 / bw, dxo = 32 - dyo * bw;
     for (int base = 0; base < nn; base += 32) {
-        const int i = base + lane;
         bool in = false;
         float locarea = 0.0f;
         double pix = 0.0, pvar = var;
-        if (i < nn) {
-            const int yo = i / bw, x = xmin + (i - yo * bw), y = ymin + yo;
+        if (yo < bh) {
+            const int x = xmin + xo, y = ymin + yo;
             float dx = x - mx, dy = y - my, r2;
             if ((r2 = dx * dx + dy * dy) < rextlim2) {
                 in = true;
+                pix = A.sub[(size_t)y * w + x];
+                int t = A.alloc[(size_t)y * w + x], x2, y2;
                 if (r2 > rintlim2) {
                     dx += offsetx;
                     dy += offsety;
-                    for (int sy = SX_APER_OVERSAMP; sy--; dy += scaley) {
-                        float dx1 = dx, dy2 = dy * dy;
-                        for (int sx = SX_APER_OVERSAMP; sx--; dx1 += scalex)
-                            if (dx1 * dx1 + dy2 < raper2) locarea += scale2;
+                    float dx2[SX_APER_OVERSAMP];
+#pragma unroll
+                    for (int k = 0; k < SX_APER_OVERSAMP; k++, dx += scalex) dx2[k] = dx * dx;
+#pragma unroll
+                    for (int sy = 0; sy < SX_APER_OVERSAMP; sy++, dy += scaley) {
+                        const float dy2 = dy * dy;
+#pragma unroll
+                        for (int k = 0; k < SX_APER_OVERSAMP; k++)
+                            if (dx2[k] + dy2 < raper2) locarea += scale2;
                     }
                 } else
                     locarea = 1.0;
-                pix = A.sub[(size_t)y * w + x];
-                int t = A.alloc[(size_t)y * w + x], x2, y2;
                 // with a weight map: the variance of the pixel actually used,
                 // 0 for a pixel replaced by 0 (src/photom.c:128-145)
                 if (A.wvar) pvar = A.wvar[(size_t)y * w + x];
@@ -305,332 +321,438 @@ __device__ void aper_warp(const EndArgs &A, int o, double mx, double my, int &fl
                 }
             }
         }
-        const double tsig = pvar * locarea, ttv = locarea * pix;
-        for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1) {
-            const int q = __ffs(m) - 1;
-            area += __shfl_sync(0xffffffffu, locarea, q);
-            sigtv += __shfl_sync(0xffffffffu, tsig, q);
-            tv += __shfl_sync(0xffffffffu, ttv, q);
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        __syncwarp();
+        if (in) {
+            const int k = __popc(m & ((1u << lane) - 1u));
+            T.t[0][k] = locarea;
+            T.t[1][k] = pvar * locarea;
+            T.t[2][k] = locarea * pix;
+        }
+        __syncwarp();
+        if (lane < 3) {
+            const int n = __popc(m);
+            const double *t = T.t[lane];
+#pragma unroll 4
+            for (int k = 0; k < n; k++) acc += t[k];
+        }
+        xo += dxo;
+        yo += dyo;
+        if (xo >= bw) {
+            xo -= bw;
+            yo++;
         }
     }
-    if (lane != 0) return;
-    if (A.O.dbkg) tv -= area * (double)A.O.dbkg[o];
-    if (A.gain > 0.0 && tv > 0.0) sigtv += tv / A.gain;
-    const float f = tv, fe = sqrt(sigtv), mg = tv > 0.0 ? -2.5 * log10(tv) + A.zp : 99.0,
-                me = tv > 0.0 ? 1.086 * sqrt(sigtv) / tv : 99.0;
-    if (k == 0) {
-        A.O.flux_aper[o] = f;
-        A.O.fluxerr_aper[o] = fe;
-        A.O.mag_aper[o] = mg;
-        A.O.magerr_aper[o] = me;
-    }
-    if (A.naper > 1) A.O.aper[(size_t)o * A.naper + k] = make_float4(f, fe, mg, me);
-}
-
-#define SX_RINT(x) (int)(floor(x + 0.5))
-
-__device__ __forceinline__ XSum xs_warp_all2(XSum s) {
-    s = xs_warp_reduce(s);
-    unsigned long long lo = (unsigned long long)s.v, hi = (unsigned long long)(s.v >> 64);
-    lo = __shfl_sync(0xffffffffu, lo, 0);
-    hi = __shfl_sync(0xffffffffu, hi, 0);
-    s.v = (__int128)(((unsigned __int128)hi << 64) | lo);
-    s.e = __shfl_sync(0xffffffffu, s.e, 0);
-    s.ovf = __shfl_sync(0xffffffffu, s.ovf, 0);
-    return s;
-}
-__device__ __forceinline__ int wsum(int v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    const double area = __shfl_sync(0xffffffffu, acc, 0);
+    if (A.O.dbkg && lane == 2) acc -= area * (double)A.O.dbkg[o];
+    return acc;
 }
 
 // ---------------------------------------------------------------------------
 // AUTO / Kron photometry, src/cuda/cudaanalyse.cu:293-592.  Pass 1 sums
 // r*pix and pix over the 6-sigma ellipse (kron radius), pass 2 the flux inside
-// kron*ellipse.  Both sums are exact, so a box may be split freely: a warp
-// takes the boxes of up to KronBufs::warp_max pixels; larger ones (a kron
-// radius that grew over a faint, elongated object can span the frame) are
-// queued and cut into KR_CHUNK-pixel work items for whole CTAs, whose
-// partial sums a warp per object merges afterwards.
+// kron*ellipse.  Both sums are exact, so a box may be split and walked freely:
+// a warp takes the boxes of up to KronBufs::warp_max pixels; larger ones (a
+// kron radius that grew over a faint, elongated object can span the frame) are
+// queued and cut into work items of whole rows for whole CTAs.  Geometry and
+// the tails in double precision are done one thread per object between and
+// after the passes.
+//
+// A warp walks a box in strips of 8 columns, 4 rows at a time: what depends on
+// the column alone (dx, and with it two of the ellipse's three terms) is
+// computed once a strip, and the strip is cut to the rows the ellipse can
+// reach there (a widened root; every pixel is still tested).
 // ---------------------------------------------------------------------------
-struct KronAcc {
+// partial sums of a work item
+struct KronPart {
     XSum s0, s1;  // pass 1: r*pix, pix;  pass 2: pix, variance
     int area, areab;
 };
 
-// what the photometry warps hand to k_end_finish (one thread per object)
+// per-object state between the photometry kernels
 struct EndRaw {
-    KronAcc p2;     // pass-2 (AUTO) sums, when have2
+    double s0, s1;        // the last pass's sums
+    int area, areab, ovf;
     float kron;
     int flags, have2;
 };
 
-__device__ __forceinline__ void kacc_init(KronAcc &c) {
-    xs_init(c.s0);
-    xs_init(c.s1);
-    c.area = c.areab = 0;
-}
-
-__device__ __forceinline__ void kacc_merge(KronAcc &c, const KronAcc &b) {
-    xs_merge(c.s0, b.s0);
-    xs_merge(c.s1, b.s1);
-    c.area += b.area;
-    c.areab += b.areab;
-}
-
-__device__ __forceinline__ void kacc_warp(KronAcc &c) {
-    c.s0 = xs_warp_all2(c.s0);
-    c.s1 = xs_warp_all2(c.s1);
-    c.area = wsum(c.area);
-    c.areab = wsum(c.areab);
-}
-
-__device__ __forceinline__ void kron_box(const EndArgs &A, double mx, double my, float dxlim, float dylim, KronGeo &g,
-                                         int &flags) {
-    if ((g.xmin = SX_RINT(mx - dxlim)) < 0) {
-        g.xmin = 0;
-        flags |= SX_OBJ_APERT_PB;
-    }
-    if ((g.xmax = SX_RINT(mx + dxlim) + 1) > A.w) {
-        g.xmax = A.w;
-        flags |= SX_OBJ_APERT_PB;
-    }
-    if ((g.ymin = SX_RINT(my - dylim)) < 0) {
-        g.ymin = 0;
-        flags |= SX_OBJ_APERT_PB;
-    }
-    if ((g.ymax = SX_RINT(my + dylim) + 1) > A.h) {
-        g.ymax = A.h;
-        flags |= SX_OBJ_APERT_PB;
-    }
-}
-
-// pass-1 ellipse and box (cudaanalyse.cu:318-357)
-__device__ __forceinline__ void kron_geo1(const EndArgs &A, int o, double mx, double my, KronGeo &g, int &flags) {
-    const double autoaper0 = 0.0;
-    const float a = A.O.a[o], b = A.O.b[o];
-    float dxlim, dylim;
-    if (SX_KRON_NSIG * sqrtf(a * b) > autoaper0 / 2.0) {
-        g.cx2 = A.O.cxx[o];
-        g.cy2 = A.O.cyy[o];
-        g.cxy = A.O.cxy[o];
-        dxlim = g.cx2 - g.cxy * g.cxy / (4.0 * g.cy2);
-        dxlim = dxlim > 0.0 ? SX_KRON_NSIG / sqrtf(dxlim) : 0.0;
-        dylim = g.cy2 - g.cxy * g.cxy / (4.0 * g.cx2);
-        dylim = dylim > 0.0 ? SX_KRON_NSIG / sqrtf(dylim) : 0.0;
-        g.klim2 = SX_KRON_NSIG * SX_KRON_NSIG;
-    } else {
-        g.cx2 = g.cy2 = 1.0;
-        g.cxy = 0.0;
-        dxlim = dylim = autoaper0 / 2.0;
-        g.klim2 = dxlim * dxlim;
-    }
-    kron_box(A, mx, my, dxlim, dylim, g, flags);
-}
-
-// kron radius from pass 1 and the pass-2 ellipse and box (cudaanalyse.cu:
-// 385-440); false when pass 1 found no pixel (no AUTO flux)
-__device__ __forceinline__ bool kron_geo2(const EndArgs &A, int o, double mx, double my, const KronAcc &p, float &kron,
-                                          KronGeo &g, int &flags) {
-    const double autoaper1 = 0.0;
-    const int areab = p.areab, area = p.area + p.areab;
-    if (!area) return false;
-    const double r1 = xs_double(p.s0), v1 = xs_double(p.s1);
-    if (r1 > 0.0 && v1 > 0.0) {
-        kron = A.autoparam0 * r1 / v1;
-        if (kron < A.autoparam1) kron = A.autoparam1;
-    } else
-        kron = A.autoparam1;
-    if ((float)areab / area > SX_CROWD_THRESHOLD) flags |= SX_OBJ_CROWDED;
-    const float a = A.O.a[o], b = A.O.b[o];
-    float dxlim, dylim;
-    if (kron * sqrtf(a * b) > autoaper1 / 2.0) {
-        g.cx2 = A.O.cxx[o];
-        g.cy2 = A.O.cyy[o];
-        g.cxy = A.O.cxy[o];
-        dxlim = g.cx2 - g.cxy * g.cxy / (4.0 * g.cy2);
-        dxlim = dxlim > 0.0 ? kron / sqrtf(dxlim) : 0.0;
-        dylim = g.cy2 - g.cxy * g.cxy / (4.0 * g.cx2);
-        dylim = dylim > 0.0 ? kron / sqrtf(dylim) : 0.0;
-        g.klim2 = kron * kron;
-    } else {
-        g.cx2 = g.cy2 = 1.0;
-        g.cxy = 0.0;
-        dxlim = dylim = autoaper1 / 2.0;
-        g.klim2 = dxlim * dxlim;
-        kron = 0.0;
-    }
-    kron_box(A, mx, my, dxlim, dylim, g, flags);
-    return true;
-}
-
-__device__ __forceinline__ int kron_npix(const KronGeo &g) { return (g.xmax - g.xmin) * (g.ymax - g.ymin); }
-
-// box pixels i0, i0+step, ... below i1 (raster index inside the box)
-template <int PASS>
-__device__ __forceinline__ void kron_range(const EndArgs &A, int o, double mx, double my, const KronGeo &g, int i0,
-                                           int i1, int step, KronAcc &c) {
-    const int w = A.w, h = A.h, bw = g.xmax - g.xmin;
-    const FastDiv bd = make_fastdiv_dev((unsigned)bw);
+// a warp's sums over rows y0 .. y1 - 1 and strips c0, c0 + cstep, ... of the
+// box: x = sum 0 in the even lanes, sum 1 in the odd ones; area, areab in all.
+// BIN: in double bins (hints: the object's peak and, for r*pix, the ellipse's
+// largest r, for the variances the frame's); *ok false when a term did not
+// fit.  Otherwise with XSum.
+template <int PASS, bool WVAR, bool BIN>
+__device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, double my, const KronGeo &g, int y0,
+                                            int y1, int c0, int cstep, XSum &out, int &area_out, int &areab_out) {
+    const int lane = threadIdx.x & 31, w = A.w, h = A.h;
+    const int cl = lane & 7, rl = lane >> 3;
     const int corrflag = (A.mask_type == 2);
-    for (int i = i0; i < i1; i += step) {
-        const int yo = (int)fdiv((unsigned)i, bd), x = g.xmin + (i - yo * bw), y = g.ymin + yo;
-        const float dx = x - mx, dy = y - my;
-        if (PASS == 1) {
-            float r2;
-            if ((r2 = g.cx2 * dx * dx + g.cy2 * dy * dy + g.cxy * dx * dy) <= g.klim2) {
-                const float pix = A.sub[(size_t)y * w + x];
-                const int t = A.alloc[(size_t)y * w + x];
-                if ((t == o || t == -1) & (pix > -SX_BIG)) {
-                    c.area++;
-                    xs_add(c.s0, sqrtf(r2) * pix);
-                    xs_add(c.s1, pix);
-                } else
-                    c.areab++;
-            }
-        } else if ((g.cx2 * dx * dx + g.cy2 * dy * dy + g.cxy * dx * dy) <= g.klim2) {
-            c.area++;
-            float pix = A.sub[(size_t)y * w + x];
-            int t = A.alloc[(size_t)y * w + x];
-            float pvar = A.wvar ? A.wvar[(size_t)y * w + x] : 0.0f;
-            if ((t >= 0 && t != o) || pix <= -SX_BIG) {
-                c.areab++;
-                int x2, y2;
-                if (corrflag && (x2 = (int)(2 * mx + 0.49999 - x)) >= 0 && x2 < w &&
-                    (y2 = (int)(2 * my + 0.49999 - y)) >= 0 && y2 < h &&
-                    ((t = A.alloc[(size_t)y2 * w + x2]) == -1 || t == o) && A.sub[(size_t)y2 * w + x2] > -SX_BIG) {
-                    pix = A.sub[(size_t)y2 * w + x2];
-                    if (A.wvar) pvar = A.wvar[(size_t)y2 * w + x2];
-                } else {
-                    pix = 0.0;
-                    pvar = 0.0f;
-                }
-            }
-            xs_add(c.s0, pix);
-            if (A.wvar) xs_add(c.s1, pvar);
+    int top0 = 0, top1 = 0;
+    if (BIN) {
+        top1 = bs_order(A.O.peak[o]);
+        top0 = PASS == 1 ? top1 + bs_order(sqrtf(g.klim2)) + 1 : top1;
+        if (WVAR) {
+            const float bsig = A.sc->backsig;
+            top1 = bs_order(bsig * bsig) + 8;
         }
     }
-}
-
-// kron_range with the exact sums in double bins (see BinSum): the hints are
-// the object's peak (and, for pass 1's r*pix, the ellipse's largest r).
-// Returns false in every lane when any lane met a term outside the bins; the
-// caller then sums with kron_range.  Pass 2 with a variance map is not binned.
-template <int PASS>
-__device__ __forceinline__ bool kron_range_bin(const EndArgs &A, int o, double mx, double my, const KronGeo &g,
-                                               int i0, int i1, int step, KronAcc &out) {
-    const int w = A.w, h = A.h, bw = g.xmax - g.xmin;
-    const FastDiv bd = make_fastdiv_dev((unsigned)bw);
-    const int corrflag = (A.mask_type == 2);
-    const int top1 = bs_order(A.O.peak[o]), top0 = top1 + bs_order(sqrtf(g.klim2)) + 1;
+    constexpr bool TWO = PASS == 1 || WVAR;
     BinSum b0, b1;
-    bs_init(b0);
-    bs_init(b1);
+    XSum x0, x1;
+    if (BIN) {
+        bs_init(b0);
+        bs_init(b1);
+    } else {
+        xs_init(x0);
+        xs_init(x1);
+    }
     int area = 0, areab = 0;
     bool ok = true;
-    for (int i = i0; i < i1; i += step) {
-        const int yo = (int)fdiv((unsigned)i, bd), x = g.xmin + (i - yo * bw), y = g.ymin + yo;
-        const float dx = x - mx, dy = y - my;
-        if (PASS == 1) {
-            float r2;
-            if ((r2 = g.cx2 * dx * dx + g.cy2 * dy * dy + g.cxy * dx * dy) <= g.klim2) {
-                const float pix = A.sub[(size_t)y * w + x];
-                const int t = A.alloc[(size_t)y * w + x];
-                if ((t == o || t == -1) & (pix > -SX_BIG)) {
+    for (int c = c0; g.xmin + 8 * c < g.xmax; c += cstep) {
+        const int x = g.xmin + 8 * c + cl;
+        const bool col = x < g.xmax;
+        const float dx = x - mx;
+        const float qa = g.cx2 * dx * dx, qb = g.cxy * dx;
+        // rows where cy2 dy^2 + qb dy + qa <= klim2 can hold: the discriminant
+        // widened by 1e-4 of its terms (they are off by 1e-6 of them), the
+        // ends by 1.5 pixels
+        int ylo = 0x7fffffff, yhi = -1;
+        if (col) {
+            const float t4 = 4.0f * g.cy2, disc = qb * qb - t4 * (qa - g.klim2) +
+                                                  1e-4f * (qb * qb + fabsf(t4) * (fabsf(qa) + g.klim2));
+            ylo = y0;
+            yhi = y1 - 1;
+            if (g.cy2 > 0.0f && disc < 0.0f) {
+                yhi = -1;
+                ylo = 0x7fffffff;
+            } else if (g.cy2 > 0.0f && disc < 1e30f) {
+                const float r = sqrtf(disc), i2 = 0.5f / g.cy2, fmy = (float)my;
+                const float lo = fmy + (-qb - r) * i2 - 1.5f, hi = fmy + (r - qb) * i2 + 1.5f;
+                if (lo > (float)ylo) ylo = (int)fminf(lo, 2e9f);
+                if (hi < (float)yhi) yhi = (int)fmaxf(hi, -1.0f) + 1;
+                yhi = min(yhi, y1 - 1);
+            }
+        }
+        ylo = __reduce_min_sync(0xffffffffu, ylo);
+        yhi = __reduce_max_sync(0xffffffffu, yhi);
+        constexpr int U = 2;  // groups of 4 rows whose loads are in flight
+        for (int yb = ylo; yb <= yhi; yb += 4 * U) {
+            bool in[U];
+            float r2[U], pixv[U], pvar[U];
+            int tv[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int y = yb + 4 * u + rl;
+                const float dy = y - my;
+                r2[u] = qa + g.cy2 * dy * dy + qb * dy;
+                in[u] = col && y <= yhi && r2[u] <= g.klim2;
+                pixv[u] = pvar[u] = 0.0f;
+                tv[u] = 0;
+                if (in[u]) {
+                    const size_t at = (size_t)y * w + x;
+                    pixv[u] = __ldg(A.sub + at);
+                    tv[u] = __ldg(A.alloc + at);
+                    if (WVAR) pvar[u] = __ldg(A.wvar + at);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (!in[u]) continue;
+                float pix = pixv[u];
+                int t = tv[u];
+                // (f > (float)-BIG as (double)f > -BIG, see seq_in)
+                if (PASS == 1) {
+                    if ((t == o || t == -1) & (pix > (float)-SX_BIG)) {
+                        area++;
+                        const float rp = sqrtf(r2[u]) * pix;
+                        if (BIN) {
+                            ok &= bs_add(b0, rp, top0);
+                            ok &= bs_add(b1, pix, top1);
+                        } else {
+                            xs_add(x0, rp);
+                            xs_add(x1, pix);
+                        }
+                    } else
+                        areab++;
+                } else {
                     area++;
-                    ok &= bs_add(b0, sqrtf(r2) * pix, top0);
-                    ok &= bs_add(b1, pix, top1);
-                } else
-                    areab++;
+                    float pv = pvar[u];
+                    if ((t >= 0 && t != o) || pix <= (float)-SX_BIG) {
+                        areab++;
+                        const int y = yb + 4 * u + rl;
+                        int x2, y2;
+                        if (corrflag && (x2 = (int)(2 * mx + 0.49999 - x)) >= 0 && x2 < w &&
+                            (y2 = (int)(2 * my + 0.49999 - y)) >= 0 && y2 < h &&
+                            ((t = A.alloc[(size_t)y2 * w + x2]) == -1 || t == o) &&
+                            A.sub[(size_t)y2 * w + x2] > (float)-SX_BIG) {
+                            pix = A.sub[(size_t)y2 * w + x2];
+                            if (WVAR) pv = A.wvar[(size_t)y2 * w + x2];
+                        } else {
+                            pix = 0.0;
+                            pv = 0.0f;
+                        }
+                    }
+                    if (BIN) {
+                        ok &= bs_add(b0, pix, top0);
+                        if (WVAR) ok &= bs_add(b1, pv, top1);
+                    } else {
+                        xs_add(x0, pix);
+                        if (WVAR) xs_add(x1, pv);
+                    }
+                }
             }
-        } else if ((g.cx2 * dx * dx + g.cy2 * dy * dy + g.cxy * dx * dy) <= g.klim2) {
-            area++;
-            float pix = A.sub[(size_t)y * w + x];
-            int t = A.alloc[(size_t)y * w + x];
-            if ((t >= 0 && t != o) || pix <= -SX_BIG) {
-                areab++;
-                int x2, y2;
-                if (corrflag && (x2 = (int)(2 * mx + 0.49999 - x)) >= 0 && x2 < w &&
-                    (y2 = (int)(2 * my + 0.49999 - y)) >= 0 && y2 < h &&
-                    ((t = A.alloc[(size_t)y2 * w + x2]) == -1 || t == o) && A.sub[(size_t)y2 * w + x2] > -SX_BIG)
-                    pix = A.sub[(size_t)y2 * w + x2];
-                else
-                    pix = 0.0;
-            }
-            ok &= bs_add(b0, pix, top1);
         }
     }
-    if (!__all_sync(0xffffffffu, ok)) return false;
-    out.s0 = bs_to_xsum(bs_warp_sum(b0));
-    if (PASS == 1)
-        out.s1 = bs_to_xsum(bs_warp_sum(b1));
-    else
-        xs_init(out.s1);
-    out.area = wsum(area);
-    out.areab = wsum(areab);
+    if (BIN && !__all_sync(0xffffffffu, ok)) return false;
+    if (BIN) {
+        // lane k mod 8: bin k of (sum 0: 0..2, sum 1: 3..5); each parity then
+        // fetches its three
+        const double v[8] = {b0.b0, b0.b1, b0.b2, TWO ? b1.b0 : 0.0, TWO ? b1.b1 : 0.0, TWO ? b1.b2 : 0.0, 0.0, 0.0};
+        const double r = warp_sum8(v, lane);
+        const int src = 3 * (lane & 1);
+        BinSum t;
+        t.b0 = __shfl_sync(0xffffffffu, r, src);
+        t.b1 = __shfl_sync(0xffffffffu, r, src + 1);
+        t.b2 = __shfl_sync(0xffffffffu, r, src + 2);
+        out = bs_to_xsum(t);
+    } else {
+        x0 = xs_warp_sum(x0);
+        x1 = xs_warp_sum(x1);
+        out = lane & 1 ? x1 : x0;
+    }
+    area_out = __reduce_add_sync(0xffffffffu, area);
+    areab_out = __reduce_add_sync(0xffffffffu, areab);
     return true;
 }
 
-// a warp's sums over box pixels i0, i0 + step, ... < i1 (every lane holds them)
-template <int PASS>
-__device__ __forceinline__ void kron_warp_sums(const EndArgs &A, int o, double mx, double my, const KronGeo &g,
-                                               int i0, int i1, int step, KronAcc &c) {
-    // at most BS_MAX_TERMS terms of the warp per bin
-    const bool binned = (PASS == 1 || !A.wvar) && (long long)(i1 - (i0 & ~31)) <= (long long)BS_MAX_TERMS * step / 32;
-    if (binned && kron_range_bin<PASS>(A, o, mx, my, g, i0, i1, step, c)) return;
-    kacc_init(c);
-    kron_range<PASS>(A, o, mx, my, g, i0, i1, step, c);
-    kacc_warp(c);
+// the same with XSum, out of line: for terms the bins do not hold
+template <int PASS, bool WVAR>
+__device__ __noinline__ void kron_strips_xsum(const EndArgs &A, int o, double mx, double my, const KronGeo &g, int y0,
+                                              int y1, int c0, int cstep, KronPart *out) {
+    XSum x;
+    int area, areab;
+    kron_strips<PASS, WVAR, false>(A, o, mx, my, g, y0, y1, c0, cstep, x, area, areab);
+    out->s0 = x;
+    out->area = area;
+    out->areab = areab;
 }
 
-// Queue object o's pass-`pass` box (warp-collective).  False when the queue is
-// full; the warp then sums the box itself.
-__device__ bool kron_defer(const EndArgs &A, int pass, int o, int flags, float kron, const KronGeo &g, int nn) {
+template <int PASS, bool WVAR>
+__device__ __forceinline__ void kron_warp(const EndArgs &A, int o, double mx, double my, const KronGeo &g, int y0,
+                                          int y1, int c0, int cstep, XSum &x, int &area, int &areab) {
+    // at most BS_MAX_TERMS terms of the warp per bin
+    const bool few = (long long)(y1 - y0) * (g.xmax - g.xmin) <= BS_MAX_TERMS;
+    if (few && kron_strips<PASS, WVAR, true>(A, o, mx, my, g, y0, y1, c0, cstep, x, area, areab)) return;
+    KronPart p;
+    kron_strips_xsum<PASS, WVAR>(A, o, mx, my, g, y0, y1, c0, cstep, &p);
+    x = p.s0;
+    area = p.area;
+    areab = p.areab;
+}
+
+// an object's sums (lane 0: sum 0, lane 1: sum 1) into its state
+__device__ __forceinline__ void kron_store(const EndArgs &A, int o, const XSum &x, int area, int areab) {
     const int lane = threadIdx.x & 31;
-    const int nch = (nn + KR_CHUNK - 1) / KR_CHUNK;
-    int k = 0, c0 = 0;
+    const double d = xs_double(x);
+    const int ovf = __any_sync(0xffffffffu, lane < 2 && x.ovf);
+    EndRaw &R = A.raw[o];
     if (lane == 0) {
-        k = atomicAdd(&A.sc->kitems[pass], 1);
-        c0 = atomicAdd(&A.sc->kchunks[pass], nch);
-    }
-    k = __shfl_sync(0xffffffffu, k, 0);
-    c0 = __shfl_sync(0xffffffffu, c0, 0);
-    const bool ok = k < A.K.icap && c0 <= A.K.ccap - nch;
-    // this warp's chunk range: item index, or -1 where the item did not fit
-    const int cend = min(c0 + nch, A.K.ccap);
-    for (int c = c0 + lane; c < cend; c += 32) A.K.chunk[pass][c] = ok ? k : -1;
-    if (lane == 0 && k < A.K.icap) {
+        R.s0 = d;
+        R.area = area;
+        R.areab = areab;
+        R.ovf = ovf;
+    } else if (lane == 1)
+        R.s1 = d;
+}
+
+// Queue object o's pass-`pass` box (one thread).  False when the queue is
+// full; its warp then sums the box.
+__device__ bool kron_defer(const EndArgs &A, int pass, int o, const KronGeo &g) {
+    const int bw = g.xmax - g.xmin, bh = g.ymax - g.ymin;
+    const int rows = max(1, KR_CHUNK / bw), nch = (bh + rows - 1) / rows;
+    const int k = atomicAdd(&A.sc->kitems[pass], 1), c0 = atomicAdd(&A.sc->kchunks[pass], nch);
+    const bool ok = k < A.K.icap && c0 >= 0 && c0 <= A.K.ccap - nch;
+    // this box's range of work items: its index, or -1 where it did not fit
+    if (c0 >= 0)
+        for (int c = c0; c < min(c0 + nch, A.K.ccap); c++) A.K.chunk[pass][c] = ok ? k : -1;
+    if (k < A.K.icap) {
         KronItem it;
         it.o = o;
-        it.flags = flags;
         it.c0 = c0;
         it.nch = ok ? nch : -1;
-        it.kron = kron;
-        it.g = g;
+        it.rows = rows;
+        it.done = 0;
         A.K.item[pass][k] = it;
     }
     return ok;
 }
 
-// catalogue columns of a survivor (lane 0 writes); p2 = pass-2 sums if any
-__device__ void end_finish(const EndArgs &A, int o, int flags, float kron, bool have2, const KronAcc &p2) {
-    if ((threadIdx.x & 31) != 0) return;
-    EndRaw R;
-    R.p2 = p2;
-    R.kron = kron;
-    R.flags = flags;
-    R.have2 = have2;
-    A.raw[o] = R;
+// apertures and pass 1, one warp per surviving object
+constexpr int EO_WARPS = 4;
+__global__ void __launch_bounds__(EO_WARPS * 32, 8) k_end_pass1(const __grid_constant__ EndArgs A) {
+    __shared__ AperTerms terms[EO_WARPS];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int o = blockIdx.x * EO_WARPS + wid;
+    if (o >= sx_count(A.n, A.n_dev)) return;
+    if (A.O.fmaster[o] >= 0) return;
+    int flags = A.O.flags[o];
+    const double mx = A.O.mx[o], my = A.O.my[o];
+    for (int k = 0; k < A.naper; k++) {
+        const double acc = aper_warp(A, o, mx, my, flags, A.apertures[k], terms[wid]);
+        if (lane == 1 || lane == 2) (&A.aper[(size_t)o * A.naper + k].x)[2 - lane] = acc;
+    }
+    const KronGeo g = A.geo[o];
+    flags |= g.flags;
+    int queued = 0;
+    if (lane == 0) {
+        A.raw[o].flags = flags;
+        if (kron_npix(g) > A.K.warp_max) queued = kron_defer(A, 0, o, g);
+    }
+    if (__shfl_sync(0xffffffffu, queued, 0)) return;
+    XSum x;
+    int area, areab;
+    kron_warp<1, false>(A, o, mx, my, g, g.ymin, g.ymax, 0, 1, x, area, areab);
+    kron_store(A, o, x, area, areab);
 }
 
-// catalogue columns of a survivor from its photometry sums: AUTO, ISOCOR and
-// ISO fluxes, magnitudes and errors, FLAGS (one thread per object, so that
-// this double-precision tail does not run on one lane of a warp)
-__global__ void k_end_finish(EndArgs A) {
+// kron radius from pass 1 and the pass-2 ellipse and box (cudaanalyse.cu:
+// 385-440), one thread per object; no AUTO flux when pass 1 found no pixel
+__global__ void k_kron_mid(const __grid_constant__ EndArgs A) {
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(A.n, A.n_dev) || A.O.fmaster[o] >= 0) return;
+    EndRaw &R = A.raw[o];
+    if (R.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
+    const int areab = R.areab, area = R.area + R.areab;
+    R.kron = 0.0f;
+    R.have2 = 0;
+    KronGeo g;
+    if (!area) return;
+    float kron;
+    const double r1 = R.s0, v1 = R.s1;
+    if (r1 > 0.0 && v1 > 0.0) {
+        kron = A.autoparam0 * r1 / v1;
+        if (kron < A.autoparam1) kron = A.autoparam1;
+    } else
+        kron = A.autoparam1;
+    if ((float)areab / area > SX_CROWD_THRESHOLD) R.flags |= SX_OBJ_CROWDED;
+    if (!kron_geo(A.w, A.h, A.O.mx[o], A.O.my[o], A.O.a[o], A.O.b[o], A.O.cxx[o], A.O.cyy[o], A.O.cxy[o], kron,
+                  kron * kron, g))
+        kron = 0.0;
+    R.kron = kron;
+    R.flags |= g.flags;
+    A.geo[o] = g;
+    // 1: summed by its warp, 2: queued
+    R.have2 = kron_npix(g) > A.K.warp_max && kron_defer(A, 1, o, g) ? 2 : 1;
+}
+
+// pass 2, one warp per surviving object
+template <bool WVAR>
+__global__ void __launch_bounds__(EO_WARPS * 32, 8) k_end_pass2(const __grid_constant__ EndArgs A) {
+    const int o = blockIdx.x * EO_WARPS + (threadIdx.x >> 5);
+    if (o >= sx_count(A.n, A.n_dev)) return;
+    if (A.O.fmaster[o] >= 0 || A.raw[o].have2 != 1) return;
+    const KronGeo g = A.geo[o];
+    XSum x;
+    int area, areab;
+    kron_warp<2, WVAR>(A, o, A.O.mx[o], A.O.my[o], g, g.ymin, g.ymax, 0, 1, x, area, areab);
+    kron_store(A, o, x, area, areab);
+}
+
+// queued boxes: one CTA per work item, its warps taking strips in turn; the
+// CTA that finishes a box's last item merges them
+template <int PASS, bool WVAR>
+__global__ void __launch_bounds__(KR_THREADS) k_kron_chunks(const __grid_constant__ EndArgs A) {
+    __shared__ KronPart red[KR_THREADS / 32];
+    __shared__ int s_last;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int nc = min(A.sc->kchunks[PASS - 1], A.K.ccap);
+    for (int c = blockIdx.x; c < nc; c += gridDim.x) {
+        const int k = A.K.chunk[PASS - 1][c];
+        if (k < 0) continue;
+        const KronItem it = A.K.item[PASS - 1][k];
+        const KronGeo g = A.geo[it.o];
+        const int y0 = g.ymin + (c - it.c0) * it.rows, y1 = min(g.ymax, y0 + it.rows);
+        XSum x;
+        int area, areab;
+        kron_warp<PASS, WVAR>(A, it.o, A.O.mx[it.o], A.O.my[it.o], g, y0, y1, wid, KR_THREADS / 32, x, area, areab);
+        if (lane == 0) {
+            red[wid].s0 = x;
+            red[wid].area = area;
+            red[wid].areab = areab;
+        } else if (lane == 1)
+            red[wid].s1 = x;
+        __syncthreads();
+        KronPart *part = A.K.part[PASS - 1];
+        if (threadIdx.x == 0) {
+            KronPart r = red[0];
+            for (int q = 1; q < KR_THREADS / 32; q++) {
+                xs_merge(r.s0, red[q].s0);
+                xs_merge(r.s1, red[q].s1);
+                r.area += red[q].area;
+                r.areab += red[q].areab;
+            }
+            part[c] = r;
+            __threadfence();
+            s_last = atomicAdd(&A.K.item[PASS - 1][k].done, 1) == it.nch - 1;
+        }
+        __syncthreads();
+        if (s_last && wid == 0) {
+            __threadfence();
+            XSum s0, s1;
+            xs_init(s0);
+            xs_init(s1);
+            int a = 0, ab = 0;
+            for (int j = lane; j < it.nch; j += 32) {
+                const volatile KronPart *q = part + it.c0 + j;
+                XSum t;
+                t.v = ((__int128)((const volatile long long *)&q->s0.v)[1] << 64) |
+                      (unsigned long long)((const volatile long long *)&q->s0.v)[0];
+                t.e = q->s0.e;
+                t.ovf = q->s0.ovf;
+                xs_merge(s0, t);
+                t.v = ((__int128)((const volatile long long *)&q->s1.v)[1] << 64) |
+                      (unsigned long long)((const volatile long long *)&q->s1.v)[0];
+                t.e = q->s1.e;
+                t.ovf = q->s1.ovf;
+                xs_merge(s1, t);
+                a += q->area;
+                ab += q->areab;
+            }
+            s0 = xs_warp_sum(s0);
+            s1 = xs_warp_sum(s1);
+            a = __reduce_add_sync(0xffffffffu, a);
+            ab = __reduce_add_sync(0xffffffffu, ab);
+            kron_store(A, it.o, lane & 1 ? s1 : s0, a, ab);
+        }
+        __syncthreads();
+    }
+}
+
+// catalogue columns of a survivor from its photometry sums: apertures, AUTO,
+// ISOCOR and ISO fluxes, magnitudes and errors, FLAGS (one thread per object,
+// so that this double-precision tail does not run on one lane of a warp)
+__global__ void k_end_finish(const __grid_constant__ EndArgs A) {
+    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= sx_count(A.n, A.n_dev) || A.O.fmaster[o] >= 0) return;
+    for (int k = 0; k < A.naper; k++) {
+        const double2 ap = A.aper[(size_t)o * A.naper + k];
+        const double tv = ap.x;
+        double sigtv = ap.y;
+        if (A.gain > 0.0 && tv > 0.0) sigtv += tv / A.gain;
+        const float f = tv, fe = sqrt(sigtv), mg = tv > 0.0 ? -2.5 * log10(tv) + A.zp : 99.0,
+                    me = tv > 0.0 ? 1.086 * sqrt(sigtv) / tv : 99.0;
+        // the first aperture fills the catalogue columns; with several, every
+        // one goes to O.aper
+        if (k == 0) {
+            A.O.flux_aper[o] = f;
+            A.O.fluxerr_aper[o] = fe;
+            A.O.mag_aper[o] = mg;
+            A.O.magerr_aper[o] = me;
+        }
+        if (A.naper > 1) A.O.aper[(size_t)o * A.naper + k] = make_float4(f, fe, mg, me);
+    }
     const EndRaw R = A.raw[o];
-    const KronAcc &p2 = R.p2;
     const bool have2 = R.have2 != 0;
     int flags = R.flags;
     float kron = R.kron;
@@ -638,13 +760,13 @@ __global__ void k_end_finish(EndArgs A) {
     const double var = backsig * backsig;
     double tv, sigtv;
     if (have2) {
-        const int area = p2.area, areab = p2.areab;
+        const int area = R.area, areab = R.areab;
         if ((float)areab > SX_CROWD_THRESHOLD * area) flags |= SX_OBJ_CROWDED;
-        tv = xs_double(p2.s0);
-        sigtv = A.wvar ? xs_double(p2.s1) : (double)area * var;
+        tv = R.s0;
+        sigtv = A.wvar ? R.s1 : (double)area * var;
         if (A.O.dbkg) tv -= area * (double)A.O.dbkg[o];
         if (A.gain > 0.0 && tv > 0.0) sigtv += tv / A.gain;
-        if (p2.s0.ovf | p2.s1.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
+        if (R.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
     } else
         tv = sigtv = 0.0;
     const float flux = A.O.flux[o], fluxerr = A.O.fluxerr[o], dthresh = A.O.dthr[o];
@@ -677,94 +799,6 @@ __global__ void k_end_finish(EndArgs A) {
     A.O.magerr_iso[o] = flux > 0.0 ? 1.086 * fluxerr_iso / flux : 99.0;
     if (A.O.peak[o] + A.O.bkg[o] >= A.satur) flags |= SX_OBJ_SATUR;
     A.O.flags[o] = flags;
-}
-
-// after pass 1 (every lane holds its sums): pass 2 in this warp or queued
-// defer_at: AUTO boxes of more pixels than this are queued for whole blocks
-__device__ void kron_after1(const EndArgs &A, int o, double mx, double my, int flags, const KronAcc &p1,
-                            int defer_at) {
-    if ((p1.s0.ovf | p1.s1.ovf) && (threadIdx.x & 31) == 0) atomicOr(&A.sc->status, SX_ST_RANGE);
-    float kron = 0.0f;
-    KronGeo g;
-    KronAcc p2;
-    kacc_init(p2);
-    if (!kron_geo2(A, o, mx, my, p1, kron, g, flags)) {
-        end_finish(A, o, flags, kron, false, p2);
-        return;
-    }
-    const int nn = kron_npix(g);
-    if (nn > defer_at && kron_defer(A, 1, o, flags, kron, g, nn)) return;
-    kron_warp_sums<2>(A, o, mx, my, g, threadIdx.x & 31, nn, 32, p2);
-    end_finish(A, o, flags, kron, true, p2);
-}
-
-// one warp per surviving object (eight CTAs of four warps per SM)
-__global__ void __launch_bounds__(128, 8) k_endobject(EndArgs A) {
-    const int lane = threadIdx.x & 31;
-    const int o = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (o >= sx_count(A.n, A.n_dev)) return;
-    if (A.O.fmaster[o] >= 0) return;
-    int flags = A.O.flags[o];
-    const double mx = A.O.mx[o], my = A.O.my[o];
-    for (int k = 0; k < A.naper; k++) aper_warp(A, o, mx, my, flags, A.apertures[k], k);
-    KronGeo g;
-    kron_geo1(A, o, mx, my, g, flags);
-    const int nn = kron_npix(g);
-    if (nn > A.K.warp_max && kron_defer(A, 0, o, flags, 0.0f, g, nn)) return;
-    KronAcc p1;
-    kron_warp_sums<1>(A, o, mx, my, g, lane, nn, 32, p1);
-    kron_after1(A, o, mx, my, flags, p1, A.K.warp_max);
-}
-
-// queued boxes: one CTA per KR_CHUNK-pixel work item, partial sums per item
-template <int PASS>
-__global__ void __launch_bounds__(KR_THREADS) k_kron_chunks(EndArgs A) {
-    __shared__ KronAcc red[KR_THREADS / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nc = min(A.sc->kchunks[PASS - 1], A.K.ccap);
-    for (int c = blockIdx.x; c < nc; c += gridDim.x) {
-        const int k = A.K.chunk[PASS - 1][c];
-        if (k < 0) continue;
-        const KronItem it = A.K.item[PASS - 1][k];
-        const int i0 = (c - it.c0) * KR_CHUNK, i1 = min(kron_npix(it.g), i0 + KR_CHUNK);
-        KronAcc acc;
-        kron_warp_sums<PASS>(A, it.o, A.O.mx[it.o], A.O.my[it.o], it.g, i0 + threadIdx.x, i1, KR_THREADS, acc);
-        if (lane == 0) red[wid] = acc;
-        __syncthreads();
-        if (wid == 0) {
-            KronAcc r;
-            kacc_init(r);
-            if (lane < KR_THREADS / 32) r = red[lane];
-            kacc_warp(r);
-            if (lane == 0) A.K.part[PASS - 1][c] = r;
-        }
-        __syncthreads();
-    }
-}
-
-// queued boxes: one warp per object merges its items' sums and continues;
-// the objects here have large Kron boxes, and their AUTO boxes of more than
-// KR_MERGE_MAX pixels go to the block queue too, so that this tail kernel
-// does not end on one warp summing thousands of pixels
-constexpr int KR_MERGE_MAX = 1024;
-
-template <int PASS>
-__global__ void k_kron_merge(EndArgs A) {
-    const int lane = threadIdx.x & 31;
-    const int n = min(A.sc->kitems[PASS - 1], A.K.icap);
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += nw) {
-        const KronItem it = A.K.item[PASS - 1][k];
-        if (it.nch < 0) continue;
-        KronAcc acc;
-        kacc_init(acc);
-        for (int j = lane; j < it.nch; j += 32) kacc_merge(acc, A.K.part[PASS - 1][it.c0 + j]);
-        kacc_warp(acc);
-        if (PASS == 1)
-            kron_after1(A, it.o, A.O.mx[it.o], A.O.my[it.o], it.flags, acc, min(A.K.warp_max, KR_MERGE_MAX));
-        else
-            end_finish(A, it.o, it.flags, it.kron, true, acc);
-    }
 }
 
 // CLASS_STAR, src/cuda/cudaanalyse.cu:2901-2920 with the network response of
@@ -800,12 +834,18 @@ __global__ void k_class_star(ObjBufs O, int n, const int *n_dev, const sexgpu_nn
 
 void launch_endobject(const EndArgs &E, int nobj, cudaStream_t st, int &launches) {
     if (nobj <= 0) return;
-    k_endobject<<<(unsigned)((nobj + 3) / 4), 128, 0, st>>>(E);
-    k_kron_chunks<1><<<KR_GRID, KR_THREADS, 0, st>>>(E);
-    k_kron_merge<1><<<KR_GRID / 2, 128, 0, st>>>(E);
-    k_kron_chunks<2><<<KR_GRID, KR_THREADS, 0, st>>>(E);
-    k_kron_merge<2><<<KR_GRID / 2, 128, 0, st>>>(E);
-    k_end_finish<<<(unsigned)((nobj + 127) / 128), 128, 0, st>>>(E);
+    const unsigned gw = (unsigned)((nobj + EO_WARPS - 1) / EO_WARPS), gt = (unsigned)((nobj + 127) / 128);
+    k_end_pass1<<<gw, EO_WARPS * 32, 0, st>>>(E);
+    k_kron_chunks<1, false><<<KR_GRID, KR_THREADS, 0, st>>>(E);
+    k_kron_mid<<<gt, 128, 0, st>>>(E);
+    if (E.wvar) {
+        k_end_pass2<true><<<gw, EO_WARPS * 32, 0, st>>>(E);
+        k_kron_chunks<2, true><<<KR_GRID, KR_THREADS, 0, st>>>(E);
+    } else {
+        k_end_pass2<false><<<gw, EO_WARPS * 32, 0, st>>>(E);
+        k_kron_chunks<2, false><<<KR_GRID, KR_THREADS, 0, st>>>(E);
+    }
+    k_end_finish<<<gt, 128, 0, st>>>(E);
     launches += 6;
     if (E.nnw) {
         k_class_star<<<(unsigned)((nobj + 127) / 128), 128, 0, st>>>(E.O, nobj, E.n_dev, E.nnw, E.seeing,

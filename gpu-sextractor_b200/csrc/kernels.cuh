@@ -93,27 +93,30 @@ struct DevCache {
 };
 
 // Kron boxes too large for one warp, summed by whole CTAs (k_post.cu)
-constexpr int KR_CHUNK = 8192;     // box pixels per CTA work item
+constexpr int KR_CHUNK = 8192;     // box pixels per CTA work item (whole rows, at least one)
 constexpr int KR_THREADS = 256;
 constexpr int KR_GRID = 2 * 148;
-constexpr int KR_ITEMS = 8192;     // queued boxes per pass
-constexpr int KR_CHUNKS = 65536;   // work items per pass (2^29 box pixels)
 constexpr int KR_WARP_MAX = 8192;  // default: larger boxes are queued
+// queued boxes and work items per pass: an eighth of the objects and 8 items
+// each, at least 8192 boxes (a crowded mosaic queues 2% of its objects; with
+// a fixed 8192 its warps were left with boxes of thousands of pixels)
+inline int kr_items(int nobj) { return nobj / 8 > 8192 ? nobj / 8 : 8192; }
+inline int kr_chunks(int nobj) { return 8 * kr_items(nobj); }
 
 struct KronGeo {
     float cx2, cy2, cxy, klim2;
     int xmin, xmax, ymin, ymax;
+    int flags;        // OBJ_APERT_PB where the frame cuts the box
 };
 struct KronItem {
-    int o, flags, c0, nch;  // object, FLAGS so far, first work item, items (-1: summed by its warp)
-    float kron;
-    KronGeo g;
+    int o, c0, nch, rows;  // object, first work item, items (-1: summed by its warp), box rows per item
+    int done;              // items finished
 };
-struct KronAcc;
+struct KronPart;
 struct KronBufs {
     KronItem *item[2];
-    int *chunk[2];    // work item -> queued box
-    KronAcc *part[2]; // work item -> partial sums
+    int *chunk[2];     // work item -> queued box
+    KronPart *part[2]; // work item -> partial sums
     int icap, ccap, warp_max;
 };
 

@@ -162,6 +162,7 @@ struct sexgpu_ctx {
     DevBuf kitem[2], kchunk[2], kpart[2];  // queued Kron boxes
     DevBuf o_sprob;                        // CLASS_STAR per object
     DevBuf o_big;                          // objects summed by whole blocks
+    DevBuf o_geo, o_apraw;                 // Kron ellipses and boxes, aperture sums
     DevBuf o_raw, o_xraw, o_eraw;          // robust preanalysis / examineiso / photometry scratch per object
     DevBuf o_dbkg, o_lstat;                // BACKPHOTO_TYPE LOCAL: annulus mode, annulus statistics
     DevBuf o_aper, aperrows;               // every aperture per object; per catalogue row
@@ -905,6 +906,8 @@ int pipe_analyse(sexgpu_ctx *ctx) {
     AA.back = B.back3;
     AA.opix = vals;
     AA.last = ps.R.last;
+    EN(o_geo, (size_t)(nobj + 1) * sizeof(KronGeo));
+    AA.geo = P<KronGeo>(ctx->o_geo);
     AA.O = O;
     AA.sc = d_sc;
     AA.w = w;
@@ -996,6 +999,9 @@ int pipe_end(sexgpu_ctx *ctx) {
     EndArgs E;
     EN(o_eraw, (size_t)(nobj + 1) * sizeof(EndRaw));
     E.raw = P<EndRaw>(ctx->o_eraw);
+    E.geo = P<KronGeo>(ctx->o_geo);
+    EN(o_apraw, (size_t)(nobj + 1) * Pm.naper * sizeof(double2));
+    E.aper = P<double2>(ctx->o_apraw);
     E.sub = A.sub;
     E.alloc = A.alloc;
     E.O = O;
@@ -1005,7 +1011,6 @@ int pipe_end(sexgpu_ctx *ctx) {
     E.n = nobj;
     E.n_dev = nobj_dev;
     E.mask_type = Pm.mask_type;
-    E.aperture = Pm.aperture;
     E.naper = Pm.naper;
     for (int k = 0; k < SEXGPU_MAXAPER; k++) E.apertures[k] = Pm.apertures[k];
     E.autoparam0 = Pm.autoparam0;
@@ -1015,15 +1020,15 @@ int pipe_end(sexgpu_ctx *ctx) {
     E.satur = Pm.satur_level;
     E.wvar = ps.wvar;
     for (int p = 0; p < 2; p++) {
-        EN(kitem[p], (size_t)KR_ITEMS * sizeof(KronItem));
-        EN(kchunk[p], (size_t)KR_CHUNKS * sizeof(int));
-        EN(kpart[p], (size_t)KR_CHUNKS * sizeof(KronAcc));
+        EN(kitem[p], (size_t)kr_items(nobj) * sizeof(KronItem));
+        EN(kchunk[p], (size_t)kr_chunks(nobj) * sizeof(int));
+        EN(kpart[p], (size_t)kr_chunks(nobj) * sizeof(KronPart));
         E.K.item[p] = P<KronItem>(ctx->kitem[p]);
         E.K.chunk[p] = P<int>(ctx->kchunk[p]);
-        E.K.part[p] = P<KronAcc>(ctx->kpart[p]);
+        E.K.part[p] = P<KronPart>(ctx->kpart[p]);
     }
-    E.K.icap = KR_ITEMS;
-    E.K.ccap = KR_CHUNKS;
+    E.K.icap = kr_items(nobj);
+    E.K.ccap = kr_chunks(nobj);
     E.K.warp_max = ctx->kron_warp_max;
     E.nnw = ctx->nnw_dev;
     E.seeing = Pm.seeing;
@@ -1437,7 +1442,7 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
                      &ctx->dback, &ctx->bu, &ctx->rownode, &ctx->rowdnode, &ctx->rowu, &ctx->colk, &ctx->coldx,
                      &ctx->rsize, &ctx->roff, &ctx->rnkept, &ctx->robjbase,
                      &ctx->rdthr, &ctx->rathr, &ctx->rzero, &ctx->rlists, &ctx->rthr, &ctx->imgm, &ctx->wvar,
-                     &ctx->wratio, &ctx->objkey, &ctx->rpix, &ctx->o_big,
+                     &ctx->wratio, &ctx->objkey, &ctx->rpix, &ctx->o_big, &ctx->o_geo, &ctx->o_apraw,
                      &ctx->o_iso, &ctx->o_sortkey, &ctx->amp, &ctx->alpha, &ctx->cellhead,
                      &ctx->vict, &ctx->svals, &ctx->order, &ctx->oitems, &ctx->rows, &ctx->sc};
     for (DevBuf *b : all) free_buf(*b);
