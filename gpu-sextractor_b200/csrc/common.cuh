@@ -216,54 +216,50 @@ __device__ __forceinline__ XSum xs_warp_sum(XSum s) {
 __device__ __forceinline__ XSum xs_warp_reduce(XSum s) { return xs_warp_sum(s); }
 
 // ---------------------------------------------------------------------------
-// Exact sums of float terms, binned form: three double bins of 16 binary
-// orders each, the top one ending at the order `top` (a hint, for instance
-// the order of the largest term expected).  A term of order e = exponent
-// field - 127 goes to bin k = (top - e) >> 4 when 0 <= k <= 2: it is a
-// multiple of 2^(top-16k-38) below 2^(top-16k+1), so up to 2^14 such terms
-// (of one bin, over every lane that adds them up) sum below 2^53 units of
-// 2^(top-16k-38), and every double addition in the bin is exact.  A nonzero
-// term outside the bins is not added and makes bs_add return false; the
-// caller then takes the sum again with XSum.  Zero and subnormal terms add
-// nothing, as in xs_add, so a valid binned sum moved into an XSum has exactly
-// the value the XSum of the same terms has.  The hint only decides which
-// terms fit: a wrong one costs a second pass, never a different result.
+// Exact sums of float terms, binned form: two double bins of W binary orders
+// each, the upper one ending at the order `top` (a hint, for instance the order
+// of the largest term expected).  A term of order e in (top - W, top] goes to
+// the upper bin, one in (top - 2W, top - W] to the lower: it is a multiple of
+// 2^(e - 23), so up to 2^t such terms (of one bin, over every lane that adds
+// them up) sum below 2^53 units when W + 23 + t <= 53, and every double
+// addition in the bin is exact.  The total is b0 + b1 rounded once, one double
+// addition.  A nonzero term outside the bins (a subnormal one included, which
+// xs_add counts as zero) makes bin_add return false; the caller then takes the
+// sum again with XSum.  The hint only decides which terms fit: a wrong one costs
+// a second pass, never a different result.
 // ---------------------------------------------------------------------------
-constexpr int BS_MAX_TERMS = 1 << 14;  // terms per sum (all lanes together)
+constexpr int BIN_MAX_BITS = 14;                  // at most 2^14 terms per sum
+constexpr int BIN_MAX_TERMS = 1 << BIN_MAX_BITS;
 
-struct BinSum {
-    double b0, b1, b2;
+struct Bin2 {
+    double b0, b1;
 };
 
-__device__ __forceinline__ void bs_init(BinSum &s) { s.b0 = s.b1 = s.b2 = 0.0; }
+__device__ __forceinline__ void bin_init(Bin2 &s) { s.b0 = s.b1 = 0.0; }
 
-__device__ __forceinline__ bool bs_add(BinSum &s, float f, int top) {
-    const unsigned u = __float_as_uint(f);
-    const int ef = (int)((u >> 23) & 0xff);
-    if (ef == 0) return true;
-    const int k = (top + 127 - ef) >> 4;
+// width of the bins for up to n <= BIN_MAX_TERMS terms
+__device__ __forceinline__ int bin_width(int n) { return 30 - (32 - __clz(max(n - 1, 1))); }
+
+// magnitude bits of the smallest term of the lower bin, for the hint `top`;
+// with a hint so small that the lower bin would reach the subnormals, no term
+// fits
+__device__ __forceinline__ unsigned bin_low(int top, int W) {
+    const int e = top + 128 - 2 * W;
+    return e > 0 ? (unsigned)min(e, 255 - 2 * W) << 23 : 0x80000000u;
+}
+
+__device__ __forceinline__ bool bin_add(Bin2 &s, float f, unsigned low, int W) {
+    const unsigned ua = __float_as_uint(f) & 0x7fffffffu, r = ua - low;
     const double d = (double)f;
     // (predicated additions: neither a branch nor an addition of 0.0 a bin)
-    asm("{ .reg .pred p; setp.eq.s32 p, %1, 0; @p add.rn.f64 %0, %0, %2; }" : "+d"(s.b0) : "r"(k), "d"(d));
-    asm("{ .reg .pred p; setp.eq.s32 p, %1, 1; @p add.rn.f64 %0, %0, %2; }" : "+d"(s.b1) : "r"(k), "d"(d));
-    asm("{ .reg .pred p; setp.eq.s32 p, %1, 2; @p add.rn.f64 %0, %0, %2; }" : "+d"(s.b2) : "r"(k), "d"(d));
-    return (unsigned)k < 3u;
+    asm("{ .reg .pred p; setp.ge.s32 p, %2, %3; @p add.rn.f64 %0, %0, %4; @!p add.rn.f64 %1, %1, %4; }"
+        : "+d"(s.b0), "+d"(s.b1)
+        : "r"((int)r), "r"(W << 23), "d"(d));
+    return r < (unsigned)(2 * W) << 23 || ua == 0u;
 }
 
 // order of a float for the hint: exponent field - 127 (-127 for 0)
 __device__ __forceinline__ int bs_order(float f) { return (int)((__float_as_uint(f) >> 23) & 0xff) - 127; }
-
-// full-warp sum of the bins (exact: each bin's terms over the warp number
-// at most BS_MAX_TERMS); valid in every lane
-__device__ __forceinline__ BinSum bs_warp_sum(BinSum s) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s.b0 += __shfl_xor_sync(0xffffffffu, s.b0, o);
-        s.b1 += __shfl_xor_sync(0xffffffffu, s.b1, o);
-        s.b2 += __shfl_xor_sync(0xffffffffu, s.b2, o);
-    }
-    return s;
-}
 
 // s += d exactly, for a double d that is a multiple of a power of two no
 // smaller than 2^-1074 (every bin sum is)
@@ -290,15 +286,9 @@ __device__ __forceinline__ void xs_add_double(XSum &s, double d) {
         s.v += t;
 }
 
-// (out of line: called once per sum and object, it keeps one copy of the
-// conversion in the instruction cache instead of one per sum)
-__device__ __noinline__ XSum bs_to_xsum(const BinSum &b) {
-    XSum x;
-    xs_init(x);
-    xs_add_double(x, b.b2);
-    xs_add_double(x, b.b1);
-    xs_add_double(x, b.b0);
-    return x;
+__device__ __forceinline__ void xs_add_bins(XSum &s, double b0, double b1) {
+    xs_add_double(s, b1);
+    xs_add_double(s, b0);
 }
 
 // ---------------------------------------------------------------------------

@@ -21,32 +21,24 @@ constexpr int AN_WARPS = 8;
 // spills, 1.65 at 2 with none; one 4096^2 frame)
 constexpr int AN_MINB = 4;
 
-__device__ __forceinline__ unsigned warp_max_u(unsigned v) {
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ int warp_min_i(int v) {
-    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ int warp_max_i(int v) {
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ int warp_sum_i(int v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ unsigned long long warp_max_ull(unsigned long long v) {
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 // fixed-order (butterfly) double sum; identical in every lane
 __device__ __forceinline__ double warp_sum_d(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ XSum xs_warp_all(XSum s) { return xs_warp_sum(s); }
+// four sums at once, each added in that same order (pairs at distance 16, 8, 4,
+// 2, 1): lanes 8k .. 8k + 7 get the sum of v[k]
+__device__ __forceinline__ double warp_sum4(const double v[4], int lane) {
+    const bool h1 = lane & 16, h2 = lane & 8;
+    const double a = (h1 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h1 ? v[0] : v[2], 16);
+    const double b = (h1 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h1 ? v[1] : v[3], 16);
+    double c = (h2 ? b : a) + __shfl_xor_sync(0xffffffffu, h2 ? a : b, 8);
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    return c;
+}
+
+constexpr int EX_TOP = 4;        // largest filtered values a lane keeps
+constexpr int EX_TOP_AREA = 16;  // DETECT_MINAREA up to which they are tried first
 
 // k-th smallest (0-based) of the cd values of n pixels, as float bits; the
 // values are positive (object pixels lie above the detection threshold), so
@@ -99,8 +91,10 @@ __device__ unsigned warp_select(const unsigned *opix, int n, const float *cd, in
 
 // what the pixel pass of examineiso hands to its finishing kernel
 struct ExamRaw {
-    XSum stv, svar;
-    double esum, emx2, emy2, emxy, s, sx, sy, sxx, sxy;
+    double err[4];      // sums of err, err x^2, err y^2, err x y (the position errors)
+    double fit[5];      // of the FWHM fit: s, sx, sy, sxx, sxy
+    double tv, svar;    // flux, variance
+    int ovf;
     float opeak, thresh0, mthresh;
     int peakpix, area;
 };
@@ -140,12 +134,7 @@ __global__ void __launch_bounds__(AN_WARPS * 32, 3) k_analyse_robust(AnaArgs A) 
         if (lane == 0) A.biglist[atomicAdd(A.counts + 5, 1)] = o;
         return;
     }
-    const unsigned *pix = A.opix + A.O.off[o];
-    PixBox b = pix_box(A.cd, A.sub, pix, lane, n, 32, A.wdiv, A.w);
-    pixbox_warp(b);
-    PixMoments M;
-    pix_moments(A.cd, A.sub, pix, 0, n, A.wdiv, A.w, b, A.O.dthr[o], M);
-    pix_moments_store(M, b, A.raw + o);
+    pix_moments_warp(A.cd, A.sub, A.opix + A.O.off[o], n, A.wdiv, A.w, A.O.dthr[o], A.raw + o);
 }
 
 __global__ void __launch_bounds__(AN_WARPS * 32, 2) k_analyse_robust_big(AnaArgs A) {
@@ -233,6 +222,24 @@ __global__ void k_robust_finish(AnaArgs A) {
     A.O.abcor[o] = abcor;
 }
 
+// an object's flux and variance with XSum (out of line: the rare path)
+__device__ __noinline__ void exam_xsum(const AnaArgs &A, const unsigned *pix, int n, double &tv, double &svar,
+                                       int &ovf) {
+    XSum s, v;
+    xs_init(s);
+    xs_init(v);
+    for (int i = threadIdx.x & 31; i < n; i += 32) {
+        const unsigned p = pix[i];
+        xs_add(s, A.sub[p]);
+        if (A.wvar) xs_add(v, A.wvar[p]);
+    }
+    s = xs_warp_sum(s);
+    v = xs_warp_sum(v);
+    tv = xs_double(s);
+    svar = xs_double(v);
+    ovf = s.ovf | v.ovf;
+}
+
 // examineiso (src/cuda/cudaanalyse.cu:2176-2581) and the CLEAN threshold
 // mthresh of every object.
 __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A) {
@@ -245,18 +252,19 @@ __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A
     const float dthresh = A.O.dthr[o], thresh = A.O.athr[o], gthresh = A.sc->thresh, backsig = A.sc->backsig;
     const double mxo = A.O.mx[o], myo = A.O.my[o];
     double dbacknoise2 = backsig * backsig;
-    unsigned pk = 0u;
-    unsigned long long best = 0ull;
+    unsigned pk = 0u, bc = 0u, bp = 0u;
     int area = 0;
-    XSum stv, svar;
-    xs_init(stv);
-    xs_init(svar);
-    // the flux in double bins (hint: the object's peak), else with XSum
-    const bool binned = n <= BS_MAX_TERMS;
+    // flux and variance in double bins (hints: the object's peak, the frame's
+    // noise), else with XSum
+    const bool binned = n <= BIN_MAX_TERMS;
     bool ok = binned;
-    BinSum btv;
-    bs_init(btv);
-    const int tv_top = bs_order(A.O.dpeak[o]);
+    const int W = bin_width(min(n, BIN_MAX_TERMS));
+    const unsigned low_tv = bin_low(bs_order(A.O.dpeak[o]), W), low_var = bin_low(bs_order(backsig * backsig) + 8, W);
+    Bin2 btv, bvar;
+    bin_init(btv);
+    bin_init(bvar);
+    // each lane's largest filtered values, for the CLEAN threshold
+    unsigned top[EX_TOP] = {};
     double esum = 0, emx2 = 0, emy2 = 0, emxy = 0;
     for (int i = lane; i < n; i += 32) {
         unsigned p = __ldg(pix + i);
@@ -264,14 +272,24 @@ __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A
         float pv = __ldg(A.sub + p), cdpix = __ldg(A.cd + p);
         pk = max(pk, f2ord(pv));
         // first maximum of cd in raster order: max cd, then smallest index
-        unsigned long long key = ((unsigned long long)f2ord(cdpix) << 32) | (unsigned)(0xffffffffu - p);
-        best = max(best, key);
+        // (a lane's pixels come in that order); cd is positive, so its bits
+        // sort like its values
+        unsigned key = __float_as_uint(cdpix);
+        if (key > bc) {
+            bc = key;
+            bp = p;
+        }
+#pragma unroll
+        for (int k = 0; k < EX_TOP; k++) {
+            const unsigned hi = max(top[k], key);
+            key = min(top[k], key);
+            top[k] = hi;
+        }
         // with a weight map: the pixel's own analysis threshold and variance
         const float pvar = A.wvar ? __ldg(A.wvar + p) : 0.0f;
         area += pv > sx_pix_thr(A.wthr, A.afac, pvar, gthresh);
-        if (binned)
-            ok &= bs_add(btv, pv, tv_top);
-        if (A.wvar) xs_add(svar, pvar);
+        ok &= bin_add(btv, pv, low_tv, W);
+        if (A.wvar) ok &= bin_add(bvar, pvar, low_var, W);
         double err = A.wvar ? (double)pvar : dbacknoise2;
         if (A.gain > 0.0 && cdpix > 0.0) err += cdpix / A.gain;
         double x = ix - mxo, y = iy - myo;
@@ -280,23 +298,45 @@ __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A
         emy2 += err * y * y;
         emxy += err * x * y;
     }
-    float peak = ord2f(warp_max_u(pk));
-    best = warp_max_ull(best);
-    area = warp_sum_i(area);
+    float peak = ord2f(__reduce_max_sync(0xffffffffu, pk));
+    const unsigned cmax = __reduce_max_sync(0xffffffffu, bc);
+    const unsigned peakpix = __reduce_min_sync(0xffffffffu, bc == cmax ? bp : 0xffffffffu);
+    area = __reduce_add_sync(0xffffffffu, area);
+    double tv, svar = 0.0;
+    int ovf = 0;
     if (__all_sync(0xffffffffu, ok)) {
-        stv = bs_to_xsum(bs_warp_sum(btv));
+        const double v[4] = {btv.b0, btv.b1, bvar.b0, bvar.b1};
+        const double r = warp_sum4(v, lane);  // lanes 0, 8, 16, 24
+        tv = __shfl_sync(0xffffffffu, r, 0) + __shfl_sync(0xffffffffu, r, 8);
+        if (A.wvar) svar = __shfl_sync(0xffffffffu, r, 16) + __shfl_sync(0xffffffffu, r, 24);
     } else {
-        for (int i = lane; i < n; i += 32) xs_add(stv, __ldg(A.sub + __ldg(pix + i)));
-        stv = xs_warp_sum(stv);
+        exam_xsum(A, pix, n, tv, svar, ovf);
     }
-    if (A.wvar) svar = xs_warp_sum(svar);
-    esum = warp_sum_d(esum);
-    emx2 = warp_sum_d(emx2);
-    emy2 = warp_sum_d(emy2);
-    emxy = warp_sum_d(emxy);
+    const double errs[4] = {esum, emx2, emy2, emxy};
+    const double err = warp_sum4(errs, lane);
+    // the minarea-th largest filtered value: the lanes' largest are taken away
+    // one by one, each lane offering its next; a lane asked for more than it
+    // kept leaves it to the radix select
     float mthresh = 0.0f;
     if (A.clean_flag && n >= A.minarea) {
-        unsigned kbits = warp_select(pix, n, A.cd, n - A.minarea, hist[wid]);
+        unsigned kbits = 0u;
+        bool found = A.minarea <= EX_TOP_AREA;
+        int left = EX_TOP;
+        for (int k = 0; found && k < A.minarea; k++) {
+            if (__any_sync(0xffffffffu, left == 0 && n > 32 * EX_TOP)) {
+                found = false;
+                break;
+            }
+            kbits = __reduce_max_sync(0xffffffffu, top[0]);
+            const unsigned has = __ballot_sync(0xffffffffu, top[0] == kbits);
+            if (lane == __ffs(has) - 1) {
+#pragma unroll
+                for (int q = 0; q < EX_TOP - 1; q++) top[q] = top[q + 1];
+                top[EX_TOP - 1] = 0u;
+                left--;
+            }
+        }
+        if (!found) kbits = warp_select(pix, n, A.cd, n - A.minarea, hist[wid]);
         mthresh = __uint_as_float(kbits) - dthresh;
     }
     // LOCAL photometry background (src/back.c:568 localback): the annulus mode,
@@ -342,34 +382,33 @@ __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A
             sxy += lpix * d2 * inverr2;
         }
     }
+    int iso_l = 0;  // lane k: iso[k]
 #pragma unroll
-    for (int k = 0; k < SX_NISO_; k++) iso[k] = warp_sum_i(iso[k]);
-    s = warp_sum_d(s);
-    sx = warp_sum_d(sx);
-    sy = warp_sum_d(sy);
-    sxx = warp_sum_d(sxx);
+    for (int k = 0; k < SX_NISO_; k++) {
+        const int t = __reduce_add_sync(0xffffffffu, iso[k]);
+        if (lane == k) iso_l = t;
+    }
+    const double fits[4] = {s, sx, sy, sxx};
+    const double fit = warp_sum4(fits, lane);
     sxy = warp_sum_d(sxy);
-    if (lane != 0) return;
-    ExamRaw X;
-    X.stv = stv;
-    X.svar = svar;
-    X.esum = esum;
-    X.emx2 = emx2;
-    X.emy2 = emy2;
-    X.emxy = emxy;
-    X.s = s;
-    X.sx = sx;
-    X.sy = sy;
-    X.sxx = sxx;
-    X.sxy = sxy;
-    X.opeak = opeak;
-    X.thresh0 = thresh0;
-    X.mthresh = mthresh;
-    X.peakpix = (int)(0xffffffffu - (unsigned)(best & 0xffffffffu));
-    X.area = area;
-    A.xraw[o] = X;
-#pragma unroll
-    for (int k = 0; k < SX_NISO_; k++) A.O.iso[(size_t)o * SX_NISO_ + k] = iso[k];
+    if (lane < SX_NISO_) A.O.iso[(size_t)o * SX_NISO_ + lane] = iso_l;
+    ExamRaw &X = A.xraw[o];
+    if ((lane & 7) == 0) {
+        X.err[lane >> 3] = err;
+        X.fit[lane >> 3] = fit;
+    }
+    if (lane == 1) {
+        X.fit[4] = sxy;
+        X.tv = tv;
+        X.svar = svar;
+    } else if (lane == 2) {
+        X.ovf = ovf;
+        X.opeak = opeak;
+        X.thresh0 = thresh0;
+        X.mthresh = mthresh;
+        X.peakpix = (int)peakpix;
+        X.area = area;
+    }
 }
 
 // examineiso, per object: position errors, fluxes, FWHM fit, background
@@ -379,9 +418,8 @@ __global__ void k_examine_finish(AnaArgs A) {
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(A.nobj, A.nobj_dev)) return;
     const ExamRaw X = A.xraw[o];
-    const XSum stv = X.stv, svar = X.svar;
-    double esum = X.esum, emx2 = X.emx2, emy2 = X.emy2, emxy = X.emxy;
-    const double s = X.s, sx = X.sx, sy = X.sy, sxx = X.sxx, sxy = X.sxy;
+    double esum = X.err[0], emx2 = X.err[1], emy2 = X.err[2], emxy = X.err[3];
+    const double s = X.fit[0], sx = X.fit[1], sy = X.fit[2], sxx = X.fit[3], sxy = X.fit[4];
     const float opeak = X.opeak, thresh0 = X.thresh0, mthresh = X.mthresh;
     const int peakpix = X.peakpix, area = X.area, n = A.O.n[o], w = A.w;
     const double mxo = A.O.mx[o], myo = A.O.my[o];
@@ -402,9 +440,9 @@ __global__ void k_examine_finish(AnaArgs A) {
             emy2 += esum;
         }
     }
-    double tvd = xs_double(stv);
+    double tvd = X.tv;
     if (A.O.dbkg) tvd -= (double)((float)n * dbkg);   // int * float: a float product
-    double sigtv = A.wvar ? xs_double(svar) : (double)n * var;
+    double sigtv = A.wvar ? X.svar : (double)n * var;
     if (A.gain > 0.0 && tvd > 0.0) sigtv += tvd / A.gain;
     float fwhm = 0.0f;
     if (thresh0 > 0.0) {
@@ -450,7 +488,7 @@ __global__ void k_examine_finish(AnaArgs A) {
     A.O.pmxy[o] = emxy;
     A.O.fwhm[o] = fwhm;
     A.O.fdnpix[o] = n;
-    if (stv.ovf | svar.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
+    if (X.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
 }
 
 // Object pixel lists, in raster order inside each object: an object's pixels

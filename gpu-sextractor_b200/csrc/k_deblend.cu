@@ -848,12 +848,7 @@ __global__ void __launch_bounds__(DT_THREADS, 3) k_da_moments(const __grid_const
         if (lane == 0) A.D.biglist[atomicAdd(A.D.counts + 4, 1)] = o;
         return;
     }
-    const unsigned *pix = A.D.ownpix + A.O.off[o];
-    PixBox b = pix_box(A.cd, A.sub, pix, lane, n, 32, A.wdiv, A.w);
-    pixbox_warp(b);
-    PixMoments M;
-    pix_moments(A.cd, A.sub, pix, 0, n, A.wdiv, A.w, b, A.O.node_dthresh[o], M);
-    pix_moments_store(M, b, A.raw + o);
+    pix_moments_warp(A.cd, A.sub, A.D.ownpix + A.O.off[o], n, A.wdiv, A.w, A.O.node_dthresh[o], A.raw + o);
 }
 
 __global__ void __launch_bounds__(DT_THREADS, 2) k_da_moments_big(const __grid_constant__ DebArgs A) {
@@ -927,13 +922,27 @@ __global__ void k_da_finish(const __grid_constant__ DebArgs A) {
     A.O.cyy[o] = (float)(xm2 / temp2);
     A.O.cxy[o] = (float)(-2 * xym / temp2);
     A.O.abcor[o] = abcor;
+    // the gatherup's copy: the centre as whole pixels and a float remainder
+    GatherObj G;
+    const double cx = xm + xmin, cy = ym + ymin;
+    G.ix = (int)floor(cx);
+    G.iy = (int)floor(cy);
+    G.fx = (float)(cx - G.ix);
+    G.fy = (float)(cy - G.iy);
+    G.cxx = (float)(ym2 / temp2);
+    G.cyy = (float)(xm2 / temp2);
+    G.cxy = (float)(-2 * xym / temp2);
+    G.abcor = abcor;
+    A.gobj[o] = G;
 }
 
 // gatherup (cudadeblend.cu:1262-1360): every other pixel to the nearest kept
 // branch in the elliptical metric, the first in order on ties.  The metric
-// ends in a double division; a branch whose single-precision distance (off by
-// less than 2^-20) is clearly above the smallest so far is passed over
-// without it.
+// takes its offsets in double and ends in a double division; a branch whose
+// single-precision distance is clearly above the smallest so far is passed
+// over without them.  The offset from whole pixels and remainder is off by
+// less than 2^-23 of 1 + |offset|, so the quadratic form, of terms that add up
+// to T, by less than 2e-6 (T + the coefficients' sum).
 __global__ void __launch_bounds__(DT_THREADS) k_da_gather(const __grid_constant__ DebArgs A) {
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     const int n = sx_count(A.nrootpix, A.nrootpix_dev);
@@ -948,11 +957,18 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_gather(const __grid_constant_
         float distmin = 1e+31f;
         for (int i = 0; i < K; i++) {
             const int q = ob + i;
+            const int4 g0 = __ldg(reinterpret_cast<const int4 *>(A.gobj + q));
+            const float4 g1 = __ldg(reinterpret_cast<const float4 *>(A.gobj + q) + 1);
+            const float abc = g1.w;
+            {
+                const float ux = (float)(x - g0.x) - __int_as_float(g0.z), uy = (float)(y - g0.y) - __int_as_float(g0.w);
+                const float qx = g1.x * ux * ux, qy = g1.y * uy * uy, qc = g1.z * ux * uy;
+                const float f = qx + qy + qc - 2e-6f * (fabsf(qx) + fabsf(qy) + fabsf(qc) + fabsf(g1.x) + fabsf(g1.y) +
+                                                        fabsf(g1.z) * (1.0f + fabsf(ux) + fabsf(uy)));
+                if (f > 1e-30f && abc > 0.0f && 0.499999f * f > distmin * abc) continue;
+            }
             const float dx = x - __ldg(A.O.mx + q), dy = y - __ldg(A.O.my + q);
-            const float f = __ldg(A.O.cxx + q) * dx * dx + __ldg(A.O.cyy + q) * dy * dy + __ldg(A.O.cxy + q) * dx * dy;
-            const float abc = __ldg(A.O.abcor + q);
-            if (f > 1e-30f && abc > 0.0f && 0.4999995f * f > distmin * abc) continue;
-            const float dist = 0.5 * f / abc;
+            const float dist = 0.5 * (g1.x * dx * dx + g1.y * dy * dy + g1.z * dx * dy) / abc;
             if (dist < distmin) {
                 distmin = dist;
                 iclst = i;

@@ -377,32 +377,35 @@ struct EndRaw {
     int flags, have2;
 };
 
+// a warp's sums: sum 0 in the even lanes, sum 1 in the odd ones, as bins or XSum
+struct KronLane {
+    bool binned;
+    double t0, t1;
+    XSum x;
+};
+
 // a warp's sums over rows y0 .. y1 - 1 and strips c0, c0 + cstep, ... of the
-// box: x = sum 0 in the even lanes, sum 1 in the odd ones; area, areab in all.
-// BIN: in double bins (hints: the object's peak and, for r*pix, the ellipse's
-// largest r, for the variances the frame's); *ok false when a term did not
-// fit.  Otherwise with XSum.
+// box; area, areab in every lane.  BIN: in double bins (hints: the object's peak
+// and, for r*pix, the ellipse's largest r, for the variances the frame's);
+// false when a term did not fit.  Otherwise with XSum.
 template <int PASS, bool WVAR, bool BIN>
 __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, double my, const KronGeo &g, int y0,
-                                            int y1, int c0, int cstep, XSum &out, int &area_out, int &areab_out) {
+                                            int y1, int c0, int cstep, KronLane &out, int &area_out, int &areab_out) {
     const int lane = threadIdx.x & 31, w = A.w, h = A.h;
     const int cl = lane & 7, rl = lane >> 3;
     const int corrflag = (A.mask_type == 2);
-    int top0 = 0, top1 = 0;
-    if (BIN) {
-        top1 = bs_order(A.O.peak[o]);
-        top0 = PASS == 1 ? top1 + bs_order(sqrtf(g.klim2)) + 1 : top1;
-        if (WVAR) {
-            const float bsig = A.sc->backsig;
-            top1 = bs_order(bsig * bsig) + 8;
-        }
-    }
     constexpr bool TWO = PASS == 1 || WVAR;
-    BinSum b0, b1;
+    const int W = bin_width(min((y1 - y0) * (g.xmax - g.xmin), BIN_MAX_TERMS));
+    unsigned low0 = 0u, low1 = 0u;
+    Bin2 b0, b1;
     XSum x0, x1;
     if (BIN) {
-        bs_init(b0);
-        bs_init(b1);
+        const int peak = bs_order(A.O.peak[o]);
+        low0 = bin_low(PASS == 1 ? peak + bs_order(sqrtf(g.klim2)) + 1 : peak, W);
+        const float bsig = A.sc->backsig;
+        low1 = bin_low(WVAR ? bs_order(bsig * bsig) + 8 : peak, W);
+        bin_init(b0);
+        bin_init(b1);
     } else {
         xs_init(x0);
         xs_init(x1);
@@ -467,8 +470,8 @@ __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, 
                         area++;
                         const float rp = sqrtf(r2[u]) * pix;
                         if (BIN) {
-                            ok &= bs_add(b0, rp, top0);
-                            ok &= bs_add(b1, pix, top1);
+                            ok &= bin_add(b0, rp, low0, W);
+                            ok &= bin_add(b1, pix, low1, W);
                         } else {
                             xs_add(x0, rp);
                             xs_add(x1, pix);
@@ -494,8 +497,8 @@ __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, 
                         }
                     }
                     if (BIN) {
-                        ok &= bs_add(b0, pix, top0);
-                        if (WVAR) ok &= bs_add(b1, pv, top1);
+                        ok &= bin_add(b0, pix, low0, W);
+                        if (WVAR) ok &= bin_add(b1, pv, low1, W);
                     } else {
                         xs_add(x0, pix);
                         if (WVAR) xs_add(x1, pv);
@@ -506,20 +509,17 @@ __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, 
     }
     if (BIN && !__all_sync(0xffffffffu, ok)) return false;
     if (BIN) {
-        // lane k mod 8: bin k of (sum 0: 0..2, sum 1: 3..5); each parity then
-        // fetches its three
-        const double v[8] = {b0.b0, b0.b1, b0.b2, TWO ? b1.b0 : 0.0, TWO ? b1.b1 : 0.0, TWO ? b1.b2 : 0.0, 0.0, 0.0};
-        const double r = warp_sum8(v, lane);
-        const int src = 3 * (lane & 1);
-        BinSum t;
-        t.b0 = __shfl_sync(0xffffffffu, r, src);
-        t.b1 = __shfl_sync(0xffffffffu, r, src + 1);
-        t.b2 = __shfl_sync(0xffffffffu, r, src + 2);
-        out = bs_to_xsum(t);
+        // lanes 8k .. 8k + 7: bin 0, 1 of sum 0, then of sum 1; each parity
+        // fetches its two
+        const double v[4] = {b0.b0, b0.b1, TWO ? b1.b0 : 0.0, TWO ? b1.b1 : 0.0};
+        const double r = warp_sum4(v, lane);
+        const int src = 16 * (lane & 1);
+        out.t0 = __shfl_sync(0xffffffffu, r, src);
+        out.t1 = __shfl_sync(0xffffffffu, r, src + 8);
     } else {
         x0 = xs_warp_sum(x0);
         x1 = xs_warp_sum(x1);
-        out = lane & 1 ? x1 : x0;
+        out.x = lane & 1 ? x1 : x0;
     }
     area_out = __reduce_add_sync(0xffffffffu, area);
     areab_out = __reduce_add_sync(0xffffffffu, areab);
@@ -530,32 +530,33 @@ __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, 
 template <int PASS, bool WVAR>
 __device__ __noinline__ void kron_strips_xsum(const EndArgs &A, int o, double mx, double my, const KronGeo &g, int y0,
                                               int y1, int c0, int cstep, KronPart *out) {
-    XSum x;
+    KronLane l;
     int area, areab;
-    kron_strips<PASS, WVAR, false>(A, o, mx, my, g, y0, y1, c0, cstep, x, area, areab);
-    out->s0 = x;
+    kron_strips<PASS, WVAR, false>(A, o, mx, my, g, y0, y1, c0, cstep, l, area, areab);
+    out->s0 = l.x;
     out->area = area;
     out->areab = areab;
 }
 
 template <int PASS, bool WVAR>
 __device__ __forceinline__ void kron_warp(const EndArgs &A, int o, double mx, double my, const KronGeo &g, int y0,
-                                          int y1, int c0, int cstep, XSum &x, int &area, int &areab) {
-    // at most BS_MAX_TERMS terms of the warp per bin
-    const bool few = (long long)(y1 - y0) * (g.xmax - g.xmin) <= BS_MAX_TERMS;
-    if (few && kron_strips<PASS, WVAR, true>(A, o, mx, my, g, y0, y1, c0, cstep, x, area, areab)) return;
+                                          int y1, int c0, int cstep, KronLane &l, int &area, int &areab) {
+    // at most BIN_MAX_TERMS terms of the warp per bin
+    l.binned = (long long)(y1 - y0) * (g.xmax - g.xmin) <= BIN_MAX_TERMS &&
+               kron_strips<PASS, WVAR, true>(A, o, mx, my, g, y0, y1, c0, cstep, l, area, areab);
+    if (l.binned) return;
     KronPart p;
     kron_strips_xsum<PASS, WVAR>(A, o, mx, my, g, y0, y1, c0, cstep, &p);
-    x = p.s0;
+    l.x = p.s0;
     area = p.area;
     areab = p.areab;
 }
 
 // an object's sums (lane 0: sum 0, lane 1: sum 1) into its state
-__device__ __forceinline__ void kron_store(const EndArgs &A, int o, const XSum &x, int area, int areab) {
+__device__ __forceinline__ void kron_store(const EndArgs &A, int o, const KronLane &l, int area, int areab) {
     const int lane = threadIdx.x & 31;
-    const double d = xs_double(x);
-    const int ovf = __any_sync(0xffffffffu, lane < 2 && x.ovf);
+    const double d = l.binned ? l.t0 + l.t1 : xs_double(l.x);
+    const int ovf = __any_sync(0xffffffffu, !l.binned && lane < 2 && l.x.ovf);
     EndRaw &R = A.raw[o];
     if (lane == 0) {
         R.s0 = d;
@@ -610,10 +611,10 @@ __global__ void __launch_bounds__(EO_WARPS * 32, 8) k_end_pass1(const __grid_con
         if (kron_npix(g) > A.K.warp_max) queued = kron_defer(A, 0, o, g);
     }
     if (__shfl_sync(0xffffffffu, queued, 0)) return;
-    XSum x;
+    KronLane l;
     int area, areab;
-    kron_warp<1, false>(A, o, mx, my, g, g.ymin, g.ymax, 0, 1, x, area, areab);
-    kron_store(A, o, x, area, areab);
+    kron_warp<1, false>(A, o, mx, my, g, g.ymin, g.ymax, 0, 1, l, area, areab);
+    kron_store(A, o, l, area, areab);
 }
 
 // kron radius from pass 1 and the pass-2 ellipse and box (cudaanalyse.cu:
@@ -653,10 +654,10 @@ __global__ void __launch_bounds__(EO_WARPS * 32, 8) k_end_pass2(const __grid_con
     if (o >= sx_count(A.n, A.n_dev)) return;
     if (A.O.fmaster[o] >= 0 || A.raw[o].have2 != 1) return;
     const KronGeo g = A.geo[o];
-    XSum x;
+    KronLane l;
     int area, areab;
-    kron_warp<2, WVAR>(A, o, A.O.mx[o], A.O.my[o], g, g.ymin, g.ymax, 0, 1, x, area, areab);
-    kron_store(A, o, x, area, areab);
+    kron_warp<2, WVAR>(A, o, A.O.mx[o], A.O.my[o], g, g.ymin, g.ymax, 0, 1, l, area, areab);
+    kron_store(A, o, l, area, areab);
 }
 
 // queued boxes: one CTA per work item, its warps taking strips in turn; the
@@ -673,15 +674,19 @@ __global__ void __launch_bounds__(KR_THREADS) k_kron_chunks(const __grid_constan
         const KronItem it = A.K.item[PASS - 1][k];
         const KronGeo g = A.geo[it.o];
         const int y0 = g.ymin + (c - it.c0) * it.rows, y1 = min(g.ymax, y0 + it.rows);
-        XSum x;
+        KronLane l;
         int area, areab;
-        kron_warp<PASS, WVAR>(A, it.o, A.O.mx[it.o], A.O.my[it.o], g, y0, y1, wid, KR_THREADS / 32, x, area, areab);
+        kron_warp<PASS, WVAR>(A, it.o, A.O.mx[it.o], A.O.my[it.o], g, y0, y1, wid, KR_THREADS / 32, l, area, areab);
+        if (l.binned) {
+            xs_init(l.x);
+            xs_add_bins(l.x, l.t0, l.t1);
+        }
         if (lane == 0) {
-            red[wid].s0 = x;
+            red[wid].s0 = l.x;
             red[wid].area = area;
             red[wid].areab = areab;
         } else if (lane == 1)
-            red[wid].s1 = x;
+            red[wid].s1 = l.x;
         __syncthreads();
         KronPart *part = A.K.part[PASS - 1];
         if (threadIdx.x == 0) {
@@ -723,7 +728,9 @@ __global__ void __launch_bounds__(KR_THREADS) k_kron_chunks(const __grid_constan
             s1 = xs_warp_sum(s1);
             a = __reduce_add_sync(0xffffffffu, a);
             ab = __reduce_add_sync(0xffffffffu, ab);
-            kron_store(A, it.o, lane & 1 ? s1 : s0, a, ab);
+            l.binned = false;
+            l.x = lane & 1 ? s1 : s0;
+            kron_store(A, it.o, l, a, ab);
         }
         __syncthreads();
     }

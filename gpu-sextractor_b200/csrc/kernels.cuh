@@ -166,6 +166,12 @@ void launch_ccl(int *lab, int *cnt, const FrameParams &P, FrameScalars *d_sc, cu
                 bool tiled);
 
 struct MomentRaw;
+// a kept branch's centre and shape, as the gatherup reads them (32 bytes)
+struct __align__(16) GatherObj {
+    int ix, iy;
+    float fx, fy;
+    float cxx, cyy, cxy, abcor;
+};
 struct DebArgs {
     const float *cd, *sub;
     const int *pos2idx;
@@ -175,6 +181,7 @@ struct DebArgs {
     DebBufs D;
     ObjBufs O;
     MomentRaw *raw;             // per-object scratch of the preanalysis
+    GatherObj *gobj;
     FrameScalars *sc;
     int *alloc;                 // W*H object id map (-1 elsewhere)
     unsigned *objkey;           // object of every element (~0: not a branch's own pixel)

@@ -4,14 +4,14 @@
 // src/cuda/cudaanalyse.cu:1686-2124.
 //
 // One warp takes a list (one block a long one).  The seven sums are kept in
-// double bins (BinSum) per lane and reduced transposed: the lanes halve the
-// set of sums they carry with each exchange, so that after three exchanges
-// every lane carries one of them (54 shuffles for the 21 bins instead of the
-// 210 of a butterfly each), and lanes 0..6 convert their sum to an XSum and
-// to a double side by side instead of one after the other.  All sums are
-// exact, so neither the order nor the split changes a result.
+// double bins (Bin2) per lane and reduced transposed: the lanes halve the set
+// of sums they carry with each exchange, so that after three exchanges every
+// lane carries one of them (36 shuffles for the 14 bins instead of the 140 of
+// a butterfly each), and lanes 0..6 round their sum side by side.  All sums
+// are exact, so neither the order nor the split changes a result.
 #pragma once
 #include "common.cuh"
+#include "kernels.cuh"
 
 namespace sx {
 
@@ -104,76 +104,59 @@ __device__ __noinline__ void pix_moments_xsum(const float *cd, const float *sub,
     *out = mine;
 }
 
-struct PixMoments {
-    XSum x;             // lane k < PM_SUMS: sum k
-    int dnpix, area2;   // every lane
-};
-
-// one warp over list entries i0 .. i1 - 1 (b: the whole list's box; dth: the
-// threshold dnpix counts above, area2 counts above the middle between it and
-// the peak)
-__device__ __forceinline__ void pix_moments(const float *cd, const float *sub, const unsigned *pix, int i0, int i1,
-                                            const FastDiv &wdiv, int w, const PixBox &b, double dth, PixMoments &M) {
+// One warp over list entries i0 .. i1 - 1, at most DA_WARP_MAX (b: the whole
+// list's box; dth: the threshold dn counts above, a2 counts above the middle
+// between it and the peak; both per lane).  Lane k < PM_SUMS gets bins t0, t1
+// of sum k; false when a term did not fit.
+__device__ __forceinline__ bool pix_moments(const float *cd, const float *sub, const unsigned *pix, int i0, int i1,
+                                            const FastDiv &wdiv, int w, const PixBox &b, double dth, double &t0,
+                                            double &t1, int &dn, int &a2) {
     const int lane = threadIdx.x & 31;
     const float peak = ord2f(b.pk);
     const double dth2 = (dth + peak) / 2.0;
+    constexpr int W = 20;  // DA_WARP_MAX = 2^10 terms
+    static_assert(DA_WARP_MAX <= 1024, "terms per bin");
     // hints of the bins: the largest values times the box sides
     const int bx = 32 - __clz(b.xmax - b.xmin), by = 32 - __clz(b.ymax - b.ymin);
-    const int tc = bs_order(ord2f(b.cpk)), tv = bs_order(peak);
-    xs_init(M.x);
-    int dn = 0, a2 = 0;
-    for (int c0 = i0; c0 < i1; c0 += BS_MAX_TERMS) {
-        const int c1 = min(i1, c0 + BS_MAX_TERMS);
-        BinSum s[PM_SUMS];
+    const int tc = bs_order(ord2f(b.cpk));
+    const unsigned l0 = bin_low(tc, W), l1 = bin_low(bs_order(peak), W), l2 = bin_low(tc + 1 + bx, W),
+                   l3 = bin_low(tc + 1 + by, W), l4 = bin_low(tc + 1 + 2 * bx, W), l5 = bin_low(tc + 1 + 2 * by, W),
+                   l6 = bin_low(tc + 1 + bx + by, W);
+    Bin2 s[PM_SUMS];
 #pragma unroll
-        for (int k = 0; k < PM_SUMS; k++) bs_init(s[k]);
-        bool ok = true;
-        for (int i = c0 + lane; i < c1; i += 32) {
-            const unsigned p = __ldg(pix + i);
-            const int yy = (int)fdiv(p, wdiv), x = (int)p - yy * w - b.xmin, y = yy - b.ymin;
-            const float cval = __ldg(cd + p), val = __ldg(sub + p);
-            dn += val > dth;
-            a2 += val > dth2;
-            ok &= bs_add(s[0], cval, tc);
-            ok &= bs_add(s[1], val, tv);
-            ok &= bs_add(s[2], cval * x, tc + 1 + bx);
-            ok &= bs_add(s[3], cval * y, tc + 1 + by);
-            ok &= bs_add(s[4], cval * x * x, tc + 1 + 2 * bx);
-            ok &= bs_add(s[5], cval * y * y, tc + 1 + 2 * by);
-            ok &= bs_add(s[6], cval * x * y, tc + 1 + bx + by);
-        }
-        XSum part;
-        if (__all_sync(0xffffffffu, ok)) {
-            BinSum t;
-            {
-                const double v[8] = {s[0].b0, s[1].b0, s[2].b0, s[3].b0, s[4].b0, s[5].b0, s[6].b0, 0.0};
-                t.b0 = warp_sum8(v, lane);
-            }
-            {
-                const double v[8] = {s[0].b1, s[1].b1, s[2].b1, s[3].b1, s[4].b1, s[5].b1, s[6].b1, 0.0};
-                t.b1 = warp_sum8(v, lane);
-            }
-            {
-                const double v[8] = {s[0].b2, s[1].b2, s[2].b2, s[3].b2, s[4].b2, s[5].b2, s[6].b2, 0.0};
-                t.b2 = warp_sum8(v, lane);
-            }
-            part = bs_to_xsum(t);
-        } else {
-            pix_moments_xsum(cd, sub, pix, c0, c1, wdiv, w, b.xmin, b.ymin, &part);
-        }
-        if (c0 == i0)
-            M.x = part;
-        else
-            xs_merge(M.x, part);
+    for (int k = 0; k < PM_SUMS; k++) bin_init(s[k]);
+    bool ok = true;
+    for (int i = i0 + lane; i < i1; i += 32) {
+        const unsigned p = __ldg(pix + i);
+        const int yy = (int)fdiv(p, wdiv), x = (int)p - yy * w - b.xmin, y = yy - b.ymin;
+        const float cval = __ldg(cd + p), val = __ldg(sub + p);
+        dn += val > dth;
+        a2 += val > dth2;
+        const float cx = cval * x, cy = cval * y;
+        ok &= bin_add(s[0], cval, l0, W);
+        ok &= bin_add(s[1], val, l1, W);
+        ok &= bin_add(s[2], cx, l2, W);
+        ok &= bin_add(s[3], cy, l3, W);
+        ok &= bin_add(s[4], cx * x, l4, W);
+        ok &= bin_add(s[5], cy * y, l5, W);
+        ok &= bin_add(s[6], cx * y, l6, W);
     }
-    M.dnpix = __reduce_add_sync(0xffffffffu, dn);
-    M.area2 = __reduce_add_sync(0xffffffffu, a2);
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    {
+        const double v[8] = {s[0].b0, s[1].b0, s[2].b0, s[3].b0, s[4].b0, s[5].b0, s[6].b0, 0.0};
+        t0 = warp_sum8(v, lane);
+    }
+    {
+        const double v[8] = {s[0].b1, s[1].b1, s[2].b1, s[3].b1, s[4].b1, s[5].b1, s[6].b1, 0.0};
+        t1 = warp_sum8(v, lane);
+    }
+    return true;
 }
 
-__device__ __forceinline__ void pix_moments_store(const PixMoments &M, const PixBox &b, MomentRaw *R) {
+// v: lane k < PM_SUMS: sum k
+__device__ __forceinline__ void pix_moments_store(double v, int ovf, int dnpix, int area2, const PixBox &b,
+                                                  MomentRaw *R) {
     const int lane = threadIdx.x & 31;
-    const int ovf = __any_sync(0xffffffffu, lane < PM_SUMS && M.x.ovf);
-    const double v = xs_double(M.x);
     if (lane == 0)
         R->rv = (float)v;
     else if (lane == 1)
@@ -183,8 +166,8 @@ __device__ __forceinline__ void pix_moments_store(const PixMoments &M, const Pix
     else if (lane == PM_SUMS) {
         R->peak = ord2f(b.pk);
         R->cpeak = ord2f(b.cpk);
-        R->dnpix = M.dnpix;
-        R->area2 = M.area2;
+        R->dnpix = dnpix;
+        R->area2 = area2;
         R->ovf = ovf;
     } else if (lane == PM_SUMS + 1) {
         R->xmin = b.xmin;
@@ -192,6 +175,27 @@ __device__ __forceinline__ void pix_moments_store(const PixMoments &M, const Pix
         R->ymin = b.ymin;
         R->ymax = b.ymax;
     }
+}
+
+// one warp over a list of n <= DA_WARP_MAX pixels
+__device__ __forceinline__ void pix_moments_warp(const float *cd, const float *sub, const unsigned *pix, int n,
+                                                 const FastDiv &wdiv, int w, double dth, MomentRaw *R) {
+    const int lane = threadIdx.x & 31;
+    PixBox b = pix_box(cd, sub, pix, lane, n, 32, wdiv, w);
+    pixbox_warp(b);
+    double t0, t1, v;
+    int dn = 0, a2 = 0, ovf = 0;
+    if (pix_moments(cd, sub, pix, 0, n, wdiv, w, b, dth, t0, t1, dn, a2)) {
+        v = t0 + t1;
+    } else {
+        XSum x;
+        pix_moments_xsum(cd, sub, pix, 0, n, wdiv, w, b.xmin, b.ymin, &x);
+        v = xs_double(x);
+        ovf = __any_sync(0xffffffffu, lane < PM_SUMS && x.ovf);
+    }
+    dn = __reduce_add_sync(0xffffffffu, dn);
+    a2 = __reduce_add_sync(0xffffffffu, a2);
+    pix_moments_store(v, ovf, dn, a2, b, R);
 }
 
 // a whole block over one list (at most 32 warps)
@@ -210,24 +214,38 @@ __device__ __forceinline__ void pix_moments_block(const float *cd, const float *
     __syncthreads();
     b = sh.box[min(lane, nw - 1)];
     pixbox_warp(b);
-    const int i0 = (int)((long long)n * wid / nw), i1 = (int)((long long)n * (wid + 1) / nw);
-    PixMoments M;
-    pix_moments(cd, sub, pix, i0, i1, wdiv, w, b, dth, M);
-    if (lane < PM_SUMS) sh.x[wid][lane] = M.x;
+    XSum x;
+    xs_init(x);
+    int dn = 0, a2 = 0;
+    for (int i0 = wid * DA_WARP_MAX; i0 < n; i0 += nw * DA_WARP_MAX) {
+        const int i1 = min(n, i0 + DA_WARP_MAX);
+        double t0, t1;
+        if (pix_moments(cd, sub, pix, i0, i1, wdiv, w, b, dth, t0, t1, dn, a2)) {
+            xs_add_bins(x, t0, t1);
+        } else {
+            XSum t;
+            pix_moments_xsum(cd, sub, pix, i0, i1, wdiv, w, b.xmin, b.ymin, &t);
+            xs_merge(x, t);
+        }
+    }
+    dn = __reduce_add_sync(0xffffffffu, dn);
+    a2 = __reduce_add_sync(0xffffffffu, a2);
+    if (lane < PM_SUMS) sh.x[wid][lane] = x;
     if (lane == 0) {
-        sh.dnpix[wid] = M.dnpix;
-        sh.area2[wid] = M.area2;
+        sh.dnpix[wid] = dn;
+        sh.area2[wid] = a2;
     }
     __syncthreads();
     if (wid == 0) {
-        xs_init(M.x);
-        M.dnpix = M.area2 = 0;
+        xs_init(x);
+        dn = a2 = 0;
         for (int k = 0; k < nw; k++) {
-            if (lane < PM_SUMS) xs_merge(M.x, sh.x[k][lane]);
-            M.dnpix += sh.dnpix[k];
-            M.area2 += sh.area2[k];
+            if (lane < PM_SUMS) xs_merge(x, sh.x[k][lane]);
+            dn += sh.dnpix[k];
+            a2 += sh.area2[k];
         }
-        pix_moments_store(M, b, R);
+        const int ovf = __any_sync(0xffffffffu, lane < PM_SUMS && x.ovf);
+        pix_moments_store(xs_double(x), ovf, dn, a2, b, R);
     }
     __syncthreads();
 }
