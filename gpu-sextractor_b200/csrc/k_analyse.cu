@@ -266,37 +266,53 @@ __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A
     // each lane's largest filtered values, for the CLEAN threshold
     unsigned top[EX_TOP] = {};
     double esum = 0, emx2 = 0, emy2 = 0, emxy = 0;
-    for (int i = lane; i < n; i += 32) {
-        unsigned p = __ldg(pix + i);
-        int iy = (int)fdiv(p, A.wdiv), ix = (int)p - iy * w;
-        float pv = __ldg(A.sub + p), cdpix = __ldg(A.cd + p);
-        pk = max(pk, f2ord(pv));
-        // first maximum of cd in raster order: max cd, then smallest index
-        // (a lane's pixels come in that order); cd is positive, so its bits
-        // sort like its values
-        unsigned key = __float_as_uint(cdpix);
-        if (key > bc) {
-            bc = key;
-            bp = p;
+    // two of a lane's pixels at a time, so that their loads overlap; added in
+    // list order
+    for (int i0 = lane; i0 < n; i0 += 64) {
+        unsigned pp[2];
+        float vv[2], cc[2], rr[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) pp[u] = i0 + 32 * u < n ? __ldg(pix + i0 + 32 * u) : 0u;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const bool in = i0 + 32 * u < n;
+            vv[u] = in ? __ldg(A.sub + pp[u]) : 0.0f;
+            cc[u] = in ? __ldg(A.cd + pp[u]) : 0.0f;
+            // with a weight map: the pixel's own analysis threshold and variance
+            rr[u] = in && A.wvar ? __ldg(A.wvar + pp[u]) : 0.0f;
         }
 #pragma unroll
-        for (int k = 0; k < EX_TOP; k++) {
-            const unsigned hi = max(top[k], key);
-            key = min(top[k], key);
-            top[k] = hi;
+        for (int u = 0; u < 2; u++) {
+            if (i0 + 32 * u >= n) break;
+            const unsigned p = pp[u];
+            const float pv = vv[u], cdpix = cc[u], pvar = rr[u];
+            int iy = (int)fdiv(p, A.wdiv), ix = (int)p - iy * w;
+            pk = max(pk, f2ord(pv));
+            // first maximum of cd in raster order: max cd, then smallest index
+            // (a lane's pixels come in that order); cd is positive, so its bits
+            // sort like its values
+            unsigned key = __float_as_uint(cdpix);
+            if (key > bc) {
+                bc = key;
+                bp = p;
+            }
+#pragma unroll
+            for (int k = 0; k < EX_TOP; k++) {
+                const unsigned hi = max(top[k], key);
+                key = min(top[k], key);
+                top[k] = hi;
+            }
+            area += pv > sx_pix_thr(A.wthr, A.afac, pvar, gthresh);
+            ok &= bin_add(btv, pv, low_tv, W);
+            if (A.wvar) ok &= bin_add(bvar, pvar, low_var, W);
+            double err = A.wvar ? (double)pvar : dbacknoise2;
+            if (A.gain > 0.0 && cdpix > 0.0) err += cdpix / A.gain;
+            double x = ix - mxo, y = iy - myo;
+            esum += err;
+            emx2 += err * x * x;
+            emy2 += err * y * y;
+            emxy += err * x * y;
         }
-        // with a weight map: the pixel's own analysis threshold and variance
-        const float pvar = A.wvar ? __ldg(A.wvar + p) : 0.0f;
-        area += pv > sx_pix_thr(A.wthr, A.afac, pvar, gthresh);
-        ok &= bin_add(btv, pv, low_tv, W);
-        if (A.wvar) ok &= bin_add(bvar, pvar, low_var, W);
-        double err = A.wvar ? (double)pvar : dbacknoise2;
-        if (A.gain > 0.0 && cdpix > 0.0) err += cdpix / A.gain;
-        double x = ix - mxo, y = iy - myo;
-        esum += err;
-        emx2 += err * x * x;
-        emy2 += err * y * y;
-        emxy += err * x * y;
     }
     float peak = ord2f(__reduce_max_sync(0xffffffffu, pk));
     const unsigned cmax = __reduce_max_sync(0xffffffffu, bc);

@@ -28,8 +28,8 @@
 //     index, exact flux in fixed-scale limbs) to the bucket of the
 //     representative and stretch it first appears in;
 //  4. the joins of each raw object are taken from the highest level down
-//     (one warp, one block with shared state, or one block on global memory,
-//     by the number of peaks) and give the kept branches;
+//     (one warp, one block with shared state, or a cluster of blocks on global
+//     memory, by the number of peaks) and give the kept branches;
 //  5. each pixel finds its kept branch by walking the joins from its peak;
 //     the branches are pre-analysed over their own pixels, and the remaining
 //     pixels gathered up.
@@ -45,6 +45,8 @@
 // 71,000 pixels in 1,400, where the largest object's levels were the time,
 // 0.99 -> 0.16 ms; a 4096 x 4096 cluster with one raw object of about 2 M
 // pixels, 64 levels, 791 -> 2.8 ms; 16384 x 16384, 108 M pixels, 38 -> 17 ms.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "pixmom.cuh"
@@ -256,29 +258,51 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_level(const __grid_constant__
     if (threadIdx.x == 0 && s_lp) atomicAdd(&A.sc->levpix, (unsigned long long)s_lp);
 }
 
-// ---- 2. joins: each pixel with its E, SW, S and SE neighbours
+// ---- 2. joins.  An edge belongs to its lower pixel (level, then element): a
+// pixel joins the peaks of all its higher neighbours at its own level, each
+// different peak once.  (Taking the four backward or forward neighbours each
+// at the lower level of the two meant twice as many walks.)
 __global__ void __launch_bounds__(DT_THREADS) k_dt_edges(const __grid_constant__ DebArgs A) {
     if (dt_failed(A)) return;
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     if (j >= sx_count(A.nrootpix, A.nrootpix_dev)) return;
     if (A.R.npk[A.rid[j]] <= 1) return;
     const int p = (int)A.rpix[j], y = (int)fdiv((unsigned)p, A.wdiv), x = p - y * A.w;
-    const int a = A.D.up[j], l = A.D.lev[j], cap = dt_cap(A);
-    int e[4];
-    e[0] = x < A.w - 1 ? __ldg(A.pos2idx + p + 1) : -1;
-    const bool down = y < A.h - 1;
-    e[1] = down && x > 0 ? __ldg(A.pos2idx + p + A.w - 1) : -1;
-    e[2] = down ? __ldg(A.pos2idx + p + A.w) : -1;
-    e[3] = down && x < A.w - 1 ? __ldg(A.pos2idx + p + A.w + 1) : -1;
-    int b[4], s[4];
+    const int a = A.D.up[j], l = A.D.lev[j];
+    const bool inner = x > 0 && y > 0 && x < A.w - 1 && y < A.h - 1;
+    int e[8];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        b[q] = e[q] >= 0 ? A.D.up[e[q]] : a;
-        s[q] = e[q] >= 0 ? min(l, (int)A.D.lev[e[q]]) : 0;
+    for (int q = 0; q < 8; q++) {
+        const int ddx[8] = {-1, 0, 1, -1, 1, -1, 0, 1}, ddy[8] = {-1, -1, -1, 0, 0, 1, 1, 1};
+        const int nx = x + ddx[q], ny = y + ddy[q];
+        e[q] = inner || (nx >= 0 && ny >= 0 && nx < A.w && ny < A.h) ? __ldg(A.pos2idx + p + ddy[q] * A.w + ddx[q]) : -1;
     }
+    int b[8];
 #pragma unroll
-    for (int q = 0; q < 4; q++)
-        if (b[q] != a) dt_join(A.D.rec, A.D.lev, a, b[q], s[q], cap, &A.sc->status);
+    for (int q = 0; q < 8; q++) {
+        b[q] = a;
+        if (e[q] >= 0) {
+            const int le = A.D.lev[e[q]];
+            if (le > l || (le == l && e[q] > j)) b[q] = A.D.up[e[q]];
+        }
+    }
+    unsigned todo = 0u;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        bool again = b[q] == a;
+#pragma unroll
+        for (int k = 0; k < q; k++) again |= b[k] == b[q];
+        if (!again) todo |= 1u << q;
+    }
+    // one join of every lane at a time, whichever neighbours they are
+    const int cap = dt_cap(A);
+    for (; todo; todo &= todo - 1u) {
+        const int q = __ffs(todo) - 1;
+        int t = b[0];
+#pragma unroll
+        for (int k = 1; k < 8; k++) t = q == k ? b[k] : t;
+        dt_join(A.D.rec, A.D.lev, a, t, l, cap, &A.sc->status);
+    }
 }
 
 // each join straight to the representative of that level, which gets a bit
@@ -317,8 +341,12 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_buckets(const __grid_constant
     }
 }
 
+constexpr int DT_FILL_RUNS = 12;
+
 // ---- 3. every pixel into the bucket of the representative and stretch it
-// first appears in; lanes of one bucket add up first
+// first appears in; lanes of one bucket add up first (taking the buckets of
+// the warp in turn: the lanes of each doing so by themselves diverged, 201 us
+// instead of 150 for 7.1 M pixels)
 __global__ void __launch_bounds__(DT_THREADS) k_dt_fill(const __grid_constant__ DebArgs A) {
     if (dt_failed(A)) return;
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
@@ -348,33 +376,42 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_fill(const __grid_constant__ 
             hi = (unsigned)(t >> DT_RADIX);
         }
     }
-    if (!__any_sync(0xffffffffu, bkt >= 0)) return;
-    // limbs of lanes with the same bucket and scale
-    const int key = bkt < 0 ? -1 : bkt;
-    const unsigned grp = __match_any_sync(0xffffffffu, key);
-    if (bkt < 0) return;
-    const int lane = threadIdx.x & 31, lead = __ffs(grp) - 1;
-    // (elements rise with the lane: the first lane has the smallest)
-    if (lane == lead) {
-        atomicAdd(A.D.bsz + bkt, __popc(grp));
-        atomicMin(A.D.bmin + bkt, e);
-    }
-    unsigned long long *acc = A.D.acc + (size_t)bkt * DT_LIMBS;
-    unsigned left = grp;
-    while (left) {  // (mostly once: lanes of one first limb)
-        const int k = __shfl_sync(grp, sh, __ffs(left) - 1);
-        const bool mine = sh == k;
-        const unsigned slo = __reduce_add_sync(grp, mine ? lo : 0u), shi = __reduce_add_sync(grp, mine ? hi : 0u);
-        if (lane == lead) {
-            if (slo) atomicAdd(acc + k, (unsigned long long)slo);
-            if (shi) atomicAdd(acc + k + 1, (unsigned long long)shi);
+    const int lane = threadIdx.x & 31;
+    // many short runs of buckets (a noisy giant): every lane by itself
+    const int prev = __shfl_up_sync(0xffffffffu, bkt, 1);
+    if (__popc(__ballot_sync(0xffffffffu, lane == 0 || prev != bkt)) > DT_FILL_RUNS) {
+        if (bkt >= 0) {
+            unsigned long long *acc = A.D.acc + (size_t)bkt * DT_LIMBS + sh;
+            atomicAdd(A.D.bsz + bkt, 1);
+            atomicMin(A.D.bmin + bkt, e);
+            if (lo) atomicAdd(acc, (unsigned long long)lo);
+            if (hi) atomicAdd(acc + 1, (unsigned long long)hi);
         }
-        left &= ~__ballot_sync(grp, mine);
+        return;
+    }
+    // one bucket (and first limb) of the warp at a time, every lane in step
+    for (unsigned left = __ballot_sync(0xffffffffu, bkt >= 0); left;) {
+        const int lead = __ffs(left) - 1;
+        const int kb = __shfl_sync(0xffffffffu, bkt, lead), ks = __shfl_sync(0xffffffffu, sh, lead);
+        const bool mine = bkt == kb && sh == ks;
+        const unsigned grp = __ballot_sync(0xffffffffu, mine);
+        const unsigned slo = __reduce_add_sync(0xffffffffu, mine ? lo : 0u),
+                       shi = __reduce_add_sync(0xffffffffu, mine ? hi : 0u);
+        if (lane == lead) {
+            // (elements rise with the lane: this one has the smallest)
+            unsigned long long *acc = A.D.acc + (size_t)bkt * DT_LIMBS + sh;
+            atomicAdd(A.D.bsz + bkt, __popc(grp));
+            atomicMin(A.D.bmin + bkt, e);
+            if (slo) atomicAdd(acc, (unsigned long long)slo);
+            if (shi) atomicAdd(acc + 1, (unsigned long long)shi);
+        }
+        left &= ~grp;
     }
 }
 
 // ---- 4. the cut
-__device__ __forceinline__ float dt_flux(const volatile unsigned long long *a, int e0) {
+template <class T>
+__device__ __forceinline__ float dt_flux(const T *a, int e0) {
     XSum s;
     __int128 v = 0;
 #pragma unroll
@@ -401,39 +438,100 @@ constexpr int DT_OK = 1, DT_OKC = 2, DT_FLAG = 4;
 // known (:1425-1776)
 __device__ __forceinline__ void dt_child(const DtState &S, int i, int k, const float thr, int debminarea, double value0,
                                          int e0) {
-    const int b = S.b0[i];
+    // (every load is issued before the first is used: in global memory each wait
+    // is most of a microsecond)
+    const int b = S.b0[i], f = S.flags[i];
+    int size = S.bsz[b], mn = S.bmin[b];
+    unsigned long long v[DT_LIMBS];
+#pragma unroll
+    for (int l = 0; l < DT_LIMBS; l++) v[l] = S.acc[(size_t)b * DT_LIMBS + l];
     if (k > 0) {
-        S.bsz[b] = S.bsz[b] + S.bsz[b + k];
-        const int mn = S.bmin[b + k];
-        if (mn < S.bmin[b]) S.bmin[b] = mn;
-        for (int l = 0; l < DT_LIMBS; l++) {
-            const unsigned long long v = S.acc[(size_t)(b + k) * DT_LIMBS + l];
-            if (v) S.acc[(size_t)b * DT_LIMBS + l] = S.acc[(size_t)b * DT_LIMBS + l] + v;
-        }
+        const int size2 = S.bsz[b + k], mn2 = S.bmin[b + k];
+        unsigned long long u[DT_LIMBS];
+#pragma unroll
+        for (int l = 0; l < DT_LIMBS; l++) u[l] = S.acc[(size_t)(b + k) * DT_LIMBS + l];
+        size += size2;
+        mn = min(mn, mn2);
+        S.bsz[b] = size;
+        S.bmin[b] = mn;
+#pragma unroll
+        for (int l = 0; l < DT_LIMBS; l++)
+            if (u[l]) {
+                v[l] += u[l];
+                S.acc[(size_t)b * DT_LIMBS + l] = v[l];
+            }
     }
-    const int size = S.bsz[b];
     bool flag = false;
     if (size >= debminarea) {
-        const float lhs = dt_flux(S.acc + (size_t)b * DT_LIMBS, e0) - thr * (float)(unsigned)size;
+        const float lhs = dt_flux(v, e0) - thr * (float)(unsigned)size;
         flag = lhs > value0;
     }
-    S.label[i] = S.bmin[b];
-    const int ok = S.flags[i] & DT_OK;
+    S.label[i] = mn;
+    const int ok = f & DT_OK;
     S.flags[i] = ok | (ok ? DT_OKC : 0) | (flag ? DT_FLAG : 0);
     S.nson[i] = flag;
 }
 
 // peak i ends here: what it stood for goes to the peak it joins
 __device__ __forceinline__ void dt_merge(const DtState &S, int i) {
-    const int q = S.par[i], b = S.b0[i], bq = S.b0[q], f = S.flags[i];
+    const int q = S.par[i], b = S.b0[i], f = S.flags[i];
+    const int bq = S.b0[q], size = S.bsz[b], mn = S.bmin[b];
+    unsigned long long v[DT_LIMBS];
+#pragma unroll
+    for (int l = 0; l < DT_LIMBS; l++) v[l] = S.acc[(size_t)b * DT_LIMBS + l];
     if (f & DT_FLAG) atomicAdd((int *)S.nson + q, 1);
     if (!(f & DT_OK)) atomicAnd((int *)S.flags + q, ~DT_OKC);
-    atomicAdd((int *)S.bsz + bq, S.bsz[b]);
-    atomicMin((int *)S.bmin + bq, S.bmin[b]);
-    for (int l = 0; l < DT_LIMBS; l++) {
-        const unsigned long long v = S.acc[(size_t)b * DT_LIMBS + l];
-        if (v) atomicAdd((unsigned long long *)S.acc + (size_t)bq * DT_LIMBS + l, v);
+    atomicAdd((int *)S.bsz + bq, size);
+    atomicMin((int *)S.bmin + bq, mn);
+#pragma unroll
+    for (int l = 0; l < DT_LIMBS; l++)
+        if (v[l]) atomicAdd((unsigned long long *)S.acc + (size_t)bq * DT_LIMBS + l, v[l]);
+}
+
+// the same for a whole warp (i < 0: nothing), where most joins of a level go to
+// one component: the lanes of the first lane's target add up first (an atomic
+// of each on the same few words was most of the time of a raw object of 2 M
+// pixels)
+__device__ __forceinline__ void dt_merge_warp(const DtState &S, int i) {
+    const int lane = threadIdx.x & 31;
+    const int q = i >= 0 ? S.par[i] : -1;
+    const unsigned all = __ballot_sync(0xffffffffu, i >= 0);
+    if (!all) return;
+    const int lead = __ffs(all) - 1, q0 = __shfl_sync(0xffffffffu, q, lead);
+    const bool mine = q == q0;
+    const unsigned grp = __ballot_sync(0xffffffffu, mine);
+    if (__popc(grp) >= 4) {
+        int b = 0, f = DT_OK, size = 0, mn = 0x7fffffff;
+        unsigned long long lim[DT_LIMBS] = {};
+        if (mine) {
+            b = S.b0[i];
+            f = S.flags[i];
+            size = S.bsz[b];
+            mn = S.bmin[b];
+#pragma unroll
+            for (int l = 0; l < DT_LIMBS; l++) lim[l] = S.acc[(size_t)b * DT_LIMBS + l];
+        }
+        size = __reduce_add_sync(0xffffffffu, size);
+        mn = __reduce_min_sync(0xffffffffu, mn);
+        const int flagged = __popc(__ballot_sync(0xffffffffu, mine && (f & DT_FLAG)));
+        const bool split = __any_sync(0xffffffffu, !(f & DT_OK));
+        const int bq = S.b0[q0];
+#pragma unroll
+        for (int l = 0; l < DT_LIMBS; l++) {
+            unsigned long long v = lim[l];
+            if (!__any_sync(0xffffffffu, v != 0ull)) continue;
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == lead) atomicAdd((unsigned long long *)S.acc + (size_t)bq * DT_LIMBS + l, v);
+        }
+        if (lane == lead) {
+            if (flagged) atomicAdd((int *)S.nson + q0, flagged);
+            if (split) atomicAnd((int *)S.flags + q0, ~DT_OKC);
+            atomicAdd((int *)S.bsz + bq, size);
+            atomicMin((int *)S.bmin + bq, mn);
+        }
+        if (mine) i = -1;
     }
+    if (i >= 0) dt_merge(S, i);
 }
 
 // is the child i of the join at (peak q) kept as an object of its own
@@ -595,16 +693,52 @@ __global__ void __launch_bounds__(NT) k_dt_cut_block(const __grid_constant__ Deb
     }
 }
 
-// the largest raw objects: one block each, state in global memory, the peaks
-// and their joins listed by level first; the kept branches are ranked by
-// k_dt_rank over the whole grid
+// the largest raw objects: one cluster of blocks each, state in global memory,
+// the peaks and their joins listed by level first; the kept branches are
+// ranked by k_dt_rank over the whole grid.  A level is three short steps over
+// its joins, each ended by a barrier of the cluster, and waits mostly on its
+// loads: a raw object of 2 M pixels and 64 levels took 1.2 ms in one block and
+// 0.86 so (1.5 before the lanes added up their joins to one component).
 constexpr int DT_HUGE_THREADS = 1024;
-__global__ void __launch_bounds__(DT_HUGE_THREADS) k_dt_cut_huge(const __grid_constant__ DebArgs A) {
-    if (dt_failed(A)) return;
-    __shared__ unsigned long long s_tot[8];
-    __shared__ int s_dead[65], s_ev[65], s_dcur[64], s_ecur[64], s_nk;
-    const int tid = threadIdx.x, NT = DT_HUGE_THREADS, nl = A.D.counts[3];
-    for (int it = blockIdx.x; it < nl; it += gridDim.x) {
+constexpr int DT_HUGE_BLOCKS = 8;
+
+struct HugeShared {
+    unsigned long long tot[DT_LIMBS];
+    int dead[65], ev[65];  // joins and the peaks they go to by level: counts, then first places
+    int dcur[64], ecur[64], nk;
+};
+
+// the warp's peaks (join level m, -1: none; levels ev of the joins it stands
+// for) added level by level to nd, ne (shared); with d, e lists, written there
+// instead, at the places the counters give (index i)
+__device__ __forceinline__ void dt_by_level(int i, int m, unsigned long long ev, int N, int *nd, int *ne, int *dlist,
+                                            int *elist) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    for (int L = 0; L < N - 1; L++) {
+        const unsigned dm = __ballot_sync(0xffffffffu, m == L), em = __ballot_sync(0xffffffffu, (int)(ev >> L) & 1);
+        if (!(dm | em)) continue;
+        int b = 0;
+        if (lane == 0 && dm) b = atomicAdd(nd + L, __popc(dm));
+        if (lane == 1 && em) b = atomicAdd(ne + L, __popc(em));
+        if (!dlist) continue;
+        const int bd = __shfl_sync(0xffffffffu, b, 0), be = __shfl_sync(0xffffffffu, b, 1);
+        if (m == L) dlist[bd + __popc(dm & below)] = i;
+        if ((ev >> L) & 1ull) elist[be + __popc(em & below)] = i;
+    }
+}
+
+__global__ void __cluster_dims__(DT_HUGE_BLOCKS, 1, 1) __launch_bounds__(DT_HUGE_THREADS)
+    k_dt_cut_huge(const __grid_constant__ DebArgs A) {
+    namespace cg = cooperative_groups;
+    __shared__ HugeShared s_own;
+    __shared__ int s_nd[64], s_ne[64];  // this block's counts by level, then its next places
+    if (dt_failed(A)) return;  // (the status is settled before this kernel: every block alike)
+    const cg::cluster_group cl = cg::this_cluster();
+    HugeShared &H = *cl.map_shared_rank(&s_own, 0);  // the cluster's first block's
+    const int tid = cl.block_rank() * DT_HUGE_THREADS + threadIdx.x, NT = DT_HUGE_THREADS * DT_HUGE_BLOCKS;
+    const int nl = A.D.counts[3];
+    for (int it = blockIdx.x / DT_HUGE_BLOCKS; it < nl; it += gridDim.x / DT_HUGE_BLOCKS) {
         const int r = A.D.lists[(size_t)3 * A.nroots + it];
         const int off = A.R.off[r], B = A.R.npk[r], NB = A.R.nbkt[r];
         const int e0 = A.sc->e0cd;
@@ -621,98 +755,124 @@ __global__ void __launch_bounds__(DT_HUGE_THREADS) k_dt_cut_huge(const __grid_co
         S.flags = A.D.g_flags + off;
         S.m = A.D.g_m + off;
         int *dlist = A.D.g_dlist + off, *elist = A.D.g_elist + off;
-        if (tid < 8) s_tot[tid] = 0ull;
-        if (tid < 65) s_dead[tid] = s_ev[tid] = 0;
-        if (tid == 0) s_nk = 0;
-        __syncthreads();
+        if (cl.block_rank() == 0) {
+            if (threadIdx.x < DT_LIMBS) s_own.tot[threadIdx.x] = 0ull;
+            if (threadIdx.x < 65) s_own.dead[threadIdx.x] = s_own.ev[threadIdx.x] = 0;
+            if (threadIdx.x == 0) s_own.nk = 0;
+        }
+        if (threadIdx.x < 64) s_nd[threadIdx.x] = s_ne[threadIdx.x] = 0;
+        cl.sync();
         unsigned long long tot[DT_LIMBS];
         for (int l = 0; l < DT_LIMBS; l++) tot[l] = 0ull;
         for (int k = tid; k < NB; k += NT)
             for (int l = 0; l < DT_LIMBS; l++) tot[l] += S.acc[(size_t)k * DT_LIMBS + l];
-        for (int l = 0; l < DT_LIMBS; l++)
-            if (tot[l]) atomicAdd(s_tot + l, tot[l]);
-        for (int i = tid; i < B; i += NT) {
-            const int d = A.D.plist[off + i];
-            const unsigned long long w = A.D.rec[d], ev = A.D.evm[d];
-            const int m = (int)(w >> 32) - 1;
-            S.evm[i] = ev;
-            S.b0[i] = A.D.boff[d] - off;
-            S.m[i] = (signed char)m;
-            S.par[i] = w ? A.D.pidx[(int)(unsigned)w] : -1;
-            S.flags[i] = DT_OK;
-            S.nson[i] = 0;
-            if (m >= 0) atomicAdd(s_dead + m, 1);
-            for (unsigned long long x = ev; x; x &= x - 1) atomicAdd(s_ev + __ffsll((long long)x) - 1, 1);
+        for (int l = 0; l < DT_LIMBS; l++) {
+            for (int o = 16; o > 0; o >>= 1) tot[l] += __shfl_xor_sync(0xffffffffu, tot[l], o);
+            if ((threadIdx.x & 31) == 0 && tot[l]) atomicAdd(H.tot + l, tot[l]);
+        }
+        for (int i0 = 0; i0 < B; i0 += NT) {
+            const int i = i0 + tid;
+            int m = -1;
+            unsigned long long ev = 0ull;
+            if (i < B) {
+                const int d = A.D.plist[off + i];
+                const unsigned long long w = A.D.rec[d];
+                ev = A.D.evm[d];
+                m = (int)(w >> 32) - 1;
+                S.evm[i] = ev;
+                S.b0[i] = A.D.boff[d] - off;
+                S.m[i] = (signed char)m;
+                S.par[i] = w ? A.D.pidx[(int)(unsigned)w] : -1;
+                S.flags[i] = DT_OK;
+                S.nson[i] = 0;
+            }
+            dt_by_level(i, m, ev, A.N, s_nd, s_ne, nullptr, nullptr);
         }
         __syncthreads();
+        if (threadIdx.x < 64) {
+            if (s_nd[threadIdx.x]) atomicAdd(H.dead + threadIdx.x, s_nd[threadIdx.x]);
+            if (s_ne[threadIdx.x]) atomicAdd(H.ev + threadIdx.x, s_ne[threadIdx.x]);
+        }
+        cl.sync();
         if (tid == 0) {
             int a = 0, b = 0;
             for (int L = 0; L < 65; L++) {
-                const int x = L < 64 ? s_dead[L] : 0, y = L < 64 ? s_ev[L] : 0;
-                s_dead[L] = a;
-                s_ev[L] = b;
+                const int x = L < 64 ? H.dead[L] : 0, y = L < 64 ? H.ev[L] : 0;
+                H.dead[L] = a;
+                H.ev[L] = b;
                 if (L < 64) {
-                    s_dcur[L] = a;
-                    s_ecur[L] = b;
+                    H.dcur[L] = a;
+                    H.ecur[L] = b;
                 }
                 a += x;
                 b += y;
             }
         }
-        __syncthreads();
-        for (int i = tid; i < B; i += NT) {
-            const int m = S.m[i];
-            if (m >= 0) dlist[atomicAdd(s_dcur + m, 1)] = i;
-            for (unsigned long long x = S.evm[i]; x; x &= x - 1)
-                elist[atomicAdd(s_ecur + __ffsll((long long)x) - 1, 1)] = i;
+        cl.sync();
+        if (threadIdx.x < 64) {
+            s_nd[threadIdx.x] = atomicAdd(H.dcur + threadIdx.x, s_nd[threadIdx.x]);
+            s_ne[threadIdx.x] = atomicAdd(H.ecur + threadIdx.x, s_ne[threadIdx.x]);
         }
         __syncthreads();
-        const double value0 = (double)dt_flux(s_tot, e0) * A.mincont;
+        for (int i0 = 0; i0 < B; i0 += NT) {
+            const int i = i0 + tid;
+            dt_by_level(i, i < B ? S.m[i] : -1, i < B ? S.evm[i] : 0ull, A.N, s_nd, s_ne, dlist, elist);
+        }
+        if (cl.block_rank() != 0) {
+            if (threadIdx.x < DT_LIMBS) s_own.tot[threadIdx.x] = H.tot[threadIdx.x];
+            if (threadIdx.x < 65) {
+                s_own.dead[threadIdx.x] = H.dead[threadIdx.x];
+                s_own.ev[threadIdx.x] = H.ev[threadIdx.x];
+            }
+        }
+        cl.sync();
+        const double value0 = (double)dt_flux(s_own.tot, e0) * A.mincont;
         for (int L = A.N - 2; L >= 0; L--) {
-            const int d0 = s_dead[L], d1 = s_dead[L + 1], v0 = s_ev[L], v1 = s_ev[L + 1];
+            const int d0 = s_own.dead[L], d1 = s_own.dead[L + 1], v0 = s_own.ev[L], v1 = s_own.ev[L + 1];
             if (d0 == d1) continue;
             const float t = thr[L + 1];
             for (int k = d0 + tid; k < d1; k += NT) {
-                const int i = dlist[k];
+                const int i = __ldcg(dlist + k);
                 dt_child(S, i, __popcll(S.evm[i]), t, A.debminarea, value0, e0);
             }
             for (int k = v0 + tid; k < v1; k += NT) {
-                const int i = elist[k];
+                const int i = __ldcg(elist + k);
                 dt_child(S, i, __popcll(S.evm[i] >> L) - 1, t, A.debminarea, value0, e0);
             }
-            __syncthreads();
-            for (int k = d0 + tid; k < d1; k += NT) dt_merge(S, dlist[k]);
-            __syncthreads();
+            cl.sync();
+            for (int k0 = d0; k0 < d1; k0 += NT) dt_merge_warp(S, k0 + tid < d1 ? __ldcg(dlist + k0 + tid) : -1);
+            cl.sync();
             for (int k = d0 + tid; k < d1; k += NT) {
-                const int i = dlist[k];
+                const int i = __ldcg(dlist + k);
                 if (dt_kept(S, i, S.par[i])) {
-                    const int q = atomicAdd(&s_nk, 1);
+                    const int q = atomicAdd(&H.nk, 1);
                     A.D.kept[off + q] = ((unsigned long long)(L + 1) << 32) | (unsigned)S.label[i];
                     A.D.krep[off + q] = A.D.plist[off + i];
                 }
             }
             for (int k = v0 + tid; k < v1; k += NT) {
-                const int i = elist[k];
+                const int i = __ldcg(elist + k);
                 if (dt_kept(S, i, i)) {
-                    const int q = atomicAdd(&s_nk, 1);
+                    const int q = atomicAdd(&H.nk, 1);
                     A.D.kept[off + q] = ((unsigned long long)(L + 1) << 32) | (unsigned)S.label[i];
                     A.D.krep[off + q] = A.D.plist[off + i];
                 }
                 const int f = S.flags[i];
                 S.flags[i] = (f & ~DT_OK) | ((f & DT_OKC) && S.nson[i] <= 1 ? DT_OK : 0);
             }
-            __syncthreads();
+            cl.sync();
         }
         for (int i = tid; i < B; i += NT)
             if (S.m[i] < 0 && (S.flags[i] & DT_OK) && A.R.size[r] >= A.debminarea) {
-                const int q = atomicAdd(&s_nk, 1);
+                const int q = atomicAdd(&H.nk, 1);
                 A.D.kept[off + q] = 0ull;
                 A.D.krep[off + q] = A.D.plist[off + i];
             }
-        __syncthreads();
-        if (tid == 0) A.R.nkept[r] = s_nk;
-        __syncthreads();
+        cl.sync();
+        if (tid == 0) A.R.nkept[r] = H.nk;
+        cl.sync();
     }
+    cl.sync();  // (no block leaves while another may still read its shared memory)
 }
 
 // kept branches of the largest raw objects in (level, label) order: the
@@ -781,7 +941,9 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_own(const __grid_constant__ D
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     const int n = sx_count(A.nrootpix, A.nrootpix_dev);
     if (blockIdx.x * DT_THREADS >= n) return;
+    __shared__ int s_wcnt[DT_THREADS / 32], s_base;
     int count = -1;
+    bool rest = false;
     if (j < n) {
         const int r = (int)A.rid[j], K = A.R.nkept[r], ob = A.R.objbase[r];
         int o = -1;
@@ -808,9 +970,24 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_own(const __grid_constant__ D
         }
         A.objkey[j] = (unsigned)o;
         if (o >= 0) A.alloc[A.rpix[j]] = o;
+        rest = o < 0;
     }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned grp = __match_any_sync(0xffffffffu, count);
-    if (count >= 0 && (int)(threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(A.O.n + count, __popc(grp));
+    if (count >= 0 && lane == __ffs(grp) - 1) atomicAdd(A.O.n + count, __popc(grp));
+    // the pixels no branch owns, listed for the gatherup (one atomic a block)
+    const unsigned rm = __ballot_sync(0xffffffffu, rest);
+    if (lane == 0) s_wcnt[wid] = __popc(rm);
+    __syncthreads();
+    int before = 0, tot = 0;
+#pragma unroll
+    for (int k = 0; k < DT_THREADS / 32; k++) {
+        if (k < wid) before += s_wcnt[k];
+        tot += s_wcnt[k];
+    }
+    if (threadIdx.x == 0 && tot) s_base = atomicAdd(A.D.counts + 7, tot);
+    __syncthreads();
+    if (rest) A.D.rest[s_base + before + __popc(rm & ((1u << lane) - 1u))] = j;
 }
 
 // lists of the branches' own pixels, inside their raw object's range (in any
@@ -944,50 +1121,51 @@ __global__ void k_da_finish(const __grid_constant__ DebArgs A) {
 // less than 2^-23 of 1 + |offset|, so the quadratic form, of terms that add up
 // to T, by less than 2e-6 (T + the coefficients' sum).
 __global__ void __launch_bounds__(DT_THREADS) k_da_gather(const __grid_constant__ DebArgs A) {
-    const int j = blockIdx.x * DT_THREADS + threadIdx.x;
-    const int n = sx_count(A.nrootpix, A.nrootpix_dev);
-    if (blockIdx.x * DT_THREADS >= n) return;
-    int o = -1, x = 0, y = 0;
-    if (j < n && (int)A.objkey[j] < 0) {
-        const int r = (int)A.rid[j], K = A.R.nkept[r], ob = A.R.objbase[r];
-        const int p = (int)A.rpix[j];
-        y = (int)fdiv((unsigned)p, A.wdiv);
-        x = p - y * A.w;
-        int iclst = 0;
-        float distmin = 1e+31f;
-        for (int i = 0; i < K; i++) {
-            const int q = ob + i;
-            const int4 g0 = __ldg(reinterpret_cast<const int4 *>(A.gobj + q));
-            const float4 g1 = __ldg(reinterpret_cast<const float4 *>(A.gobj + q) + 1);
-            const float abc = g1.w;
-            {
-                const float ux = (float)(x - g0.x) - __int_as_float(g0.z), uy = (float)(y - g0.y) - __int_as_float(g0.w);
-                const float qx = g1.x * ux * ux, qy = g1.y * uy * uy, qc = g1.z * ux * uy;
-                const float f = qx + qy + qc - 2e-6f * (fabsf(qx) + fabsf(qy) + fabsf(qc) + fabsf(g1.x) + fabsf(g1.y) +
-                                                        fabsf(g1.z) * (1.0f + fabsf(ux) + fabsf(uy)));
-                if (f > 1e-30f && abc > 0.0f && 0.499999f * f > distmin * abc) continue;
+    const int n = A.D.counts[7], nround = (n + 31) & ~31;
+    for (int i0 = blockIdx.x * DT_THREADS + threadIdx.x; i0 < nround; i0 += gridDim.x * DT_THREADS) {
+        int o = -1, x = 0, y = 0;
+        if (i0 < n) {
+            const int j = A.D.rest[i0];
+            const int r = (int)A.rid[j], K = A.R.nkept[r], ob = A.R.objbase[r];
+            const int p = (int)A.rpix[j];
+            y = (int)fdiv((unsigned)p, A.wdiv);
+            x = p - y * A.w;
+            int iclst = 0;
+            float distmin = 1e+31f;
+            for (int i = 0; i < K; i++) {
+                const int q = ob + i;
+                const int4 g0 = __ldg(reinterpret_cast<const int4 *>(A.gobj + q));
+                const float4 g1 = __ldg(reinterpret_cast<const float4 *>(A.gobj + q) + 1);
+                const float abc = g1.w;
+                {
+                    const float ux = (float)(x - g0.x) - __int_as_float(g0.z), uy = (float)(y - g0.y) - __int_as_float(g0.w);
+                    const float qx = g1.x * ux * ux, qy = g1.y * uy * uy, qc = g1.z * ux * uy;
+                    const float f = qx + qy + qc - 2e-6f * (fabsf(qx) + fabsf(qy) + fabsf(qc) + fabsf(g1.x) + fabsf(g1.y) +
+                                                            fabsf(g1.z) * (1.0f + fabsf(ux) + fabsf(uy)));
+                    if (f > 1e-30f && abc > 0.0f && 0.499999f * f > distmin * abc) continue;
+                }
+                const float dx = x - __ldg(A.O.mx + q), dy = y - __ldg(A.O.my + q);
+                const float dist = 0.5 * (g1.x * dx * dx + g1.y * dy * dy + g1.z * dx * dy) / abc;
+                if (dist < distmin) {
+                    distmin = dist;
+                    iclst = i;
+                }
             }
-            const float dx = x - __ldg(A.O.mx + q), dy = y - __ldg(A.O.my + q);
-            const float dist = 0.5 * (g1.x * dx * dx + g1.y * dy * dy + g1.z * dx * dy) / abc;
-            if (dist < distmin) {
-                distmin = dist;
-                iclst = i;
-            }
+            o = ob + iclst;
+            A.alloc[p] = o;
         }
-        o = ob + iclst;
-        A.alloc[p] = o;
-    }
-    // the objects grow by them: their pixel counts and boxes
-    const unsigned grp = __match_any_sync(0xffffffffu, o);
-    if (o < 0) return;
-    const int x0 = __reduce_min_sync(grp, x), x1 = __reduce_max_sync(grp, x);
-    const int y0 = __reduce_min_sync(grp, y), y1 = __reduce_max_sync(grp, y);
-    if ((int)(threadIdx.x & 31) == __ffs(grp) - 1) {
-        atomicAdd(A.O.n + o, __popc(grp));
-        if (x0 < A.O.xmin[o]) atomicMin(A.O.xmin + o, x0);
-        if (x1 > A.O.xmax[o]) atomicMax(A.O.xmax + o, x1);
-        if (y0 < A.O.ymin[o]) atomicMin(A.O.ymin + o, y0);
-        if (y1 > A.O.ymax[o]) atomicMax(A.O.ymax + o, y1);
+        // the objects grow by them: their pixel counts and boxes
+        const unsigned grp = __match_any_sync(0xffffffffu, o);
+        if (o < 0) continue;
+        const int x0 = __reduce_min_sync(grp, x), x1 = __reduce_max_sync(grp, x);
+        const int y0 = __reduce_min_sync(grp, y), y1 = __reduce_max_sync(grp, y);
+        if ((int)(threadIdx.x & 31) == __ffs(grp) - 1) {
+            atomicAdd(A.O.n + o, __popc(grp));
+            if (x0 < A.O.xmin[o]) atomicMin(A.O.xmin + o, x0);
+            if (x1 > A.O.xmax[o]) atomicMax(A.O.xmax + o, x1);
+            if (y0 < A.O.ymin[o]) atomicMin(A.O.ymin + o, y0);
+            if (y1 > A.O.ymax[o]) atomicMax(A.O.ymax + o, y1);
+        }
     }
 }
 
@@ -1027,7 +1205,7 @@ int launch_deblend_tree(const DebArgs &A, cudaStream_t st) {
     k_dt_cut_warp<<<dt_grid((A.nroots + DT_CUT_WARPS - 1) / DT_CUT_WARPS, 8), DT_CUT_WARPS * 32, 0, st>>>(A);
     k_dt_cut_block<256><<<dt_grid(A.nroots, 4), 256, dt_smem(DT_MID_PEAKS), st>>>(A, 1, DT_MID_PEAKS);
     k_dt_cut_block<512><<<dt_grid(A.nroots, 1), 512, dt_smem(DT_BIG_PEAKS), st>>>(A, 2, DT_BIG_PEAKS);
-    k_dt_cut_huge<<<dt_grid(A.nroots, 1), DT_HUGE_THREADS, 0, st>>>(A);
+    k_dt_cut_huge<<<(unsigned)std::min((long long)A.nroots, 8ll) * DT_HUGE_BLOCKS, DT_HUGE_THREADS, 0, st>>>(A);
     k_dt_rank<<<dt_grid(A.nrootpix / DT_THREADS + 1, 4), DT_THREADS, 0, st>>>(A);
     return 12;
 }
@@ -1044,7 +1222,7 @@ int launch_deblend_assign(const DebArgs &A, cudaStream_t st) {
     k_da_moments<<<gw, DT_THREADS, 0, st>>>(A);
     k_da_moments_big<<<dt_grid(A.nobj, 2), DT_THREADS, 0, st>>>(A);
     k_da_finish<<<go, DT_THREADS, 0, st>>>(A);
-    k_da_gather<<<gp, DT_THREADS, 0, st>>>(A);
+    k_da_gather<<<dt_grid(gp, 8), DT_THREADS, 0, st>>>(A);
     return 8;
 }
 

@@ -47,6 +47,7 @@ struct DebBufs {
     unsigned long long *acc;            // flux limbs
     int *olev;                          // kept branches in order: level
     unsigned *ownpix;                   // the branches' own pixels
+    int *rest;                          // elements no branch owns
     // the same, for the raw objects whose joins are taken in global memory
     unsigned long long *kept, *g_evm;
     int *krep, *g_b0, *g_par, *g_nson, *g_label, *g_flags, *g_dlist, *g_elist;
@@ -56,8 +57,8 @@ struct DebBufs {
     int *biglist;                       // objects whose pixels a whole block sums
 };
 // raw objects of at most this many peaks: joins taken by one warp, a block of
-// 256 threads, a block of 512 (state in shared memory); more: a block of 1024
-// on global memory
+// 256 threads, a block of 512 (state in shared memory); more: a cluster of
+// blocks on global memory
 constexpr int DT_WARP_PEAKS = 32;
 constexpr int DT_MID_PEAKS = 320;
 constexpr int DT_BIG_PEAKS = 1536;

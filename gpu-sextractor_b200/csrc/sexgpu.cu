@@ -153,7 +153,7 @@ struct sexgpu_ctx {
     DevBuf rsize, roff, rnkept, robjbase, rdthr, rathr, rzero, rlists, rthr;
     // deblend scratch
     DevBuf objkey, rpix;
-    enum { D_UP, D_LEV, D_REC, D_EVM, D_BOFF, D_PIDX, D_KOWN, D_PEAKS, D_PLIST, D_BSZ, D_BMIN, D_ACC, D_OLEV, D_OWNPIX,
+    enum { D_UP, D_LEV, D_REC, D_EVM, D_BOFF, D_PIDX, D_KOWN, D_PEAKS, D_PLIST, D_BSZ, D_BMIN, D_ACC, D_OLEV, D_OWNPIX, D_REST,
            D_KEPT, D_GEVM, D_KREP, D_GB0, D_GPAR, D_GNSON, D_GLABEL, D_GFLAGS, D_GDLIST, D_GELIST, D_GM, D_COUNT };
     DevBuf deb;  // all of them
     // objects
@@ -769,7 +769,7 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     int rc = SEXGPU_OK;
     // ---- deblending
     static const size_t elem[sexgpu_ctx::D_COUNT] = {
-        4, 1, 8, 8, 4, 4, 8, 4, 4, 4, 4, 8 * DT_LIMBS, 4, 4, 8, 8, 4, 4, 4, 4, 4, 4, 4, 4, 1};
+        4, 1, 8, 8, 4, 4, 8, 4, 4, 4, 4, 8 * DT_LIMBS, 4, 4, 4, 8, 8, 4, 4, 4, 4, 4, 4, 4, 4, 1};
     const size_t M = (size_t)nrootpix + 1, NR = (size_t)nroots + 1;
     size_t at[sexgpu_ctx::D_COUNT], bytes = 0;
     for (int k = 0; k < sexgpu_ctx::D_COUNT; k++) {
@@ -811,6 +811,7 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     D.acc = reinterpret_cast<unsigned long long *>(deb + at[sexgpu_ctx::D_ACC]);
     D.olev = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_OLEV]);
     D.ownpix = reinterpret_cast<unsigned *>(deb + at[sexgpu_ctx::D_OWNPIX]);
+    D.rest = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_REST]);
     D.kept = reinterpret_cast<unsigned long long *>(deb + at[sexgpu_ctx::D_KEPT]);
     D.g_evm = reinterpret_cast<unsigned long long *>(deb + at[sexgpu_ctx::D_GEVM]);
     D.krep = reinterpret_cast<int *>(deb + at[sexgpu_ctx::D_KREP]);
