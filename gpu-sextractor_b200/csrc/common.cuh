@@ -6,7 +6,38 @@
 #pragma once
 
 #include <cstdint>
+#include <utility>
 #include <cuda_runtime.h>
+
+// ---------------------------------------------------------------------------
+// Launches.  A frame is 70 short kernels in one stream, most of them a few
+// microseconds on small frames, each depending on the one before.  They are
+// launched with programmatic stream serialization: the next kernel's blocks are
+// set up while the current one drains, and wait for its end (sx_pdl, the first
+// statement of every kernel) before they touch anything.  The order of all
+// memory operations is that of the plain launches.  160 x 160 frame 0.64 ->
+// 0.53 ms, 1024 x 1024 through a captured graph 0.84 -> 0.74, 4096 x 4096 4.22
+// -> 4.10.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void sx_pdl() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline void sx_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
 
 #define SX_BIG 1e+30
 // blank (NaN) input pixels read as -BIG, like the FITS reader's blank value

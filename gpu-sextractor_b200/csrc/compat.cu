@@ -56,6 +56,7 @@ bool compat_ready(const char *what, int stage) {
 }
 
 __global__ void k_compat_thresholds(FrameScalars *sc, float dthresh, float thresh) {
+    sx_pdl();
     sc->dthresh = dthresh;
     sc->thresh = thresh;
     sc->e0cd = fexpo(dthresh);
@@ -63,6 +64,7 @@ __global__ void k_compat_thresholds(FrameScalars *sc, float dthresh, float thres
 
 // one record per object, in object index order
 __global__ void k_compat_rows(ObjBufs O, int n, sexgpu_outobj *rows) {
+    sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= n) return;
     sexgpu_outobj q;
@@ -223,7 +225,7 @@ void run_detection(float dthresh, float thresh, int minarea, size_t *numValidObj
         compat_fail("run_detection", rc);
         return;
     }
-    k_compat_thresholds<<<1, 1, 0, ctx->stream>>>(P<FrameScalars>(ctx->sc), dthresh, thresh);
+    sx_launch(k_compat_thresholds, 1, 1, 0, ctx->stream, P<FrameScalars>(ctx->sc), dthresh, thresh);
     rc = pipe_detect(ctx);
     if (rc) {
         compat_fail("run_detection", rc);
@@ -345,7 +347,8 @@ void endobject_gpu(void *prefs, void *brain, void *flagobj2, sexgpu_outobj *outo
     if (!rc && numobj > 0) {
         rc = ensure(ctx, ctx->rows, (size_t)numobj * sizeof(sexgpu_outobj));
         if (!rc) {
-            k_compat_rows<<<grid1(numobj, 128), 128, 0, ctx->stream>>>(ctx->O, numobj, P<sexgpu_outobj>(ctx->rows));
+            sx_launch(k_compat_rows, grid1(numobj, 128), 128, 0, ctx->stream, ctx->O, numobj,
+                      P<sexgpu_outobj>(ctx->rows));
             if (outobj &&
                 cudaMemcpyAsync(outobj, ctx->rows.p, (size_t)numobj * sizeof(sexgpu_outobj), cudaMemcpyDeviceToHost,
                                 ctx->stream) != cudaSuccess)

@@ -126,6 +126,7 @@ struct AnaArgs {
 // correction are finished by k_robust_finish, one thread per object, so that
 // the double-precision tail does not run on one lane of a warp.
 __global__ void __launch_bounds__(AN_WARPS * 32, 3) k_analyse_robust(AnaArgs A) {
+    sx_pdl();
     const int lane = threadIdx.x & 31;
     const int o = blockIdx.x * AN_WARPS + (threadIdx.x >> 5);
     if (o >= sx_count(A.nobj, A.nobj_dev) || A.O.level[o] == 0) return;
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(AN_WARPS * 32, 3) k_analyse_robust(AnaArgs A) 
 }
 
 __global__ void __launch_bounds__(AN_WARPS * 32, 2) k_analyse_robust_big(AnaArgs A) {
+    sx_pdl();
     __shared__ PixBlock sh;
     const int nb = A.counts[5];
     for (int i = blockIdx.x; i < nb; i += gridDim.x) {
@@ -147,6 +149,7 @@ __global__ void __launch_bounds__(AN_WARPS * 32, 2) k_analyse_robust_big(AnaArgs
 }
 
 __global__ void k_robust_finish(AnaArgs A) {
+    sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(A.nobj, A.nobj_dev) || A.O.level[o] == 0) return;
     const MomentRaw R = A.raw[o];
@@ -243,6 +246,7 @@ __device__ __noinline__ void exam_xsum(const AnaArgs &A, const unsigned *pix, in
 // examineiso (src/cuda/cudaanalyse.cu:2176-2581) and the CLEAN threshold
 // mthresh of every object.
 __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A) {
+    sx_pdl();
     __shared__ __align__(16) unsigned hist[AN_WARPS][256];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int o = blockIdx.x * AN_WARPS + wid;
@@ -431,6 +435,7 @@ __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A
 // (one thread per object, so that this double-precision tail does not run on
 // one lane of a warp)
 __global__ void k_examine_finish(AnaArgs A) {
+    sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(A.nobj, A.nobj_dev)) return;
     const ExamRaw X = A.xraw[o];
@@ -553,6 +558,7 @@ struct ListArgs {
 };
 
 __global__ void __launch_bounds__(OL_THREADS) k_obj_lists(const ListArgs A) {
+    sx_pdl();
     const int lane = threadIdx.x & 31, o = (blockIdx.x * OL_THREADS + threadIdx.x) >> 5;
     if (o >= sx_count(A.nobj, A.nobj_dev)) return;
     const int x0 = A.O.xmin[o], y0 = A.O.ymin[o], bw = A.O.xmax[o] - x0 + 1, bh = A.O.ymax[o] - y0 + 1;
@@ -596,6 +602,7 @@ __global__ void __launch_bounds__(OL_THREADS) k_obj_lists(const ListArgs A) {
 }
 
 __global__ void __launch_bounds__(OL_THREADS) k_obj_list_count(const ListArgs A) {
+    sx_pdl();
     __shared__ int s_n;
     const int n = min(*A.nitems, OL_ITEMS);
     for (int c = blockIdx.x; c < n; c += gridDim.x) {
@@ -616,6 +623,7 @@ __global__ void __launch_bounds__(OL_THREADS) k_obj_list_count(const ListArgs A)
 }
 
 __global__ void __launch_bounds__(OL_THREADS) k_obj_list_write(const ListArgs A) {
+    sx_pdl();
     __shared__ int s_base, s_warp[2][OL_THREADS / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int n = min(*A.nitems, OL_ITEMS);
@@ -654,28 +662,26 @@ __global__ void __launch_bounds__(OL_THREADS) k_obj_list_write(const ListArgs A)
 int launch_obj_lists(const ListArgs &A, cudaStream_t st) {
     if (A.nobj <= 0) return 0;
     const unsigned per = OL_THREADS / 32;
-    k_obj_lists<<<(A.nobj + per - 1) / per, OL_THREADS, 0, st>>>(A);
-    k_obj_list_count<<<dt_grid(A.nobj, 4), OL_THREADS, 0, st>>>(A);
-    k_obj_list_write<<<dt_grid(A.nobj, 4), OL_THREADS, 0, st>>>(A);
+    sx_launch(k_obj_lists, (A.nobj + per - 1) / per, OL_THREADS, 0, st, A);
+    sx_launch(k_obj_list_count, dt_grid(A.nobj, 4), OL_THREADS, 0, st, A);
+    sx_launch(k_obj_list_write, dt_grid(A.nobj, 4), OL_THREADS, 0, st, A);
     return 3;
 }
 
 void launch_analyse(const AnaArgs &A, cudaStream_t st) {
     if (A.nobj <= 0) return;
     const unsigned grid = (A.nobj + AN_WARPS - 1) / AN_WARPS;
-    k_analyse_robust<<<grid, AN_WARPS * 32, 0, st>>>(A);
-    k_analyse_robust_big<<<dt_grid(A.nobj, 2), AN_WARPS * 32, 0, st>>>(A);
-    k_robust_finish<<<(unsigned)((A.nobj + 127) / 128), 128, 0, st>>>(A);
+    sx_launch(k_analyse_robust, grid, AN_WARPS * 32, 0, st, A);
+    sx_launch(k_analyse_robust_big, dt_grid(A.nobj, 2), AN_WARPS * 32, 0, st, A);
+    sx_launch(k_robust_finish, (unsigned)((A.nobj + 127) / 128), 128, 0, st, A);
     if (A.O.dbkg) {
-        k_local_stat<<<(unsigned)((A.nobj + GW_WARPS - 1) / GW_WARPS), 32 * GW_WARPS, 0, st>>>(
-            A.sub, A.w, A.h, A.bp_thick, A.O.xmin, A.O.xmax, A.O.ymin, A.O.ymax, A.nobj, A.nobj_dev, A.O.lstat,
-            A.O.dbkg);
-        k_local_guess<<<(unsigned)A.nobj, GUESS_THREADS, 0, st>>>(A.sub, A.w, A.h, A.bp_thick, A.O.xmin, A.O.xmax,
-                                                                   A.O.ymin, A.O.ymax, A.nobj, A.nobj_dev, A.O.lstat,
-                                                                   A.O.dbkg);
+        sx_launch(k_local_stat, (unsigned)((A.nobj + GW_WARPS - 1) / GW_WARPS), 32 * GW_WARPS, 0, st, A.sub, A.w,
+                  A.h, A.bp_thick, A.O.xmin, A.O.xmax, A.O.ymin, A.O.ymax, A.nobj, A.nobj_dev, A.O.lstat, A.O.dbkg);
+        sx_launch(k_local_guess, (unsigned)A.nobj, GUESS_THREADS, 0, st, A.sub, A.w, A.h, A.bp_thick, A.O.xmin,
+                  A.O.xmax, A.O.ymin, A.O.ymax, A.nobj, A.nobj_dev, A.O.lstat, A.O.dbkg);
     }
-    k_examineiso<<<grid, AN_WARPS * 32, 0, st>>>(A);
-    k_examine_finish<<<(unsigned)((A.nobj + 127) / 128), 128, 0, st>>>(A);
+    sx_launch(k_examineiso, grid, AN_WARPS * 32, 0, st, A);
+    sx_launch(k_examine_finish, (unsigned)((A.nobj + 127) / 128), 128, 0, st, A);
 }
 
 }  // namespace sx

@@ -288,6 +288,7 @@ __device__ __forceinline__ void mesh_geometry(int m, int w, int h, int bw, int b
 template <bool VEC>
 __global__ void __launch_bounds__(32) k_mesh_stat(const float *__restrict__ img, int w, int h, int bw, int bh, int nbx,
                                                   int nby, MeshStat *__restrict__ ms) {
+    sx_pdl();
     __shared__ __align__(16) float stage[32 * SEQ_PITCH];
     const int m = blockIdx.x;
     int x0, y0, mw, mh, nv;
@@ -413,6 +414,7 @@ __global__ void __launch_bounds__(GUESS_THREADS) k_mesh_guess(const float *__res
                                                                 int bh, int nbx, int nby,
                                                                 const MeshStat *__restrict__ ms,
                                                                 float *__restrict__ back, float *__restrict__ sig) {
+    sx_pdl();
     __shared__ int hist[SX_QUANTIF_NMAXLEVELS + 2];
     __shared__ int pfx[SX_QUANTIF_NMAXLEVELS + 2];   // pfx[i] = sum_{k<i} hist[k]
     int m = blockIdx.x;
@@ -637,6 +639,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(32 * GW_WARPS) k_mesh_mode(const float *__restrict__ img, int w, int h, int bw, int bh,
                                                              int nbx, int nby, float *__restrict__ back,
                                                              float *__restrict__ sig) {
+    sx_pdl();
     __shared__ GuessWarpSmem smem[GW_WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int m = blockIdx.x * GW_WARPS + wid;
@@ -749,6 +752,7 @@ __global__ void __launch_bounds__(32 * GW_WARPS) k_local_stat(const float *__res
                                                               const int *__restrict__ ymin,
                                                               const int *__restrict__ ymax, int n, const int *n_dev,
                                                               MeshStat *__restrict__ ls, float *__restrict__ dbkg) {
+    sx_pdl();
     __shared__ GuessWarpSmem smem[GW_WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int o = blockIdx.x * GW_WARPS + wid;
@@ -786,6 +790,7 @@ __global__ void __launch_bounds__(GUESS_THREADS) k_local_guess(const float *__re
                                                                  const int *__restrict__ ymax, int n,
                                                                  const int *n_dev,
                                                                  const MeshStat *__restrict__ ls, float *dbkg) {
+    sx_pdl();
     __shared__ int hist[SX_QUANTIF_NMAXLEVELS + 2];
     __shared__ int pfx[SX_QUANTIF_NMAXLEVELS + 2];
     const int o = blockIdx.x;
@@ -825,6 +830,7 @@ __global__ void __launch_bounds__(GUESS_THREADS) k_local_guess(const float *__re
 // Writes back2 (all meshes) and fixes sigma in place for bad meshes.
 __global__ void k_mesh_badfill(const float *__restrict__ back, float *__restrict__ sigma, float *__restrict__ back2,
                                int nx, int ny) {
+    sx_pdl();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nx * ny) return;
     float b = back[i];
@@ -869,6 +875,7 @@ __device__ __forceinline__ float median_small(float *v, int n) {
 __global__ void k_mesh_median(const float *__restrict__ back, const float *__restrict__ sigma,
                               float *__restrict__ back3, float *__restrict__ sigma3, int nx, int ny, int npx,
                               int npy, float fthresh) {
+    sx_pdl();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nx * ny) return;
     int px = i % nx, py = i / nx;
@@ -986,6 +993,7 @@ __device__ float median_of(const float *v, int m, int n, unsigned lowkey, unsign
 __global__ void k_back_medians(const float *__restrict__ back3, const float *__restrict__ sigma3, int nb,
                                FrameScalars *sc, int back_type, float back_value, int thresh_type,
                                double dthr, double athr) {
+    sx_pdl();
     __shared__ unsigned hist[256];
     __shared__ unsigned s_npos;
     if (blockIdx.x == 0) {
@@ -1039,6 +1047,7 @@ constexpr int SPL_MAX = 768;   // longest line kept there; longer ones use the g
 // of the columns longer than SPL_MAX
 __global__ void __launch_bounds__(32) k_back_spline(const float *__restrict__ map, float *__restrict__ dmap,
                                                     float *__restrict__ u, int nbx, int nby) {
+    sx_pdl();
     extern __shared__ float spl[];
     const int x = blockIdx.x * 32 + threadIdx.x;
     if (x >= nbx) return;
@@ -1076,6 +1085,7 @@ __global__ void __launch_bounds__(32) k_back_spline(const float *__restrict__ ma
 __global__ void k_rms_map(const float *__restrict__ node, const float *__restrict__ dnode, const int *__restrict__ colk,
                           const float *__restrict__ coldx, int nbx, int w, long long n, float *__restrict__ out,
                           int square) {
+    sx_pdl();
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const int y = (int)(p / w), x = (int)(p - (long long)y * w);
@@ -1128,6 +1138,7 @@ __global__ void __launch_bounds__(SPL_THREADS) k_row_nodes(const float *__restri
                                                            const float *__restrict__ dback, int nbx, int nby,
                                                            int backh, int h, float *__restrict__ node,
                                                            float *__restrict__ dnode) {
+    sx_pdl();
     extern __shared__ float spl[];  // SPL_ROWS x (nbx | 1) nodes, as many u, the d of every column
     const int y0 = blockIdx.x * SPL_ROWS, rows = min(SPL_ROWS, h - y0), pitch = nbx | 1;
     float *su = spl + SPL_ROWS * pitch, *sd = su + SPL_ROWS * pitch;
@@ -1174,6 +1185,7 @@ __global__ void __launch_bounds__(SPL_THREADS) k_row_nodes(const float *__restri
 __global__ void k_row_nodes_long(const float *__restrict__ back, const float *__restrict__ dback, int nbx, int nby,
                                  int backh, int h, float *__restrict__ node, float *__restrict__ dnode,
                                  float *__restrict__ u) {
+    sx_pdl();
     const int y = blockIdx.x * blockDim.x + threadIdx.x;
     if (y >= h) return;
     float *nd = node + (size_t)y * nbx, *dnd = dnode + (size_t)y * nbx, *uu = u + (size_t)y * nbx;
@@ -1214,12 +1226,12 @@ void launch_map_nodes(const float *map, float *dmap, float *u, int nbx, int nby,
         return 1;
     });
     const size_t sb = nby <= SPL_MAX ? (size_t)64 * nby * 4 : 0;
-    k_back_spline<<<(nbx + 31) / 32, 32, sb, st>>>(map, dmap, u, nbx, nby);
+    sx_launch(k_back_spline, (nbx + 31) / 32, 32, sb, st, map, dmap, u, nbx, nby);
     if (nbx <= SPL_MAX)
-        k_row_nodes<<<(h + SPL_ROWS - 1) / SPL_ROWS, SPL_THREADS, (size_t)(2 * SPL_ROWS + 1) * (nbx | 1) * 4, st>>>(
-            map, dmap, nbx, nby, bh, h, node, dnode);
+        sx_launch(k_row_nodes, (h + SPL_ROWS - 1) / SPL_ROWS, SPL_THREADS, (size_t)(2 * SPL_ROWS + 1) * (nbx | 1) *
+                  4, st, map, dmap, nbx, nby, bh, h, node, dnode);
     else
-        k_row_nodes_long<<<(h + 127) / 128, 128, 0, st>>>(map, dmap, nbx, nby, bh, h, node, dnode, rowu);
+        sx_launch(k_row_nodes_long, (h + 127) / 128, 128, 0, st, map, dmap, nbx, nby, bh, h, node, dnode, rowu);
 }
 
 // ---------------------------------------------------------------------------
@@ -1228,6 +1240,7 @@ void launch_map_nodes(const float *map, float *dmap, float *u, int nbx, int nby,
 // ---------------------------------------------------------------------------
 __global__ void k_weight_mask(const float *__restrict__ img, const float *__restrict__ wmap, int wtype,
                               float *__restrict__ imgm, long long n) {
+    sx_pdl();
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p < n) imgm[p] = sx_rel_var(__ldg(wmap + p), wtype) < 1e30f ? __ldg(img + p) : -1e30f;
 }
@@ -1236,6 +1249,7 @@ __global__ void k_weight_mask(const float *__restrict__ img, const float *__rest
 // pixels; ratio = mesh rms / sqrt(mean) for a usable mesh, -1 otherwise
 __global__ void k_weight_ratio(const float *__restrict__ wmap, int wtype, int w, int h, int bw, int bh, int nbx,
                                int nby, const float *__restrict__ sigma, float *__restrict__ ratio) {
+    sx_pdl();
     const int lane = threadIdx.x & 31;
     const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (m >= nbx * nby) return;
@@ -1268,6 +1282,7 @@ __global__ void k_weight_ratio(const float *__restrict__ wmap, int wtype, int w,
 
 // sigfac: median of the usable meshes' ratios (hmedian, src/misc.c:30), 1 if none
 __global__ void k_weight_sigfac(const float *__restrict__ ratio, int nb, FrameScalars *sc) {
+    sx_pdl();
     __shared__ unsigned hist[256];
     __shared__ unsigned s_npos;
     if (threadIdx.x == 0) s_npos = 0;
@@ -1285,13 +1300,14 @@ __global__ void k_weight_sigfac(const float *__restrict__ ratio, int nb, FrameSc
 
 __global__ void k_weight_var(const float *__restrict__ wmap, int wtype, const FrameScalars *sc,
                              float *__restrict__ wvar, long long n) {
+    sx_pdl();
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const float sigfac = sc->sigfac, sigfac2 = sigfac * sigfac;
     if (p < n) wvar[p] = sx_calib_var(__ldg(wmap + p), wtype, sigfac2);
 }
 
 void launch_weight_mask(const float *img, const float *wmap, int wtype, float *imgm, long long n, cudaStream_t st) {
-    if (n > 0) k_weight_mask<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(img, wmap, wtype, imgm, n);
+    if (n > 0) sx_launch(k_weight_mask, (unsigned)((n + 255) / 256), 256, 0, st, img, wmap, wtype, imgm, n);
 }
 
 // after launch_background: sigfac from the filtered mesh rms map, then the
@@ -1301,11 +1317,11 @@ void launch_weight_var(const BackBufs &B, const float *wmap, const FrameParams &
     const int nb = P.nbx * P.nby;
     const long long n = (long long)P.w * P.h;
     if (P.wtype != 2) {
-        k_weight_ratio<<<(nb + 3) / 4, 128, 0, st>>>(wmap, P.wtype, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.sigma3,
-                                                     ratio);
-        k_weight_sigfac<<<1, 1024, 0, st>>>(ratio, nb, d_sc);
+        sx_launch(k_weight_ratio, (nb + 3) / 4, 128, 0, st, wmap, P.wtype, P.w, P.h, P.bw, P.bh, P.nbx, P.nby,
+                  B.sigma3, ratio);
+        sx_launch(k_weight_sigfac, 1, 1024, 0, st, ratio, nb, d_sc);
     }
-    k_weight_var<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(wmap, P.wtype, d_sc, wvar, n);
+    sx_launch(k_weight_var, (unsigned)((n + 255) / 256), 256, 0, st, wmap, P.wtype, d_sc, wvar, n);
 }
 
 void launch_background(BackBufs &B, const float *img, const FrameParams &P, FrameScalars *d_sc,
@@ -1316,22 +1332,25 @@ void launch_background(BackBufs &B, const float *img, const FrameParams &P, Fram
     if ((long long)P.bw * P.bh < 65536) {
         const unsigned g = (unsigned)((nb + GW_WARPS - 1) / GW_WARPS);
         if (vec)
-            k_mesh_mode<true><<<g, 32 * GW_WARPS, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.back, B.sigma);
+            sx_launch(k_mesh_mode<true>, g, 32 * GW_WARPS, 0, st, img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.back,
+                      B.sigma);
         else
-            k_mesh_mode<false><<<g, 32 * GW_WARPS, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.back, B.sigma);
+            sx_launch(k_mesh_mode<false>, g, 32 * GW_WARPS, 0, st, img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.back,
+                      B.sigma);
     } else {
         if (vec)
-            k_mesh_stat<true><<<nb, 32, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms);
+            sx_launch(k_mesh_stat<true>, nb, 32, 0, st, img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms);
         else
-            k_mesh_stat<false><<<nb, 32, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms);
-        k_mesh_guess<<<nb, GUESS_THREADS, 0, st>>>(img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms, B.back, B.sigma);
+            sx_launch(k_mesh_stat<false>, nb, 32, 0, st, img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms);
+        sx_launch(k_mesh_guess, nb, GUESS_THREADS, 0, st, img, P.w, P.h, P.bw, P.bh, P.nbx, P.nby, B.ms, B.back,
+                  B.sigma);
         launches += 1;
     }
-    k_mesh_badfill<<<(nb + 127) / 128, 128, 0, st>>>(B.back, B.sigma, B.back2, P.nbx, P.nby);
-    k_mesh_median<<<(nb + 127) / 128, 128, 0, st>>>(B.back2, B.sigma, B.back3, B.sigma3, P.nbx, P.nby, P.nfx / 2,
-                                                   P.nfy / 2, P.fthresh);
-    k_back_medians<<<2, 1024, 0, st>>>(B.back3, B.sigma3, nb, d_sc, P.back_type, P.back_value, P.thresh_type,
-                                       P.detect_thresh, P.analysis_thresh);
+    sx_launch(k_mesh_badfill, (nb + 127) / 128, 128, 0, st, B.back, B.sigma, B.back2, P.nbx, P.nby);
+    sx_launch(k_mesh_median, (nb + 127) / 128, 128, 0, st, B.back2, B.sigma, B.back3, B.sigma3, P.nbx, P.nby, P.nfx /
+              2, P.nfy / 2, P.fthresh);
+    sx_launch(k_back_medians, 2, 1024, 0, st, B.back3, B.sigma3, nb, d_sc, P.back_type, P.back_value, P.thresh_type,
+              P.detect_thresh, P.analysis_thresh);
     launch_map_nodes(B.back3, B.dback, B.u, P.nbx, P.nby, P.bh, P.h, B.rownode, B.rowdnode, B.rowu, st);
     launches += 6;
 }

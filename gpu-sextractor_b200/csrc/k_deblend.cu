@@ -113,6 +113,7 @@ __device__ __forceinline__ void dt_join(unsigned long long *rec, const unsigned 
 // a weight map a pixel outside the object can, and then only the neighbours
 // with a list index count (pixels of two raw objects are never adjacent).
 __global__ void __launch_bounds__(DT_THREADS) k_dt_up(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     const bool in = j < sx_count(A.nrootpix, A.nrootpix_dev);
     bool peak = false;
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_up(const __grid_constant__ De
 // puts it on the list of its class: one peak (done here), up to 32 peaks (one
 // warp), more (blocks).
 __global__ void __launch_bounds__(DT_THREADS) k_dt_thresholds(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const long long t = (long long)blockIdx.x * DT_THREADS + threadIdx.x;
     const int r = (int)(t / A.N), i = (int)(t - (long long)r * A.N);
     if (r >= sx_count(A.nroots, A.nroots_dev)) return;
@@ -217,6 +219,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_thresholds(const __grid_const
 
 // level of every pixel (the highest threshold it reaches) and its peak
 __global__ void __launch_bounds__(DT_THREADS) k_dt_level(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     __shared__ unsigned s_lp;
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     const int n = sx_count(A.nrootpix, A.nrootpix_dev);
@@ -263,6 +266,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_level(const __grid_constant__
 // different peak once.  (Taking the four backward or forward neighbours each
 // at the lower level of the two meant twice as many walks.)
 __global__ void __launch_bounds__(DT_THREADS) k_dt_edges(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     if (dt_failed(A)) return;
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     if (j >= sx_count(A.nrootpix, A.nrootpix_dev)) return;
@@ -308,6 +312,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_edges(const __grid_constant__
 // each join straight to the representative of that level, which gets a bit
 // for it
 __global__ void __launch_bounds__(DT_THREADS) k_dt_flatten(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     if (dt_failed(A)) return;
     const int n = A.sc->npeaks;
     for (int i = blockIdx.x * DT_THREADS + threadIdx.x; i < n; i += gridDim.x * DT_THREADS) {
@@ -325,6 +330,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_flatten(const __grid_constant
 // raw object of P pixels has at most P of them (peaks are never adjacent, and
 // no more joins than peaks)
 __global__ void __launch_bounds__(DT_THREADS) k_dt_buckets(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     if (dt_failed(A)) return;
     const int n = A.sc->npeaks;
     for (int i = blockIdx.x * DT_THREADS + threadIdx.x; i < n; i += gridDim.x * DT_THREADS) {
@@ -348,6 +354,7 @@ constexpr int DT_FILL_RUNS = 12;
 // the warp in turn: the lanes of each doing so by themselves diverged, 201 us
 // instead of 150 for 7.1 M pixels)
 __global__ void __launch_bounds__(DT_THREADS) k_dt_fill(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     if (dt_failed(A)) return;
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     const int n = sx_count(A.nrootpix, A.nrootpix_dev);
@@ -672,6 +679,7 @@ __device__ __forceinline__ void dt_cut(const DebArgs &A, const int r, unsigned c
 // one warp per raw object of up to DT_WARP_PEAKS peaks
 constexpr int DT_CUT_WARPS = 4;
 __global__ void __launch_bounds__(DT_CUT_WARPS * 32) k_dt_cut_warp(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     if (dt_failed(A)) return;
     __shared__ __align__(16) unsigned char smem[DT_CUT_WARPS][dt_smem(DT_WARP_PEAKS)];
     __shared__ unsigned long long s_all[DT_CUT_WARPS][8];
@@ -683,6 +691,7 @@ __global__ void __launch_bounds__(DT_CUT_WARPS * 32) k_dt_cut_warp(const __grid_
 // one block per raw object of up to cap peaks
 template <int NT>
 __global__ void __launch_bounds__(NT) k_dt_cut_block(const __grid_constant__ DebArgs A, int list, int cap) {
+    sx_pdl();
     if (dt_failed(A)) return;
     extern __shared__ __align__(16) unsigned char dt_smem_buf[];
     __shared__ unsigned long long s_all[8];
@@ -730,6 +739,7 @@ __device__ __forceinline__ void dt_by_level(int i, int m, unsigned long long ev,
 
 __global__ void __cluster_dims__(DT_HUGE_BLOCKS, 1, 1) __launch_bounds__(DT_HUGE_THREADS)
     k_dt_cut_huge(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     namespace cg = cooperative_groups;
     __shared__ HugeShared s_own;
     __shared__ int s_nd[64], s_ne[64];  // this block's counts by level, then its next places
@@ -879,6 +889,7 @@ __global__ void __cluster_dims__(DT_HUGE_BLOCKS, 1, 1) __launch_bounds__(DT_HUGE
 // whole grid counts, one thread per branch (a cluster's raw object of 2 M
 // pixels keeps thousands)
 __global__ void __launch_bounds__(DT_THREADS) k_dt_rank(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     if (dt_failed(A)) return;
     const int nl = A.D.counts[3];
     for (int it = 0; it < nl; it++) {
@@ -898,6 +909,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_rank(const __grid_constant__ 
 
 // DEBLEND_NTHRESH 1: no level above the detection threshold
 __global__ void __launch_bounds__(DT_THREADS) k_dt_whole(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const int r = blockIdx.x * DT_THREADS + threadIdx.x;
     if (r >= sx_count(A.nroots, A.nroots_dev)) return;
     A.R.nkept[r] = 1;
@@ -912,6 +924,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_whole(const __grid_constant__
 // the branch's own pixels and O.npix the fill of that list until later stages
 // set them.
 __global__ void __launch_bounds__(DT_THREADS) k_da_objects(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const int lane = threadIdx.x & 31, r = (blockIdx.x * DT_THREADS + threadIdx.x) >> 5;
     if (r >= sx_count(A.nroots, A.nroots_dev)) return;
     const int K = A.R.nkept[r], ob = A.R.objbase[r], off = A.R.off[r], P = A.R.size[r];
@@ -938,6 +951,7 @@ __device__ __forceinline__ bool da_whole(const DebArgs &A, int r, int K) {
 // from where the previous one of the chain joined it); a kept branch (L,
 // peak) owns the pixel when the peak covers L on the chain.
 __global__ void __launch_bounds__(DT_THREADS) k_da_own(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     const int n = sx_count(A.nrootpix, A.nrootpix_dev);
     if (blockIdx.x * DT_THREADS >= n) return;
@@ -993,6 +1007,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_own(const __grid_constant__ D
 // lists of the branches' own pixels, inside their raw object's range (in any
 // order: every sum over them is exact)
 __global__ void __launch_bounds__(DT_THREADS) k_da_starts(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const int o = blockIdx.x * DT_THREADS + threadIdx.x;
     if (o >= sx_count(A.nobj, A.nobj_dev)) return;
     const int r = A.O.root[o], n = A.O.n[o];
@@ -1000,6 +1015,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_starts(const __grid_constant_
 }
 
 __global__ void __launch_bounds__(DT_THREADS) k_da_scatter(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const int j = blockIdx.x * DT_THREADS + threadIdx.x;
     const int n = sx_count(A.nrootpix, A.nrootpix_dev);
     if (blockIdx.x * DT_THREADS >= n) return;
@@ -1018,6 +1034,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_da_scatter(const __grid_constant
 // DA_WARP_MAX pixels; the ellipse is finished by k_da_finish, one thread per
 // object
 __global__ void __launch_bounds__(DT_THREADS, 3) k_da_moments(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const int o = (blockIdx.x * DT_THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (o >= sx_count(A.nobj, A.nobj_dev)) return;
     const int n = A.O.n[o];
@@ -1029,6 +1046,7 @@ __global__ void __launch_bounds__(DT_THREADS, 3) k_da_moments(const __grid_const
 }
 
 __global__ void __launch_bounds__(DT_THREADS, 2) k_da_moments_big(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     __shared__ PixBlock sh;
     const int nb = A.D.counts[4];
     for (int i = blockIdx.x; i < nb; i += gridDim.x) {
@@ -1038,6 +1056,7 @@ __global__ void __launch_bounds__(DT_THREADS, 2) k_da_moments_big(const __grid_c
 }
 
 __global__ void k_da_finish(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(A.nobj, A.nobj_dev)) return;
     const MomentRaw R = A.raw[o];
@@ -1121,6 +1140,7 @@ __global__ void k_da_finish(const __grid_constant__ DebArgs A) {
 // less than 2^-23 of 1 + |offset|, so the quadratic form, of terms that add up
 // to T, by less than 2e-6 (T + the coefficients' sum).
 __global__ void __launch_bounds__(DT_THREADS) k_da_gather(const __grid_constant__ DebArgs A) {
+    sx_pdl();
     const int n = A.D.counts[7], nround = (n + 31) & ~31;
     for (int i0 = blockIdx.x * DT_THREADS + threadIdx.x; i0 < nround; i0 += gridDim.x * DT_THREADS) {
         int o = -1, x = 0, y = 0;
@@ -1191,22 +1211,23 @@ int launch_deblend_tree(const DebArgs &A, cudaStream_t st) {
     const unsigned gp = (unsigned)((A.nrootpix + DT_THREADS - 1) / DT_THREADS);
     const unsigned gt = (unsigned)(((long long)A.nroots * A.N + DT_THREADS - 1) / DT_THREADS);
     const unsigned gk = dt_grid((A.nrootpix / 2 + DT_THREADS) / DT_THREADS, 8);
-    k_dt_up<<<gp, DT_THREADS, 0, st>>>(A);
-    k_dt_thresholds<<<gt, DT_THREADS, 0, st>>>(A);
-    k_dt_level<<<gp, DT_THREADS, 0, st>>>(A);
+    sx_launch(k_dt_up, gp, DT_THREADS, 0, st, A);
+    sx_launch(k_dt_thresholds, gt, DT_THREADS, 0, st, A);
+    sx_launch(k_dt_level, gp, DT_THREADS, 0, st, A);
     if (A.N < 2) {  // one level: every raw object is one branch
-        k_dt_whole<<<(A.nroots + DT_THREADS - 1) / DT_THREADS, DT_THREADS, 0, st>>>(A);
+        sx_launch(k_dt_whole, (A.nroots + DT_THREADS - 1) / DT_THREADS, DT_THREADS, 0, st, A);
         return 4;
     }
-    k_dt_edges<<<gp, DT_THREADS, 0, st>>>(A);
-    k_dt_flatten<<<gk, DT_THREADS, 0, st>>>(A);
-    k_dt_buckets<<<gk, DT_THREADS, 0, st>>>(A);
-    k_dt_fill<<<gp, DT_THREADS, 0, st>>>(A);
-    k_dt_cut_warp<<<dt_grid((A.nroots + DT_CUT_WARPS - 1) / DT_CUT_WARPS, 8), DT_CUT_WARPS * 32, 0, st>>>(A);
-    k_dt_cut_block<256><<<dt_grid(A.nroots, 4), 256, dt_smem(DT_MID_PEAKS), st>>>(A, 1, DT_MID_PEAKS);
-    k_dt_cut_block<512><<<dt_grid(A.nroots, 1), 512, dt_smem(DT_BIG_PEAKS), st>>>(A, 2, DT_BIG_PEAKS);
-    k_dt_cut_huge<<<(unsigned)std::min((long long)A.nroots, 8ll) * DT_HUGE_BLOCKS, DT_HUGE_THREADS, 0, st>>>(A);
-    k_dt_rank<<<dt_grid(A.nrootpix / DT_THREADS + 1, 4), DT_THREADS, 0, st>>>(A);
+    sx_launch(k_dt_edges, gp, DT_THREADS, 0, st, A);
+    sx_launch(k_dt_flatten, gk, DT_THREADS, 0, st, A);
+    sx_launch(k_dt_buckets, gk, DT_THREADS, 0, st, A);
+    sx_launch(k_dt_fill, gp, DT_THREADS, 0, st, A);
+    sx_launch(k_dt_cut_warp, dt_grid((A.nroots + DT_CUT_WARPS - 1) / DT_CUT_WARPS, 8), DT_CUT_WARPS * 32, 0, st, A);
+    sx_launch(k_dt_cut_block<256>, dt_grid(A.nroots, 4), 256, dt_smem(DT_MID_PEAKS), st, A, 1, DT_MID_PEAKS);
+    sx_launch(k_dt_cut_block<512>, dt_grid(A.nroots, 1), 512, dt_smem(DT_BIG_PEAKS), st, A, 2, DT_BIG_PEAKS);
+    sx_launch(k_dt_cut_huge, (unsigned)std::min((long long)A.nroots, 8ll) * DT_HUGE_BLOCKS, DT_HUGE_THREADS, 0, st,
+              A);
+    sx_launch(k_dt_rank, dt_grid(A.nrootpix / DT_THREADS + 1, 4), DT_THREADS, 0, st, A);
     return 12;
 }
 
@@ -1215,14 +1236,14 @@ int launch_deblend_assign(const DebArgs &A, cudaStream_t st) {
     const unsigned gp = (unsigned)((A.nrootpix + DT_THREADS - 1) / DT_THREADS);
     const unsigned go = (unsigned)((std::max(A.nobj, 1) + DT_THREADS - 1) / DT_THREADS);
     const unsigned gw = (unsigned)((std::max(A.nobj, 1) + DT_THREADS / 32 - 1) / (DT_THREADS / 32));
-    k_da_objects<<<(A.nroots + DT_THREADS / 32 - 1) / (DT_THREADS / 32), DT_THREADS, 0, st>>>(A);
-    k_da_own<<<gp, DT_THREADS, 0, st>>>(A);
-    k_da_starts<<<go, DT_THREADS, 0, st>>>(A);
-    k_da_scatter<<<gp, DT_THREADS, 0, st>>>(A);
-    k_da_moments<<<gw, DT_THREADS, 0, st>>>(A);
-    k_da_moments_big<<<dt_grid(A.nobj, 2), DT_THREADS, 0, st>>>(A);
-    k_da_finish<<<go, DT_THREADS, 0, st>>>(A);
-    k_da_gather<<<dt_grid(gp, 8), DT_THREADS, 0, st>>>(A);
+    sx_launch(k_da_objects, (A.nroots + DT_THREADS / 32 - 1) / (DT_THREADS / 32), DT_THREADS, 0, st, A);
+    sx_launch(k_da_own, gp, DT_THREADS, 0, st, A);
+    sx_launch(k_da_starts, go, DT_THREADS, 0, st, A);
+    sx_launch(k_da_scatter, gp, DT_THREADS, 0, st, A);
+    sx_launch(k_da_moments, gw, DT_THREADS, 0, st, A);
+    sx_launch(k_da_moments_big, dt_grid(A.nobj, 2), DT_THREADS, 0, st, A);
+    sx_launch(k_da_finish, go, DT_THREADS, 0, st, A);
+    sx_launch(k_da_gather, dt_grid(gp, 8), DT_THREADS, 0, st, A);
     return 8;
 }
 

@@ -42,6 +42,7 @@ __device__ __forceinline__ float bkg_at(int x, int y, const BackBufs &B, int nbx
 // image (src/readimage.c:114); backmean everywhere for an absolute background.
 __global__ void k_back_map(BackBufs B, int nbx, int back_type, const FrameScalars *sc, int w, long long n,
                            float *__restrict__ out) {
+    sx_pdl();
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const int y = (int)(p / w), x = (int)(p - (long long)y * w);
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(SF_TX *SF_TY) k_sub_filter(const float *__rest
                                                               const float *__restrict__ mask, int mw, int mh,
                                                               const float *__restrict__ wvar, int wthr, double dfac,
                                                               FrameScalars *sc) {
+    sx_pdl();
     extern __shared__ float tile[];
     const int rx = mw / 2, ry = mh / 2;
     const int TWp = SF_TW + mw - 1, THp = SF_TH + mh - 1;
@@ -250,6 +252,7 @@ template <int MW, int MH, bool WEIGHTED>
 __global__ void __launch_bounds__(ST_THREADS, 4) k_sub_filter_pipe(const __grid_constant__ CUtensorMap tmap,
                                                                 const __grid_constant__ SpArgs A,
                                                                 const __grid_constant__ ConvTaps taps) {
+    sx_pdl();
     extern __shared__ __align__(128) float sp_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
     __shared__ float s_nd[ST_MAXBH][SP_NK], s_dnd[ST_MAXBH][SP_NK];
@@ -553,7 +556,7 @@ bool launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const 
             slot.store(((long long)smem << 8) | per, std::memory_order_relaxed);                        \
         }                                                                                               \
         const int grid = std::max(1, std::min(A.ntiles, sx_share(nsm * per)));                         \
-        kern<<<grid, ST_THREADS, smem, st>>>(tmap, A, taps);                                            \
+        sx_launch(kern, grid, ST_THREADS, smem, st, tmap, A, taps);                                            \
     } while (0)
 #define SP_MASK(wt)                    \
     if (mw == mh && mw == 1)           \
@@ -583,8 +586,8 @@ bool launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const 
     dim3 grid((P.w + SF_TW - 1) / SF_TW, (P.h + SF_TH - 1) / SF_TH);
     dim3 block(SF_TX, SF_TY);
     size_t smem = sizeof(float) * (SF_TW + mw - 1) * (SF_TH + mh - 1);
-    k_sub_filter<<<grid, block, smem, st>>>(img, sub, cd, lab, B, P.w, P.h, P.nbx, P.back_type, M.dev, mw, mh, d_var,
-                                            P.wthr, P.detect_thresh, d_sc);
+    sx_launch(k_sub_filter, grid, block, smem, st, img, sub, cd, lab, B, P.w, P.h, P.nbx, P.back_type, M.dev, mw, mh,
+              d_var, P.wthr, P.detect_thresh, d_sc);
     launches += 1;
     return false;
 }
@@ -602,6 +605,7 @@ constexpr int CC_TW = 32, CC_TH = 16;
 // in shared memory.  Every link goes to a smaller tile index, so each tile
 // component ends at its smallest pixel.
 __global__ void __launch_bounds__(CC_TW *CC_TH) k_ccl_local(int *__restrict__ lab, int w, int h) {
+    sx_pdl();
     __shared__ int L[CC_TH * CC_TW];
     __shared__ unsigned rowm[CC_TH];
     const int lx = threadIdx.x, ly = threadIdx.y, t = ly * CC_TW + lx;
@@ -671,6 +675,7 @@ __device__ __forceinline__ void gunion(int *L, int a, int b, int *status, int lo
 // first/last column of a tile look at their backward neighbours in other tiles
 template <int TW, int TH>
 __global__ void k_ccl_border(int *__restrict__ lab, int w, int h, int *status, int loop_cap) {
+    sx_pdl();
     int tilesx = (w + TW - 1) / TW;
     int tile = blockIdx.x, k = threadIdx.x;           // k < TW + TH
     int tx0 = (tile % tilesx) * TW, ty0 = (tile / tilesx) * TH;
@@ -699,6 +704,7 @@ __global__ void k_ccl_border(int *__restrict__ lab, int w, int h, int *status, i
 // the last column of each tile also looks NE into the next tile (row y-1)
 template <int TW, int TH>
 __global__ void k_ccl_border_ne(int *__restrict__ lab, int w, int h, int *status, int loop_cap) {
+    sx_pdl();
     int tilesx = (w + TW - 1) / TW;
     int tile = blockIdx.x, k = threadIdx.x;  // k in [1, TH)
     if (k == 0 || k >= TH) return;
@@ -715,6 +721,7 @@ __global__ void k_ccl_border_ne(int *__restrict__ lab, int w, int h, int *status
 // writes) or the pixel's root, so a concurrent walk through it still reads an
 // ancestor (the walks only read).
 __global__ void k_ccl_flatten(int *__restrict__ lab, long long n, int *__restrict__ cnt, int *status, int loop_cap) {
+    sx_pdl();
     const long long base = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     const bool vec = base + 3 < n && (reinterpret_cast<uintptr_t>(lab) & 15) == 0;
     int l[4], r[4];
@@ -759,19 +766,19 @@ void launch_ccl(int *lab, int *cnt, const FrameParams &P, FrameScalars *d_sc, cu
     int *status = &d_sc->status;
     if (tiled) {
         const int ntiles = ((P.w + ST_TW - 1) / ST_TW) * ((P.h + ST_TH - 1) / ST_TH);
-        k_ccl_border<ST_TW, ST_TH><<<ntiles, ST_TW + ST_TH, 0, st>>>(lab, P.w, P.h, status, P.loop_cap);
-        k_ccl_border_ne<ST_TW, ST_TH><<<ntiles, ST_TH, 0, st>>>(lab, P.w, P.h, status, P.loop_cap);
+        sx_launch(k_ccl_border<ST_TW, ST_TH>, ntiles, ST_TW + ST_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
+        sx_launch(k_ccl_border_ne<ST_TW, ST_TH>, ntiles, ST_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
         launches += 3;
     } else {
         dim3 grid((P.w + CC_TW - 1) / CC_TW, (P.h + CC_TH - 1) / CC_TH);
-        k_ccl_local<<<grid, dim3(CC_TW, CC_TH), 0, st>>>(lab, P.w, P.h);
+        sx_launch(k_ccl_local, grid, dim3(CC_TW, CC_TH), 0, st, lab, P.w, P.h);
         const int ntiles = grid.x * grid.y;
-        k_ccl_border<CC_TW, CC_TH><<<ntiles, CC_TW + CC_TH, 0, st>>>(lab, P.w, P.h, status, P.loop_cap);
-        k_ccl_border_ne<CC_TW, CC_TH><<<ntiles, CC_TH, 0, st>>>(lab, P.w, P.h, status, P.loop_cap);
+        sx_launch(k_ccl_border<CC_TW, CC_TH>, ntiles, CC_TW + CC_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
+        sx_launch(k_ccl_border_ne<CC_TW, CC_TH>, ntiles, CC_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
         launches += 4;
     }
     long long n = (long long)P.w * P.h;
-    k_ccl_flatten<<<(unsigned)((n + 1023) / 1024), 256, 0, st>>>(lab, n, cnt, status, P.loop_cap);
+    sx_launch(k_ccl_flatten, (unsigned)((n + 1023) / 1024), 256, 0, st, lab, n, cnt, status, P.loop_cap);
 }
 
 }  // namespace sx

@@ -21,6 +21,7 @@ __device__ __forceinline__ unsigned fits_bswap32(unsigned x) { return __byte_per
 template <int BITPIX>
 __global__ void k_fits_to_float(const unsigned char *__restrict__ raw, float *__restrict__ out, long long n, float bs,
                                 float bz, int has_blank, long long blank) {
+    sx_pdl();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         float v;
@@ -54,11 +55,11 @@ bool launch_fits_to_float(const void *d_raw, int bitpix, double bscale, double b
     const unsigned grid = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 16);
     const unsigned char *raw = static_cast<const unsigned char *>(d_raw);
     switch (bitpix) {
-    case 8: k_fits_to_float<8><<<grid, 256, 0, st>>>(raw, d_out, n, bs, bz, has_blank, blank); return true;
-    case 16: k_fits_to_float<16><<<grid, 256, 0, st>>>(raw, d_out, n, bs, bz, has_blank, blank); return true;
-    case 32: k_fits_to_float<32><<<grid, 256, 0, st>>>(raw, d_out, n, bs, bz, has_blank, blank); return true;
-    case -32: k_fits_to_float<-32><<<grid, 256, 0, st>>>(raw, d_out, n, bs, bz, has_blank, blank); return true;
-    case -64: k_fits_to_float<-64><<<grid, 256, 0, st>>>(raw, d_out, n, bs, bz, has_blank, blank); return true;
+    case 8: sx_launch(k_fits_to_float<8>, grid, 256, 0, st, raw, d_out, n, bs, bz, has_blank, blank); return true;
+    case 16: sx_launch(k_fits_to_float<16>, grid, 256, 0, st, raw, d_out, n, bs, bz, has_blank, blank); return true;
+    case 32: sx_launch(k_fits_to_float<32>, grid, 256, 0, st, raw, d_out, n, bs, bz, has_blank, blank); return true;
+    case -32: sx_launch(k_fits_to_float<-32>, grid, 256, 0, st, raw, d_out, n, bs, bz, has_blank, blank); return true;
+    case -64: sx_launch(k_fits_to_float<-64>, grid, 256, 0, st, raw, d_out, n, bs, bz, has_blank, blank); return true;
     }
     return false;
 }

@@ -34,6 +34,7 @@ __device__ __forceinline__ int clean_cell(double mx, double my, int gx, int gy) 
 }
 
 __global__ void k_clean_count(ObjBufs O, int n, const int *n_dev, int *cellcnt, int gx, int gy) {
+    sx_pdl();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= sx_count(n, n_dev)) return;
     O.master[i] = 0x7fffffff;
@@ -42,6 +43,7 @@ __global__ void k_clean_count(ObjBufs O, int n, const int *n_dev, int *cellcnt, 
 
 __global__ void k_clean_pack(ObjBufs O, int n, const int *n_dev, double beta, const int *cellstart, int *cellcur,
                              CleanObj *packed, int gx, int gy) {
+    sx_pdl();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= sx_count(n, n_dev)) return;
     CleanObj c;
@@ -100,6 +102,7 @@ __global__ void __launch_bounds__(CL_PAIR_WARPS * 32) k_clean_pairs(const CleanO
                                                                     const int *n_dev, double beta,
                                                                     const int *__restrict__ cellstart,
                                                                     int *master, int gx, int gy) {
+    sx_pdl();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int k = blockIdx.x;
     if (k >= sx_count(n, n_dev)) return;
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(CL_PAIR_WARPS * 32) k_clean_pairs(const CleanO
 // bound set for a failure test (0: n); running out sets SX_ST_LOOP.  Every
 // survivor counts its victims (vcnt, zeroed before).
 __global__ void k_clean_chain(ObjBufs O, int n, const int *n_dev, int *vcnt, int *status, int cap) {
+    sx_pdl();
     n = sx_count(n, n_dev);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -148,6 +152,7 @@ __global__ void k_clean_chain(ObjBufs O, int n, const int *n_dev, int *vcnt, int
 // to its rank among them in vsort.  A victim compares itself with the others
 // of its survivor only, usually a handful.
 __global__ void k_victim_scatter(ObjBufs O, int n, const int *n_dev, const int *voff, int *vfill, int *vlist) {
+    sx_pdl();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= sx_count(n, n_dev)) return;
     const int m = O.fmaster[i];
@@ -156,6 +161,7 @@ __global__ void k_victim_scatter(ObjBufs O, int n, const int *n_dev, const int *
 
 __global__ void k_victim_rank(ObjBufs O, int n, const int *n_dev, const int *voff, const int *vcnt, const int *vlist,
                               int *vsort) {
+    sx_pdl();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= sx_count(n, n_dev)) return;
     const int m = O.fmaster[i];
@@ -168,6 +174,7 @@ __global__ void k_victim_rank(ObjBufs O, int n, const int *n_dev, const int *vof
 
 // each survivor merges its victims in index order (src/clean.c:234-287)
 __global__ void k_clean_merge(ObjBufs O, int n, const int *n_dev, const int *voff, const int *vcnt, const int *vsort) {
+    sx_pdl();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= sx_count(n, n_dev)) return;
     const int v0 = voff[m], v1 = v0 + vcnt[m];
@@ -197,6 +204,7 @@ __global__ void k_clean_merge(ObjBufs O, int n, const int *n_dev, const int *vof
 // pixels of cleaned objects belong to their master in the allocation map (one
 // warp per object)
 __global__ void k_alloc_victims(ObjBufs O, const unsigned *opix, int *alloc, int n, const int *n_dev) {
+    sx_pdl();
     const int o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (o >= sx_count(n, n_dev)) return;
     const int m = O.fmaster[o];
@@ -592,6 +600,7 @@ __device__ bool kron_defer(const EndArgs &A, int pass, int o, const KronGeo &g) 
 // apertures and pass 1, one warp per surviving object
 constexpr int EO_WARPS = 4;
 __global__ void __launch_bounds__(EO_WARPS * 32, 8) k_end_pass1(const __grid_constant__ EndArgs A) {
+    sx_pdl();
     __shared__ AperTerms terms[EO_WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int o = blockIdx.x * EO_WARPS + wid;
@@ -620,6 +629,7 @@ __global__ void __launch_bounds__(EO_WARPS * 32, 8) k_end_pass1(const __grid_con
 // kron radius from pass 1 and the pass-2 ellipse and box (cudaanalyse.cu:
 // 385-440), one thread per object; no AUTO flux when pass 1 found no pixel
 __global__ void k_kron_mid(const __grid_constant__ EndArgs A) {
+    sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(A.n, A.n_dev) || A.O.fmaster[o] >= 0) return;
     EndRaw &R = A.raw[o];
@@ -650,6 +660,7 @@ __global__ void k_kron_mid(const __grid_constant__ EndArgs A) {
 // pass 2, one warp per surviving object
 template <bool WVAR>
 __global__ void __launch_bounds__(EO_WARPS * 32, 8) k_end_pass2(const __grid_constant__ EndArgs A) {
+    sx_pdl();
     const int o = blockIdx.x * EO_WARPS + (threadIdx.x >> 5);
     if (o >= sx_count(A.n, A.n_dev)) return;
     if (A.O.fmaster[o] >= 0 || A.raw[o].have2 != 1) return;
@@ -664,6 +675,7 @@ __global__ void __launch_bounds__(EO_WARPS * 32, 8) k_end_pass2(const __grid_con
 // CTA that finishes a box's last item merges them
 template <int PASS, bool WVAR>
 __global__ void __launch_bounds__(KR_THREADS) k_kron_chunks(const __grid_constant__ EndArgs A) {
+    sx_pdl();
     __shared__ KronPart red[KR_THREADS / 32];
     __shared__ int s_last;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -740,6 +752,7 @@ __global__ void __launch_bounds__(KR_THREADS) k_kron_chunks(const __grid_constan
 // ISOCOR and ISO fluxes, magnitudes and errors, FLAGS (one thread per object,
 // so that this double-precision tail does not run on one lane of a warp)
 __global__ void k_end_finish(const __grid_constant__ EndArgs A) {
+    sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(A.n, A.n_dev) || A.O.fmaster[o] >= 0) return;
     for (int k = 0; k < A.naper; k++) {
@@ -814,6 +827,7 @@ __global__ void k_end_finish(const __grid_constant__ EndArgs A) {
 // seeing; every layer applies the logistic function; double arithmetic.
 __global__ void k_class_star(ObjBufs O, int n, const int *n_dev, const sexgpu_nnw *__restrict__ net, double fwhm,
                              double pixscale) {
+    sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(n, n_dev) || O.fmaster[o] >= 0) return;
     double fac2 = fwhm / pixscale;
@@ -842,21 +856,21 @@ __global__ void k_class_star(ObjBufs O, int n, const int *n_dev, const sexgpu_nn
 void launch_endobject(const EndArgs &E, int nobj, cudaStream_t st, int &launches) {
     if (nobj <= 0) return;
     const unsigned gw = (unsigned)((nobj + EO_WARPS - 1) / EO_WARPS), gt = (unsigned)((nobj + 127) / 128);
-    k_end_pass1<<<gw, EO_WARPS * 32, 0, st>>>(E);
-    k_kron_chunks<1, false><<<KR_GRID, KR_THREADS, 0, st>>>(E);
-    k_kron_mid<<<gt, 128, 0, st>>>(E);
+    sx_launch(k_end_pass1, gw, EO_WARPS * 32, 0, st, E);
+    sx_launch(k_kron_chunks<1, false>, KR_GRID, KR_THREADS, 0, st, E);
+    sx_launch(k_kron_mid, gt, 128, 0, st, E);
     if (E.wvar) {
-        k_end_pass2<true><<<gw, EO_WARPS * 32, 0, st>>>(E);
-        k_kron_chunks<2, true><<<KR_GRID, KR_THREADS, 0, st>>>(E);
+        sx_launch(k_end_pass2<true>, gw, EO_WARPS * 32, 0, st, E);
+        sx_launch(k_kron_chunks<2, true>, KR_GRID, KR_THREADS, 0, st, E);
     } else {
-        k_end_pass2<false><<<gw, EO_WARPS * 32, 0, st>>>(E);
-        k_kron_chunks<2, false><<<KR_GRID, KR_THREADS, 0, st>>>(E);
+        sx_launch(k_end_pass2<false>, gw, EO_WARPS * 32, 0, st, E);
+        sx_launch(k_kron_chunks<2, false>, KR_GRID, KR_THREADS, 0, st, E);
     }
-    k_end_finish<<<gt, 128, 0, st>>>(E);
+    sx_launch(k_end_finish, gt, 128, 0, st, E);
     launches += 6;
     if (E.nnw) {
-        k_class_star<<<(unsigned)((nobj + 127) / 128), 128, 0, st>>>(E.O, nobj, E.n_dev, E.nnw, E.seeing,
-                                                                      E.pixscale);
+        sx_launch(k_class_star, (unsigned)((nobj + 127) / 128), 128, 0, st, E.O, nobj, E.n_dev, E.nnw, E.seeing,
+                  E.pixscale);
         launches += 1;
     }
 }
@@ -873,6 +887,7 @@ void launch_endobject(const EndArgs &E, int nobj, cudaStream_t st, int &launches
 constexpr int NO_TILE = 1024;  // elements; 3 to 20 raw objects of a crowded frame
 
 __global__ void k_surv_flags(ObjBufs O, int n, const int *n_dev, int *flag) {
+    sx_pdl();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < sx_count(n, n_dev)) flag[i] = O.fmaster[i] < 0 ? 1 : 0;
 }
@@ -885,6 +900,7 @@ struct OrderBufs {
 
 __global__ void k_order_roots(ObjBufs O, RootBufs R, const int *pos2idx, int w, int nroots, const int *nroots_dev,
                               OrderBufs Q) {
+    sx_pdl();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= sx_count(nroots, nroots_dev)) return;
     const int K = R.nkept[r], ob = R.objbase[r];
@@ -903,6 +919,7 @@ __global__ void k_order_roots(ObjBufs O, RootBufs R, const int *pos2idx, int w, 
 // index order)
 __global__ void k_order_objs(ObjBufs O, RootBufs R, int n, const int *n_dev, int numbering, OrderBufs Q,
                              unsigned *order) {
+    sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= sx_count(n, n_dev)) return;
     if (O.fmaster[o] >= 0) {
@@ -921,6 +938,7 @@ __global__ void k_order_objs(ObjBufs O, RootBufs R, int n, const int *n_dev, int
 }
 
 __global__ void k_write_rows(ObjBufs O, const unsigned *vals, int ns, const int *ns_dev, sexgpu_object *rows) {
+    sx_pdl();
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= sx_count(ns, ns_dev)) return;
     int o = (int)vals[k];
@@ -1001,6 +1019,7 @@ __global__ void k_write_rows(ObjBufs O, const unsigned *vals, int ns, const int 
 
 // every aperture of the catalogue rows, in catalogue order (naper per row)
 __global__ void k_write_apers(ObjBufs O, const unsigned *order, int ns, int naper, float4 *out) {
+    sx_pdl();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= ns) return;
     const int o = (int)order[r];
@@ -1012,6 +1031,7 @@ __global__ void k_write_apers(ObjBufs O, const unsigned *order, int ns, int nape
 
 // segmentation map: NUMBER of the owning object, 0 elsewhere
 __global__ void k_segmap(const int *alloc, const int *number, int *seg, long long npix) {
+    sx_pdl();
     long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npix) return;
     int a = alloc[p];

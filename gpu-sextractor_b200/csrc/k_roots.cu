@@ -21,6 +21,7 @@ namespace sx {
 __global__ void k_root_thresholds(const int *__restrict__ lab, const int *__restrict__ cnt,
                                   const int *__restrict__ rid, long long n, int minarea, const float *__restrict__ wvar,
                                   int wthr, double dfac, double afac, FrameScalars *sc, int *rdthr, int *rathr) {
+    sx_pdl();
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int r = -1, idt = 0x7fffffff, iat = 0x7fffffff, e = 0x7fffffff;
     if (p < n) {
@@ -54,6 +55,7 @@ __global__ void k_root_thresholds(const int *__restrict__ lab, const int *__rest
 // without a weight map every raw object has the global thresholds
 __global__ void k_root_thresholds_global(int nroots, const int *nroots_dev, const FrameScalars *sc, float *rdthr,
                                          float *rathr) {
+    sx_pdl();
     nroots = sx_count(nroots, nroots_dev);
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r < nroots) {
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_tile_counts(const int *__
                                                                   const int *__restrict__ cnt, long long n,
                                                                   int minarea, int *__restrict__ troots,
                                                                   int *__restrict__ tkept) {
+    sx_pdl();
     __shared__ int sh[32];
     const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
     int cr = 0, ck = 0, r[SCAN_ITEMS], kp[SCAN_ITEMS], l[SCAN_ITEMS];
@@ -117,6 +120,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_tile_counts(const int *__
 __global__ void __launch_bounds__(SCAN_THREADS) k_root_number(const int *__restrict__ lab, const int *__restrict__ cnt,
                                                              long long n, int minarea, const int *__restrict__ toff,
                                                              int *__restrict__ rid, int *__restrict__ rsize) {
+    sx_pdl();
     __shared__ int sh[32];
     const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
     int fr[SCAN_ITEMS], kp[SCAN_ITEMS], l[SCAN_ITEMS], c = 0;
@@ -143,6 +147,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_compact(const int *__rest
                                                               const int *__restrict__ rid, unsigned *__restrict__ erid,
                                                               unsigned *__restrict__ epix, int *__restrict__ alloc,
                                                               int *__restrict__ pos2idx) {
+    sx_pdl();
     __shared__ int sh[32];
     const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
     int fk[SCAN_ITEMS], lb[SCAN_ITEMS], fr[SCAN_ITEMS], c = 0;

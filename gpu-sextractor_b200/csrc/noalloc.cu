@@ -78,6 +78,7 @@ static cudaError_t scratch_on_current_device(unsigned char **out) {
 // reference's float additions from the last restart of the sequence, so it
 // equals the value of the sequential loop.
 __global__ void k_col_table(int width, int nbx, int backw, int *colk, float *coldx) {
+    sx_pdl();
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= width) return;
     if (nbx <= 1) {
@@ -115,6 +116,7 @@ __global__ void k_col_table(int width, int nbx, int backw, int *colk, float *col
 // background subtraction only (the subtraction half of k_sub_filter)
 __global__ void k_sub_only(const float *__restrict__ img, float *__restrict__ sub, sx::BackBufs B, int w, int h,
                            int nbx, int back_type, const FrameScalars *sc) {
+    sx_pdl();
     long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= (long long)w * h) return;
     int x = (int)(p % w), y = (int)(p / w);
@@ -164,11 +166,11 @@ extern "C" int sexgpu_background_noalloc(const float *d_img, float *d_sub, int w
     B.colk = (int *)(base + OFF_COLK);
     B.coldx = (float *)(base + OFF_COLDX);
     int nl = 0;
-    k_init_scalars<<<1, 1, 0, st>>>(d_sc);  // the pipeline's initial scalars (sigfac 1)
-    k_col_table<<<(w + 255) / 256, 256, 0, st>>>(w, Pm.nbx, Pm.bw, B.colk, B.coldx);
+    sx_launch(k_init_scalars, 1, 1, 0, st, d_sc);  // the pipeline's initial scalars (sigfac 1)
+    sx_launch(k_col_table, (w + 255) / 256, 256, 0, st, w, Pm.nbx, Pm.bw, B.colk, B.coldx);
     sx::launch_background(B, d_img, Pm, d_sc, st, nl);
     long long n = (long long)w * h;
-    k_sub_only<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_img, d_sub, B, w, h, Pm.nbx, Pm.back_type, d_sc);
+    sx_launch(k_sub_only, (unsigned)((n + 255) / 256), 256, 0, st, d_img, d_sub, B, w, h, Pm.nbx, Pm.back_type, d_sc);
     if (cudaGetLastError() != cudaSuccess) return SEXGPU_ERR_CUDA;
     if (sum) {
         FrameScalars hs;

@@ -44,6 +44,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *sh_warp, int &to
 __device__ __forceinline__ int dev_count(int n, const int *n_dev) { return n_dev ? min(n, max(*n_dev, 0)) : n; }
 
 __global__ void k_tile_sums(const int *__restrict__ in, int n, int *__restrict__ sums, const int *n_dev) {
+    sx_pdl();
     __shared__ int sh[32];
     n = dev_count(n, n_dev);
     long long base = (long long)blockIdx.x * SCAN_TILE;
@@ -60,6 +61,7 @@ __global__ void k_tile_sums(const int *__restrict__ in, int n, int *__restrict__
 
 __global__ void k_tile_scan(const int *__restrict__ in, int *__restrict__ out, int n,
                             const int *__restrict__ offs, int *total, const int *n_dev) {
+    sx_pdl();
     __shared__ int sh[32];
     n = dev_count(n, n_dev);
     long long base = (long long)blockIdx.x * SCAN_TILE;
@@ -95,6 +97,7 @@ struct ScanArray {
 };
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_one(const ScanArray A, const ScanArray B, int n, const int *n_dev) {
+    sx_pdl();
     __shared__ int sh[32];
     const ScanArray S = blockIdx.x ? B : A;
     n = dev_count(n, n_dev);
@@ -139,14 +142,14 @@ int exclusive_scan(const int *in, int *out, long long n, int *total, int *tmp, c
     }
     if (n <= SCAN_ONE_MAX) {
         const ScanArray A{in, out, total};
-        k_scan_one<<<1, SCAN_THREADS, 0, st>>>(A, A, (int)n, n_dev);
+        sx_launch(k_scan_one, 1, SCAN_THREADS, 0, st, A, A, (int)n, n_dev);
         return 1;
     }
     const int nt = (int)((n + SCAN_TILE - 1) / SCAN_TILE);
     int *sums = tmp, *offs = tmp + nt;
-    k_tile_sums<<<nt, SCAN_THREADS, 0, st>>>(in, (int)n, sums, n_dev);
+    sx_launch(k_tile_sums, nt, SCAN_THREADS, 0, st, in, (int)n, sums, n_dev);
     const int k = exclusive_scan(sums, offs, nt, nullptr, tmp + 2 * nt + 2, st, nullptr);
-    k_tile_scan<<<nt, SCAN_THREADS, 0, st>>>(in, out, (int)n, offs, total, n_dev);
+    sx_launch(k_tile_scan, nt, SCAN_THREADS, 0, st, in, out, (int)n, offs, total, n_dev);
     return 2 + k;
 }
 
@@ -155,8 +158,8 @@ int exclusive_scan(const int *in, int *out, long long n, int *total, int *tmp, c
 int exclusive_scan2(const int *in0, int *out0, int *total0, const int *in1, int *out1, int *total1, long long n,
                     int *tmp, cudaStream_t st) {
     if (n > 0 && n <= SCAN_ONE_MAX) {
-        k_scan_one<<<2, SCAN_THREADS, 0, st>>>(ScanArray{in0, out0, total0}, ScanArray{in1, out1, total1}, (int)n,
-                                               nullptr);
+        sx_launch(k_scan_one, 2, SCAN_THREADS, 0, st, ScanArray{in0, out0, total0}, ScanArray{in1, out1, total1},
+                  (int)n, nullptr);
         return 1;
     }
     return exclusive_scan(in0, out0, n, total0, tmp, st, nullptr) + exclusive_scan(in1, out1, n, total1, tmp, st, nullptr);

@@ -380,6 +380,7 @@ void make_params(const sexgpu_config *cfg, int w, int h, FrameParams &P) {
 }
 
 __global__ void k_init_scalars(FrameScalars *sc) {
+    sx_pdl();
     FrameScalars z;
     memset(&z, 0, sizeof(z));
     z.e0sub = 1000;
@@ -393,6 +394,7 @@ __global__ void k_init_scalars(FrameScalars *sc) {
 // read to 0, so that the rest of the frame does nothing; the status tells the
 // host afterwards.
 __global__ void k_gate(FrameScalars *sc, int check_thr, int cap_roots, int cap_rootpix, int cap_obj) {
+    sx_pdl();
     int st = sc->status;
     if (check_thr && (sc->dthresh <= 0.0f || sc->thresh <= 0.0f)) st |= SX_ST_THRESH;
     if (sc->nroots > cap_roots || sc->nrootpix > cap_rootpix || sc->nobj > cap_obj) st |= SX_ST_CAPACITY;
@@ -635,7 +637,7 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
 
     stage_begin(ctx);
     int nl = 0;
-    k_init_scalars<<<1, 1, 0, st>>>(d_sc);
+    sx_launch(k_init_scalars, 1, 1, 0, st, d_sc);
     ps.wvar = nullptr;
     if (d_wmap) {
         // pixels of unusable weight are blank for the background and the detection
@@ -663,8 +665,8 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
         EN(rmsdnode, (size_t)h * Pm.nbx * 4);
         launch_map_nodes(B.sigma3, P<float>(ctx->rmsd), P<float>(ctx->rmsu), Pm.nbx, Pm.nby, Pm.bh, h,
                          P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), P<float>(ctx->rmsu), st);
-        k_rms_map<<<grid1(N, 256), 256, 0, st>>>(P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), B.colk, B.coldx,
-                                                Pm.nbx, w, N, P<float>(ctx->wvar), 1);
+        sx_launch(k_rms_map, grid1(N, 256), 256, 0, st, P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), B.colk,
+                  B.coldx, Pm.nbx, w, N, P<float>(ctx->wvar), 1);
         ps.wvar = P<float>(ctx->wvar);
         nl += 3;
     }
@@ -700,7 +702,7 @@ int pipe_detect(sexgpu_ctx *ctx) {
     // (pos holds the two count arrays and the two offset arrays)
     const int ntile = (int)((N + SCAN_TILE - 1) / SCAN_TILE);
     int *troots = pos, *tkept = pos + ntile, *troff = pos + 2 * ntile, *tkoff = pos + 3 * ntile;
-    k_root_tile_counts<<<ntile, SCAN_THREADS, 0, st>>>(lab, cnt, N, Pm.minarea, troots, tkept);
+    sx_launch(k_root_tile_counts, ntile, SCAN_THREADS, 0, st, lab, cnt, N, Pm.minarea, troots, tkept);
     nl = 1 + exclusive_scan2(troots, troff, &d_sc->nroots, tkept, tkoff, &d_sc->nrootpix, ntile, tmp, st);
     // roots (the capacity in the capacity form) and the length of the root
     // arrays: in the capacity form, the most roots the frame can hold (each
@@ -710,7 +712,7 @@ int pipe_detect(sexgpu_ctx *ctx) {
         nroots = ps.cap_roots;
         nrootpix = ps.cap_rootpix;
         rlen = (int)(N / std::max(Pm.minarea, 1));
-        k_gate<<<1, 1, 0, st>>>(d_sc, 1, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
+        sx_launch(k_gate, 1, 1, 0, st, d_sc, 1, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
     } else {
         rc = read_scalars(ctx);
         if (rc) return rc;
@@ -737,19 +739,18 @@ int pipe_detect(sexgpu_ctx *ctx) {
     R.objbase = P<int>(ctx->robjbase);
     R.dthresh = P<float>(ctx->rdthr);
     R.thresh = P<float>(ctx->rathr);
-    k_root_number<<<ntile, SCAN_THREADS, 0, st>>>(lab, cnt, N, Pm.minarea, troff, flag, R.size);
+    sx_launch(k_root_number, ntile, SCAN_THREADS, 0, st, lab, cnt, N, Pm.minarea, troff, flag, R.size);
     nl += 3 + exclusive_scan(R.size, R.off, nroots, nullptr, tmp, st, nroots_dev);
-    k_root_compact<<<ntile, SCAN_THREADS, 0, st>>>(lab, cnt, N, Pm.minarea, tkoff, flag, P<unsigned>(ctx->keys),
-                                                   P<unsigned>(ctx->rpix), P<int>(ctx->alloc), P<int>(ctx->pos2idx));
+    sx_launch(k_root_compact, ntile, SCAN_THREADS, 0, st, lab, cnt, N, Pm.minarea, tkoff, flag,
+              P<unsigned>(ctx->keys), P<unsigned>(ctx->rpix), P<int>(ctx->alloc), P<int>(ctx->pos2idx));
     if (ps.wvar) {
         CK(cudaMemsetAsync(R.dthresh, 0x7f, (size_t)(nroots + 1) * 4, st));
         CK(cudaMemsetAsync(R.thresh, 0x7f, (size_t)(nroots + 1) * 4, st));
-        k_root_thresholds<<<grid1(N, 256), 256, 0, st>>>(lab, cnt, flag, N, Pm.minarea, ps.wvar, Pm.wthr,
-                                                         Pm.detect_thresh, Pm.analysis_thresh, d_sc,
-                                                         (int *)R.dthresh, (int *)R.thresh);
+        sx_launch(k_root_thresholds, grid1(N, 256), 256, 0, st, lab, cnt, flag, N, Pm.minarea, ps.wvar, Pm.wthr,
+                  Pm.detect_thresh, Pm.analysis_thresh, d_sc, (int *)R.dthresh, (int *)R.thresh);
     } else {
-        k_root_thresholds_global<<<grid1(nroots, 256), 256, 0, st>>>(nroots, nroots_dev, d_sc, R.dthresh,
-                                                                       R.thresh);
+        sx_launch(k_root_thresholds_global, grid1(nroots, 256), 256, 0, st, nroots, nroots_dev, d_sc, R.dthresh,
+                  R.thresh);
     }
     stage_mark(ctx, "roots", nl);
     ps.stage = 2;
@@ -846,7 +847,7 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     int nobj;
     if (ps.capf) {
         nobj = ps.cap_obj;
-        k_gate<<<1, 1, 0, st>>>(d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
+        sx_launch(k_gate, 1, 1, 0, st, d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
     } else {
         rc = read_scalars(ctx);
         if (rc) return rc;
@@ -962,18 +963,18 @@ int pipe_clean(sexgpu_ctx *ctx) {
         CK(cudaMemsetAsync(cellcnt, 0, (2 * (size_t)(ncell + 1) + 2 * n1) * 4, st));
         const int *nobj_dev = ps.capf ? &d_sc->nobj : nullptr;
         const unsigned g = grid1(nobj, 128);
-        k_clean_count<<<g, 128, 0, st>>>(O, nobj, nobj_dev, cellcnt, gx, gy);
+        sx_launch(k_clean_count, g, 128, 0, st, O, nobj, nobj_dev, cellcnt, gx, gy);
         nl += exclusive_scan(cellcnt, cellcnt, ncell + 1, nullptr, tmp, st);
-        k_clean_pack<<<g, 128, 0, st>>>(O, nobj, nobj_dev, Pm.clean_param, cellcnt, cellcur, P<CleanObj>(ctx->amp), gx,
-                                        gy);
-        k_clean_pairs<<<(unsigned)nobj, CL_PAIR_WARPS * 32, 0, st>>>(P<CleanObj>(ctx->amp), nobj, nobj_dev,
-                                                                      Pm.clean_param, cellcnt, O.master, gx, gy);
-        k_clean_chain<<<g, 128, 0, st>>>(O, nobj, nobj_dev, vcnt, &d_sc->status, Pm.loop_cap);
+        sx_launch(k_clean_pack, g, 128, 0, st, O, nobj, nobj_dev, Pm.clean_param, cellcnt, cellcur,
+                  P<CleanObj>(ctx->amp), gx, gy);
+        sx_launch(k_clean_pairs, (unsigned)nobj, CL_PAIR_WARPS * 32, 0, st, P<CleanObj>(ctx->amp), nobj, nobj_dev,
+                  Pm.clean_param, cellcnt, O.master, gx, gy);
+        sx_launch(k_clean_chain, g, 128, 0, st, O, nobj, nobj_dev, vcnt, &d_sc->status, Pm.loop_cap);
         nl += exclusive_scan(vcnt, voff, nobj, nullptr, tmp, st, nobj_dev);
-        k_victim_scatter<<<g, 128, 0, st>>>(O, nobj, nobj_dev, voff, vfill, vlist);
-        k_victim_rank<<<g, 128, 0, st>>>(O, nobj, nobj_dev, voff, vcnt, vlist, vsort);
-        k_clean_merge<<<g, 128, 0, st>>>(O, nobj, nobj_dev, voff, vcnt, vsort);
-        k_alloc_victims<<<grid1((long long)nobj * 32, 256), 256, 0, st>>>(O, vals, A.alloc, nobj, nobj_dev);
+        sx_launch(k_victim_scatter, g, 128, 0, st, O, nobj, nobj_dev, voff, vfill, vlist);
+        sx_launch(k_victim_rank, g, 128, 0, st, O, nobj, nobj_dev, voff, vcnt, vlist, vsort);
+        sx_launch(k_clean_merge, g, 128, 0, st, O, nobj, nobj_dev, voff, vcnt, vsort);
+        sx_launch(k_alloc_victims, grid1((long long)nobj * 32, 256), 256, 0, st, O, vals, A.alloc, nobj, nobj_dev);
         nl += 8;
     } else if (nobj > 0) {
         CK(cudaMemsetAsync(O.fmaster, 0xff, (size_t)nobj * 4, st));
@@ -996,7 +997,7 @@ int pipe_end(sexgpu_ctx *ctx) {
     int *tmp = P<int>(ctx->scan_tmp);
     // an error so far empties the frame (the host reads the status at its end)
     constexpr int NOCAP = 0x7fffffff;
-    k_gate<<<1, 1, 0, st>>>(d_sc, 0, NOCAP, NOCAP, NOCAP);
+    sx_launch(k_gate, 1, 1, 0, st, d_sc, 0, NOCAP, NOCAP, NOCAP);
     const int *nobj_dev = &d_sc->nobj;
     // ---- photometry / FLAGS
     EndArgs E;
@@ -1054,21 +1055,22 @@ int pipe_end(sexgpu_ctx *ctx) {
     int *const pos = Q.ns + nr1;
     Q.pos = pos;
     CK(cudaMemsetAsync(Q.tcnt, 0, 2 * (size_t)nt * 4, st));
-    k_surv_flags<<<grid1(nobj, 256), 256, 0, st>>>(O, nobj, nobj_dev, pos);
+    sx_launch(k_surv_flags, grid1(nobj, 256), 256, 0, st, O, nobj, nobj_dev, pos);
     nl = 3 + exclusive_scan(pos, pos, nobj, &d_sc->nsurv, tmp, st, nobj_dev);
     if (Pm.numbering == 0) {
-        k_order_roots<<<grid1(ps.nroots, 128), 128, 0, st>>>(O, R, P<int>(ctx->pos2idx), w, ps.nroots,
-                                                             &d_sc->nroots, Q);
+        sx_launch(k_order_roots, grid1(ps.nroots, 128), 128, 0, st, O, R, P<int>(ctx->pos2idx), w, ps.nroots,
+                  &d_sc->nroots, Q);
         nl += 1 + exclusive_scan(Q.tcnt, Q.tcnt, nt, nullptr, tmp, st);
     }
-    k_order_objs<<<grid1(nobj, 128), 128, 0, st>>>(O, R, nobj, nobj_dev, Pm.numbering, Q, P<unsigned>(ctx->svals));
+    sx_launch(k_order_objs, grid1(nobj, 128), 128, 0, st, O, R, nobj, nobj_dev, Pm.numbering, Q,
+              P<unsigned>(ctx->svals));
     // rows for every object: the survivors' count stays on the device until
     // the end of the frame
     const int ns = nobj;
     const int *ns_dev = &d_sc->nsurv;
     EN(rows, (size_t)(ns + 1) * sizeof(sexgpu_object));
-    k_write_rows<<<grid1(ns + 1, 128), 128, 0, st>>>(O, P<unsigned>(ctx->svals), ns, ns_dev,
-                                                     P<sexgpu_object>(ctx->rows));
+    sx_launch(k_write_rows, grid1(ns + 1, 128), 128, 0, st, O, P<unsigned>(ctx->svals), ns, ns_dev,
+              P<sexgpu_object>(ctx->rows));
     stage_mark(ctx, "catalog", nl);
     CK(cudaGetLastError());
     if (ps.capf) {
@@ -1573,7 +1575,7 @@ int sexgpu_copy_results(sexgpu_ctx *ctx, sexgpu_object *objs, int max_objects, i
     }
     if (segmap && N > 0) {
         EN(seg, N * 4);
-        k_segmap<<<grid1(N, 256), 256, 0, st>>>(P<int>(ctx->alloc), ctx->O.number, P<int>(ctx->seg), N);
+        sx_launch(k_segmap, grid1(N, 256), 256, 0, st, P<int>(ctx->alloc), ctx->O.number, P<int>(ctx->seg), N);
         CK(cudaMemcpyAsync(segmap, ctx->seg.p, N * 4, cudaMemcpyDeviceToHost, st));
     }
     if (sub && N > 0) CK(cudaMemcpyAsync(sub, ctx->sub.p, N * 4, cudaMemcpyDeviceToHost, st));
@@ -1690,8 +1692,8 @@ int sexgpu_background_rms(sexgpu_ctx *ctx, float *rms) {
     EN(rmsmap, (size_t)N * 4);
     launch_map_nodes(ps.B.sigma3, P<float>(ctx->rmsd), P<float>(ctx->rmsu), Pm.nbx, Pm.nby, Pm.bh, h,
                      P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), P<float>(ctx->rmsu), st);
-    k_rms_map<<<grid1(N, 256), 256, 0, st>>>(P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), ps.B.colk, ps.B.coldx,
-                                            Pm.nbx, w, N, P<float>(ctx->rmsmap), 0);
+    sx_launch(k_rms_map, grid1(N, 256), 256, 0, st, P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), ps.B.colk,
+              ps.B.coldx, Pm.nbx, w, N, P<float>(ctx->rmsmap), 0);
     CK(cudaMemcpyAsync(rms, ctx->rmsmap.p, (size_t)N * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     return SEXGPU_OK;
@@ -1712,8 +1714,8 @@ int sexgpu_copy_apertures(sexgpu_ctx *ctx, float *out, int max_rows, int *nrows,
     if (ns == 0) return SEXGPU_OK;
     cudaStream_t st = ctx->stream;
     EN(aperrows, (size_t)ns * na * sizeof(float4));
-    k_write_apers<<<grid1(ns, 128), 128, 0, st>>>(ctx->O, P<unsigned>(ctx->svals), ns, na,
-                                                  P<float4>(ctx->aperrows));
+    sx_launch(k_write_apers, grid1(ns, 128), 128, 0, st, ctx->O, P<unsigned>(ctx->svals), ns, na,
+              P<float4>(ctx->aperrows));
     CK(cudaMemcpyAsync(out, ctx->aperrows.p, (size_t)ns * na * sizeof(float4), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     return SEXGPU_OK;
@@ -1731,8 +1733,8 @@ int sexgpu_background_map(sexgpu_ctx *ctx, float *back) {
     const FrameParams &Pm = ps.Pm;
     const long long N = (long long)Pm.w * Pm.h;
     EN(rmsmap, (size_t)N * 4);
-    k_back_map<<<grid1(N, 256), 256, 0, st>>>(ps.B, Pm.nbx, Pm.back_type, P<FrameScalars>(ctx->sc), Pm.w, N,
-                                             P<float>(ctx->rmsmap));
+    sx_launch(k_back_map, grid1(N, 256), 256, 0, st, ps.B, Pm.nbx, Pm.back_type, P<FrameScalars>(ctx->sc), Pm.w, N,
+              P<float>(ctx->rmsmap));
     CK(cudaMemcpyAsync(back, ctx->rmsmap.p, (size_t)N * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     return SEXGPU_OK;
@@ -1790,7 +1792,7 @@ int sexgpu_background(sexgpu_ctx *ctx, float *img, int w, int h, const sexgpu_co
     if (rc) return rc;
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int nl = 0;
-    k_init_scalars<<<1, 1, 0, st>>>(d_sc);
+    sx_launch(k_init_scalars, 1, 1, 0, st, d_sc);
     launch_background(B, P<float>(ctx->img), Pm, d_sc, st, nl);
     launch_sub_filter(P<float>(ctx->img), P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), B, Pm, d_sc,
                       nullptr, ctx->cmask, st, nl);
