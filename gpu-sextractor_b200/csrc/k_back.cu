@@ -1238,11 +1238,42 @@ void launch_map_nodes(const float *map, float *dmap, float *u, int nbx, int nby,
 // weight maps: blank the unusable pixels, then (after the background) the
 // scale factor sigfac and the calibrated variance map
 // ---------------------------------------------------------------------------
-__global__ void k_weight_mask(const float *__restrict__ img, const float *__restrict__ wmap, int wtype,
-                              float *__restrict__ imgm, long long n) {
+// Maps are read and written once: four pixels (16 bytes) at a time where the
+// arrays are aligned, two such words in flight per thread.  One pixel a thread,
+// these passes over a 16384 x 16384 frame took 1.18 (mask) and 0.75 ms
+// (variance); the bytes take 0.49 and 0.33.
+constexpr int WM_PIX = 2048;  // pixels per block of 256 threads
+
+template <class F>
+__device__ __forceinline__ void map_words(long long n, bool vec, F f) {
+    const long long base = (long long)blockIdx.x * WM_PIX;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const long long p = base + u * 1024 + threadIdx.x * 4;
+        if (vec && p + 3 < n)
+            f(p, true);
+        else
+            for (int k = 0; k < 4; k++)
+                if (p + k < n) f(p + k, false);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_weight_mask(const float *__restrict__ img, const float *__restrict__ wmap,
+                                                     int wtype, float *__restrict__ imgm, long long n) {
     sx_pdl();
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) imgm[p] = sx_rel_var(__ldg(wmap + p), wtype) < 1e30f ? __ldg(img + p) : -1e30f;
+    const bool vec = ((reinterpret_cast<uintptr_t>(img) | reinterpret_cast<uintptr_t>(wmap) |
+                       reinterpret_cast<uintptr_t>(imgm)) & 15) == 0;
+    auto one = [&](float v, float w) { return sx_rel_var(w, wtype) < 1e30f ? v : -1e30f; };
+    map_words(n, vec, [&](long long p, bool four) {
+        if (four) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(img + p)),
+                         w = __ldg(reinterpret_cast<const float4 *>(wmap + p));
+            *reinterpret_cast<float4 *>(imgm + p) =
+                make_float4(one(v.x, w.x), one(v.y, w.y), one(v.z, w.z), one(v.w, w.w));
+        } else {
+            imgm[p] = one(__ldg(img + p), __ldg(wmap + p));
+        }
+    });
 }
 
 // one warp per mesh: exact mean of the relative variance over its usable
@@ -1298,16 +1329,25 @@ __global__ void k_weight_sigfac(const float *__restrict__ ratio, int nb, FrameSc
     if (threadIdx.x == 0) sc->sigfac = f;
 }
 
-__global__ void k_weight_var(const float *__restrict__ wmap, int wtype, const FrameScalars *sc,
-                             float *__restrict__ wvar, long long n) {
+__global__ void __launch_bounds__(256) k_weight_var(const float *__restrict__ wmap, int wtype, const FrameScalars *sc,
+                                                    float *__restrict__ wvar, long long n) {
     sx_pdl();
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const float sigfac = sc->sigfac, sigfac2 = sigfac * sigfac;
-    if (p < n) wvar[p] = sx_calib_var(__ldg(wmap + p), wtype, sigfac2);
+    const bool vec = ((reinterpret_cast<uintptr_t>(wmap) | reinterpret_cast<uintptr_t>(wvar)) & 15) == 0;
+    map_words(n, vec, [&](long long p, bool four) {
+        if (four) {
+            const float4 v = __ldg(reinterpret_cast<const float4 *>(wmap + p));
+            *reinterpret_cast<float4 *>(wvar + p) =
+                make_float4(sx_calib_var(v.x, wtype, sigfac2), sx_calib_var(v.y, wtype, sigfac2),
+                            sx_calib_var(v.z, wtype, sigfac2), sx_calib_var(v.w, wtype, sigfac2));
+        } else {
+            wvar[p] = sx_calib_var(__ldg(wmap + p), wtype, sigfac2);
+        }
+    });
 }
 
 void launch_weight_mask(const float *img, const float *wmap, int wtype, float *imgm, long long n, cudaStream_t st) {
-    if (n > 0) sx_launch(k_weight_mask, (unsigned)((n + 255) / 256), 256, 0, st, img, wmap, wtype, imgm, n);
+    if (n > 0) sx_launch(k_weight_mask, (unsigned)((n + WM_PIX - 1) / WM_PIX), 256, 0, st, img, wmap, wtype, imgm, n);
 }
 
 // after launch_background: sigfac from the filtered mesh rms map, then the
@@ -1321,7 +1361,7 @@ void launch_weight_var(const BackBufs &B, const float *wmap, const FrameParams &
                   B.sigma3, ratio);
         sx_launch(k_weight_sigfac, 1, 1024, 0, st, ratio, nb, d_sc);
     }
-    sx_launch(k_weight_var, (unsigned)((n + 255) / 256), 256, 0, st, wmap, P.wtype, d_sc, wvar, n);
+    sx_launch(k_weight_var, (unsigned)((n + WM_PIX - 1) / WM_PIX), 256, 0, st, wmap, P.wtype, d_sc, wvar, n);
 }
 
 void launch_background(BackBufs &B, const float *img, const FrameParams &P, FrameScalars *d_sc,

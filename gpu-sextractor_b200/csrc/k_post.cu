@@ -1029,13 +1029,19 @@ __global__ void k_write_apers(ObjBufs O, const unsigned *order, int ns, int nape
                                                              O.magerr_aper[o]);
 }
 
-// segmentation map: NUMBER of the owning object, 0 elsewhere
-__global__ void k_segmap(const int *alloc, const int *number, int *seg, long long npix) {
+// segmentation map: NUMBER of the owning object, 0 elsewhere; four pixels a
+// thread (both maps are 16-byte aligned buffers of the context)
+__global__ void __launch_bounds__(256) k_segmap(const int *alloc, const int *number, int *seg, long long npix) {
     sx_pdl();
-    long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long p = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
     if (p >= npix) return;
-    int a = alloc[p];
-    seg[p] = (a >= 0 && a != SX_ALLOC_OTHER) ? number[a] : 0;
+    auto num = [&](int a) { return a >= 0 && a != SX_ALLOC_OTHER ? __ldg(number + a) : 0; };
+    if (p + 3 < npix) {
+        const int4 a = *reinterpret_cast<const int4 *>(alloc + p);
+        *reinterpret_cast<int4 *>(seg + p) = make_int4(num(a.x), num(a.y), num(a.z), num(a.w));
+    } else {
+        for (long long q = p; q < npix; q++) seg[q] = num(alloc[q]);
+    }
 }
 
 }  // namespace sx

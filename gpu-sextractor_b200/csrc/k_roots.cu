@@ -13,43 +13,54 @@
 
 namespace sx {
 
-// Each raw object's thresholds: the smallest detection and analysis threshold
-// of its pixels (the global ones without a weight map); rdthr/rathr start at a
-// large positive float and are lowered through their bit patterns (positive
-// floats order like their bits).  The fixed-point scale of the exact branch
-// sums, sc->e0cd, becomes the exponent of the smallest of them.
-__global__ void k_root_thresholds(const int *__restrict__ lab, const int *__restrict__ cnt,
-                                  const int *__restrict__ rid, long long n, int minarea, const float *__restrict__ wvar,
-                                  int wthr, double dfac, double afac, FrameScalars *sc, int *rdthr, int *rathr) {
+// Each raw object's thresholds with a weight map: the smallest detection and
+// analysis threshold of its pixels.  A threshold is a factor times the root of
+// the variance, rounded, and so grows with the variance: the smallest variance
+// of the object's pixels gives both.  It is found over the compacted pixels
+// (positive floats order like their bits; in the warp first, since neighbouring
+// pixels mostly share their raw object, then by an atomic where it would lower
+// the value).  Two square roots in double and the labels of every pixel of the
+// frame took 2.6 ms of a 16384 x 16384 frame.
+__global__ void __launch_bounds__(256) k_root_minvar(const unsigned *__restrict__ erid,
+                                                     const unsigned *__restrict__ epix, int n, const int *n_dev,
+                                                     const float *__restrict__ wvar, int *__restrict__ rvar) {
     sx_pdl();
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int r = -1, idt = 0x7fffffff, iat = 0x7fffffff, e = 0x7fffffff;
-    if (p < n) {
-        const int l = lab[p];
-        if (l >= 0 && cnt[l] >= minarea) {
-            r = rid[l];
-            const float v = wvar ? __ldg(wvar + p) : 0.0f;
-            const float dt = sx_pix_thr(wthr, dfac, v, sc->dthresh), at = sx_pix_thr(wthr, afac, v, sc->thresh);
-            idt = __float_as_int(dt);
-            iat = __float_as_int(at);
+    const int j = blockIdx.x * 256 + threadIdx.x;
+    n = sx_count(n, n_dev);
+    if (blockIdx.x * 256 >= n) return;
+    int r = -1, v = 0x7fffffff;
+    if (j < n) {
+        r = (int)erid[j];
+        const float x = __ldg(wvar + epix[j]);
+        if (x >= 0.0f) v = __float_as_int(fabsf(x));
+    }
+    const unsigned grp = __match_any_sync(0xffffffffu, r);
+    if (r < 0) return;
+    v = __reduce_min_sync(grp, v);
+    if ((int)(threadIdx.x & 31) == __ffs(grp) - 1 && v < __ldcg(rvar + r)) atomicMin(rvar + r, v);
+}
+
+// the thresholds from those variances (in place of rvar); the fixed-point scale
+// of the exact branch sums, sc->e0cd, becomes the exponent of the smallest
+__global__ void k_root_thresholds(int nroots, const int *nroots_dev, double dfac, double afac, FrameScalars *sc,
+                                  float *rdthr, float *rathr) {
+    sx_pdl();
+    nroots = sx_count(nroots, nroots_dev);
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    int e = 0x7fffffff;
+    if (r < nroots) {
+        const int v = reinterpret_cast<const int *>(rdthr)[r];
+        float dt = __int_as_float(0x7f7f7f7f), at = dt;  // no usable variance
+        if (v < 0x7f7f7f7f) {
+            dt = sx_pix_thr(true, dfac, __int_as_float(v), 0.0f);
+            at = sx_pix_thr(true, afac, __int_as_float(v), 0.0f);
             e = fexpo(dt);
         }
+        rdthr[r] = dt;
+        rathr[r] = at;
     }
-    // the minima are taken in the warp first (neighbouring pixels mostly
-    // share their raw object), then one atomic per raw object and warp, and
-    // only where it would lower the value (the frame's minimum is one address:
-    // an atomic of every warp on it took 7 ms of a 16384 x 16384 frame)
     e = __reduce_min_sync(0xffffffffu, e);
     if ((threadIdx.x & 31) == 0 && e < *(volatile int *)&sc->e0cd) atomicMin(&sc->e0cd, e);
-    const unsigned grp = __match_any_sync(0xffffffffu, r);
-    if (r >= 0) {
-        idt = __reduce_min_sync(grp, idt);
-        iat = __reduce_min_sync(grp, iat);
-        if ((int)(threadIdx.x & 31) == __ffs(grp) - 1) {
-            if (idt < __ldcg(rdthr + r)) atomicMin(rdthr + r, idt);
-            if (iat < __ldcg(rathr + r)) atomicMin(rathr + r, iat);
-        }
-    }
 }
 
 // without a weight map every raw object has the global thresholds

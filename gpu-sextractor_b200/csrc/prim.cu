@@ -102,22 +102,49 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_one(const ScanArray A, co
     const ScanArray S = blockIdx.x ? B : A;
     n = dev_count(n, n_dev);
     int carry = 0;
+    // 16-byte words where the arrays are aligned (a thread's elements are
+    // consecutive: one at a time, a warp's loads touched 32 lines each)
+    const bool vec = ((reinterpret_cast<uintptr_t>(S.in) | reinterpret_cast<uintptr_t>(S.out)) & 15) == 0;
     for (int t0 = 0; t0 < n; t0 += SCAN_ONE_TILE) {
         const int base = t0 + threadIdx.x * SCAN_ONE_ITEMS;
+        const bool whole = vec && base + SCAN_ONE_ITEMS <= n;
         int v[SCAN_ONE_ITEMS], acc = 0;
+        if (whole) {
 #pragma unroll
-        for (int k = 0; k < SCAN_ONE_ITEMS; k++) {
-            v[k] = base + k < n ? S.in[base + k] : 0;
-            acc += v[k];
+            for (int k = 0; k < SCAN_ONE_ITEMS; k += 4) {
+                const int4 q = *reinterpret_cast<const int4 *>(S.in + base + k);
+                v[k] = q.x;
+                v[k + 1] = q.y;
+                v[k + 2] = q.z;
+                v[k + 3] = q.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < SCAN_ONE_ITEMS; k++) v[k] = base + k < n ? S.in[base + k] : 0;
         }
+#pragma unroll
+        for (int k = 0; k < SCAN_ONE_ITEMS; k++) acc += v[k];
         int tot;
         int pre = block_exclusive_scan(acc, sh, tot) + carry;
-#pragma unroll
-        for (int k = 0; k < SCAN_ONE_ITEMS; k++) {
-            if (base + k < n) S.out[base + k] = pre;
-            pre += v[k];
-        }
         carry += tot;
+        if (whole) {
+#pragma unroll
+            for (int k = 0; k < SCAN_ONE_ITEMS; k += 4) {
+                int4 q;
+                q.x = pre;
+                q.y = q.x + v[k];
+                q.z = q.y + v[k + 1];
+                q.w = q.z + v[k + 2];
+                pre = q.w + v[k + 3];
+                *reinterpret_cast<int4 *>(S.out + base + k) = q;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < SCAN_ONE_ITEMS; k++) {
+                if (base + k < n) S.out[base + k] = pre;
+                pre += v[k];
+            }
+        }
     }
     if (S.total && threadIdx.x == 0) *S.total = carry;
 }

@@ -743,11 +743,13 @@ int pipe_detect(sexgpu_ctx *ctx) {
     nl += 3 + exclusive_scan(R.size, R.off, nroots, nullptr, tmp, st, nroots_dev);
     sx_launch(k_root_compact, ntile, SCAN_THREADS, 0, st, lab, cnt, N, Pm.minarea, tkoff, flag,
               P<unsigned>(ctx->keys), P<unsigned>(ctx->rpix), P<int>(ctx->alloc), P<int>(ctx->pos2idx));
-    if (ps.wvar) {
+    if (ps.wvar && Pm.wthr) {
         CK(cudaMemsetAsync(R.dthresh, 0x7f, (size_t)(nroots + 1) * 4, st));
-        CK(cudaMemsetAsync(R.thresh, 0x7f, (size_t)(nroots + 1) * 4, st));
-        sx_launch(k_root_thresholds, grid1(N, 256), 256, 0, st, lab, cnt, flag, N, Pm.minarea, ps.wvar, Pm.wthr,
-                  Pm.detect_thresh, Pm.analysis_thresh, d_sc, (int *)R.dthresh, (int *)R.thresh);
+        sx_launch(k_root_minvar, grid1(nrootpix, 256), 256, 0, st, P<unsigned>(ctx->keys), P<unsigned>(ctx->rpix),
+                  nrootpix, ps.capf ? &d_sc->nrootpix : nullptr, ps.wvar, (int *)R.dthresh);
+        sx_launch(k_root_thresholds, grid1(nroots, 256), 256, 0, st, nroots, nroots_dev, Pm.detect_thresh,
+                  Pm.analysis_thresh, d_sc, R.dthresh, R.thresh);
+        nl += 1;
     } else {
         sx_launch(k_root_thresholds_global, grid1(nroots, 256), 256, 0, st, nroots, nroots_dev, d_sc, R.dthresh,
                   R.thresh);
@@ -1575,7 +1577,7 @@ int sexgpu_copy_results(sexgpu_ctx *ctx, sexgpu_object *objs, int max_objects, i
     }
     if (segmap && N > 0) {
         EN(seg, N * 4);
-        sx_launch(k_segmap, grid1(N, 256), 256, 0, st, P<int>(ctx->alloc), ctx->O.number, P<int>(ctx->seg), N);
+        sx_launch(k_segmap, grid1(N, 1024), 256, 0, st, P<int>(ctx->alloc), ctx->O.number, P<int>(ctx->seg), N);
         CK(cudaMemcpyAsync(segmap, ctx->seg.p, N * 4, cudaMemcpyDeviceToHost, st));
     }
     if (sub && N > 0) CK(cudaMemcpyAsync(sub, ctx->sub.p, N * 4, cudaMemcpyDeviceToHost, st));
