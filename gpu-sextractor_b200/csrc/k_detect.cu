@@ -21,10 +21,6 @@ struct ConvTaps {
     float m[121];
 };
 
-constexpr int SF_TW = 32;   // output tile width
-constexpr int SF_TH = 16;   // output tile height
-constexpr int SF_TX = 32, SF_TY = 8;
-
 // background at (x, y) from the per-row node splines (src/back.c:863-899)
 __device__ __forceinline__ float bkg_at(int x, int y, const BackBufs &B, int nbx, int back_type, float backmean) {
     if (back_type == 1) return backmean;
@@ -49,135 +45,39 @@ __global__ void k_back_map(BackBufs B, int nbx, int back_type, const FrameScalar
     out[p] = bkg_at(x, y, B, nbx, back_type, sc->backmean);
 }
 
-__global__ void __launch_bounds__(SF_TX *SF_TY) k_sub_filter(const float *__restrict__ img, float *__restrict__ sub,
-                                                              float *__restrict__ cd, int *__restrict__ lab,
-                                                              BackBufs B, int w, int h, int nbx, int back_type,
-                                                              const float *__restrict__ mask, int mw, int mh,
-                                                              const float *__restrict__ wvar, int wthr, double dfac,
-                                                              FrameScalars *sc) {
-    sx_pdl();
-    extern __shared__ float tile[];
-    const int rx = mw / 2, ry = mh / 2;
-    const int TWp = SF_TW + mw - 1, THp = SF_TH + mh - 1;
-    const int x0 = blockIdx.x * SF_TW, y0 = blockIdx.y * SF_TH;
-    const float backmean = sc->backmean, dthresh = sc->dthresh;
-    const int tid = threadIdx.y * SF_TX + threadIdx.x;
-    int emin = 1000;
-    for (int i = tid; i < TWp * THp; i += SF_TX * SF_TY) {
-        int ty = i / TWp, tx = i - ty * TWp;
-        int gx = x0 - rx + tx, gy = y0 - ry + ty;
-        float s = 0.0f;
-        if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
-            float raw = sx_unblank(__ldg(img + (size_t)gy * w + gx));
-            s = raw - bkg_at(gx, gy, B, nbx, back_type, backmean);
-            if (tx >= rx && tx < rx + SF_TW && ty >= ry && ty < ry + SF_TH) {
-                sub[(size_t)gy * w + gx] = s;
-                unsigned ef = (__float_as_uint(s) >> 23) & 0xff;
-                if (ef) emin = min(emin, (int)ef - 127);
-            }
-        }
-        tile[i] = s;
-    }
-    __syncthreads();
-    int nabove = 0;
-    for (int r = threadIdx.y; r < SF_TH; r += SF_TY) {
-        int gx = x0 + threadIdx.x, gy = y0 + r;
-        bool in = gx < w && gy < h;
-        float acc = 0.0f;
-        if (in) {
-            const float *t0 = tile + r * TWp + threadIdx.x;
-            for (int j = 0; j < mh; j++) {
-                const float *tr = t0 + j * TWp;
-                const float *mk = mask + j * mw;
-                for (int i = 0; i < mw; i++) acc += mk[i] * tr[i];
-            }
-            size_t p = (size_t)gy * w + gx;
-            cd[p] = acc;
-            const float v = wvar ? __ldg(wvar + p) : 0.0f;
-            bool fg = !(wvar && !(v < 1e30f)) && acc >= sx_pix_thr(wthr, dfac, v, dthresh);
-            lab[p] = fg ? (int)p : -1;
-            nabove += fg;
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        nabove += __shfl_down_sync(0xffffffffu, nabove, o);
-        emin = min(emin, __shfl_down_sync(0xffffffffu, emin, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (nabove) atomicAdd(&sc->npix_above, nabove);
-        if (emin < 1000) atomicMin(&sc->e0sub, emin);
-    }
-}
-
 // ---------------------------------------------------------------------------
-// The same stage with the frame tile (halo included) brought into shared
-// memory by one TMA load (cp.async.bulk.tensor, zero fill outside the frame),
-// 64x32 output pixels per CTA and the tile's spline column table staged in
-// shared memory.  Needs rows of a multiple of 16 bytes and a 16-byte aligned
-// frame; other frames take k_sub_filter.
+// Background subtraction, detection filter, threshold and tile-local labels in
+// one pass over the frame.
+//
+// Bound by issue slots (a 7x7 mask is 98 separately rounded multiplies and adds
+// a pixel against 16 bytes), so the rest of the work is kept to few
+// instructions: 64 x 32 output tiles on persistent CTAs, the next tile (halo
+// included) in flight into a second buffer while this one is computed.  A
+// thread subtracts the background from quads of one column position, whose
+// spline constants stay in its registers for all the tile's rows, then filters
+// 4 columns x 2 rows from 16-byte shared-memory words and writes 16-byte words;
+// tiles without foreground skip the labelling.  With one column of 8 rows a
+// thread, one pixel a store and lanes 18 to 31 idle over the background,
+// 4096 x 4096 pixels with a 7x7 mask took 233 us and 336 warp instructions per
+// 32 pixels, now 133 us and 193 (98 of them the mask's); a crowded field under
+// a 5x5 mask 304, now 169 us; a weighted 16384 x 16384 frame 5.9, now 3.4 ms.
+// Multiplies and adds of register pairs save a quarter of the instructions but
+// no time (138 us: the pairs go through the pipe at half the rate).
+//
+// Frames whose rows are not a multiple of 16 bytes, or that do not start on a
+// 16-byte boundary, cannot be brought in by TMA: for those (TMA = false) the
+// tile comes by 4-byte asynchronous copies and the results go out a pixel at a
+// time.  Under a kernel of their own, labelled in a pass of its own, a frame of
+// 1023 x 1023 took 35 us here and 34 us for its components, now 17 and 18.
 // ---------------------------------------------------------------------------
 constexpr int ST_TW = 64, ST_TH = 32, ST_THREADS = 256;
-constexpr int ST_MAXBW = ST_TW + 2 * 16, ST_MAXBH = ST_TH + 2 * 15;  // masks up to 31x31
-constexpr unsigned ST_WAIT_LIMIT = 1u << 24;                       // polls of the load barrier
-
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-constexpr int ST_RPT = 8;  // output rows per thread (64 columns x 4 row groups x 8 rows)
-
-// Convolution of one output column segment (rows r0..r0+ST_RPT-1) from the
-// shared tile.  Each input row is read once and added into every output row
-// it serves; an output receives its terms in mask row-major order (mask rows
-// in increasing order, columns left to right), as convolve() adds them.
-template <int MW, int MH>
-__device__ __forceinline__ void conv_rows(const ConvTaps &taps, const float *__restrict__ tile, int bw, int c0, int r0,
-                                          float *acc) {
-#pragma unroll
-    for (int k = 0; k < ST_RPT; k++) acc[k] = 0.0f;
-#pragma unroll
-    for (int R = 0; R < ST_RPT + MH - 1; R++) {
-        float v[MW];
-        const float *row = tile + (r0 + R) * bw + c0;
-#pragma unroll
-        for (int i = 0; i < MW; i++) v[i] = row[i];
-#pragma unroll
-        for (int k = 0; k < ST_RPT; k++) {
-            const int j = R - k;
-            if (j >= 0 && j < MH) {
-#pragma unroll
-                for (int i = 0; i < MW; i++) acc[k] += taps.m[j * MW + i] * v[i];
-            }
-        }
-    }
-}
-
-// any mask size (runtime loops, same order)
-__device__ __forceinline__ void conv_rows_any(const float *__restrict__ mask, const float *__restrict__ tile, int bw,
-                                              int c0, int r0, int mw, int mh, float *acc) {
-    for (int k = 0; k < ST_RPT; k++) {
-        const float *t0 = tile + (r0 + k) * bw + c0;
-        float s = 0.0f;
-        for (int j = 0; j < mh; j++) {
-            const float *tr = t0 + j * bw;
-            const float *mk = mask + j * mw;
-            for (int i = 0; i < mw; i++) s += mk[i] * tr[i];
-        }
-        acc[k] = s;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Persistent form: each CTA walks tiles t, t + G, ... with two tile buffers;
-// the TMA load of the next tile is in flight while the current one is
-// subtracted, filtered and thresholded.  Per tile the spline column constants
-// (segment, dx, 1 - dx and the two cubic factors, all the float values the
-// per-pixel formula uses) sit in each lane's registers (a lane keeps its four
-// columns for the whole tile) and the row nodes of the tile's rows are staged
-// in shared memory, so the per-pixel background is shared-memory reads and
-// float arithmetic in the reference's order.
-// ---------------------------------------------------------------------------
-constexpr int SP_NK = 16;  // staged spline nodes per row (segments touching a tile + 1)
+constexpr int ST_MAXBH = ST_TH + 2 * 15;      // masks up to 31x31
+constexpr unsigned ST_WAIT_LIMIT = 1u << 24;  // polls of the load barrier
+constexpr int ST_QR = 2;                      // output rows of a thread's quads (16 quads x 16 row pairs)
+constexpr int SP_NK = 16;                     // staged spline nodes per row (segments touching a tile + 1)
 
 struct SpArgs {
+    const float *img;
     float *sub, *cd;
     int *lab;
     BackBufs B;
@@ -186,6 +86,64 @@ struct SpArgs {
     const float *mask, *wvar;
     FrameScalars *sc;
 };
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+// Convolution of one quad of output columns in rows r0, r0 + 1 from the shared
+// tile.  Each input row is read once and added into the output rows it serves;
+// an output receives its terms in mask row-major order (mask rows in increasing
+// order, columns left to right), as convolve() adds them.
+template <int MW, int MH>
+__device__ __forceinline__ void conv_quad(const ConvTaps &taps, const float *__restrict__ tile, int bw, int quad,
+                                          int r0, float (&acc)[ST_QR][4]) {
+    constexpr int RXA = ((MW / 2) + 3) & ~3, OFF = RXA - MW / 2, NQ = (OFF + MW + 2) / 4 + 1;
+#pragma unroll
+    for (int k = 0; k < ST_QR; k++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[k][c] = 0.0f;
+#pragma unroll
+    for (int R = 0; R < ST_QR + MH - 1; R++) {
+        float v[4 * NQ];
+        const float4 *row = reinterpret_cast<const float4 *>(tile + (r0 + R) * bw) + quad;
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const float4 f = row[q];
+            v[4 * q] = f.x;
+            v[4 * q + 1] = f.y;
+            v[4 * q + 2] = f.z;
+            v[4 * q + 3] = f.w;
+        }
+#pragma unroll
+        for (int k = 0; k < ST_QR; k++) {
+            const int j = R - k;
+            if (j >= 0 && j < MH) {
+#pragma unroll
+                for (int i = 0; i < MW; i++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) acc[k][c] += taps.m[j * MW + i] * v[OFF + i + c];
+            }
+        }
+    }
+}
+
+// any mask size (runtime loops, same order); c0: tile column of the first tap
+__device__ __forceinline__ void conv_quad_any(const float *__restrict__ mask, const float *__restrict__ tile, int bw,
+                                              int c0, int r0, int mw, int mh, float (&acc)[ST_QR][4]) {
+#pragma unroll
+    for (int k = 0; k < ST_QR; k++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[k][c] = 0.0f;
+    for (int j = 0; j < mh; j++) {
+        const float *t0 = tile + (r0 + j) * bw + c0;
+        for (int i = 0; i < mw; i++) {
+            const float m = __ldg(mask + j * mw + i);
+#pragma unroll
+            for (int k = 0; k < ST_QR; k++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) acc[k][c] += m * t0[k * bw + i + c];
+        }
+    }
+}
 
 __device__ __forceinline__ void sp_issue(const CUtensorMap *tmap, float *buf, unsigned bar, int x, int y,
                                          unsigned bytes) {
@@ -198,6 +156,24 @@ __device__ __forceinline__ void sp_issue(const CUtensorMap *tmap, float *buf, un
         : "memory");
 }
 
+// the tile at (x, y) by 4-byte asynchronous copies, a warp per row; zero outside
+// the frame (a copy of no bytes fills its destination with zeros)
+__device__ __forceinline__ void sp_copy(const SpArgs &A, float *buf, int x, int y, int bw, int bh) {
+    const int lane = threadIdx.x & 31;
+    for (int ty = threadIdx.x >> 5; ty < bh; ty += ST_THREADS / 32) {
+        const int gy = y + ty;
+        const bool rin = gy >= 0 && gy < A.h;
+        const float *row = A.img + (size_t)(rin ? gy : 0) * A.w;
+        for (int tx = lane; tx < bw; tx += 32) {
+            const int gx = x + tx;
+            const bool in = rin && gx >= 0 && gx < A.w;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(buf + ty * bw + tx)),
+                         "l"(row + (in ? gx : 0)), "r"(in ? 4 : 0)
+                         : "memory");
+        }
+    }
+}
+
 __device__ __forceinline__ bool sp_wait(unsigned bar, unsigned parity) {
     unsigned done = 0;
     for (unsigned it = 0; it < ST_WAIT_LIMIT && !done; it++)
@@ -207,6 +183,21 @@ __device__ __forceinline__ bool sp_wait(unsigned bar, unsigned parity) {
             : "r"(bar), "r"(parity)
             : "memory");
     return done != 0;
+}
+
+// acc >= the pixel's threshold, the float nearest to fac * sqrt(var) in double:
+// an approximate threshold (its error below 5e-7 of it) decides unless acc is
+// within 1e-5 of it, so that the double-precision root is rarely taken
+__device__ __forceinline__ bool above_pix_thr(float acc, bool wthr, double fac, float var, float global) {
+    if (!wthr) return acc >= global;
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(var));
+    const float t = (float)fac * r;
+    if (t > 1e-30f && t < 1e30f) {
+        if (acc > t * 1.00001f) return true;
+        if (acc < t * 0.99999f) return false;
+    }
+    return acc >= sx_pix_thr(true, fac, var, global);
 }
 
 // ---- union-find in shared memory (tile-local components)
@@ -231,227 +222,285 @@ __device__ __forceinline__ void sunion(int *L, int a, int b) {
     }
 }
 
-// runs of foreground bits in a row mask
-__device__ __forceinline__ int run_start(unsigned starts, int b) {  // start bit of the run holding bit b
-    return 31 - __clz(starts & (0xffffffffu >> (31 - b)));
-}
-__device__ __forceinline__ int run_end(unsigned m, int b) {  // last bit of the run holding bit b
-    return b + __ffsll(~(unsigned long long)(m >> b)) - 2;     // 64-bit: a run may reach bit 31
-}
-
-// the same on 64-bit row masks (the subtract/filter kernel's 64-pixel tile rows)
-__device__ __forceinline__ int run_start64(unsigned long long starts, int b) {
+// runs of foreground bits in a 64-pixel row mask
+__device__ __forceinline__ int run_start64(unsigned long long starts, int b) {  // start of the run holding bit b
     return 63 - __clzll((long long)(starts & (~0ull >> (63 - b))));
 }
-__device__ __forceinline__ int run_end64(unsigned long long m, int b) {
+__device__ __forceinline__ int run_end64(unsigned long long m, int b) {  // last bit of the run holding bit b
     const unsigned long long r = ~(m >> b);
     return r ? b + __ffsll((long long)r) - 2 : 63;
 }
 
-template <int MW, int MH, bool WEIGHTED>
-__global__ void __launch_bounds__(ST_THREADS, 4) k_sub_filter_pipe(const __grid_constant__ CUtensorMap tmap,
-                                                                const __grid_constant__ SpArgs A,
-                                                                const __grid_constant__ ConvTaps taps) {
+template <int MW, int MH, bool WEIGHTED, bool TMA>
+__global__ void __launch_bounds__(ST_THREADS, 4) k_sub_filter(const __grid_constant__ CUtensorMap tmap,
+                                                           const __grid_constant__ SpArgs A,
+                                                           const __grid_constant__ ConvTaps taps) {
     sx_pdl();
     extern __shared__ __align__(128) float sp_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
-    __shared__ float s_nd[ST_MAXBH][SP_NK], s_dnd[ST_MAXBH][SP_NK];
-    __shared__ int s_kmin, s_nk;
-    __shared__ unsigned s_rowh[ST_TH][2];  // tile rows' foreground, two 32-bit halves
-    __shared__ int s_L[ST_TH * ST_TW];     // tile-local union-find
+    __shared__ float2 s_nd[ST_MAXBH][SP_NK + 1];   // spline nodes (value, second derivative) of the tile's rows
+    __shared__ unsigned long long s_row[ST_TH];    // the tile rows' foreground
+    __shared__ int s_L[ST_TH * ST_TW];             // tile-local union-find, set at the runs' first pixels
     const int mw = MW > 0 ? MW : A.mw, mh = MH > 0 ? MH : A.mh;
-    const int rx = mw / 2, ry = mh / 2, rxa = A.rxa;
+    const int rx = mw / 2, ry = mh / 2, rxa = MW > 0 ? ((MW / 2) + 3) & ~3 : A.rxa;
     const int bw = ST_TW + 2 * rxa, bh = ST_TH + 2 * ry;
     const int tsz = (bw * bh + 31) & ~31;  // floats per tile buffer (128-byte multiple)
     float *const buf0 = sp_smem, *const buf1 = sp_smem + tsz;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
     const int w = A.w, h = A.h;
     const unsigned bar0 = smem_u32(&bars[0]), bar1 = smem_u32(&bars[1]);
     const unsigned tbytes = (unsigned)(bw * bh * 4);
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0), "r"(1));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar1), "r"(1));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (TMA) {
+        if (tid == 0) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0), "r"(1));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar1), "r"(1));
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncthreads();
     }
-    __syncthreads();
+    auto load = [&](int t, int b) {  // tile t into buffer b
+        const int x = (t % A.tilesx) * ST_TW - rxa, y = (t / A.tilesx) * ST_TH - ry;
+        if (TMA) {
+            if (tid == 0 && t < A.ntiles) sp_issue(&tmap, b ? buf1 : buf0, b ? bar1 : bar0, x, y, tbytes);
+        } else {
+            if (t < A.ntiles) sp_copy(A, b ? buf1 : buf0, x, y, bw, bh);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+    };
     int t = blockIdx.x;
-    if (tid == 0 && t < A.ntiles)
-        sp_issue(&tmap, buf0, bar0, (t % A.tilesx) * ST_TW - rxa, (t / A.tilesx) * ST_TH - ry, tbytes);
+    load(t, 0);
     const float backmean = A.sc->backmean, dthresh = A.sc->dthresh;
-    int emin = 1000, nabove = 0;
+    const bool spline = A.back_type != 1 && A.nbx > 1;
+    // the background's part: one quad of the tile's columns, every rpp-th row
+    const int nq = bw / 4, rpp = ST_THREADS / nq, brow = tid / nq, bq = tid - brow * nq;
+    const bool bcol = brow < rpp, binner = 4 * bq >= rxa && 4 * bq < rxa + ST_TW;
+    // the filter's part: one quad of the output columns in two rows
+    const int qc = tid & 15, r0 = (tid >> 4) * ST_QR;
+    int nabove = 0;
     bool failed = false;
     for (int it = 0; t < A.ntiles; it++, t += gridDim.x) {
         const int cur = it & 1;
         float *const tile = cur ? buf1 : buf0;
         const int x0 = (t % A.tilesx) * ST_TW, y0 = (t / A.tilesx) * ST_TH;
-        // next tile into the other buffer (free: the previous iteration ended
-        // with a barrier after its last read)
-        const int tn = t + gridDim.x;
-        if (tid == 0 && tn < A.ntiles)
-            sp_issue(&tmap, cur ? buf0 : buf1, cur ? bar0 : bar1, (tn % A.tilesx) * ST_TW - rxa,
-                     (tn / A.tilesx) * ST_TH - ry, tbytes);
-        // spline row nodes of this tile's rows, while the load is in flight
-        const int gxa = x0 - rxa;
-        const bool spline = A.back_type != 1 && A.nbx > 1;
-        if (spline && tid == 0) {
-            const int ka = A.B.colk[max(gxa, 0)], kb = A.B.colk[min(gxa + bw, w) - 1];
-            s_kmin = ka;
-            s_nk = kb - ka + 2;
-        }
-        __syncthreads();
-        const int kmin = spline ? s_kmin : 0, nk = spline ? s_nk : 0;
-        const bool staged = nk <= SP_NK;
-        if (spline && staged)
-            for (int i = tid; i < bh * nk; i += ST_THREADS) {
-                const int ty = i / nk, j = i - ty * nk, gy = y0 - ry + ty;
-                const int k = min(kmin + j, A.nbx - 1);
-                const bool in = gy >= 0 && gy < h;
-                s_nd[ty][j] = in ? A.B.rownode[(size_t)gy * A.nbx + k] : 0.0f;
-                s_dnd[ty][j] = in ? A.B.rowdnode[(size_t)gy * A.nbx + k] : 0.0f;
-            }
-        // this lane's tile columns: 4*lane .. 4*lane+3 (lanes beyond the tile idle)
-        int ck[4];
+        // next tile into the other buffer (free: its last reads came before
+        // this iteration's predecessor's barrier after the filter)
+        load(t + gridDim.x, cur ^ 1);
+        // while the load is in flight, the spline nodes of this tile's rows and
+        // the column constants of this thread's quad
+        const int gxa = x0 - rxa, qx = gxa + 4 * bq;
+        const int nin = bcol && qx >= 0 ? min(max(w - qx, 0), 4) : 0;  // its columns in the frame
+        int kmin = 0, k0 = 0;
+        bool staged = true, step[4];
         float cdx[4], cb[4], cx[4], cdd[4];
-        bool cin[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int tx = 4 * lane + q, gx = gxa + tx;
-            cin[q] = tx < bw && gx >= 0 && gx < w;
-            const int gxc = min(max(gx, 0), w - 1);
-            const float dx = A.B.coldx[gxc];
-            ck[q] = A.B.colk[gxc] - kmin;
-            cx[q] = dx;
-            cdx[q] = 1 - dx;
-            cb[q] = cdx[q] * cdx[q] - 1;
-            cdd[q] = dx * dx - 1;
-        }
-        // every thread polls; the outcome is made uniform before anyone acts on it
-        if (!__syncthreads_and(sp_wait(cur ? bar1 : bar0, (unsigned)((it >> 1) & 1)))) {
-            failed = true;
-            break;
-        }
-        // subtract the background in place, one warp per tile row, four
-        // columns per lane; outside the frame the value is 0
-        for (int ty = wid; ty < bh; ty += ST_THREADS / 32) {
-            const int gy = y0 - ry + ty;
-            if (4 * lane >= bw) continue;
-            float4 *tp = reinterpret_cast<float4 *>(tile + ty * bw) + lane;
-            float4 v = *tp;
-            float *vv = reinterpret_cast<float *>(&v);
-            const bool rin = gy >= 0 && gy < h;
-            const bool inner = ty >= ry && ty < ry + ST_TH;
-            float *srow = A.sub + (size_t)(rin ? gy : 0) * w;
+        if (spline) {
+            kmin = __ldg(A.B.colk + max(gxa, 0));
+            const int nk = __ldg(A.B.colk + min(gxa + bw, w) - 1) - kmin + 2;
+            staged = nk <= SP_NK;
+            if (staged)
+                for (int j = tid & 3; j < nk; j += 4)
+                    for (int ty = tid >> 2; ty < bh; ty += ST_THREADS / 4) {
+                        const int gy = y0 - ry + ty;
+                        const size_t o = (size_t)gy * A.nbx + min(kmin + j, A.nbx - 1);
+                        if (gy >= 0 && gy < h) s_nd[ty][j] = make_float2(__ldg(A.B.rownode + o), __ldg(A.B.rowdnode + o));
+                    }
+            int kp = 0;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                float s = 0.0f;
-                if (rin && cin[q]) {
-                    float b;
-                    if (!spline) {
-                        b = A.back_type == 1 ? backmean : __ldg(A.B.rownode + (size_t)gy * A.nbx);
-                    } else if (staged) {
-                        const int k = ck[q];
-                        b = (float)(cdx[q] * (s_nd[ty][k] + cb[q] * s_dnd[ty][k]) +
-                                    cx[q] * (s_nd[ty][k + 1] + cdd[q] * s_dnd[ty][k + 1]));
-                    } else {
-                        const float *nd = A.B.rownode + (size_t)gy * A.nbx, *dnd = A.B.rowdnode + (size_t)gy * A.nbx;
-                        const int k = ck[q] + kmin;
-                        b = (float)(cdx[q] * (__ldg(nd + k) + cb[q] * __ldg(dnd + k)) +
-                                    cx[q] * (__ldg(nd + k + 1) + cdd[q] * __ldg(dnd + k + 1)));
-                    }
-                    s = sx_unblank(vv[q]) - b;
-                    const int tx = 4 * lane + q;
-                    if (inner && tx >= rxa && tx < rxa + ST_TW) {
-                        srow[gxa + tx] = s;
-                        const unsigned ef = (__float_as_uint(s) >> 23) & 0xff;
-                        if (ef) emin = min(emin, (int)ef - 127);
-                    }
-                }
-                vv[q] = s;
+                const int x = min(max(qx + q, 0), w - 1);
+                const float dx = __ldg(A.B.coldx + x);
+                const int k = __ldg(A.B.colk + x) - kmin;
+                if (q == 0) k0 = k;
+                step[q] = q > 0 && k != kp;  // the next segment begins here
+                kp = k;
+                cx[q] = dx;
+                cdx[q] = 1 - dx;
+                cb[q] = cdx[q] * cdx[q] - 1;
+                cdd[q] = dx * dx - 1;
             }
-            *tp = v;
         }
-        __syncthreads();
-        // convolution, threshold, label seed: one column, ST_RPT rows per thread
-        const int cxo = tid & (ST_TW - 1), r0 = (tid / ST_TW) * ST_RPT;
-        float acc[ST_RPT];
-        if constexpr (MW > 0)
-            conv_rows<MW, MH>(taps, tile, bw, cxo + rxa - rx, r0, acc);
-        else
-            conv_rows_any(A.mask, tile, bw, cxo + rxa - rx, r0, mw, mh, acc);
-        const int gx = x0 + cxo;
-        unsigned fgb = 0u;  // bit k: pixel (cxo, r0 + k) above its threshold
+        if (TMA) {
+            // every thread polls; the outcome is made uniform before anyone acts on it
+            if (!__syncthreads_and(sp_wait(cur ? bar1 : bar0, (unsigned)((it >> 1) & 1)))) {
+                failed = true;
+                break;
+            }
+        } else {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+        }
+        // subtract the background in place; outside the frame the loads left 0
+        if (nin > 0)
+            for (int ty = brow; ty < bh; ty += rpp) {
+                const int gy = y0 - ry + ty;
+                if (gy < 0 || gy >= h) continue;
+                float4 *tp = reinterpret_cast<float4 *>(tile + ty * bw) + bq;
+                float4 v4 = *tp;
+                float v[4] = {v4.x, v4.y, v4.z, v4.w}, b[4];
+                if (!spline) {
+                    b[0] = A.back_type == 1 ? backmean : __ldg(A.B.rownode + (size_t)gy * A.nbx);
+                    b[1] = b[2] = b[3] = b[0];
+                } else if (staged) {
+                    const float2 *nd = s_nd[ty] + k0;
+                    float2 lo = nd[0], hi = nd[1];
 #pragma unroll
-        for (int k = 0; k < ST_RPT; k++) {
-            const int gy = y0 + r0 + k;
-            if (gx < w && gy < h) {
-                const int p = gy * w + gx;
-                A.cd[p] = acc[k];
-                bool fg;
-                if (WEIGHTED) {
-                    const float v = __ldg(A.wvar + p);
-                    fg = (v < 1e30f) && acc[k] >= sx_pix_thr(A.wthr, A.dfac, v, dthresh);
+                    for (int q = 0; q < 4; q++) {
+                        if (step[q]) {
+                            nd++;
+                            lo = hi;
+                            hi = nd[1];
+                        }
+                        b[q] = cdx[q] * (lo.x + cb[q] * lo.y) + cx[q] * (hi.x + cdd[q] * hi.y);
+                    }
                 } else {
-                    fg = acc[k] >= dthresh;
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        b[q] = bkg_at(min(qx + q, w - 1), gy, A.B, A.nbx, A.back_type, backmean);
                 }
-                fgb |= (unsigned)fg << k;
-                nabove += fg;
+#pragma unroll
+                for (int q = 0; q < 4; q++) v[q] = TMA || q < nin ? sx_unblank(v[q]) - b[q] : 0.0f;
+                v4 = make_float4(v[0], v[1], v[2], v[3]);
+                *tp = v4;
+                if (binner && ty >= ry && ty < ry + ST_TH) {
+                    float *out = A.sub + (size_t)gy * w + qx;
+                    if (TMA) {
+                        *reinterpret_cast<float4 *>(out) = v4;
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; q++)
+                            if (q < nin) out[q] = v[q];
+                    }
+                }
+            }
+        __syncthreads();
+        // convolution and threshold
+        float acc[ST_QR][4];
+        if constexpr (MW > 0)
+            conv_quad<MW, MH>(taps, tile, bw, qc, r0, acc);
+        else
+            conv_quad_any(A.mask, tile, bw, 4 * qc + rxa - rx, r0, mw, mh, acc);
+        const int gx = x0 + 4 * qc, ncol = min(max(w - gx, 0), 4);
+        unsigned nib[ST_QR];  // bit c of nib[k]: pixel (gx + c, r0 + k) at or above its threshold
+#pragma unroll
+        for (int k = 0; k < ST_QR; k++) {
+            const int gy = y0 + r0 + k;
+            nib[k] = 0u;
+            if (gy < h && ncol > 0) {
+                const size_t p = (size_t)gy * w + gx;
+                float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                if (TMA) {
+                    *reinterpret_cast<float4 *>(A.cd + p) = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+                    if (WEIGHTED) {
+                        const float4 f = __ldg(reinterpret_cast<const float4 *>(A.wvar + p));
+                        v[0] = f.x;
+                        v[1] = f.y;
+                        v[2] = f.z;
+                        v[3] = f.w;
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        if (c < ncol) {
+                            A.cd[p + c] = acc[k][c];
+                            if (WEIGHTED) v[c] = __ldg(A.wvar + p + c);
+                        }
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    bool fg;
+                    if (WEIGHTED)
+                        fg = (v[c] < 1e30f) && above_pix_thr(acc[k][c], A.wthr, A.dfac, v[c], dthresh);
+                    else
+                        fg = acc[k][c] >= dthresh;
+                    if (TMA || c < ncol) nib[k] |= (unsigned)fg << c;
+                }
+                nabove += __popc(nib[k]);
             }
         }
         // Components within the tile (the first step of the CCL, done here
         // while the tile's foreground is on chip): each tile row's foreground
-        // as 64 bits from two ballots; the pixels of a horizontal run join
-        // the run's first pixel; a run joins the runs of the row above that
-        // touch it or its diagonal ends.  Every link goes to a smaller tile
-        // index, so a tile component ends at its smallest pixel, which is
-        // written as the label of each of its pixels (global index).
+        // as 64 bits, gathered from the 16 lanes of the row; the pixels of a
+        // horizontal run have the run's first pixel as their tile label; a run
+        // joins the runs of the row above that touch it or its diagonal ends.
+        // Every link goes to a smaller tile index, so a tile component ends at
+        // its smallest pixel, which is written as the label of each of its
+        // pixels (global index).
+        unsigned long long m[ST_QR];
+        const bool wany = __any_sync(0xffffffffu, (nib[0] | nib[1]) != 0u);
 #pragma unroll
-        for (int k = 0; k < ST_RPT; k++) {
-            const unsigned m = __ballot_sync(0xffffffffu, (fgb >> k) & 1u);
-            if (lane == 0) s_rowh[r0 + k][cxo >> 5] = m;
-        }
-        __syncthreads();
+        for (int k = 0; k < ST_QR; k++) {
+            m[k] = 0ull;
+            if (wany) {
+                unsigned a = nib[k] << (4 * (lane & 7));
+                a |= __shfl_xor_sync(0xffffffffu, a, 1);
+                a |= __shfl_xor_sync(0xffffffffu, a, 2);
+                a |= __shfl_xor_sync(0xffffffffu, a, 4);
+                const unsigned o = __shfl_xor_sync(0xffffffffu, a, 8);
+                m[k] = lane & 8 ? ((unsigned long long)a << 32) | o : ((unsigned long long)o << 32) | a;
+                const unsigned long long st = m[k] & ~(m[k] << 1);
 #pragma unroll
-        for (int k = 0; k < ST_RPT; k++) {
-            const int ty = r0 + k, t = ty * ST_TW + cxo;
-            const unsigned long long m = ((unsigned long long)s_rowh[ty][1] << 32) | s_rowh[ty][0];
-            s_L[t] = (fgb >> k) & 1u ? ty * ST_TW + run_start64(m & ~(m << 1), cxo) : -1;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < ST_RPT; k++) {
-            const int ty = r0 + k;
-            if (!((fgb >> k) & 1u) || ty == 0) continue;
-            const unsigned long long m = ((unsigned long long)s_rowh[ty][1] << 32) | s_rowh[ty][0];
-            if (!((m >> cxo) & 1ull) || (cxo > 0 && ((m >> (cxo - 1)) & 1ull))) continue;  // run starts only
-            const int e = run_end64(m, cxo);
-            const int s1 = cxo > 0 ? cxo - 1 : 0, e1 = e < 63 ? e + 1 : 63;
-            const unsigned long long dil = (e1 == 63 ? ~0ull : ((2ull << e1) - 1ull)) & ~((1ull << s1) - 1ull);
-            const unsigned long long mp = ((unsigned long long)s_rowh[ty - 1][1] << 32) | s_rowh[ty - 1][0];
-            const unsigned long long sp = mp & ~(mp << 1);
-            unsigned long long ov = mp & dil;
-            while (ov) {
-                const int b = __ffsll((long long)ov) - 1;
-                sunion(s_L, ty * ST_TW + cxo, (ty - 1) * ST_TW + run_start64(sp, b));
-                const int eb = run_end64(mp, b);
-                ov = eb >= 63 ? 0ull : ov & ~((2ull << eb) - 1ull);
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < ST_RPT; k++) {
-            const int gy = y0 + r0 + k;
-            if (gx < w && gy < h) {
-                int l = -1;
-                if ((fgb >> k) & 1u) {
-                    const int r = sfind(s_L, (r0 + k) * ST_TW + cxo);
-                    l = (y0 + r / ST_TW) * w + x0 + r % ST_TW;
+                for (int c = 0; c < 4; c++) {
+                    const int b = 4 * qc + c, i = (r0 + k) * ST_TW + b;
+                    if ((st >> b) & 1ull) s_L[i] = i;
                 }
-                A.lab[gy * w + gx] = l;
+            }
+            if (qc == 0) s_row[r0 + k] = m[k];
+        }
+        const bool any = __syncthreads_or(wany);
+        if (any) {
+#pragma unroll
+            for (int k = 0; k < ST_QR; k++) {
+                const int ty = r0 + k;
+                const unsigned long long mk = m[k], st = mk & ~(mk << 1);
+                unsigned mine = ty > 0 ? (unsigned)(st >> (4 * qc)) & 15u : 0u;
+                if (!mine) continue;
+                const unsigned long long mp = k ? m[0] : s_row[ty - 1], sp = mp & ~(mp << 1);
+                while (mine) {
+                    const int b = 4 * qc + __ffs(mine) - 1;
+                    mine &= mine - 1;
+                    const int e = run_end64(mk, b);
+                    const int s1 = b > 0 ? b - 1 : 0, e1 = e < 63 ? e + 1 : 63;
+                    const unsigned long long dil =
+                        (e1 == 63 ? ~0ull : ((2ull << e1) - 1ull)) & ~((1ull << s1) - 1ull);
+                    unsigned long long ov = mp & dil;
+                    while (ov) {
+                        const int o = __ffsll((long long)ov) - 1;
+                        sunion(s_L, ty * ST_TW + b, (ty - 1) * ST_TW + run_start64(sp, o));
+                        const int eo = run_end64(mp, o);
+                        ov = eo >= 63 ? 0ull : ov & ~((2ull << eo) - 1ull);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int k = 0; k < ST_QR; k++) {
+            const int gy = y0 + r0 + k;
+            if (gy >= h || ncol == 0) continue;
+            int l[4] = {-1, -1, -1, -1};
+            if (nib[k]) {
+                const unsigned long long st = m[k] & ~(m[k] << 1);
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    if (!((nib[k] >> c) & 1u)) continue;
+                    if (c > 0 && ((nib[k] >> (c - 1)) & 1u)) {
+                        l[c] = l[c - 1];
+                    } else {
+                        const int r = sfind(s_L, (r0 + k) * ST_TW + run_start64(st, 4 * qc + c));
+                        l[c] = (y0 + r / ST_TW) * w + x0 + r % ST_TW;
+                    }
+                }
+            }
+            int *out = A.lab + (size_t)gy * w + gx;
+            if (TMA) {
+                *reinterpret_cast<int4 *>(out) = make_int4(l[0], l[1], l[2], l[3]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (c < ncol) out[c] = l[c];
             }
         }
-        __syncthreads();
     }
-    if (failed) {
+    if (TMA && failed) {
         // A load did not complete in time: report it, and give the copies
         // still in flight one more bounded wait before the CTA exits.  A copy
         // that outlasts that wait too may still write into shared memory after
@@ -466,14 +515,8 @@ __global__ void __launch_bounds__(ST_THREADS, 4) k_sub_filter_pipe(const __grid_
         }
         return;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        nabove += __shfl_down_sync(0xffffffffu, nabove, o);
-        emin = min(emin, __shfl_down_sync(0xffffffffu, emin, o));
-    }
-    if (lane == 0) {
-        if (nabove) atomicAdd(&A.sc->npix_above, nabove);
-        if (emin < 1000) atomicMin(&A.sc->e0sub, emin);
-    }
+    nabove = __reduce_add_sync(0xffffffffu, nabove);
+    if (lane == 0 && nabove) atomicAdd(&A.sc->npix_above, nabove);
 }
 
 // a 2D float tensor map of the frame with the tile box of this mask, or false
@@ -499,145 +542,93 @@ static bool make_frame_tmap(CUtensorMap *m, const float *img, int w, int h, int 
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Returns true when the labels written are already tile-local components
-// (the subtract/filter pipeline's 64 x 32 tiles), false when they are seeds
-// (every foreground pixel its own label).
-bool launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const BackBufs &B, const FrameParams &P,
+// (smem << 8) | resident CTAs of each instance, per device
+template <int MW, int MH, bool WEIGHTED, bool TMA>
+static void sp_launch(const CUtensorMap &tmap, const SpArgs &A, const ConvTaps &taps, size_t smem, cudaStream_t st) {
+    static DevCache nsm_cache;
+    const int nsm = nsm_cache.get([](int dev) {
+        int n = 148;
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? n : 148;
+    });
+    auto kern = k_sub_filter<MW, MH, WEIGHTED, TMA>;
+    static std::atomic<long long> cached[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::atomic<long long> &slot = cached[dev >= 0 && dev < 64 ? dev : 0];
+    const long long c = slot.load(std::memory_order_relaxed);
+    int per = (int)(c & 255);
+    if ((c >> 8) != (long long)smem) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        per = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, ST_THREADS, smem);
+        per = std::min(std::max(per, 1), 255);
+        slot.store(((long long)smem << 8) | per, std::memory_order_relaxed);
+    }
+    const int grid = std::max(1, std::min(A.ntiles, sx_share(nsm * per)));
+    sx_launch(kern, grid, ST_THREADS, smem, st, tmap, A, taps);
+}
+
+template <bool WEIGHTED, bool TMA>
+static void sp_launch_mask(const CUtensorMap &tmap, const SpArgs &A, const ConvTaps &taps, size_t smem,
+                           cudaStream_t st) {
+    const int m = A.mw == A.mh ? A.mw : 0;
+    switch (m) {
+        case 1: sp_launch<1, 1, WEIGHTED, TMA>(tmap, A, taps, smem, st); break;
+        case 3: sp_launch<3, 3, WEIGHTED, TMA>(tmap, A, taps, smem, st); break;
+        case 5: sp_launch<5, 5, WEIGHTED, TMA>(tmap, A, taps, smem, st); break;
+        case 7: sp_launch<7, 7, WEIGHTED, TMA>(tmap, A, taps, smem, st); break;
+        case 9: sp_launch<9, 9, WEIGHTED, TMA>(tmap, A, taps, smem, st); break;
+        case 11: sp_launch<11, 11, WEIGHTED, TMA>(tmap, A, taps, smem, st); break;
+        default: sp_launch<0, 0, WEIGHTED, TMA>(tmap, A, taps, smem, st);
+    }
+}
+
+// Subtracted and filtered frame, and as labels the components within each
+// ST_TW x ST_TH tile.
+void launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const BackBufs &B, const FrameParams &P,
                        FrameScalars *d_sc, const float *d_var, const ConvMask &M, cudaStream_t st, int &launches) {
     const int mw = M.mw, mh = M.mh;
     const int rxa = ((mw / 2) + 3) & ~3;  // halo width rounded up to 16 bytes
+    SpArgs A;
+    A.img = img;
+    A.sub = sub;
+    A.cd = cd;
+    A.lab = lab;
+    A.B = B;
+    A.w = P.w;
+    A.h = P.h;
+    A.nbx = P.nbx;
+    A.back_type = P.back_type;
+    A.mw = mw;
+    A.mh = mh;
+    A.rxa = rxa;
+    A.wthr = P.wthr;
+    A.tilesx = (P.w + ST_TW - 1) / ST_TW;
+    A.ntiles = A.tilesx * ((P.h + ST_TH - 1) / ST_TH);
+    A.dfac = P.detect_thresh;
+    A.mask = M.dev;
+    A.wvar = d_var;
+    A.sc = d_sc;
+    ConvTaps taps;
+    memset(&taps, 0, sizeof(taps));
+    if (mw * mh <= 121) memcpy(taps.m, M.host, sizeof(float) * mw * mh);
+    const int bw = ST_TW + 2 * rxa, bh = ST_TH + 2 * (mh / 2);
+    const size_t smem = 2 * sizeof(float) * (size_t)((bw * bh + 31) & ~31);
     CUtensorMap tmap;
-    if (make_frame_tmap(&tmap, img, P.w, P.h, rxa, mh / 2)) {
-        SpArgs A;
-        A.sub = sub;
-        A.cd = cd;
-        A.lab = lab;
-        A.B = B;
-        A.w = P.w;
-        A.h = P.h;
-        A.nbx = P.nbx;
-        A.back_type = P.back_type;
-        A.mw = mw;
-        A.mh = mh;
-        A.rxa = rxa;
-        A.wthr = P.wthr;
-        A.tilesx = (P.w + ST_TW - 1) / ST_TW;
-        A.ntiles = A.tilesx * ((P.h + ST_TH - 1) / ST_TH);
-        A.dfac = P.detect_thresh;
-        A.mask = M.dev;
-        A.wvar = d_var;
-        A.sc = d_sc;
-        ConvTaps taps;
-        memset(&taps, 0, sizeof(taps));
-        if (mw * mh <= 121) memcpy(taps.m, M.host, sizeof(float) * mw * mh);
-        const int bw = ST_TW + 2 * rxa, bh = ST_TH + 2 * (mh / 2);
-        const size_t smem = 2 * sizeof(float) * (size_t)((bw * bh + 31) & ~31);
-        static DevCache nsm_cache;
-        const int nsm = nsm_cache.get([](int dev) {
-            int n = 148;
-            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-            return n > 0 ? n : 148;
-        });
-#define SP_LAUNCH(a, b, wt)                                                                              \
-    do {                                                                                                \
-        auto kern = k_sub_filter_pipe<a, b, wt>;                                                        \
-        /* (smem << 8) | resident CTAs of this instance, per device */                                 \
-        static std::atomic<long long> cached[64];                                                       \
-        int dev_ = 0;                                                                                   \
-        cudaGetDevice(&dev_);                                                                           \
-        std::atomic<long long> &slot = cached[dev_ >= 0 && dev_ < 64 ? dev_ : 0];                      \
-        long long c = slot.load(std::memory_order_relaxed);                                             \
-        int per = (int)(c & 255);                                                                       \
-        if ((c >> 8) != (long long)smem) {                                                              \
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);        \
-            per = 1;                                                                                    \
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, ST_THREADS, smem);                \
-            per = std::min(std::max(per, 1), 255);                                                      \
-            slot.store(((long long)smem << 8) | per, std::memory_order_relaxed);                        \
-        }                                                                                               \
-        const int grid = std::max(1, std::min(A.ntiles, sx_share(nsm * per)));                         \
-        sx_launch(kern, grid, ST_THREADS, smem, st, tmap, A, taps);                                            \
-    } while (0)
-#define SP_MASK(wt)                    \
-    if (mw == mh && mw == 1)           \
-        SP_LAUNCH(1, 1, wt);           \
-    else if (mw == mh && mw == 3)      \
-        SP_LAUNCH(3, 3, wt);           \
-    else if (mw == mh && mw == 5)      \
-        SP_LAUNCH(5, 5, wt);           \
-    else if (mw == mh && mw == 7)      \
-        SP_LAUNCH(7, 7, wt);           \
-    else if (mw == mh && mw == 9)      \
-        SP_LAUNCH(9, 9, wt);           \
-    else if (mw == mh && mw == 11)     \
-        SP_LAUNCH(11, 11, wt);         \
-    else                               \
-        SP_LAUNCH(0, 0, wt)
-        if (d_var) {
-            SP_MASK(true);
-        } else {
-            SP_MASK(false);
-        }
-#undef SP_MASK
-#undef SP_LAUNCH
-        launches += 1;
-        return true;
-    }
-    dim3 grid((P.w + SF_TW - 1) / SF_TW, (P.h + SF_TH - 1) / SF_TH);
-    dim3 block(SF_TX, SF_TY);
-    size_t smem = sizeof(float) * (SF_TW + mw - 1) * (SF_TH + mh - 1);
-    sx_launch(k_sub_filter, grid, block, smem, st, img, sub, cd, lab, B, P.w, P.h, P.nbx, P.back_type, M.dev, mw, mh,
-              d_var, P.wthr, P.detect_thresh, d_sc);
+    memset(&tmap, 0, sizeof(tmap));
+    const bool tma = make_frame_tmap(&tmap, img, P.w, P.h, rxa, mh / 2);
+    if (d_var)
+        tma ? sp_launch_mask<true, true>(tmap, A, taps, smem, st) : sp_launch_mask<true, false>(tmap, A, taps, smem, st);
+    else
+        tma ? sp_launch_mask<false, true>(tmap, A, taps, smem, st)
+            : sp_launch_mask<false, false>(tmap, A, taps, smem, st);
     launches += 1;
-    return false;
 }
 
 // ---------------------------------------------------------------------------
 // union-find CCL
 // ---------------------------------------------------------------------------
-constexpr int CC_TW = 32, CC_TH = 16;
-
-// Labels within one 32 x CC_TH tile, one warp per tile row (frames that the
-// subtract/filter kernel could not label itself).  A row's foreground is one
-// ballot; pixels of a horizontal run are connected through the run's first
-// pixel (bit arithmetic, no unions); a run joins the runs of the row above
-// that touch it or its two diagonal ends (8-connected) with one union each,
-// in shared memory.  Every link goes to a smaller tile index, so each tile
-// component ends at its smallest pixel.
-__global__ void __launch_bounds__(CC_TW *CC_TH) k_ccl_local(int *__restrict__ lab, int w, int h) {
-    sx_pdl();
-    __shared__ int L[CC_TH * CC_TW];
-    __shared__ unsigned rowm[CC_TH];
-    const int lx = threadIdx.x, ly = threadIdx.y, t = ly * CC_TW + lx;
-    const int gx = blockIdx.x * CC_TW + lx, gy = blockIdx.y * CC_TH + ly;
-    const bool in = gx < w && gy < h;
-    const bool fg = in && lab[(size_t)gy * w + gx] >= 0;
-    const unsigned m = __ballot_sync(0xffffffffu, fg);
-    const unsigned starts = m & ~(m << 1);
-    if (lx == 0) rowm[ly] = m;
-    L[t] = fg ? ly * CC_TW + run_start(starts, lx) : -1;
-    __syncthreads();
-    if (fg && ly > 0 && ((starts >> lx) & 1u)) {
-        const int e = run_end(m, lx);
-        const int s1 = lx > 0 ? lx - 1 : 0, e1 = e < 31 ? e + 1 : 31;
-        const unsigned dil = (unsigned)((2ull << e1) - 1ull) & ~((1u << s1) - 1u);
-        const unsigned mp = rowm[ly - 1], sp = mp & ~(mp << 1);
-        unsigned ov = mp & dil;
-        while (ov) {
-            const int b = __ffs(ov) - 1;
-            sunion(L, t, (ly - 1) * CC_TW + run_start(sp, b));
-            const int eb = run_end(mp, b);
-            ov = eb >= 31 ? 0u : ov & ~((2u << eb) - 1u);
-        }
-    }
-    __syncthreads();
-    if (fg) {
-        int r = sfind(L, t);
-        int rx = blockIdx.x * CC_TW + (r % CC_TW), ry = blockIdx.y * CC_TH + (r / CC_TW);
-        lab[(size_t)gy * w + gx] = ry * w + rx;
-    }
-}
-
 // walk to the root; a walk longer than cap steps sets SX_ST_LOOP and stops
 __device__ __forceinline__ int gfind(const int *L, int a, int cap, int *status) {
     for (int n = 0; n <= cap; n++) {
@@ -758,25 +749,13 @@ __global__ void k_ccl_flatten(int *__restrict__ lab, long long n, int *__restric
 }
 
 // cnt: zeroed, w*h ints; receives the size of every component at its root
-// tiled: the labels are already the tile-local components of the
-// subtract/filter pipeline's ST_TW x ST_TH tiles (else seeds, labelled here
-// in CC_TW x CC_TH tiles first)
-void launch_ccl(int *lab, int *cnt, const FrameParams &P, FrameScalars *d_sc, cudaStream_t st, int &launches,
-                bool tiled) {
+// lab: the tile-local components of k_sub_filter's tiles
+void launch_ccl(int *lab, int *cnt, const FrameParams &P, FrameScalars *d_sc, cudaStream_t st, int &launches) {
     int *status = &d_sc->status;
-    if (tiled) {
-        const int ntiles = ((P.w + ST_TW - 1) / ST_TW) * ((P.h + ST_TH - 1) / ST_TH);
-        sx_launch(k_ccl_border<ST_TW, ST_TH>, ntiles, ST_TW + ST_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
-        sx_launch(k_ccl_border_ne<ST_TW, ST_TH>, ntiles, ST_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
-        launches += 3;
-    } else {
-        dim3 grid((P.w + CC_TW - 1) / CC_TW, (P.h + CC_TH - 1) / CC_TH);
-        sx_launch(k_ccl_local, grid, dim3(CC_TW, CC_TH), 0, st, lab, P.w, P.h);
-        const int ntiles = grid.x * grid.y;
-        sx_launch(k_ccl_border<CC_TW, CC_TH>, ntiles, CC_TW + CC_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
-        sx_launch(k_ccl_border_ne<CC_TW, CC_TH>, ntiles, CC_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
-        launches += 4;
-    }
+    const int ntiles = ((P.w + ST_TW - 1) / ST_TW) * ((P.h + ST_TH - 1) / ST_TH);
+    sx_launch(k_ccl_border<ST_TW, ST_TH>, ntiles, ST_TW + ST_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
+    sx_launch(k_ccl_border_ne<ST_TW, ST_TH>, ntiles, ST_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
+    launches += 3;
     long long n = (long long)P.w * P.h;
     sx_launch(k_ccl_flatten, (unsigned)((n + 1023) / 1024), 256, 0, st, lab, n, cnt, status, P.loop_cap);
 }

@@ -159,12 +159,11 @@ struct ConvMask {
     int mw, mh;
 };
 
-bool launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const BackBufs &B,
+void launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const BackBufs &B,
                        const FrameParams &P, FrameScalars *d_sc, const float *d_var, const ConvMask &M,
                        cudaStream_t st, int &launches);
 
-void launch_ccl(int *lab, int *cnt, const FrameParams &P, FrameScalars *d_sc, cudaStream_t st, int &launches,
-                bool tiled);
+void launch_ccl(int *lab, int *cnt, const FrameParams &P, FrameScalars *d_sc, cudaStream_t st, int &launches);
 
 struct MomentRaw;
 // a kept branch's centre and shape, as the gatherup reads them (32 bytes)

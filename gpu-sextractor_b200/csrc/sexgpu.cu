@@ -383,7 +383,6 @@ __global__ void k_init_scalars(FrameScalars *sc) {
     sx_pdl();
     FrameScalars z;
     memset(&z, 0, sizeof(z));
-    z.e0sub = 1000;
     z.sigfac = 1.0f;
     *sc = z;
 }
@@ -687,14 +686,14 @@ int pipe_detect(sexgpu_ctx *ctx) {
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int *tmp = P<int>(ctx->scan_tmp);
     int rc = SEXGPU_OK, nl = 0;
-    const bool tiled = launch_sub_filter(d_img, P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), B, Pm, d_sc, ps.wvar,
-                      ctx->cmask, st, nl);
+    launch_sub_filter(d_img, P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), B, Pm, d_sc, ps.wvar, ctx->cmask,
+                      st, nl);
     stage_mark(ctx, "sub_filter", nl);
 
     nl = 0;
     int *lab = P<int>(ctx->lab), *cnt = P<int>(ctx->cnt), *flag = P<int>(ctx->flag), *pos = P<int>(ctx->pos);
     CK(cudaMemsetAsync(cnt, 0, N * 4, st));
-    launch_ccl(lab, cnt, Pm, d_sc, st, nl, tiled);  // labels to roots, component sizes at the roots
+    launch_ccl(lab, cnt, Pm, d_sc, st, nl);  // labels to roots, component sizes at the roots
     stage_mark(ctx, "ccl", nl);
 
     // ---- raw objects
@@ -1831,7 +1830,6 @@ int sexgpu_filter(sexgpu_ctx *ctx, const float *sub, int w, int h, const float *
     memset(&z, 0, sizeof(z));
     z.backmean = 0.0f;
     z.dthresh = 1e30f;
-    z.e0sub = 1000;
     CK(cudaMemcpyAsync(ctx->sc.p, &z, sizeof(z), cudaMemcpyHostToDevice, st));
     BackBufs B;
     memset(&B, 0, sizeof(B));

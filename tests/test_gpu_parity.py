@@ -429,3 +429,39 @@ def test_lists_and_catalogue_order(gpu_ctx, w, h, minarea):
         g = run_both(gpu_ctx, img, filter_flag=0, back_type=1, back_value=0.0, thresh_type=1, detect_thresh=3.2,
                      analysis_thresh=3.2, detect_minarea=minarea, numbering=numbering, deblend_mincont=0.001)
         assert len(g) > 10
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (3, 2), (63, 33), (64, 32), (65, 31), (68, 36), (132, 97), (257, 65)])
+@pytest.mark.parametrize("mw,mh", [(1, 1), (3, 3), (5, 5), (7, 7), (9, 9), (11, 11), (4, 6), (2, 1), (31, 31)])
+def test_filter_at_tile_edges(gpu_ctx, w, h, mw, mh):
+    """Frames of one tile, of whole tiles and just beyond, with rows that are
+    and are not a multiple of 16 bytes, under every specialised mask size, even
+    sizes and the largest mask: bit for bit."""
+    rng = np.random.default_rng(100 * w + mw)
+    sub = rng.normal(0, 10, (h, w)).astype(np.float32)
+    m = rng.uniform(-0.2, 1.0, (mh, mw)).astype(np.float32)
+    assert np.array_equal(gpu_ctx.filter(sub, m), O.filter_image(sub, m))
+
+
+@pytest.mark.parametrize("w,h", [(7, 5), (63, 33), (64, 32), (65, 31), (68, 36), (132, 97), (257, 65)])
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("bs,thr", [(3, 0.3), (64, 0.1), (40, 1.5)])
+def test_components_at_tile_edges(gpu_ctx, masks, w, h, weighted, bs, thr):
+    """Noise cut near its mean, so that components wind through the tiles and
+    over their borders, with meshes narrower than four pixels (more spline
+    segments than a tile row has staged nodes) and wider than a tile; with and
+    without a variance map that marks unusable pixels."""
+    rng = np.random.default_rng(w * 1000 + h + bs)
+    img = rng.normal(100.0, 10.0, (h, w)).astype(np.float32)
+    kw = dict(back_size=bs, filter_flag=0, detect_thresh=thr, analysis_thresh=thr, detect_minarea=1,
+              deblend_nthresh=4, deblend_mincont=0.5, clean_flag=0)
+    if weighted:
+        var = rng.uniform(50.0, 150.0, (h, w)).astype(np.float32)
+        var[rng.random((h, w)) < 0.05] = 1e30
+        g, gseg, gs = gpu_ctx.extract(img, weight=var, weight_type=1, **kw)
+        o, oseg, os_ = O.extract(img, weight=var, weight_type=1, **kw)
+        assert gs.npix_above == os_.npix_above
+        assert np.array_equal(gseg, oseg)
+        compare_catalogs(g, o)
+    else:
+        run_both(gpu_ctx, img, **kw)
