@@ -220,7 +220,7 @@ void run_detection(float dthresh, float thresh, int minarea, size_t *numValidObj
         Pm.filter_flag = 0;
         Pm.conv_w = Pm.conv_h = 1;
     }
-    int rc = load_mask(ctx, s.mask_w > 0 ? s.mask.data() : nullptr, s.mask_w, s.mask_w);
+    int rc = load_tables(ctx, Pm, s.mask_w > 0 ? s.mask.data() : nullptr, s.mask_w, s.mask_w, ctx->ps.B);
     if (rc) {
         compat_fail("run_detection", rc);
         return;

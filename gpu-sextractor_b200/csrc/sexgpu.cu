@@ -47,7 +47,6 @@ struct DevBuf {
 struct StageRec {
     const char *name;
     int launches;
-    cudaEvent_t ev;
 };
 
 }  // namespace
@@ -148,7 +147,7 @@ struct sexgpu_ctx {
     // scan / sort scratch
     DevBuf scan_tmp, keys, vals;  // scan scratch; raw object of every element; object pixel lists
     // background
-    DevBuf ms, back, sigma, back2, back3, sigma3, dback, bu, rownode, rowdnode, rowu, colk, coldx;
+    DevBuf ms, back, sigma, back2, back3, sigma3, dback, bu, rownode, rowdnode, rowu;
     // roots
     DevBuf rsize, roff, rnkept, robjbase, rdthr, rathr, rzero, rlists, rthr;
     // deblend scratch
@@ -180,17 +179,15 @@ struct sexgpu_ctx {
     unsigned long long graph_epoch = 0;  // bumped whenever a graph is captured or dropped
     unsigned long long last_entry = 0;   // id of the graph entry of the last extraction (0: none)
     BatchGraph *bgraph = nullptr;        // one-launch form of the last batch (sexgpu_extract_batch)
-    FrameScalars *hsc_pin = nullptr;     // pinned copy of the frame scalars (capacity form)
+    FrameScalars *hsc_pin = nullptr;     // page-locked copy of the frame scalars
     int last_graph = 0;                  // the last extraction replayed a graph
     int last_kernels = 0;                // kernel launches of the last extraction
     DevBuf sc;
     FrameScalars hsc;
     ObjBufs O;
-    std::vector<int> colk_h;
-    std::vector<float> coldx_h;
     int last_w = 0, last_h = 0, last_nobj = 0, last_ns = 0;
     std::vector<StageRec> stages;
-    cudaEvent_t ev0 = nullptr;
+    std::vector<cudaEvent_t> stage_ev;  // [0]: the frame's begin, [k + 1]: the end of stage k
     std::vector<float> stage_ms;
     std::vector<std::string> stage_names;
     std::vector<int> stage_launches;
@@ -206,7 +203,8 @@ struct sexgpu_ctx {
     size_t stage_bytes = 0;
     void *rows_host = nullptr;          // pinned staging of a batch worker's catalogue rows
     size_t rows_bytes = 0;
-    DevBuf dmask;                       // detection mask of the current extraction
+    DevBuf tabs;                        // column tables and detection mask of the current extraction
+    std::vector<char> tabs_h;
     std::vector<float> hmask;
     ConvMask cmask{nullptr, nullptr, 1, 1};
 };
@@ -256,15 +254,23 @@ int ensure(sexgpu_ctx *ctx, DevBuf &b, size_t bytes) {
 template <class T> T *P(DevBuf &b) { return (T *)b.p; }
 
 // stage timing (plain form only: a graph has no per-stage events)
+// the k-th event of the frame (the events are kept from frame to frame)
+void stage_event(sexgpu_ctx *ctx, size_t k) {
+    while (ctx->stage_ev.size() <= k) {
+        cudaEvent_t e = nullptr;
+        cudaEventCreate(&e);
+        ctx->stage_ev.push_back(e);
+    }
+    cudaEventRecord(ctx->stage_ev[k], ctx->stream);
+}
+
 void stage_begin(sexgpu_ctx *ctx) {
     ctx->stage_names.clear();
     ctx->stage_launches.clear();
     ctx->stage_ms.clear();
     if (ctx->ps.capf) return;  // (no event calls while the stages may be captured)
-    for (auto &s : ctx->stages) cudaEventDestroy(s.ev);
     ctx->stages.clear();
-    if (!ctx->ev0) cudaEventCreate(&ctx->ev0);
-    cudaEventRecord(ctx->ev0, ctx->stream);
+    stage_event(ctx, 0);
 }
 
 void stage_mark(sexgpu_ctx *ctx, const char *name, int launches) {
@@ -272,31 +278,28 @@ void stage_mark(sexgpu_ctx *ctx, const char *name, int launches) {
     StageRec s;
     s.name = name;
     s.launches = launches;
-    cudaEventCreate(&s.ev);
-    cudaEventRecord(s.ev, ctx->stream);
     ctx->stages.push_back(s);
+    stage_event(ctx, ctx->stages.size());
 }
 
 void stage_collect(sexgpu_ctx *ctx) {
     ctx->stage_ms.clear();
     ctx->stage_names.clear();
     ctx->stage_launches.clear();
-    cudaEvent_t prev = ctx->ev0;
-    for (auto &s : ctx->stages) {
+    for (size_t k = 0; k < ctx->stages.size(); k++) {
         float ms = 0.f;
-        cudaEventElapsedTime(&ms, prev, s.ev);
+        cudaEventElapsedTime(&ms, ctx->stage_ev[k], ctx->stage_ev[k + 1]);
         ctx->stage_ms.push_back(ms);
-        ctx->stage_names.push_back(s.name);
-        ctx->stage_launches.push_back(s.launches);
-        prev = s.ev;
+        ctx->stage_names.push_back(ctx->stages[k].name);
+        ctx->stage_launches.push_back(ctx->stages[k].launches);
     }
 }
 
 // x-interpolation table of src/back.c:863-899 (segment index and dx of
 // every column), the same float arithmetic as the reference's loop
-void column_table(int width, int nbx, int backw, std::vector<int> &colk, std::vector<float> &coldx) {
-    colk.assign(width, 0);
-    coldx.assign(width, 0.f);
+void column_table(int width, int nbx, int backw, int *colk, float *coldx) {
+    std::fill(colk, colk + width, 0);
+    std::fill(coldx, coldx + width, 0.f);
     if (nbx <= 1) return;
     int nx = backw, changepoint = nx / 2, x = 0, i = 0, k = 0;
     float xstep = 1.0 / nx;
@@ -416,9 +419,20 @@ cudaError_t stream_wait(sexgpu_ctx *ctx, cudaStream_t st) {
     return e == cudaSuccess ? cudaEventSynchronize(ctx->ev_block) : e;
 }
 
+// the context's page-locked copy of the frame scalars
+int pin_scalars(sexgpu_ctx *ctx) {
+    if (ctx->hsc_pin || cudaMallocHost((void **)&ctx->hsc_pin, sizeof(FrameScalars)) == cudaSuccess) return SEXGPU_OK;
+    cudaGetLastError();
+    ctx->hsc_pin = nullptr;
+    ctx->err = "pinned host allocation failed";
+    return SEXGPU_ERR_NOMEM;
+}
+
 int read_scalars(sexgpu_ctx *ctx) {
-    CK(cudaMemcpyAsync(&ctx->hsc, ctx->sc.p, sizeof(FrameScalars), cudaMemcpyDeviceToHost, ctx->stream));
+    if (int rc = pin_scalars(ctx)) return rc;
+    CK(cudaMemcpyAsync(ctx->hsc_pin, ctx->sc.p, sizeof(FrameScalars), cudaMemcpyDeviceToHost, ctx->stream));
     CK(stream_wait(ctx, ctx->stream));
+    ctx->hsc = *ctx->hsc_pin;
     if (ctx->hsc.status & SX_ST_LOAD) {
         ctx->err = "a tile load did not complete in time; destroy this context";
         return SEXGPU_ERR_LOAD;
@@ -434,22 +448,36 @@ int read_scalars(sexgpu_ctx *ctx) {
     return SEXGPU_OK;
 }
 
-// the detection mask of this context's next extraction (host and device copy)
-int load_mask(sexgpu_ctx *ctx, const float *mask, int mw, int mh) {
+// The tables that a frame's kernels read, in one block: the segment index and
+// dx of every column, then the detection mask (w ints, w floats, the mask).
+void fill_tables(std::vector<char> &tabs, const FrameParams &Pm, const float *mask, size_t nmask) {
+    tabs.resize((size_t)8 * Pm.w + 4 * nmask);
+    column_table(Pm.w, Pm.nbx, Pm.bw, reinterpret_cast<int *>(tabs.data()),
+                 reinterpret_cast<float *>(tabs.data() + (size_t)4 * Pm.w));
+    memcpy(tabs.data() + (size_t)8 * Pm.w, mask, 4 * nmask);
+}
+
+size_t tables_bytes(int w) { return (size_t)8 * w + 4 * SX_MAXCONV * SX_MAXCONV; }
+
+// ... of this context's next extraction, by one upload; a frame that is being
+// captured reads the graph's device copy
+int load_tables(sexgpu_ctx *ctx, const FrameParams &Pm, const float *mask, int mw, int mh, BackBufs &B) {
     static const float one = 1.0f;
     if (!mask) {
         mask = &one;
         mw = mh = 1;
     }
     ctx->hmask.assign(mask, mask + (size_t)mw * mh);
-    EN(dmask, sizeof(float) * SX_MAXCONV * SX_MAXCONV);
-    if (ctx->ps.cst) {  // being captured: the graph's device copy
-        ctx->cmask.dev = reinterpret_cast<const float *>(ctx->ps.cst + (size_t)8 * ctx->ps.w);
-    } else {
-        CK(cudaMemcpyAsync(ctx->dmask.p, ctx->hmask.data(), sizeof(float) * mw * mh, cudaMemcpyHostToDevice,
-                           ctx->stream));
-        ctx->cmask.dev = P<float>(ctx->dmask);
+    unsigned char *dev = ctx->ps.cst;
+    if (!dev) {
+        EN(tabs, tables_bytes(Pm.w));
+        dev = P<unsigned char>(ctx->tabs);
+        fill_tables(ctx->tabs_h, Pm, mask, ctx->hmask.size());
+        CK(cudaMemcpyAsync(dev, ctx->tabs_h.data(), ctx->tabs_h.size(), cudaMemcpyHostToDevice, ctx->stream));
     }
+    B.colk = reinterpret_cast<int *>(dev);
+    B.coldx = reinterpret_cast<float *>(dev + (size_t)4 * Pm.w);
+    ctx->cmask.dev = reinterpret_cast<const float *>(dev + (size_t)8 * Pm.w);
     ctx->cmask.host = ctx->hmask.data();
     ctx->cmask.mw = mw;
     ctx->cmask.mh = mh;
@@ -603,8 +631,6 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
     EN(rownode, (size_t)h * Pm.nbx * 4);
     EN(rowdnode, (size_t)h * Pm.nbx * 4);
     EN(rowu, (size_t)h * Pm.nbx * 4);
-    EN(colk, w * 4);
-    EN(coldx, w * 4);
     EN(sc, sizeof(FrameScalars));
     BackBufs &B = ps.B;
     B.ms = P<MeshStat>(ctx->ms);
@@ -618,20 +644,10 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
     B.rownode = P<float>(ctx->rownode);
     B.rowdnode = P<float>(ctx->rowdnode);
     B.rowu = P<float>(ctx->rowu);
-    B.colk = P<int>(ctx->colk);
-    B.coldx = P<float>(ctx->coldx);
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int *tmp = P<int>(ctx->scan_tmp);
 
-    if (ps.cst) {  // being captured: the graph's device copy
-        B.colk = reinterpret_cast<int *>(ps.cst);
-        B.coldx = reinterpret_cast<float *>(ps.cst + (size_t)w * 4);
-    } else {
-        column_table(w, Pm.nbx, Pm.bw, ctx->colk_h, ctx->coldx_h);
-        CK(cudaMemcpyAsync(B.colk, ctx->colk_h.data(), w * 4, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(B.coldx, ctx->coldx_h.data(), w * 4, cudaMemcpyHostToDevice, st));
-    }
-    rc = load_mask(ctx, cfg->filter_flag ? cfg->conv : nullptr, cfg->conv_w, cfg->conv_h);
+    rc = load_tables(ctx, Pm, cfg->filter_flag ? cfg->conv : nullptr, cfg->conv_w, cfg->conv_h, B);
     if (rc) return rc;
 
     stage_begin(ctx);
@@ -1218,25 +1234,18 @@ void capture_graph(sexgpu_ctx *ctx, GraphEntry &e, const float *d_img, const flo
     cudaStream_t st = ctx->stream;
     // the frame's constants into the entry's own device memory before the
     // capture; the graph reads them there
-    if (!e.cst && cudaMalloc((void **)&e.cst, (size_t)8 * w + 4 * SX_MAXCONV * SX_MAXCONV) != cudaSuccess) {
+    if (!e.cst && cudaMalloc((void **)&e.cst, tables_bytes(w)) != cudaSuccess) {
         cudaGetLastError();
         e.cst = nullptr;
         e.no_graph = true;
         return;
     }
-    {
-        std::vector<int> ck;
-        std::vector<float> cdx;
-        column_table(w, e.Pm.nbx, e.Pm.bw, ck, cdx);
-        const float *m = e.mask.data();
-        const size_t mbytes = sizeof(float) * e.mask.size();
-        if (cudaMemcpy(e.cst, ck.data(), (size_t)w * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(e.cst + (size_t)w * 4, cdx.data(), (size_t)w * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(e.cst + (size_t)8 * w, m, mbytes, cudaMemcpyHostToDevice) != cudaSuccess) {
-            cudaGetLastError();
-            e.no_graph = true;
-            return;
-        }
+    std::vector<char> tabs;
+    fill_tables(tabs, e.Pm, e.mask.data(), e.mask.size());
+    if (cudaMemcpy(e.cst, tabs.data(), tabs.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        e.no_graph = true;
+        return;
     }
     const unsigned long long gen0 = ctx->gen;
     cudaGraph_t g = nullptr;
@@ -1336,14 +1345,7 @@ int run_graph(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, i
         if (!rc) learn_caps(ctx, *e, N, Pm.minarea);
         return rc;
     }
-    if (!ctx->hsc_pin) {
-        if (cudaMallocHost((void **)&ctx->hsc_pin, sizeof(FrameScalars)) != cudaSuccess) {
-            cudaGetLastError();
-            ctx->hsc_pin = nullptr;
-            ctx->err = "pinned host allocation failed";
-            return SEXGPU_ERR_NOMEM;
-        }
-    }
+    if (int rc = pin_scalars(ctx)) return rc;
     cudaStream_t st = ctx->stream;
     const bool replay = e->exec && e->gen == ctx->gen;
     int rc = SEXGPU_OK;
@@ -1445,7 +1447,7 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     DevBuf *all[] = {&ctx->img, &ctx->sub, &ctx->cd, &ctx->lab, &ctx->cnt, &ctx->flag, &ctx->pos, &ctx->alloc,
                      &ctx->seg, &ctx->pos2idx, &ctx->var, &ctx->scan_tmp, &ctx->keys, &ctx->vals, &ctx->ms, &ctx->back, &ctx->sigma, &ctx->back2, &ctx->back3, &ctx->sigma3,
-                     &ctx->dback, &ctx->bu, &ctx->rownode, &ctx->rowdnode, &ctx->rowu, &ctx->colk, &ctx->coldx,
+                     &ctx->dback, &ctx->bu, &ctx->rownode, &ctx->rowdnode, &ctx->rowu,
                      &ctx->rsize, &ctx->roff, &ctx->rnkept, &ctx->robjbase,
                      &ctx->rdthr, &ctx->rathr, &ctx->rzero, &ctx->rlists, &ctx->rthr, &ctx->imgm, &ctx->wvar,
                      &ctx->wratio, &ctx->objkey, &ctx->rpix, &ctx->o_big, &ctx->o_geo, &ctx->o_apraw, &ctx->o_gobj,
@@ -1476,9 +1478,8 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
     free_buf(ctx->rmsu);
     free_buf(ctx->rmsmap);
     free_buf(ctx->dnnw);
-    free_buf(ctx->dmask);
-    for (auto &s : ctx->stages) cudaEventDestroy(s.ev);
-    if (ctx->ev0) cudaEventDestroy(ctx->ev0);
+    free_buf(ctx->tabs);
+    for (cudaEvent_t e : ctx->stage_ev) cudaEventDestroy(e);
     if (ctx->ev_block) cudaEventDestroy(ctx->ev_block);
     free_batch_graph(ctx);
     for (GraphEntry &e : ctx->graphs) drop_graph(ctx, e);
@@ -1768,8 +1769,6 @@ int sexgpu_background(sexgpu_ctx *ctx, float *img, int w, int h, const sexgpu_co
     EN(rownode, (size_t)h * Pm.nbx * 4);
     EN(rowdnode, (size_t)h * Pm.nbx * 4);
     EN(rowu, (size_t)h * Pm.nbx * 4);
-    EN(colk, w * 4);
-    EN(coldx, w * 4);
     EN(sc, sizeof(FrameScalars));
     BackBufs B;
     B.ms = P<MeshStat>(ctx->ms);
@@ -1783,14 +1782,9 @@ int sexgpu_background(sexgpu_ctx *ctx, float *img, int w, int h, const sexgpu_co
     B.rownode = P<float>(ctx->rownode);
     B.rowdnode = P<float>(ctx->rowdnode);
     B.rowu = P<float>(ctx->rowu);
-    B.colk = P<int>(ctx->colk);
-    B.coldx = P<float>(ctx->coldx);
-    column_table(w, Pm.nbx, Pm.bw, ctx->colk_h, ctx->coldx_h);
-    CK(cudaMemcpyAsync(B.colk, ctx->colk_h.data(), w * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(B.coldx, ctx->coldx_h.data(), w * 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ctx->img.p, img, N * 4, cudaMemcpyHostToDevice, st));
-    rc = load_mask(ctx, nullptr, 1, 1);
+    rc = load_tables(ctx, Pm, nullptr, 1, 1, B);
     if (rc) return rc;
+    CK(cudaMemcpyAsync(ctx->img.p, img, N * 4, cudaMemcpyHostToDevice, st));
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int nl = 0;
     sx_launch(k_init_scalars, 1, 1, 0, st, d_sc);
@@ -1821,11 +1815,7 @@ int sexgpu_filter(sexgpu_ctx *ctx, const float *sub, int w, int h, const float *
     EN(lab, N * 4);
     EN(sc, sizeof(FrameScalars));
     EN(rownode, 16);
-    EN(colk, 16);
-    EN(coldx, 16);
     CK(cudaMemcpyAsync(ctx->img.p, sub, N * 4, cudaMemcpyHostToDevice, st));
-    int rc = load_mask(ctx, mask, mw, mh);
-    if (rc) return rc;
     FrameScalars z;
     memset(&z, 0, sizeof(z));
     z.backmean = 0.0f;
@@ -1834,8 +1824,6 @@ int sexgpu_filter(sexgpu_ctx *ctx, const float *sub, int w, int h, const float *
     BackBufs B;
     memset(&B, 0, sizeof(B));
     B.rownode = P<float>(ctx->rownode);
-    B.colk = P<int>(ctx->colk);
-    B.coldx = P<float>(ctx->coldx);
     FrameParams Pm;
     memset(&Pm, 0, sizeof(Pm));
     Pm.w = w;
@@ -1845,6 +1833,8 @@ int sexgpu_filter(sexgpu_ctx *ctx, const float *sub, int w, int h, const float *
     Pm.filter_flag = 1;
     Pm.conv_w = mw;
     Pm.conv_h = mh;
+    int rc = load_tables(ctx, Pm, mask, mw, mh, B);
+    if (rc) return rc;
     int nl = 0;
     launch_sub_filter(P<float>(ctx->img), P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), B, Pm,
                       P<FrameScalars>(ctx->sc), nullptr, ctx->cmask, st, nl);

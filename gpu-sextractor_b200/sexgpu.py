@@ -255,21 +255,26 @@ class Context:
         h, w = img.shape
         if max_objects is None:
             max_objects = w * h // max(1, cfg.detect_minarea) // 2 + 16
-        objs = np.zeros(max_objects, OBJECT_DTYPE)
-        seg = np.zeros((h, w), np.int32) if segmap else None
         n = C.c_int()
         s = Summary()
-        sub = np.zeros_like(img) if want_maps else None
-        cd = np.zeros_like(img) if want_maps else None
         rc = lib().sexgpu_extract(self.h, _f(img), _f(wmap) if wmap is not None else None, w, h, C.byref(cfg),
-                                  objs.ctypes.data_as(C.c_void_p), max_objects, C.byref(n),
-                                  seg.ctypes.data_as(C.c_void_p) if segmap else None,
-                                  _f(sub) if want_maps else None,
-                                  _f(cd) if want_maps else None, C.byref(s))
+                                  None, 0, C.byref(n), None, None, None, C.byref(s))
         _check(rc, self.h, "sexgpu_extract")
-        if want_maps:
-            return objs[:n.value], seg, s, sub, cd
-        return objs[:n.value], seg, s
+        objs, seg, sub, cd = self._results("sexgpu_extract", n.value, max_objects, (h, w), segmap, want_maps)
+        return (objs, seg, s, sub, cd) if want_maps else (objs, seg, s)
+
+    def _results(self, what, n, max_objects, shape, segmap=False, maps=False):
+        """The catalogue of n rows (and the maps) of the extraction that `what`
+        just made, in arrays of their size; more than max_objects rows are an
+        error, as in the library's one-call forms."""
+        objs = np.empty(min(n, max_objects), OBJECT_DTYPE)
+        seg = np.empty(shape, np.int32) if segmap else None
+        sub, cd = (np.empty(shape, np.float32), np.empty(shape, np.float32)) if maps else (None, None)
+        rc = lib().sexgpu_copy_results(self.h, objs.ctypes.data_as(C.c_void_p), max_objects, None,
+                                       seg.ctypes.data_as(C.c_void_p) if segmap else None,
+                                       _f(sub) if maps else None, _f(cd) if maps else None)
+        _check(rc, self.h, what)
+        return objs, seg, sub, cd
 
     def extract_fits(self, data, bitpix, w, h, bscale=1.0, bzero=0.0, blank=None, max_objects=None,
                      want_maps=False, segmap=True, weight=None, **kw):
@@ -286,21 +291,14 @@ class Context:
         wmap = np.ascontiguousarray(weight, np.float32) if weight is not None else None
         if max_objects is None:
             max_objects = w * h // max(1, cfg.detect_minarea) // 2 + 16
-        objs = np.zeros(max_objects, OBJECT_DTYPE)
-        seg = np.zeros((h, w), np.int32) if segmap else None
         n = C.c_int()
         s = Summary()
-        sub = np.zeros((h, w), np.float32) if want_maps else None
-        cd = np.zeros((h, w), np.float32) if want_maps else None
         rc = lib().sexgpu_extract_fits(self.h, raw.ctypes.data_as(C.c_void_p), C.byref(fmt),
                                        _f(wmap) if wmap is not None else None, w, h, C.byref(cfg),
-                                       objs.ctypes.data_as(C.c_void_p), max_objects, C.byref(n),
-                                       seg.ctypes.data_as(C.c_void_p) if segmap else None,
-                                       _f(sub) if want_maps else None, _f(cd) if want_maps else None, C.byref(s))
+                                       None, 0, C.byref(n), None, None, None, C.byref(s))
         _check(rc, self.h, "sexgpu_extract_fits")
-        if want_maps:
-            return objs[:n.value], seg, s, sub, cd
-        return objs[:n.value], seg, s
+        objs, seg, sub, cd = self._results("sexgpu_extract_fits", n.value, max_objects, (h, w), segmap, want_maps)
+        return (objs, seg, s, sub, cd) if want_maps else (objs, seg, s)
 
     def apertures(self):
         """Every aperture of the last extraction's catalogue rows: float32
@@ -338,7 +336,7 @@ class Context:
         return s
 
     def copy_results(self, max_objects, segmap=False, shape=None):
-        objs = np.zeros(max_objects, OBJECT_DTYPE)
+        objs = np.empty(max_objects, OBJECT_DTYPE)
         n = C.c_int()
         seg = np.zeros(shape, np.int32) if segmap else None
         rc = lib().sexgpu_copy_results(self.h, objs.ctypes.data_as(C.c_void_p), max_objects, C.byref(n),
@@ -386,7 +384,7 @@ class Context:
             cfg = make_config(**kw)
             h, w = img.shape
             cap = max_objects or (w * h // max(1, cfg.detect_minarea) // 2 + 16)
-            objs = np.zeros(cap, OBJECT_DTYPE)
+            objs = np.empty(cap, OBJECT_DTYPE)
             keep.append((img, cfg, objs, wmap))
             f = arr[i]
             f.img, f.w, f.h, f.cfg = _f(img), w, h, C.pointer(cfg)
@@ -421,15 +419,13 @@ class Context:
         img = self._queued[0][0] if getattr(self, "_queued", None) else None
         if max_objects is None:
             max_objects = (img.size // max(1, cfg.detect_minarea) // 2 + 16) if img is not None else 16
-        objs = np.zeros(max_objects, OBJECT_DTYPE)
         n = C.c_int()
         s = Summary()
-        rc = lib().sexgpu_stream_next(self.h, C.byref(cfg), objs.ctypes.data_as(C.c_void_p), max_objects,
-                                      C.byref(n), C.byref(s))
+        rc = lib().sexgpu_stream_next(self.h, C.byref(cfg), None, 0, C.byref(n), C.byref(s))
         if getattr(self, "_queued", None):
             self._queued.pop(0)
         _check(rc, self.h, "sexgpu_stream_next")
-        return objs[:n.value], s
+        return self._results("sexgpu_stream_next", n.value, max_objects, None)[0], s
 
     def graph_stats(self):
         """(replayed, kernels, kinds) of the last extraction (sexgpu_graph_stats)."""

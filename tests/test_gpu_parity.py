@@ -465,3 +465,29 @@ def test_components_at_tile_edges(gpu_ctx, masks, w, h, weighted, bs, thr):
         compare_catalogs(g, o)
     else:
         run_both(gpu_ctx, img, **kw)
+
+
+@pytest.mark.parametrize("w,h,nsrc", [(64, 48, 0), (333, 257, 60), (1024, 700, 900)])
+def test_results_sized_by_count(gpu_ctx, w, h, nsrc):
+    """Rows and maps that are fetched after the extraction into arrays of their
+    size are those of the one-call form; a limit of exactly the rows is enough,
+    one less is an error."""
+    import ctypes as C
+
+    import sexgpu
+    img = synth.frame_c0(seed=w + nsrc, w=w, h=h, nsrc=nsrc) if nsrc else np.full((h, w), 7.0, np.float32)
+    g, gseg, gs, sub, cd = gpu_ctx.extract(img, want_maps=True)
+    cfg, n = sexgpu.make_config(), C.c_int()
+    rows, seg = np.zeros(len(g) + 3, sexgpu.OBJECT_DTYPE), np.zeros((h, w), np.int32)
+    sub1, cd1 = np.zeros((h, w), np.float32), np.zeros((h, w), np.float32)
+    f = [a.ctypes.data_as(C.POINTER(C.c_float)) for a in (img, sub1, cd1)]
+    assert sexgpu.lib().sexgpu_extract(gpu_ctx.h, f[0], None, w, h, C.byref(cfg), rows.ctypes.data_as(C.c_void_p),
+                                       len(rows), C.byref(n), seg.ctypes.data_as(C.c_void_p), f[1], f[2],
+                                       None) == sexgpu.OK
+    assert n.value == len(g) == gs.nobj
+    assert np.array_equal(rows[:len(g)].view(np.uint8), g.view(np.uint8)) and not rows[len(g):].view(np.uint8).any()
+    assert np.array_equal(seg, gseg) and np.array_equal(sub1, sub) and np.array_equal(cd1, cd)
+    assert len(gpu_ctx.extract(img, max_objects=len(g))[0]) == len(g)
+    if len(g):
+        with pytest.raises(RuntimeError):
+            gpu_ctx.extract(img, max_objects=len(g) - 1)
