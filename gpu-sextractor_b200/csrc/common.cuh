@@ -398,12 +398,6 @@ inline FastDiv make_fastdiv(unsigned d) {
     f.m = d > 1 ? (~0ull) / d + 1 : 0ull;
     return f;
 }
-__device__ __forceinline__ FastDiv make_fastdiv_dev(unsigned d) {
-    FastDiv f;
-    f.d = d;
-    f.m = d > 1 ? (~0ull) / d + 1 : 0ull;
-    return f;
-}
 __device__ __forceinline__ unsigned fdiv(unsigned p, const FastDiv &f) {
     return f.m ? (unsigned)__umul64hi((unsigned long long)p, f.m) : p;
 }

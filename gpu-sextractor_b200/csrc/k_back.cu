@@ -45,6 +45,23 @@ namespace sx {
 constexpr int SEQ_G = 16;                          // pixels of a lane's stretch
 constexpr int SEQ_CHUNK = 32 * SEQ_G;              // pixels taken at a time
 constexpr int SEQ_PITCH = SEQ_G + 4;               // staged stretches: 16-byte reads on distinct banks
+constexpr int SEQ_STAGE = 32 * SEQ_PITCH;          // floats of a staged chunk
+
+// asynchronous copies into shared memory, and the wait for all but the newest
+// N groups of this lane's
+__device__ __forceinline__ void cp_async4(float *dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async16(float *dst, const float *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 
 struct SeqSums {
     double sum, sq;
@@ -63,40 +80,44 @@ __device__ __forceinline__ bool seq_in(float f, float lcut, float hcut) {
     return (!VALID || f > (float)-SX_BIG) && f <= hcut && f >= lcut;
 }
 
-// LOAD: chunk(v) loads the sequence's next SEQ_CHUNK pixels, SEQ_G per lane
-// (NaN beyond the end), store(stage, v) puts them at their places of the
-// staged stretches; stage: 32 * SEQ_PITCH floats of this warp, 16-byte
-// aligned.  amin: for pass 1, what pass 0 found (its pixels are among them).
+// LOAD: fetch<G, STRETCH>(dst) starts the copies of the sequence's next 32 G
+// pixels (NaN beyond the end) to dst, as they come or into their lanes'
+// stretches, as one group.  Each chunk is on its way while the one before it is
+// taken (with a chunk loaded, stored and taken in turn, DRAM and L2 latency were
+// a tenth of the background stage of a frame of few meshes: 0.199 ms for 128 x 128
+// meshes of 4096 x 4096 pixels, 0.176 so).  stage: 2 SEQ_STAGE floats of
+// this warp, 16-byte aligned.  amin: for pass 1, what pass 0 found (its pixels
+// are among them).
 template <int PASS, bool VALID, class LOAD>
 __device__ __forceinline__ SeqSums seq_sums(LOAD load, int n, float lcut, float hcut, unsigned amin, float *stage) {
     const int lane = threadIdx.x & 31;
     double S = 0.0, m = 0.0;
     int cnt = 0;
+    load.template fetch<SEQ_G, true>(stage);
+    const float *cur = stage;
     for (int c0 = 0; c0 < n; c0 += SEQ_CHUNK) {
-        float v[SEQ_G];
-        load.chunk(v);
-#pragma unroll
-        for (int g = 0; g < SEQ_G; g++) {
-            const bool in = seq_in<PASS, VALID>(v[g], lcut, hcut);
-            v[g] = in ? v[g] : 0.0f;
-            cnt += in;
-            if (PASS == 0) amin = min(amin, (__float_as_uint(v[g]) & 0x7fffffffu) - 1u);
+        if (c0 + SEQ_CHUNK < n) {
+            load.template fetch<SEQ_G, true>(cur == stage ? stage + SEQ_STAGE : stage);
+            cp_wait<1>();
+        } else {
+            cp_wait<0>();
         }
-        LOAD::store(stage, v);
         __syncwarp();
-        const float4 *mine = reinterpret_cast<const float4 *>(stage + lane * SEQ_PITCH);
+        const float4 *mine = reinterpret_cast<const float4 *>(cur + lane * SEQ_PITCH);
         double d[SEQ_G];
 #pragma unroll
         for (int g = 0; g < SEQ_G / 4; g++) {
-            const float4 f = mine[g];
-            d[4 * g] = (double)f.x;
-            d[4 * g + 1] = (double)f.y;
-            d[4 * g + 2] = (double)f.z;
-            d[4 * g + 3] = (double)f.w;
-            m += d[4 * g];
-            m += d[4 * g + 1];
-            m += d[4 * g + 2];
-            m += d[4 * g + 3];
+            const float4 f4 = mine[g];
+            const float f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const bool in = seq_in<PASS, VALID>(f[k], lcut, hcut);
+                const float v = in ? f[k] : 0.0f;
+                cnt += in;
+                if (PASS == 0) amin = min(amin, (__float_as_uint(v) & 0x7fffffffu) - 1u);
+                d[4 * g + k] = (double)v;
+                m += d[4 * g + k];
+            }
         }
         for (int first = 0; first < 32;) {
             // S in [2^k, 2 * 2^k)
@@ -138,16 +159,17 @@ __device__ __forceinline__ SeqSums seq_sums(LOAD load, int n, float lcut, float 
                 if (stop > 0) S = __shfl_sync(0xffffffffu, after, stop - 1);
             }
             if (stop < 32) {
-                const float *st = stage + stop * SEQ_PITCH;
+                const float *st = cur + stop * SEQ_PITCH;
 #pragma unroll
                 for (int g = 0; g < SEQ_G; g++) {
-                    const double x = (double)st[g];
+                    const double x = seq_in<PASS, VALID>(st[g], lcut, hcut) ? (double)st[g] : 0.0;
                     S = fma(x, x, S);
                 }
             }
             first = stop + 1;
         }
-        __syncwarp();
+        __syncwarp();  // (every lane has read this chunk: its place takes the next but one)
+        cur = cur == stage ? stage + SEQ_STAGE : stage;
     }
     SeqSums r;
     r.sq = S;
@@ -168,15 +190,16 @@ template <int PASS, bool VALID, class LOAD>
 __device__ __noinline__ double seq_sum_slow(LOAD load, int n, float lcut, float hcut, float *stage) {
     double m = 0.0;
     for (int c0 = 0; c0 < n; c0 += SEQ_CHUNK) {
-        float v[SEQ_G];
-        load.chunk(v);
-        for (int g = 0; g < SEQ_G; g++) v[g] = seq_in<PASS, VALID>(v[g], lcut, hcut) ? v[g] : 0.0f;
-        __syncwarp();
-        LOAD::store(stage, v);
+        load.template fetch<SEQ_G, true>(stage);
+        cp_wait<0>();
         __syncwarp();
         for (int l = 0; l < 32; l++)
 #pragma unroll
-            for (int k = 0; k < SEQ_G; k++) m += (double)stage[l * SEQ_PITCH + k];
+            for (int k = 0; k < SEQ_G; k++) {
+                const float f = stage[l * SEQ_PITCH + k];
+                m += seq_in<PASS, VALID>(f, lcut, hcut) ? (double)f : 0.0;
+            }
+        __syncwarp();
     }
     return m;
 }
@@ -215,15 +238,19 @@ __device__ __forceinline__ void seq_stat(const LOAD &load, int n, float minpix, 
     o.qzero = mean - SX_QUANTIF_NSIGMA * sigma;
 }
 
-// staged place of chunk pixel i
-__device__ __forceinline__ int seq_slot(int i) { return (i / SEQ_G) * SEQ_PITCH + i % SEQ_G; }
+// place of pixel i of a fetch
+template <bool STRETCH>
+__device__ __forceinline__ int seq_slot(int i) {
+    return STRETCH ? (i / SEQ_G) * SEQ_PITCH + i % SEQ_G : i;
+}
 
-// the pixels of a mw x mh mesh in row-major order, SEQ_CHUNK at a time: lane
-// l loads words l, l + 32, ... of a chunk, of four pixels (VEC: frame and mesh
+// the pixels of a mw x mh mesh in row-major order: lane l copies words l,
+// l + 32, ... of a fetch, of four pixels (VEC: frame and mesh
 // width multiples of 4, frame 16-byte aligned) or one
 template <bool VEC>
 struct MeshLoad {
     static constexpr int V = VEC ? 4 : 1;
+    static constexpr bool REGS = VEC;  // the histogram's pixels go through registers
     const float *origin;
     int off, left, col, mw, step, wrap, dcol;
     __device__ __forceinline__ MeshLoad(const float *origin_, int w, int mw_, int mh) {
@@ -238,39 +265,48 @@ struct MeshLoad {
         wrap = w - mw;
         left = mw * mh - V * lane;
     }
-    __device__ __forceinline__ void chunk(float *v) {
-        // beyond the mesh: NaN, which every test rejects as it does a NaN pixel
-        const float nan = __int_as_float(0x7fffffff);
-#pragma unroll
-        for (int g = 0; g < SEQ_G / V; g++) {
-            if (VEC) {
-                const float4 f = left > 0 ? __ldg(reinterpret_cast<const float4 *>(origin + off))
-                                          : make_float4(nan, nan, nan, nan);
-                v[4 * g] = f.x;
-                v[4 * g + 1] = f.y;
-                v[4 * g + 2] = f.z;
-                v[4 * g + 3] = f.w;
-            } else {
-                v[g] = left > 0 ? __ldg(origin + off) : nan;
-            }
-            left -= 32 * V;
-            col += dcol;
-            off += step;
-            if (col >= mw) {
-                col -= mw;
-                off += wrap;
-            }
+    __device__ __forceinline__ void next() {
+        left -= 32 * V;
+        col += dcol;
+        off += step;
+        if (col >= mw) {
+            col -= mw;
+            off += wrap;
         }
     }
-    static __device__ __forceinline__ void store(float *stage, const float *v) {
-        const int lane = threadIdx.x & 31;
+    template <int G, bool STRETCH>
+    __device__ __forceinline__ void fetch(float *dst) {
+        dst += seq_slot<STRETCH>(V * (threadIdx.x & 31));
+        const bool whole = VEC && left > 32 * V * (G / V - 1);
 #pragma unroll
-        for (int g = 0; g < SEQ_G / V; g++) {
-            if (VEC)
-                *reinterpret_cast<float4 *>(stage + seq_slot(4 * (lane + 32 * g))) =
-                    make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-            else
-                stage[seq_slot(lane + 32 * g)] = v[g];
+        for (int g = 0; g < G / V; g++) {
+            float *to = dst + seq_slot<STRETCH>(32 * V * g);
+            if (whole || left > 0) {
+                if (VEC)
+                    cp_async16(to, origin + off);
+                else
+                    cp_async4(to, origin + off);
+            } else {
+                // beyond the mesh: NaN, which every test rejects as it does a NaN pixel
+                for (int k = 0; k < V; k++) to[k] = __int_as_float(0x7fffffff);
+            }
+            next();
+        }
+        cp_commit();
+    }
+    // the same into registers (VEC)
+    template <int G>
+    __device__ __forceinline__ void take(float (&v)[G]) {
+        const float nan = __int_as_float(0x7fffffff);
+#pragma unroll
+        for (int g = 0; g < G / 4; g++) {
+            const float4 f = left > 0 ? __ldg(reinterpret_cast<const float4 *>(origin + off))
+                                      : make_float4(nan, nan, nan, nan);
+            v[4 * g] = f.x;
+            v[4 * g + 1] = f.y;
+            v[4 * g + 2] = f.z;
+            v[4 * g + 3] = f.w;
+            next();
         }
     }
 };
@@ -289,7 +325,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(32) k_mesh_stat(const float *__restrict__ img, int w, int h, int bw, int bh, int nbx,
                                                   int nby, MeshStat *__restrict__ ms) {
     sx_pdl();
-    __shared__ __align__(16) float stage[32 * SEQ_PITCH];
+    __shared__ __align__(16) float stage[2 * SEQ_STAGE];
     const int m = blockIdx.x;
     int x0, y0, mw, mh, nv;
     mesh_geometry(m, w, h, bw, bh, nbx, nby, x0, y0, mw, mh);
@@ -614,23 +650,56 @@ __device__ __forceinline__ void gw_guess(GuessWarpSmem &S, const MeshStat &bm, f
     sg = sig_ * bm.qscale;
 }
 
-// the histogram of the n pixels of a sequence and its mode, by one warp
+// The histogram of the n pixels of a sequence and its mode, by one warp, the
+// next pixels on their way while these are counted: in registers, or through
+// two buffers in the place of the chunk sums, which are not in use yet.
+constexpr int GW_FETCH = 8;  // pixels of a lane at a time
+static_assert(sizeof(GuessWarpSmem) - sizeof(unsigned) * GW_WORDS >= 2 * 32 * GW_FETCH * sizeof(float) &&
+                  sizeof(unsigned) * GW_WORDS >= 2 * SEQ_STAGE * sizeof(float) && GW_WORDS % 4 == 0,
+              "staged pixels fit the histogram's memory");
+
 template <bool VALID, class LOAD>
 __device__ __forceinline__ void gw_mode(LOAD load, int n, GuessWarpSmem &S, const MeshStat &bm, float &mode, float &sg) {
     const int lane = threadIdx.x & 31;
-    for (int i = lane; i < GW_WORDS; i += 32) S.hw[i] = 0u;
-    __syncwarp();
     const int nlevels = bm.nlevels;
     const float qscale = bm.qscale;
     const float cste = 0.499999 - bm.qzero / qscale;
-    for (int k0 = 0; k0 < n; k0 += SEQ_CHUNK) {
-        float v[SEQ_G];
-        load.chunk(v);
+    if constexpr (LOAD::REGS) {
+        float v[SEQ_G], nv[SEQ_G];
+        load.take(nv);
+        for (int i = lane; i < GW_WORDS; i += 32) S.hw[i] = 0u;
+        __syncwarp();
+        for (int k0 = 0; k0 < n; k0 += SEQ_CHUNK) {
 #pragma unroll
-        for (int g = 0; g < SEQ_G; g++)
-            if (!VALID || v[g] > (float)-SX_BIG) gw_count(S, v[g], qscale, cste, nlevels);
+            for (int g = 0; g < SEQ_G; g++) v[g] = nv[g];
+            load.take(nv);
+#pragma unroll
+            for (int g = 0; g < SEQ_G; g++)
+                if (!VALID || v[g] > (float)-SX_BIG) gw_count(S, v[g], qscale, cste, nlevels);
+        }
+        __syncwarp();
+    } else {
+        float *const stage = reinterpret_cast<float *>(S.hw + GW_WORDS), *cur = stage;
+        load.template fetch<GW_FETCH, false>(stage);
+        for (int i = lane; i < GW_WORDS; i += 32) S.hw[i] = 0u;
+        for (int k0 = 0; k0 < n; k0 += 32 * GW_FETCH) {
+            float *const other = cur == stage ? stage + 32 * GW_FETCH : stage;
+            if (k0 + 32 * GW_FETCH < n) {
+                load.template fetch<GW_FETCH, false>(other);
+                cp_wait<1>();
+            } else {
+                cp_wait<0>();
+            }
+            __syncwarp();
+#pragma unroll
+            for (int g = 0; g < GW_FETCH; g++) {
+                const float v = cur[lane + 32 * g];
+                if (!VALID || v > (float)-SX_BIG) gw_count(S, v, qscale, cste, nlevels);
+            }
+            __syncwarp();
+            cur = other;
+        }
     }
-    __syncwarp();
     gw_guess(S, bm, mode, sg);
 }
 
@@ -695,50 +764,57 @@ __device__ __forceinline__ int local_npix(const LocalBox &B, int pbs) {
     return (B.bymax - B.bymin) * 2 * pbs + ((B.iymin - B.bymin) + (B.bymax - B.iymax)) * (B.ixmax - B.ixmin);
 }
 
-// the annulus pixels lane, lane + 32, ... in the reference's collection order
+// The annulus pixels lane, lane + 32, ... in the reference's collection order:
+// three rectangles, the first (both strips) with a gap in its rows.  One copy
+// after the other in a short loop: with sixteen at a time, each with its
+// divisions, in three places, the warps waited for instructions more than half
+// the time and the annuli of a 2501 x 1999 frame took 0.68 ms, now 0.56; the largest annuli, one
+// warp each, last longest.
 struct LocalLoad {
+    static constexpr bool REGS = false;
     const float *sub;
-    int w, i, n, ns, pbs, iw, bxmin, bymin, ixmin, ixmax, iymin, iymax;
-    FastDiv dsw, diw;
-    __device__ __forceinline__ LocalLoad(const float *sub_, int w_, const LocalBox &B, int pbs_) {
-        sub = sub_;
-        w = w_;
-        pbs = pbs_;
-        i = threadIdx.x & 31;
+    int w, n, i, reg, W, end, col, off, dcol, step, split, gap;  // split: first column beyond the gap
+    LocalBox B;
+    int pbs;
+    __device__ __forceinline__ LocalLoad(const float *sub_, int w_, const LocalBox &B_, int pbs_)
+        : sub(sub_), w(w_), i(threadIdx.x & 31), B(B_), pbs(pbs_) {
         n = local_npix(B, pbs);
-        ns = (B.bymax - B.bymin) * 2 * pbs;
-        iw = B.ixmax - B.ixmin;
-        bxmin = B.bxmin;
-        bymin = B.bymin;
-        ixmin = B.ixmin;
-        ixmax = B.ixmax;
-        iymin = B.iymin;
-        iymax = B.iymax;
-        dsw = make_fastdiv_dev((unsigned)(2 * pbs));
-        diw = make_fastdiv_dev((unsigned)iw);
+        enter(0);
     }
-    __device__ __forceinline__ void chunk(float *v) {
-#pragma unroll
-        for (int g = 0; g < SEQ_G; g++, i += 32) {
-            v[g] = __int_as_float(0x7fffffff);
+    // to this lane's place in rectangle r
+    __device__ __forceinline__ void enter(int r) {
+        const int ns = (B.bymax - B.bymin) * 2 * pbs, iw = B.ixmax - B.ixmin, nt = (B.iymin - B.bymin) * iw;
+        reg = r;
+        W = max(r ? iw : 2 * pbs, 1);
+        end = r == 0 ? ns : r == 1 ? ns + nt : n;
+        split = r ? 0x7fffffff : pbs;
+        gap = B.ixmax - pbs - B.bxmin;
+        const int k = i - (r == 0 ? 0 : r == 1 ? ns : ns + nt), row = k / W, drow = 32 / W;
+        col = k - row * W;
+        off = ((r < 2 ? B.bymin : B.iymax) + row) * w + (r ? B.ixmin : B.bxmin);
+        dcol = 32 - drow * W;
+        step = drow * w;
+    }
+    template <int G, bool STRETCH>
+    __device__ __forceinline__ void fetch(float *dst) {
+        dst += seq_slot<STRETCH>(threadIdx.x & 31);
+#pragma unroll 1
+        for (int g = 0; g < G; g++, dst += seq_slot<STRETCH>(32)) {
             if (i < n) {
-                int x, y;
-                if (i < ns) {
-                    const int r = (int)fdiv((unsigned)i, dsw), c = i - r * 2 * pbs;
-                    y = bymin + r;
-                    x = c < pbs ? bxmin + c : ixmax + c - pbs;
-                } else {
-                    const int k = i - ns, r = (int)fdiv((unsigned)k, diw);
-                    x = ixmin + k - r * iw;
-                    y = r < iymin - bymin ? bymin + r : iymax + r - (iymin - bymin);
-                }
-                v[g] = __ldg(sub + (size_t)y * w + x);
+                while (i >= end) enter(reg + 1);
+                cp_async4(dst, sub + off + col + (col >= split ? gap : 0));
+            } else {
+                *dst = __int_as_float(0x7fffffff);
+            }
+            i += 32;
+            col += dcol;
+            off += step;
+            if (col >= W) {
+                col -= W;
+                off += w;
             }
         }
-    }
-    static __device__ __forceinline__ void store(float *stage, const float *v) {
-#pragma unroll
-        for (int g = 0; g < SEQ_G; g++) stage[seq_slot((threadIdx.x & 31) + 32 * g)] = v[g];
+        cp_commit();
     }
 };
 
