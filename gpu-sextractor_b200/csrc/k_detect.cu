@@ -79,7 +79,7 @@ constexpr int SP_NK = 16;                     // staged spline nodes per row (se
 struct SpArgs {
     const float *img;
     float *sub, *cd;
-    int *lab;
+    int *lab, *cnt;  // cnt: set to 0 at every tile component's label pixel, or null
     BackBufs B;
     int w, h, nbx, back_type, mw, mh, rxa, wthr, tilesx, ntiles;
     double dfac;
@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(ST_THREADS, 4) k_sub_filter(const __grid_const
                     } else {
                         const int r = sfind(s_L, (r0 + k) * ST_TW + run_start64(st, 4 * qc + c));
                         l[c] = (y0 + r / ST_TW) * w + x0 + r % ST_TW;
+                        if (A.cnt && l[c] == gy * w + gx + c) A.cnt[l[c]] = 0;
                     }
                 }
             }
@@ -585,9 +586,10 @@ static void sp_launch_mask(const CUtensorMap &tmap, const SpArgs &A, const ConvT
 }
 
 // Subtracted and filtered frame, and as labels the components within each
-// ST_TW x ST_TH tile.
-void launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const BackBufs &B, const FrameParams &P,
-                       FrameScalars *d_sc, const float *d_var, const ConvMask &M, cudaStream_t st, int &launches) {
+// ST_TW x ST_TH tile; cnt (or null) is zeroed at the labels' pixels.
+void launch_sub_filter(const float *img, float *sub, float *cd, int *lab, int *cnt, const BackBufs &B,
+                       const FrameParams &P, FrameScalars *d_sc, const float *d_var, const ConvMask &M,
+                       cudaStream_t st, int &launches) {
     const int mw = M.mw, mh = M.mh;
     const int rxa = ((mw / 2) + 3) & ~3;  // halo width rounded up to 16 bytes
     SpArgs A;
@@ -595,6 +597,7 @@ void launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const 
     A.sub = sub;
     A.cd = cd;
     A.lab = lab;
+    A.cnt = cnt;
     A.B = B;
     A.w = P.w;
     A.h = P.h;
@@ -663,46 +666,30 @@ __device__ __forceinline__ void gunion(int *L, int a, int b, int *status, int lo
 }
 
 // unions across tile borders (TW x TH tiles): pixels on the first row or
-// first/last column of a tile look at their backward neighbours in other tiles
+// first/last column of a tile look at their backward neighbours in other
+// tiles, those on the last column at the NE one (row y - 1 of the next tile)
 template <int TW, int TH>
 __global__ void k_ccl_border(int *__restrict__ lab, int w, int h, int *status, int loop_cap) {
     sx_pdl();
-    int tilesx = (w + TW - 1) / TW;
-    int tile = blockIdx.x, k = threadIdx.x;           // k < TW + TH
-    int tx0 = (tile % tilesx) * TW, ty0 = (tile / tilesx) * TH;
-    int x, y;
-    if (k < TW) {
-        x = tx0 + k;
-        y = ty0;
-    } else {
-        x = tx0;
-        y = ty0 + (k - TW) + 1;
-        if (k - TW + 1 >= TH) return;
-    }
+    const int tilesx = (w + TW - 1) / TW, tile = blockIdx.x, k = threadIdx.x;  // k < TW + 2 (TH - 1)
+    const int tx0 = (tile % tilesx) * TW, ty0 = (tile / tilesx) * TH;
+    const bool east = k >= TW + TH - 1;
+    const int x = k < TW ? tx0 + k : east ? tx0 + TW - 1 : tx0, y = k < TW ? ty0 : ty0 + 1 + (k - TW) % (TH - 1);
     if (x >= w || y >= h) return;
-    int p = y * w + x;
+    const int p = y * w + x;
     if (lab[p] < 0) return;
+    if (east) {
+        if (x < w - 1 && lab[p - w + 1] >= 0) gunion(lab, p, p - w + 1, status, loop_cap);
+        return;
+    }
     // W neighbour (other tile when x is the tile's first column)
     if (x == tx0 && x > 0 && lab[p - 1] >= 0) gunion(lab, p, p - 1, status, loop_cap);
     if (y > 0) {
         // NW: other tile when x or y is on the tile's first column/row
         if (x > 0 && (x == tx0 || y == ty0) && lab[p - w - 1] >= 0) gunion(lab, p, p - w - 1, status, loop_cap);
         if (y == ty0 && lab[p - w] >= 0) gunion(lab, p, p - w, status, loop_cap);
-        if (x < w - 1 && (y == ty0 || x == tx0 + TW - 1) && lab[p - w + 1] >= 0) gunion(lab, p, p - w + 1, status, loop_cap);
+        if (x < w - 1 && y == ty0 && lab[p - w + 1] >= 0) gunion(lab, p, p - w + 1, status, loop_cap);
     }
-}
-
-// the last column of each tile also looks NE into the next tile (row y-1)
-template <int TW, int TH>
-__global__ void k_ccl_border_ne(int *__restrict__ lab, int w, int h, int *status, int loop_cap) {
-    sx_pdl();
-    int tilesx = (w + TW - 1) / TW;
-    int tile = blockIdx.x, k = threadIdx.x;  // k in [1, TH)
-    if (k == 0 || k >= TH) return;
-    int x = (tile % tilesx) * TW + TW - 1, y = (tile / tilesx) * TH + k;
-    if (x >= w - 1 || y >= h) return;
-    int p = y * w + x;
-    if (lab[p] >= 0 && lab[p - w + 1] >= 0) gunion(lab, p, p - w + 1, status, loop_cap);
 }
 
 // every pixel to its root, and the component sizes: lanes of a warp holding
@@ -748,14 +735,13 @@ __global__ void k_ccl_flatten(int *__restrict__ lab, long long n, int *__restric
     }
 }
 
-// cnt: zeroed, w*h ints; receives the size of every component at its root
+// cnt: w*h ints, zeroed at the components' labels; receives the size of every component at its root
 // lab: the tile-local components of k_sub_filter's tiles
 void launch_ccl(int *lab, int *cnt, const FrameParams &P, FrameScalars *d_sc, cudaStream_t st, int &launches) {
     int *status = &d_sc->status;
     const int ntiles = ((P.w + ST_TW - 1) / ST_TW) * ((P.h + ST_TH - 1) / ST_TH);
-    sx_launch(k_ccl_border<ST_TW, ST_TH>, ntiles, ST_TW + ST_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
-    sx_launch(k_ccl_border_ne<ST_TW, ST_TH>, ntiles, ST_TH, 0, st, lab, P.w, P.h, status, P.loop_cap);
-    launches += 3;
+    sx_launch(k_ccl_border<ST_TW, ST_TH>, ntiles, ST_TW + 2 * (ST_TH - 1), 0, st, lab, P.w, P.h, status, P.loop_cap);
+    launches += 2;
     long long n = (long long)P.w * P.h;
     sx_launch(k_ccl_flatten, (unsigned)((n + 1023) / 1024), 256, 0, st, lab, n, cnt, status, P.loop_cap);
 }

@@ -151,12 +151,18 @@ __global__ void k_clean_chain(ObjBufs O, int n, const int *n_dev, int *vcnt, int
 // in any order (voff: exclusive sums of vcnt; vfill zeroed before), then each
 // to its rank among them in vsort.  A victim compares itself with the others
 // of its survivor only, usually a handful.
-__global__ void k_victim_scatter(ObjBufs O, int n, const int *n_dev, const int *voff, int *vfill, int *vlist) {
+// The pixels of a victim belong to its survivor in the allocation map (one warp
+// per object).
+__global__ void k_victim_scatter(ObjBufs O, int n, const int *n_dev, const int *voff, int *vfill, int *vlist,
+                                 const unsigned *opix, int *alloc) {
     sx_pdl();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= sx_count(n, n_dev)) return;
     const int m = O.fmaster[i];
-    if (m >= 0) vlist[voff[m] + atomicAdd(vfill + m, 1)] = i;
+    if (m < 0) return;
+    if (lane == 0) vlist[voff[m] + atomicAdd(vfill + m, 1)] = i;
+    const int off = O.off[i], cnt = O.n[i];
+    for (int k = lane; k < cnt; k += 32) alloc[opix[off + k]] = m;
 }
 
 __global__ void k_victim_rank(ObjBufs O, int n, const int *n_dev, const int *voff, const int *vcnt, const int *vlist,
@@ -201,18 +207,6 @@ __global__ void k_clean_merge(ObjBufs O, int n, const int *n_dev, const int *vof
     }
 }
 
-// pixels of cleaned objects belong to their master in the allocation map (one
-// warp per object)
-__global__ void k_alloc_victims(ObjBufs O, const unsigned *opix, int *alloc, int n, const int *n_dev) {
-    sx_pdl();
-    const int o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (o >= sx_count(n, n_dev)) return;
-    const int m = O.fmaster[o];
-    if (m < 0) return;
-    const int off = O.off[o], cnt = O.n[o];
-    for (int i = threadIdx.x & 31; i < cnt; i += 32) alloc[opix[off + i]] = m;
-}
-
 // ---------------------------------------------------------------------------
 // photometry and FLAGS of the survivors
 // ---------------------------------------------------------------------------
@@ -220,6 +214,7 @@ struct EndRaw;
 
 struct EndArgs {
     EndRaw *raw;    // per-object state between the photometry kernels
+    int *surv;      // per object: 1 for a survivor of CLEAN, 0 for a victim (k_end_finish)
     KronGeo *geo;   // per object: the next pass's ellipse and box (pass 1's from k_examine_finish)
     double2 *aper;  // per object and aperture: flux, variance
     const float *sub;
@@ -754,7 +749,10 @@ __global__ void __launch_bounds__(KR_THREADS) k_kron_chunks(const __grid_constan
 __global__ void k_end_finish(const __grid_constant__ EndArgs A) {
     sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= sx_count(A.n, A.n_dev) || A.O.fmaster[o] >= 0) return;
+    if (o >= sx_count(A.n, A.n_dev)) return;
+    const bool victim = A.O.fmaster[o] >= 0;
+    A.surv[o] = victim ? 0 : 1;
+    if (victim) return;
     for (int k = 0; k < A.naper; k++) {
         const double2 ap = A.aper[(size_t)o * A.naper + k];
         const double tv = ap.x;
@@ -885,12 +883,6 @@ void launch_endobject(const EndArgs &E, int nobj, cudaStream_t st, int &launches
 // element tiles before its own, and those of the raw objects of its tile whose
 // element is smaller (a linked list of a few).
 constexpr int NO_TILE = 1024;  // elements; 3 to 20 raw objects of a crowded frame
-
-__global__ void k_surv_flags(ObjBufs O, int n, const int *n_dev, int *flag) {
-    sx_pdl();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < sx_count(n, n_dev)) flag[i] = O.fmaster[i] < 0 ? 1 : 0;
-}
 
 struct OrderBufs {
     const int *pos;         // exclusive sums of the survivor flags

@@ -63,18 +63,6 @@ __global__ void k_root_thresholds(int nroots, const int *nroots_dev, double dfac
     if ((threadIdx.x & 31) == 0 && e < *(volatile int *)&sc->e0cd) atomicMin(&sc->e0cd, e);
 }
 
-// without a weight map every raw object has the global thresholds
-__global__ void k_root_thresholds_global(int nroots, const int *nroots_dev, const FrameScalars *sc, float *rdthr,
-                                         float *rathr) {
-    sx_pdl();
-    nroots = sx_count(nroots, nroots_dev);
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nroots) {
-        rdthr[r] = sc->dthresh;
-        rathr[r] = sc->thresh;
-    }
-}
-
 // ---- the raw-object numbering and the kept-pixel compaction as two scans
 // whose inputs are computed on the fly (a root: lab[p] == p with at least
 // minarea pixels; a kept pixel: its root has at least minarea pixels).  The
@@ -127,10 +115,13 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_tile_counts(const int *__
     if (threadIdx.x == 0) tkept[blockIdx.x] = tot;
 }
 
-// roots numbered in raster order: rid at the root pixel, and size
+// roots numbered in raster order: rid at the root pixel, and size; their
+// thresholds start as the global ones, or (minvar) as the largest variance
 __global__ void __launch_bounds__(SCAN_THREADS) k_root_number(const int *__restrict__ lab, const int *__restrict__ cnt,
                                                              long long n, int minarea, const int *__restrict__ toff,
-                                                             int *__restrict__ rid, int *__restrict__ rsize) {
+                                                             int *__restrict__ rid, int *__restrict__ rsize,
+                                                             const FrameScalars *sc, bool minvar,
+                                                             float *__restrict__ rdthr, float *__restrict__ rathr) {
     sx_pdl();
     __shared__ int sh[32];
     const long long base = (long long)blockIdx.x * SCAN_TILE + (long long)threadIdx.x * SCAN_ITEMS;
@@ -138,6 +129,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_number(const int *__restr
     root_kept_flags4(lab, cnt, base, n, minarea, fr, kp, l);
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; k++) c += fr[k];
+    const float dthr = minvar ? __int_as_float(0x7f7f7f7f) : sc->dthresh, athr = sc->thresh;
     int tot;
     int id = block_exclusive_scan(c, sh, tot) + toff[blockIdx.x];
 #pragma unroll
@@ -146,6 +138,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_root_number(const int *__restr
             const long long p = base + k;
             rid[p] = id;
             rsize[id] = cnt[p];
+            rdthr[id] = dthr;
+            rathr[id] = athr;
             id++;
         }
 }

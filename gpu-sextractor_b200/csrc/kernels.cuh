@@ -159,7 +159,7 @@ struct ConvMask {
     int mw, mh;
 };
 
-void launch_sub_filter(const float *img, float *sub, float *cd, int *lab, const BackBufs &B,
+void launch_sub_filter(const float *img, float *sub, float *cd, int *lab, int *cnt, const BackBufs &B,
                        const FrameParams &P, FrameScalars *d_sc, const float *d_var, const ConvMask &M,
                        cudaStream_t st, int &launches);
 

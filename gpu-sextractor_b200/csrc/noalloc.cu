@@ -166,7 +166,6 @@ extern "C" int sexgpu_background_noalloc(const float *d_img, float *d_sub, int w
     B.colk = (int *)(base + OFF_COLK);
     B.coldx = (float *)(base + OFF_COLDX);
     int nl = 0;
-    sx_launch(k_init_scalars, 1, 1, 0, st, d_sc);  // the pipeline's initial scalars (sigfac 1)
     sx_launch(k_col_table, (w + 255) / 256, 256, 0, st, w, Pm.nbx, Pm.bw, B.colk, B.coldx);
     sx::launch_background(B, d_img, Pm, d_sc, st, nl);
     long long n = (long long)w * h;

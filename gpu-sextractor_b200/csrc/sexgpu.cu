@@ -156,7 +156,7 @@ struct sexgpu_ctx {
            D_KEPT, D_GEVM, D_KREP, D_GB0, D_GPAR, D_GNSON, D_GLABEL, D_GFLAGS, D_GDLIST, D_GELIST, D_GM, D_COUNT };
     DevBuf deb;  // all of them
     // objects
-    DevBuf o_i[20], o_f[32], o_d[10], o_iso, o_sortkey, amp, alpha, cellhead, vict, svals, order, rows;
+    DevBuf o_i[20], o_f[32], o_d[10], o_iso, amp, zeros, vict, svals, order, rows;
     DevBuf oitems;                         // bands of large objects' boxes (pixel lists)
     DevBuf kitem[2], kchunk[2], kpart[2];  // queued Kron boxes
     DevBuf o_sprob;                        // CLASS_STAR per object
@@ -380,14 +380,6 @@ void make_params(const sexgpu_config *cfg, int w, int h, FrameParams &P) {
     P.bp_local = cfg->back_photo_type == 1;
     P.bp_thick = cfg->back_photo_thick;
     P.loop_cap = 0;
-}
-
-__global__ void k_init_scalars(FrameScalars *sc) {
-    sx_pdl();
-    FrameScalars z;
-    memset(&z, 0, sizeof(z));
-    z.sigfac = 1.0f;
-    *sc = z;
 }
 
 // Capacity form: the checks the plain form makes on the host between stages.
@@ -652,7 +644,6 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
 
     stage_begin(ctx);
     int nl = 0;
-    sx_launch(k_init_scalars, 1, 1, 0, st, d_sc);
     ps.wvar = nullptr;
     if (d_wmap) {
         // pixels of unusable weight are blank for the background and the detection
@@ -679,7 +670,7 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
         EN(rmsnode, (size_t)h * Pm.nbx * 4);
         EN(rmsdnode, (size_t)h * Pm.nbx * 4);
         launch_map_nodes(B.sigma3, P<float>(ctx->rmsd), P<float>(ctx->rmsu), Pm.nbx, Pm.nby, Pm.bh, h,
-                         P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), P<float>(ctx->rmsu), st);
+                         P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), P<float>(ctx->rmsu), MedianArgs{}, st);
         sx_launch(k_rms_map, grid1(N, 256), 256, 0, st, P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), B.colk,
                   B.coldx, Pm.nbx, w, N, P<float>(ctx->wvar), 1);
         ps.wvar = P<float>(ctx->wvar);
@@ -702,13 +693,11 @@ int pipe_detect(sexgpu_ctx *ctx) {
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int *tmp = P<int>(ctx->scan_tmp);
     int rc = SEXGPU_OK, nl = 0;
-    launch_sub_filter(d_img, P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), B, Pm, d_sc, ps.wvar, ctx->cmask,
-                      st, nl);
+    int *lab = P<int>(ctx->lab), *cnt = P<int>(ctx->cnt), *flag = P<int>(ctx->flag), *pos = P<int>(ctx->pos);
+    launch_sub_filter(d_img, P<float>(ctx->sub), P<float>(ctx->cd), lab, cnt, B, Pm, d_sc, ps.wvar, ctx->cmask, st, nl);
     stage_mark(ctx, "sub_filter", nl);
 
     nl = 0;
-    int *lab = P<int>(ctx->lab), *cnt = P<int>(ctx->cnt), *flag = P<int>(ctx->flag), *pos = P<int>(ctx->pos);
-    CK(cudaMemsetAsync(cnt, 0, N * 4, st));
     launch_ccl(lab, cnt, Pm, d_sc, st, nl);  // labels to roots, component sizes at the roots
     stage_mark(ctx, "ccl", nl);
 
@@ -754,25 +743,36 @@ int pipe_detect(sexgpu_ctx *ctx) {
     R.objbase = P<int>(ctx->robjbase);
     R.dthresh = P<float>(ctx->rdthr);
     R.thresh = P<float>(ctx->rathr);
-    sx_launch(k_root_number, ntile, SCAN_THREADS, 0, st, lab, cnt, N, Pm.minarea, troff, flag, R.size);
-    nl += 3 + exclusive_scan(R.size, R.off, nroots, nullptr, tmp, st, nroots_dev);
+    // what the deblending counts per raw object, zeroed here (a copy or memset
+    // between two kernels keeps the second from starting early)
+    const size_t nzero = 6 * ((size_t)nroots + 1) + DT_NCOUNTS;
+    EN(rzero, nzero * 4);
+    CK(cudaMemsetAsync(ctx->rzero.p, 0, nzero * 4, st));
+    const bool minvar = ps.wvar && Pm.wthr;
+    sx_launch(k_root_number, ntile, SCAN_THREADS, 0, st, lab, cnt, N, Pm.minarea, troff, flag, R.size, d_sc, minvar,
+              R.dthresh, R.thresh);
+    nl += 2 + exclusive_scan(R.size, R.off, nroots, nullptr, tmp, st, nroots_dev);
     sx_launch(k_root_compact, ntile, SCAN_THREADS, 0, st, lab, cnt, N, Pm.minarea, tkoff, flag,
               P<unsigned>(ctx->keys), P<unsigned>(ctx->rpix), P<int>(ctx->alloc), P<int>(ctx->pos2idx));
-    if (ps.wvar && Pm.wthr) {
-        CK(cudaMemsetAsync(R.dthresh, 0x7f, (size_t)(nroots + 1) * 4, st));
+    if (minvar) {
         sx_launch(k_root_minvar, grid1(nrootpix, 256), 256, 0, st, P<unsigned>(ctx->keys), P<unsigned>(ctx->rpix),
                   nrootpix, ps.capf ? &d_sc->nrootpix : nullptr, ps.wvar, (int *)R.dthresh);
         sx_launch(k_root_thresholds, grid1(nroots, 256), 256, 0, st, nroots, nroots_dev, Pm.detect_thresh,
                   Pm.analysis_thresh, d_sc, R.dthresh, R.thresh);
-        nl += 1;
-    } else {
-        sx_launch(k_root_thresholds_global, grid1(nroots, 256), 256, 0, st, nroots, nroots_dev, d_sc, R.dthresh,
-                  R.thresh);
+        nl += 2;
     }
     stage_mark(ctx, "roots", nl);
     ps.stage = 2;
     return SEXGPU_OK;
 }
+
+// counters of CLEAN (whether it will run or not): cells (then starts) and their
+// fills, victims and fills
+size_t clean_cells(int w, int h) { return (size_t)((int)(w / CL_CELL) + 2) * ((int)(h / CL_CELL) + 2); }
+size_t clean_zeros(int w, int h, int nobj) {
+    return nobj > 0 ? 2 * (clean_cells(w, h) + 1) + 2 * ((size_t)nobj + 1) : 0;
+}
+int order_tiles(int nrootpix) { return nrootpix / NO_TILE + 1; }
 
 int pipe_deblend(sexgpu_ctx *ctx) {
     PipeState &ps = ctx->ps;
@@ -798,10 +798,8 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     unsigned char *const deb = P<unsigned char>(ctx->deb);
     // per raw object, zeroed: completion key, peak, counts of peaks, buckets
     // and own pixels; then the list lengths
-    EN(rzero, (6 * NR + DT_NCOUNTS) * 4);
     EN(rlists, 4 * NR * 4);
     EN(rthr, NR * Pm.nthresh * 4);
-    CK(cudaMemsetAsync(ctx->rzero.p, 0, (6 * NR + DT_NCOUNTS) * 4, st));
     R.last = P<unsigned long long>(ctx->rzero);
     R.peak = P<unsigned>(ctx->rzero) + 2 * NR;
     R.npk = P<int>(ctx->rzero) + 3 * NR;
@@ -882,6 +880,10 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     A.gobj = P<GatherObj>(ctx->o_gobj);
     A.nobj = nobj;
     A.nobj_dev = ps.capf ? &d_sc->nobj : nullptr;
+    // what CLEAN and the catalogue order count, zeroed here
+    const size_t nzero = clean_zeros(w, h, nobj) + 2 * (size_t)order_tiles(nrootpix);
+    EN(zeros, nzero * 4);
+    CK(cudaMemsetAsync(ctx->zeros.p, 0, nzero * 4, st));
     D.biglist = P<int>(ctx->o_big);
     nl += launch_deblend_assign(A, st);
     stage_mark(ctx, "deblend", nl);
@@ -970,14 +972,11 @@ int pipe_clean(sexgpu_ctx *ctx) {
     if (Pm.clean_flag && nobj > 0) {
         const int gx = (int)(w / CL_CELL) + 2, gy = (int)(h / CL_CELL) + 2, ncell = gx * gy;
         const size_t n1 = (size_t)nobj + 1;
-        // zeroed: cell counts (then starts) and fills, victim counts and fills
-        EN(cellhead, (2 * (size_t)(ncell + 1) + 2 * n1) * 4);
         EN(vict, 3 * n1 * 4);
         EN(amp, n1 * sizeof(CleanObj));
-        int *cellcnt = P<int>(ctx->cellhead), *cellcur = cellcnt + ncell + 1, *vcnt = cellcur + ncell + 1,
+        int *cellcnt = P<int>(ctx->zeros), *cellcur = cellcnt + ncell + 1, *vcnt = cellcur + ncell + 1,
             *vfill = vcnt + n1;
         int *voff = P<int>(ctx->vict), *vlist = voff + n1, *vsort = vlist + n1;
-        CK(cudaMemsetAsync(cellcnt, 0, (2 * (size_t)(ncell + 1) + 2 * n1) * 4, st));
         const int *nobj_dev = ps.capf ? &d_sc->nobj : nullptr;
         const unsigned g = grid1(nobj, 128);
         sx_launch(k_clean_count, g, 128, 0, st, O, nobj, nobj_dev, cellcnt, gx, gy);
@@ -988,11 +987,11 @@ int pipe_clean(sexgpu_ctx *ctx) {
                   Pm.clean_param, cellcnt, O.master, gx, gy);
         sx_launch(k_clean_chain, g, 128, 0, st, O, nobj, nobj_dev, vcnt, &d_sc->status, Pm.loop_cap);
         nl += exclusive_scan(vcnt, voff, nobj, nullptr, tmp, st, nobj_dev);
-        sx_launch(k_victim_scatter, g, 128, 0, st, O, nobj, nobj_dev, voff, vfill, vlist);
+        sx_launch(k_victim_scatter, grid1((long long)nobj * 32, 256), 256, 0, st, O, nobj, nobj_dev, voff, vfill,
+                  vlist, vals, A.alloc);
         sx_launch(k_victim_rank, g, 128, 0, st, O, nobj, nobj_dev, voff, vcnt, vlist, vsort);
         sx_launch(k_clean_merge, g, 128, 0, st, O, nobj, nobj_dev, voff, vcnt, vsort);
-        sx_launch(k_alloc_victims, grid1((long long)nobj * 32, 256), 256, 0, st, O, vals, A.alloc, nobj, nobj_dev);
-        nl += 8;
+        nl += 7;
     } else if (nobj > 0) {
         CK(cudaMemsetAsync(O.fmaster, 0xff, (size_t)nobj * 4, st));
     }
@@ -1054,26 +1053,25 @@ int pipe_end(sexgpu_ctx *ctx) {
     E.nnw = ctx->nnw_dev;
     E.seeing = Pm.seeing;
     E.pixscale = Pm.pixscale;
+    const size_t n1 = (size_t)nobj + 1, nr1 = (size_t)ps.nroots + 1;
+    const int nt = order_tiles(ps.nrootpix);
+    EN(order, (3 * nr1 + n1) * 4);
+    OrderBufs Q;
+    Q.tcnt = P<int>(ctx->zeros) + clean_zeros(w, h, nobj);
+    Q.thead = Q.tcnt + nt;
+    Q.next = P<int>(ctx->order);
+    Q.elem = Q.next + nr1;
+    Q.ns = Q.elem + nr1;
+    int *const pos = Q.ns + nr1;
+    Q.pos = pos;
+    E.surv = pos;
     int nl = 1;
     launch_endobject(E, nobj, st, nl);
     stage_mark(ctx, "endobject", nl);
 
     // ---- catalogue order
-    const size_t n1 = (size_t)nobj + 1, nr1 = (size_t)ps.nroots + 1;
-    const int nt = ps.nrootpix / NO_TILE + 1;
     EN(svals, n1 * 4);
-    EN(order, (2 * (size_t)nt + 3 * nr1 + n1) * 4);
-    OrderBufs Q;
-    Q.tcnt = P<int>(ctx->order);
-    Q.thead = Q.tcnt + nt;
-    Q.next = Q.thead + nt;
-    Q.elem = Q.next + nr1;
-    Q.ns = Q.elem + nr1;
-    int *const pos = Q.ns + nr1;
-    Q.pos = pos;
-    CK(cudaMemsetAsync(Q.tcnt, 0, 2 * (size_t)nt * 4, st));
-    sx_launch(k_surv_flags, grid1(nobj, 256), 256, 0, st, O, nobj, nobj_dev, pos);
-    nl = 3 + exclusive_scan(pos, pos, nobj, &d_sc->nsurv, tmp, st, nobj_dev);
+    nl = 2 + exclusive_scan(pos, pos, nobj, &d_sc->nsurv, tmp, st, nobj_dev);
     if (Pm.numbering == 0) {
         sx_launch(k_order_roots, grid1(ps.nroots, 128), 128, 0, st, O, R, P<int>(ctx->pos2idx), w, ps.nroots,
                   &d_sc->nroots, Q);
@@ -1451,7 +1449,7 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
                      &ctx->rsize, &ctx->roff, &ctx->rnkept, &ctx->robjbase,
                      &ctx->rdthr, &ctx->rathr, &ctx->rzero, &ctx->rlists, &ctx->rthr, &ctx->imgm, &ctx->wvar,
                      &ctx->wratio, &ctx->objkey, &ctx->rpix, &ctx->o_big, &ctx->o_geo, &ctx->o_apraw, &ctx->o_gobj,
-                     &ctx->o_iso, &ctx->o_sortkey, &ctx->amp, &ctx->alpha, &ctx->cellhead,
+                     &ctx->o_iso, &ctx->amp, &ctx->zeros,
                      &ctx->vict, &ctx->svals, &ctx->order, &ctx->oitems, &ctx->rows, &ctx->sc};
     for (DevBuf *b : all) free_buf(*b);
     free_buf(ctx->deb);
@@ -1693,7 +1691,7 @@ int sexgpu_background_rms(sexgpu_ctx *ctx, float *rms) {
     EN(rmsdnode, (size_t)h * Pm.nbx * 4);
     EN(rmsmap, (size_t)N * 4);
     launch_map_nodes(ps.B.sigma3, P<float>(ctx->rmsd), P<float>(ctx->rmsu), Pm.nbx, Pm.nby, Pm.bh, h,
-                     P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), P<float>(ctx->rmsu), st);
+                     P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), P<float>(ctx->rmsu), MedianArgs{}, st);
     sx_launch(k_rms_map, grid1(N, 256), 256, 0, st, P<float>(ctx->rmsnode), P<float>(ctx->rmsdnode), ps.B.colk,
               ps.B.coldx, Pm.nbx, w, N, P<float>(ctx->rmsmap), 0);
     CK(cudaMemcpyAsync(rms, ctx->rmsmap.p, (size_t)N * 4, cudaMemcpyDeviceToHost, st));
@@ -1787,9 +1785,8 @@ int sexgpu_background(sexgpu_ctx *ctx, float *img, int w, int h, const sexgpu_co
     CK(cudaMemcpyAsync(ctx->img.p, img, N * 4, cudaMemcpyHostToDevice, st));
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int nl = 0;
-    sx_launch(k_init_scalars, 1, 1, 0, st, d_sc);
     launch_background(B, P<float>(ctx->img), Pm, d_sc, st, nl);
-    launch_sub_filter(P<float>(ctx->img), P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), B, Pm, d_sc,
+    launch_sub_filter(P<float>(ctx->img), P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), nullptr, B, Pm, d_sc,
                       nullptr, ctx->cmask, st, nl);
     CK(cudaMemcpyAsync(img, ctx->sub.p, N * 4, cudaMemcpyDeviceToHost, st));
     if (back) CK(cudaMemcpyAsync(back, B.back3, nb * 4, cudaMemcpyDeviceToHost, st));
@@ -1836,7 +1833,7 @@ int sexgpu_filter(sexgpu_ctx *ctx, const float *sub, int w, int h, const float *
     int rc = load_tables(ctx, Pm, mask, mw, mh, B);
     if (rc) return rc;
     int nl = 0;
-    launch_sub_filter(P<float>(ctx->img), P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), B, Pm,
+    launch_sub_filter(P<float>(ctx->img), P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), nullptr, B, Pm,
                       P<FrameScalars>(ctx->sc), nullptr, ctx->cmask, st, nl);
     CK(cudaMemcpyAsync(cd, ctx->cd.p, N * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
