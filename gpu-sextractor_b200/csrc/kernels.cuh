@@ -94,10 +94,13 @@ struct DevCache {
 };
 
 // Kron boxes too large for one warp, summed by whole CTAs (k_post.cu)
-constexpr int KR_CHUNK = 8192;     // box pixels per CTA work item (whole rows, at least one)
-constexpr int KR_THREADS = 256;
-constexpr int KR_GRID = 2 * 148;
-constexpr int KR_WARP_MAX = 8192;  // default: larger boxes are queued
+constexpr int KR_CHUNK = 4096;     // box pixels per CTA work item (whole rows, at least one)
+// Larger boxes than this are queued, unless the caller has set a size: the fewer
+// objects there are, the sooner the longest box of a warp is what a pass waits
+// for.  Photometry of 3900 objects on 1024 x 1024 pixels: 0.086 ms at 1024, 0.105
+// at 2048, 0.19 at 8192; 19,500 (cluster): 0.37, 0.34, 0.34; 68,000: 1.40 (the
+// queue overflows), 0.62, 0.65; 780,000: 13.7, 11.4, 10.5 (10.46 at 6144).
+inline int kr_warp_max(int nobj) { return nobj <= 8192 ? 1024 : nobj <= 131072 ? 2048 : 6144; }
 // queued boxes and work items per pass: an eighth of the objects and 8 items
 // each, at least 8192 boxes (a crowded mosaic queues 2% of its objects; with
 // a fixed 8192 its warps were left with boxes of thousands of pixels)

@@ -170,7 +170,7 @@ struct sexgpu_ctx {
     DevBuf rmsd, rmsnode, rmsdnode, rmsu, rmsmap;  // background rms map (sexgpu_background_rms)
     DevBuf dnnw;                           // this context's copy of the CLASS_STAR network
     const sexgpu_nnw *nnw_dev = nullptr;   // network used (this context's or, for a batch worker, its owner's)
-    int kron_warp_max = KR_WARP_MAX;
+    int kron_warp_max = 0;  // 0: kr_warp_max of the object count
     int loop_cap = 0;  // "loop_cap" parameter: cap on device walks, for failure tests (0: built-in caps)
     int graph_mode = 0;                  // "graph" parameter: extract through captured graphs
     unsigned long long gen = 0;          // bumped by every device allocation (graphs hold pointers)
@@ -1011,9 +1011,6 @@ int pipe_end(sexgpu_ctx *ctx) {
     ObjBufs &O = ctx->O;
     FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
     int *tmp = P<int>(ctx->scan_tmp);
-    // an error so far empties the frame (the host reads the status at its end)
-    constexpr int NOCAP = 0x7fffffff;
-    sx_launch(k_gate, 1, 1, 0, st, d_sc, 0, NOCAP, NOCAP, NOCAP);
     const int *nobj_dev = &d_sc->nobj;
     // ---- photometry / FLAGS
     EndArgs E;
@@ -1049,7 +1046,7 @@ int pipe_end(sexgpu_ctx *ctx) {
     }
     E.K.icap = kr_items(nobj);
     E.K.ccap = kr_chunks(nobj);
-    E.K.warp_max = ctx->kron_warp_max;
+    E.K.warp_max = ctx->kron_warp_max > 0 ? ctx->kron_warp_max : kr_warp_max(nobj);
     E.nnw = ctx->nnw_dev;
     E.seeing = Pm.seeing;
     E.pixscale = Pm.pixscale;
@@ -1065,7 +1062,7 @@ int pipe_end(sexgpu_ctx *ctx) {
     int *const pos = Q.ns + nr1;
     Q.pos = pos;
     E.surv = pos;
-    int nl = 1;
+    int nl = 0;
     launch_endobject(E, nobj, st, nl);
     stage_mark(ctx, "endobject", nl);
 

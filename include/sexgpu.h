@@ -358,7 +358,7 @@ int sexgpu_stage_times(sexgpu_ctx *ctx, sexgpu_stage *stages, int max);
 /* Execution parameters of this context (and of its batch workers); results
  * do not depend on them.  "kron_warp_max": AUTO-photometry boxes of more
  * pixels than this are summed by whole thread blocks instead of one warp
- * (default 8192, >= 1).  "batch_grid_div": the persistent grids of
+ * (>= 1; default: 1024, 2048 or 6144, by the number of objects).  "batch_grid_div": the persistent grids of
  * sexgpu_extract_batch's workers use 1/n of the resident capacity each
  * (default 1).  "batch_sync": 1 (default) makes the batch workers wait for
  * their streams on blocking events, which leaves the host cores to the other
