@@ -314,9 +314,10 @@ def run_gpu(args):
                                   "dram__bytes_write.sum over the stage's launches, one frame)",
                 "algorithmic_bytes": algo,
                 "stage_ms": {s[0]: round(s[2], 4) for s in stages}}
-    # algorithmic bytes of a frame (24N pixel stages + 8 B per pixel and
-    # deblending level + 16 B per object pixel + 64 B per catalogue row)
-    frame_bytes = 24 * N + 8 * int(summ.level_pix) + 16 * int(summ.nraw_pix) + 64 * int(summ.nobj)
+    # algorithmic bytes of a frame (24N pixel stages + 16 B per raw-object pixel
+    # for the deblending and 16 B for the analysis and photometry + 64 B per
+    # catalogue row)
+    frame_bytes = 24 * N + 32 * int(summ.nraw_pix) + 64 * int(summ.nobj)
     line = {
         "metric": METRIC, "value": round(frames_dev, 3), "unit": "frames/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms_dev, 4),
@@ -484,16 +485,17 @@ def run_batch(ctx, frames, reps=5, workers=8, maxobj=400000):
 # DRAM bytes (read + write) per c1 frame of each stage's launches, from one
 # ncu launch-list capture of bench.py --profile-case c1 (its summary is kept
 # under profiles/)
-NCU_TRAFFIC = {"background": 134_700_000, "sub_filter": 207_900_000, "ccl": 168_700_000, "roots": 671_800_000,
-               "deblend": 715_500_000, "analyse": 406_900_000, "clean": 14_900_000, "endobject": 212_400_000,
-               "catalog": 24_000_000}
+NCU_TRAFFIC = {"background": 67_800_000, "sub_filter": 211_500_000, "ccl": 138_500_000, "roots": 349_300_000,
+               "deblend": 1_378_900_000, "analyse": 418_500_000, "clean": 17_000_000, "endobject": 392_400_000,
+               "catalog": 26_400_000}
 
 
 def algorithmic_bytes(stage, N, s):
     """Compulsory bytes of one launch set of a stage: the frame read by the
     background; frame in, subtracted and filtered frames and label seeds out
-    for sub_filter; labels read and written by the CCL; 8 bytes (pixel index
-    and filtered value) per pixel and deblending level."""
+    for sub_filter; labels read and written by the CCL; 16 bytes (pixel index,
+    raw object and filtered value in, owner out) per raw-object pixel for the
+    deblending, which does not visit a pixel once per level."""
     if stage == "background":
         return 4 * N                       # frame read once
     if stage == "sub_filter":
@@ -503,7 +505,7 @@ def algorithmic_bytes(stage, N, s):
     if stage == "roots":
         return 24 * N
     if stage == "deblend":
-        return 8 * int(s.level_pix)        # index + cd per pixel and level
+        return 16 * int(s.nraw_pix)
     return 4 * N
 
 
@@ -569,8 +571,8 @@ C4_WORKLOAD = ("c4: one 16384x16384 float32 frame with 2.5 M injected sources (c
 def stage_bytes(stage, N, s, weighted):
     """Compulsory bytes of a stage of one extraction: pixel stages from the
     frame size N, object stages from the counts the extraction reports
-    (raw-object pixels P, pixel-levels of the deblending, catalogue rows)."""
-    P, L, M = int(s.nraw_pix), int(s.level_pix), int(s.nobj)
+    (raw-object pixels P, catalogue rows M)."""
+    P, M = int(s.nraw_pix), int(s.nobj)
     if stage == "background":
         return 4 * N + (8 * N if weighted else 0)   # frame; weight map read + variance written
     if stage == "sub_filter":
@@ -579,9 +581,7 @@ def stage_bytes(stage, N, s, weighted):
         return 8 * N
     if stage == "roots":
         return 24 * N
-    if stage == "deblend":
-        return 8 * L
-    if stage in ("analyse", "endobject"):
+    if stage in ("deblend", "analyse", "endobject"):
         return 16 * P
     return 64 * M
 

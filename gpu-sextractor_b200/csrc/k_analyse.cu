@@ -18,7 +18,8 @@ constexpr int AN_WARPS = 8;
 // four resident CTAs per SM (at most 64 registers, a few spilled): these
 // kernels wait on pixel-list loads, and residency hides that better than
 // registers saved (analyse stage 1.37 ms at 4 CTAs/SM, 1.45 at 3 with fewer
-// spills, 1.65 at 2 with none; one 4096^2 frame)
+// spills, 1.65 at 2 with none, one crowded 4096^2 frame when its sums were
+// 128-bit; 0.54 ms at 4 now)
 constexpr int AN_MINB = 4;
 
 // fixed-order (butterfly) double sum; identical in every lane

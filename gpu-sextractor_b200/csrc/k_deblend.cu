@@ -41,10 +41,10 @@
 // entries a pixel, L1/L2 hits) and the latency of the join loop in 4.
 // Measured (deblend stage, plain form) against the level-by-level union-find
 // of one block or warp per raw object that stood here before: 4096 x 4096
-// crowded, 7.1 M pixels in 36,000 raw objects, 3.12 -> 1.45 ms; 1023 x 1021,
+// crowded, 7.1 M pixels in 36,000 raw objects, 3.12 -> 1.34 ms; 1023 x 1021,
 // 71,000 pixels in 1,400, where the largest object's levels were the time,
-// 0.99 -> 0.16 ms; a 4096 x 4096 cluster with one raw object of about 2 M
-// pixels, 64 levels, 791 -> 2.8 ms; 16384 x 16384, 108 M pixels, 38 -> 17 ms.
+// 0.99 -> 0.115 ms; a 4096 x 4096 cluster with one raw object of about 2 M
+// pixels, 64 levels, 791 -> 2.7 ms; 16384 x 16384, 108 M pixels, 38 -> 15.9 ms.
 #include <cooperative_groups.h>
 
 #include "common.cuh"

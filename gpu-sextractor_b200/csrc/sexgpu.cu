@@ -676,7 +676,7 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
         ps.wvar = P<float>(ctx->wvar);
         nl += 3;
     }
-    stage_mark(ctx, "background", nl + 1);
+    stage_mark(ctx, "background", nl);
     ps.stage = 1;
     return SEXGPU_OK;
 }
