@@ -491,3 +491,24 @@ def test_results_sized_by_count(gpu_ctx, w, h, nsrc):
     if len(g):
         with pytest.raises(RuntimeError):
             gpu_ctx.extract(img, max_objects=len(g) - 1)
+
+
+@pytest.mark.parametrize("w,h,bs", [(333, 140, 37), (520, 300, 256), (512, 130, 128), (260, 64, 64)])
+@pytest.mark.parametrize("wtype", [1, 3])
+@pytest.mark.parametrize("spread", [0.1, 9.0])
+def test_weight_scale_of_meshes(gpu_ctx, w, h, bs, wtype, spread):
+    """The mean relative variance of a mesh is its exact sum rounded once, for
+    rows that are and are not a multiple of 16 bytes, meshes of more pixels than
+    the double bins hold, variances over more binades than they span, and meshes
+    of mostly unusable pixels."""
+    rng = np.random.default_rng(w + bs + wtype)
+    img = rng.normal(300.0, 10.0, (h, w)).astype(np.float32)
+    wmap = np.exp(rng.normal(0.0, spread, (h, w))).clip(1e-6, 1e12).astype(np.float32)
+    bad = 1e30 if wtype == 1 else 0.0
+    wmap[rng.random((h, w)) < 0.1] = bad
+    wmap[: h // 3, : w // 2][rng.random((h // 3, w // 2)) < 0.6] = bad
+    kw = dict(back_size=bs, weight_type=wtype, filter_flag=0, detect_thresh=3.0, analysis_thresh=3.0)
+    _, gseg, gs = gpu_ctx.extract(img, weight=wmap, **kw)
+    _, oseg, os_ = O.extract(img, weight=wmap, **kw)
+    assert gs.sigfac == os_.sigfac and gs.npix_above == os_.npix_above
+    assert np.array_equal(gseg, oseg)
