@@ -175,6 +175,13 @@ struct __align__(16) GatherObj {
     float fx, fy;
     float cxx, cyy, cxy, abcor;
 };
+// ... and a bound: the distance of a pixel 16 or more away is above lam times the
+// square of its offset from (ix, iy) (lam 0: no bound)
+struct __align__(16) GatherBound {
+    int ix, iy;
+    float lam;
+    int pad;
+};
 struct DebArgs {
     const float *cd, *sub;
     const int *pos2idx;
@@ -185,6 +192,7 @@ struct DebArgs {
     ObjBufs O;
     MomentRaw *raw;             // per-object scratch of the preanalysis
     GatherObj *gobj;
+    GatherBound *gbound;
     FrameScalars *sc;
     int *alloc;                 // W*H object id map (-1 elsewhere)
     unsigned *objkey;           // object of every element (~0: not a branch's own pixel)

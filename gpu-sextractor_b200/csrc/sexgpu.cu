@@ -161,7 +161,7 @@ struct sexgpu_ctx {
     DevBuf kitem[2], kchunk[2], kpart[2];  // queued Kron boxes
     DevBuf o_sprob;                        // CLASS_STAR per object
     DevBuf o_big;                          // objects summed by whole blocks
-    DevBuf o_geo, o_apraw, o_gobj;         // Kron ellipses and boxes, aperture sums, gatherup's shapes
+    DevBuf o_geo, o_apraw, o_gobj, o_gbnd; // Kron ellipses and boxes, aperture sums, gatherup's shapes and bounds
     DevBuf o_raw, o_xraw, o_eraw;          // robust preanalysis / examineiso / photometry scratch per object
     DevBuf o_dbkg, o_lstat;                // BACKPHOTO_TYPE LOCAL: annulus mode, annulus statistics
     DevBuf o_aper, aperrows;               // every aperture per object; per catalogue row
@@ -878,6 +878,8 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     A.raw = P<MomentRaw>(ctx->o_raw);
     EN(o_gobj, (size_t)(nobj + 1) * sizeof(GatherObj));
     A.gobj = P<GatherObj>(ctx->o_gobj);
+    EN(o_gbnd, (size_t)(nobj + 1) * sizeof(GatherBound));
+    A.gbound = P<GatherBound>(ctx->o_gbnd);
     A.nobj = nobj;
     A.nobj_dev = ps.capf ? &d_sc->nobj : nullptr;
     // what CLEAN and the catalogue order count, zeroed here
@@ -1445,7 +1447,7 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
                      &ctx->dback, &ctx->bu, &ctx->rownode, &ctx->rowdnode, &ctx->rowu,
                      &ctx->rsize, &ctx->roff, &ctx->rnkept, &ctx->robjbase,
                      &ctx->rdthr, &ctx->rathr, &ctx->rzero, &ctx->rlists, &ctx->rthr, &ctx->imgm, &ctx->wvar,
-                     &ctx->wratio, &ctx->objkey, &ctx->rpix, &ctx->o_big, &ctx->o_geo, &ctx->o_apraw, &ctx->o_gobj,
+                     &ctx->wratio, &ctx->objkey, &ctx->rpix, &ctx->o_big, &ctx->o_geo, &ctx->o_apraw, &ctx->o_gobj, &ctx->o_gbnd,
                      &ctx->o_iso, &ctx->amp, &ctx->zeros,
                      &ctx->vict, &ctx->svals, &ctx->order, &ctx->oitems, &ctx->rows, &ctx->sc};
     for (DevBuf *b : all) free_buf(*b);
