@@ -181,7 +181,7 @@ void back_estimate(int back_size, float backfthresh, float *backmean, float *bac
     s.cfg.conv_w = s.cfg.conv_h = 0;
     sexgpu_ctx *ctx = s.ctx;
     int rc = pipe_begin(ctx, P<float>(ctx->img), nullptr, s.w, s.h, &s.cfg);
-    if (!rc) rc = read_scalars(ctx);
+    if (!rc) rc = read_scalars(ctx, ctx->bk);
     if (rc) {
         compat_fail("back_estimate", rc);
         return;
@@ -220,12 +220,12 @@ void run_detection(float dthresh, float thresh, int minarea, size_t *numValidObj
         Pm.filter_flag = 0;
         Pm.conv_w = Pm.conv_h = 1;
     }
-    int rc = load_tables(ctx, Pm, s.mask_w > 0 ? s.mask.data() : nullptr, s.mask_w, s.mask_w, ctx->ps.B);
+    int rc = load_tables(ctx, ctx->bk, Pm, s.mask_w > 0 ? s.mask.data() : nullptr, s.mask_w, s.mask_w, ctx->ps.B);
     if (rc) {
         compat_fail("run_detection", rc);
         return;
     }
-    sx_launch(k_compat_thresholds, 1, 1, 0, ctx->stream, P<FrameScalars>(ctx->sc), dthresh, thresh);
+    sx_launch(k_compat_thresholds, 1, 1, 0, ctx->stream, P<FrameScalars>(ctx->bk.sc), dthresh, thresh);
     rc = pipe_detect(ctx);
     if (rc) {
         compat_fail("run_detection", rc);

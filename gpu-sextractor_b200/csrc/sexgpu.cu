@@ -49,6 +49,12 @@ struct StageRec {
     int launches;
 };
 
+// device buffers of one background and its filter: mesh maps, splines, row
+// nodes, column tables and detection mask
+struct BackDev {
+    DevBuf ms, back, sigma, back2, back3, sigma3, dback, u, rownode, rowdnode, rowu, tabs, sc;
+};
+
 }  // namespace
 
 namespace {
@@ -146,8 +152,10 @@ struct sexgpu_ctx {
     cudaEvent_t qev[2] = {nullptr, nullptr};
     // scan / sort scratch
     DevBuf scan_tmp, keys, vals;  // scan scratch; raw object of every element; object pixel lists
-    // background
-    DevBuf ms, back, sigma, back2, back3, sigma3, dback, bu, rownode, rowdnode, rowu;
+    // the current extraction's background (its maps are read after it,
+    // sexgpu_background_map / _rms), and that of the calls that are no
+    // extraction (sexgpu_background, sexgpu_filter)
+    BackDev bk, call;
     // roots
     DevBuf rsize, roff, rnkept, robjbase, rdthr, rathr, rzero, rlists, rthr;
     // deblend scratch
@@ -182,7 +190,6 @@ struct sexgpu_ctx {
     FrameScalars *hsc_pin = nullptr;     // page-locked copy of the frame scalars
     int last_graph = 0;                  // the last extraction replayed a graph
     int last_kernels = 0;                // kernel launches of the last extraction
-    DevBuf sc;
     FrameScalars hsc;
     ObjBufs O;
     int last_w = 0, last_h = 0, last_nobj = 0, last_ns = 0;
@@ -203,7 +210,6 @@ struct sexgpu_ctx {
     size_t stage_bytes = 0;
     void *rows_host = nullptr;          // pinned staging of a batch worker's catalogue rows
     size_t rows_bytes = 0;
-    DevBuf tabs;                        // column tables and detection mask of the current extraction
     std::vector<char> tabs_h;
     std::vector<float> hmask;
     ConvMask cmask{nullptr, nullptr, 1, 1};
@@ -420,9 +426,9 @@ int pin_scalars(sexgpu_ctx *ctx) {
     return SEXGPU_ERR_NOMEM;
 }
 
-int read_scalars(sexgpu_ctx *ctx) {
+int read_scalars(sexgpu_ctx *ctx, const BackDev &d) {
     if (int rc = pin_scalars(ctx)) return rc;
-    CK(cudaMemcpyAsync(ctx->hsc_pin, ctx->sc.p, sizeof(FrameScalars), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->hsc_pin, d.sc.p, sizeof(FrameScalars), cudaMemcpyDeviceToHost, ctx->stream));
     CK(stream_wait(ctx, ctx->stream));
     ctx->hsc = *ctx->hsc_pin;
     if (ctx->hsc.status & SX_ST_LOAD) {
@@ -440,6 +446,31 @@ int read_scalars(sexgpu_ctx *ctx) {
     return SEXGPU_OK;
 }
 
+// the buffers of a background of Pm's frame
+int back_bufs(sexgpu_ctx *ctx, BackDev &d, const FrameParams &Pm, BackBufs &B) {
+    const size_t nb = (size_t)Pm.nbx * Pm.nby, nodes = (size_t)Pm.h * Pm.nbx * 4;
+    const struct {
+        DevBuf *b;
+        size_t bytes;
+    } need[] = {{&d.ms, nb * sizeof(MeshStat)}, {&d.back, nb * 4},     {&d.sigma, nb * 4},   {&d.back2, nb * 4},
+                {&d.back3, nb * 4},             {&d.sigma3, nb * 4},   {&d.dback, nb * 4},   {&d.u, nb * 4 + 64},
+                {&d.rownode, nodes},            {&d.rowdnode, nodes},  {&d.rowu, nodes},     {&d.sc, sizeof(FrameScalars)}};
+    for (const auto &n : need)
+        if (int rc = ensure(ctx, *n.b, n.bytes)) return rc;
+    B.ms = P<MeshStat>(d.ms);
+    B.back = P<float>(d.back);
+    B.sigma = P<float>(d.sigma);
+    B.back2 = P<float>(d.back2);
+    B.back3 = P<float>(d.back3);
+    B.sigma3 = P<float>(d.sigma3);
+    B.dback = P<float>(d.dback);
+    B.u = P<float>(d.u);
+    B.rownode = P<float>(d.rownode);
+    B.rowdnode = P<float>(d.rowdnode);
+    B.rowu = P<float>(d.rowu);
+    return SEXGPU_OK;
+}
+
 // The tables that a frame's kernels read, in one block: the segment index and
 // dx of every column, then the detection mask (w ints, w floats, the mask).
 void fill_tables(std::vector<char> &tabs, const FrameParams &Pm, const float *mask, size_t nmask) {
@@ -451,9 +482,9 @@ void fill_tables(std::vector<char> &tabs, const FrameParams &Pm, const float *ma
 
 size_t tables_bytes(int w) { return (size_t)8 * w + 4 * SX_MAXCONV * SX_MAXCONV; }
 
-// ... of this context's next extraction, by one upload; a frame that is being
-// captured reads the graph's device copy
-int load_tables(sexgpu_ctx *ctx, const FrameParams &Pm, const float *mask, int mw, int mh, BackBufs &B) {
+// ... of this context's next extraction or other call (d: its buffers), by one
+// upload; a frame that is being captured reads the graph's device copy
+int load_tables(sexgpu_ctx *ctx, BackDev &d, const FrameParams &Pm, const float *mask, int mw, int mh, BackBufs &B) {
     static const float one = 1.0f;
     if (!mask) {
         mask = &one;
@@ -462,8 +493,8 @@ int load_tables(sexgpu_ctx *ctx, const FrameParams &Pm, const float *mask, int m
     ctx->hmask.assign(mask, mask + (size_t)mw * mh);
     unsigned char *dev = ctx->ps.cst;
     if (!dev) {
-        EN(tabs, tables_bytes(Pm.w));
-        dev = P<unsigned char>(ctx->tabs);
+        if (int rc = ensure(ctx, d.tabs, tables_bytes(Pm.w))) return rc;
+        dev = P<unsigned char>(d.tabs);
         fill_tables(ctx->tabs_h, Pm, mask, ctx->hmask.size());
         CK(cudaMemcpyAsync(dev, ctx->tabs_h.data(), ctx->tabs_h.size(), cudaMemcpyHostToDevice, ctx->stream));
     }
@@ -612,34 +643,12 @@ int pipe_begin(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, int w, 
     EN(rpix, N * 4);
     EN(objkey, N * 4);
     EN(scan_tmp, (scan_temp_ints(N) + 64) * 4);
-    EN(ms, nb * sizeof(MeshStat));
-    EN(back, nb * 4);
-    EN(sigma, nb * 4);
-    EN(back2, nb * 4);
-    EN(back3, nb * 4);
-    EN(sigma3, nb * 4);
-    EN(dback, nb * 4);
-    EN(bu, (size_t)nb * 4 + 64);
-    EN(rownode, (size_t)h * Pm.nbx * 4);
-    EN(rowdnode, (size_t)h * Pm.nbx * 4);
-    EN(rowu, (size_t)h * Pm.nbx * 4);
-    EN(sc, sizeof(FrameScalars));
     BackBufs &B = ps.B;
-    B.ms = P<MeshStat>(ctx->ms);
-    B.back = P<float>(ctx->back);
-    B.sigma = P<float>(ctx->sigma);
-    B.back2 = P<float>(ctx->back2);
-    B.back3 = P<float>(ctx->back3);
-    B.sigma3 = P<float>(ctx->sigma3);
-    B.dback = P<float>(ctx->dback);
-    B.u = P<float>(ctx->bu);
-    B.rownode = P<float>(ctx->rownode);
-    B.rowdnode = P<float>(ctx->rowdnode);
-    B.rowu = P<float>(ctx->rowu);
-    FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
+    if ((rc = back_bufs(ctx, ctx->bk, Pm, B))) return rc;
+    FrameScalars *d_sc = P<FrameScalars>(ctx->bk.sc);
     int *tmp = P<int>(ctx->scan_tmp);
 
-    rc = load_tables(ctx, Pm, cfg->filter_flag ? cfg->conv : nullptr, cfg->conv_w, cfg->conv_h, B);
+    rc = load_tables(ctx, ctx->bk, Pm, cfg->filter_flag ? cfg->conv : nullptr, cfg->conv_w, cfg->conv_h, B);
     if (rc) return rc;
 
     stage_begin(ctx);
@@ -690,7 +699,7 @@ int pipe_detect(sexgpu_ctx *ctx) {
     const long long N = (long long)w * h;
     const float *d_img = ps.d_img;
     BackBufs &B = ps.B;
-    FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
+    FrameScalars *d_sc = P<FrameScalars>(ctx->bk.sc);
     int *tmp = P<int>(ctx->scan_tmp);
     int rc = SEXGPU_OK, nl = 0;
     int *lab = P<int>(ctx->lab), *cnt = P<int>(ctx->cnt), *flag = P<int>(ctx->flag), *pos = P<int>(ctx->pos);
@@ -718,7 +727,7 @@ int pipe_detect(sexgpu_ctx *ctx) {
         rlen = (int)(N / std::max(Pm.minarea, 1));
         sx_launch(k_gate, 1, 1, 0, st, d_sc, 1, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
     } else {
-        rc = read_scalars(ctx);
+        rc = read_scalars(ctx, ctx->bk);
         if (rc) return rc;
         if (ctx->hsc.dthresh <= 0.0f || ctx->hsc.thresh <= 0.0f) {
             ctx->err = "zero or negative threshold";
@@ -781,7 +790,7 @@ int pipe_deblend(sexgpu_ctx *ctx) {
     const FrameParams &Pm = ps.Pm;
     const int w = ps.w, h = ps.h, nroots = ps.nroots, nrootpix = ps.nrootpix;
     RootBufs &R = ps.R;
-    FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
+    FrameScalars *d_sc = P<FrameScalars>(ctx->bk.sc);
     int *tmp = P<int>(ctx->scan_tmp);
     unsigned *rpix = P<unsigned>(ctx->rpix);
     int rc = SEXGPU_OK;
@@ -864,7 +873,7 @@ int pipe_deblend(sexgpu_ctx *ctx) {
         nobj = ps.cap_obj;
         sx_launch(k_gate, 1, 1, 0, st, d_sc, 0, ps.cap_roots, ps.cap_rootpix, ps.cap_obj);
     } else {
-        rc = read_scalars(ctx);
+        rc = read_scalars(ctx, ctx->bk);
         if (rc) return rc;
         nobj = ctx->hsc.nobj;
     }
@@ -901,7 +910,7 @@ int pipe_analyse(sexgpu_ctx *ctx) {
     const int w = ps.w, h = ps.h, nobj = ps.nobj;
     const DebArgs &A = ps.A;
     const BackBufs &B = ps.B;
-    FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
+    FrameScalars *d_sc = P<FrameScalars>(ctx->bk.sc);
     int *tmp = P<int>(ctx->scan_tmp);
     unsigned *vals = P<unsigned>(ctx->vals);
     // ---- object pixel lists (raster order inside each object)
@@ -966,7 +975,7 @@ int pipe_clean(sexgpu_ctx *ctx) {
     const int w = ps.w, h = ps.h, nobj = ps.nobj;
     const DebArgs &A = ps.A;
     ObjBufs &O = ctx->O;
-    FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
+    FrameScalars *d_sc = P<FrameScalars>(ctx->bk.sc);
     int *tmp = P<int>(ctx->scan_tmp);
     unsigned *vals = P<unsigned>(ctx->vals);
     // ---- CLEAN
@@ -1011,7 +1020,7 @@ int pipe_end(sexgpu_ctx *ctx) {
     const DebArgs &A = ps.A;
     const RootBufs &R = ps.R;
     ObjBufs &O = ctx->O;
-    FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
+    FrameScalars *d_sc = P<FrameScalars>(ctx->bk.sc);
     int *tmp = P<int>(ctx->scan_tmp);
     const int *nobj_dev = &d_sc->nobj;
     // ---- photometry / FLAGS
@@ -1095,7 +1104,7 @@ int pipe_end(sexgpu_ctx *ctx) {
         ps.stage = 6;
         return SEXGPU_OK;
     }
-    const int rc = read_scalars(ctx);
+    const int rc = read_scalars(ctx, ctx->bk);
     if (rc) return rc;
     stage_collect(ctx);
     ctx->last_w = w;
@@ -1443,13 +1452,12 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     DevBuf *all[] = {&ctx->img, &ctx->sub, &ctx->cd, &ctx->lab, &ctx->cnt, &ctx->flag, &ctx->pos, &ctx->alloc,
-                     &ctx->seg, &ctx->pos2idx, &ctx->var, &ctx->scan_tmp, &ctx->keys, &ctx->vals, &ctx->ms, &ctx->back, &ctx->sigma, &ctx->back2, &ctx->back3, &ctx->sigma3,
-                     &ctx->dback, &ctx->bu, &ctx->rownode, &ctx->rowdnode, &ctx->rowu,
+                     &ctx->seg, &ctx->pos2idx, &ctx->var, &ctx->scan_tmp, &ctx->keys, &ctx->vals,
                      &ctx->rsize, &ctx->roff, &ctx->rnkept, &ctx->robjbase,
                      &ctx->rdthr, &ctx->rathr, &ctx->rzero, &ctx->rlists, &ctx->rthr, &ctx->imgm, &ctx->wvar,
                      &ctx->wratio, &ctx->objkey, &ctx->rpix, &ctx->o_big, &ctx->o_geo, &ctx->o_apraw, &ctx->o_gobj, &ctx->o_gbnd,
                      &ctx->o_iso, &ctx->amp, &ctx->zeros,
-                     &ctx->vict, &ctx->svals, &ctx->order, &ctx->oitems, &ctx->rows, &ctx->sc};
+                     &ctx->vict, &ctx->svals, &ctx->order, &ctx->oitems, &ctx->rows};
     for (DevBuf *b : all) free_buf(*b);
     free_buf(ctx->deb);
     for (auto &b : ctx->o_i) free_buf(b);
@@ -1475,7 +1483,10 @@ int sexgpu_destroy(sexgpu_ctx *ctx) {
     free_buf(ctx->rmsu);
     free_buf(ctx->rmsmap);
     free_buf(ctx->dnnw);
-    free_buf(ctx->tabs);
+    for (BackDev *d : {&ctx->bk, &ctx->call})
+        for (DevBuf *b : {&d->ms, &d->back, &d->sigma, &d->back2, &d->back3, &d->sigma3, &d->dback, &d->u, &d->rownode,
+                          &d->rowdnode, &d->rowu, &d->tabs, &d->sc})
+            free_buf(*b);
     for (cudaEvent_t e : ctx->stage_ev) cudaEventDestroy(e);
     if (ctx->ev_block) cudaEventDestroy(ctx->ev_block);
     free_batch_graph(ctx);
@@ -1732,7 +1743,7 @@ int sexgpu_background_map(sexgpu_ctx *ctx, float *back) {
     const FrameParams &Pm = ps.Pm;
     const long long N = (long long)Pm.w * Pm.h;
     EN(rmsmap, (size_t)N * 4);
-    sx_launch(k_back_map, grid1(N, 256), 256, 0, st, ps.B, Pm.nbx, Pm.back_type, P<FrameScalars>(ctx->sc), Pm.w, N,
+    sx_launch(k_back_map, grid1(N, 256), 256, 0, st, ps.B, Pm.nbx, Pm.back_type, P<FrameScalars>(ctx->bk.sc), Pm.w, N,
               P<float>(ctx->rmsmap));
     CK(cudaMemcpyAsync(back, ctx->rmsmap.p, (size_t)N * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1755,34 +1766,13 @@ int sexgpu_background(sexgpu_ctx *ctx, float *img, int w, int h, const sexgpu_co
     EN(sub, N * 4);
     EN(cd, N * 4);
     EN(lab, N * 4);
-    EN(ms, nb * sizeof(MeshStat));
-    EN(back, nb * 4);
-    EN(sigma, nb * 4);
-    EN(back2, nb * 4);
-    EN(back3, nb * 4);
-    EN(sigma3, nb * 4);
-    EN(dback, nb * 4);
-    EN(bu, (size_t)nb * 4 + 64);
-    EN(rownode, (size_t)h * Pm.nbx * 4);
-    EN(rowdnode, (size_t)h * Pm.nbx * 4);
-    EN(rowu, (size_t)h * Pm.nbx * 4);
-    EN(sc, sizeof(FrameScalars));
+    // (in buffers of its own: the maps of the last extraction stay as they are)
     BackBufs B;
-    B.ms = P<MeshStat>(ctx->ms);
-    B.back = P<float>(ctx->back);
-    B.sigma = P<float>(ctx->sigma);
-    B.back2 = P<float>(ctx->back2);
-    B.back3 = P<float>(ctx->back3);
-    B.sigma3 = P<float>(ctx->sigma3);
-    B.dback = P<float>(ctx->dback);
-    B.u = P<float>(ctx->bu);
-    B.rownode = P<float>(ctx->rownode);
-    B.rowdnode = P<float>(ctx->rowdnode);
-    B.rowu = P<float>(ctx->rowu);
-    rc = load_tables(ctx, Pm, nullptr, 1, 1, B);
+    if ((rc = back_bufs(ctx, ctx->call, Pm, B))) return rc;
+    rc = load_tables(ctx, ctx->call, Pm, nullptr, 1, 1, B);
     if (rc) return rc;
     CK(cudaMemcpyAsync(ctx->img.p, img, N * 4, cudaMemcpyHostToDevice, st));
-    FrameScalars *d_sc = P<FrameScalars>(ctx->sc);
+    FrameScalars *d_sc = P<FrameScalars>(ctx->call.sc);
     int nl = 0;
     launch_background(B, P<float>(ctx->img), Pm, d_sc, st, nl);
     launch_sub_filter(P<float>(ctx->img), P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), nullptr, B, Pm, d_sc,
@@ -1790,7 +1780,7 @@ int sexgpu_background(sexgpu_ctx *ctx, float *img, int w, int h, const sexgpu_co
     CK(cudaMemcpyAsync(img, ctx->sub.p, N * 4, cudaMemcpyDeviceToHost, st));
     if (back) CK(cudaMemcpyAsync(back, B.back3, nb * 4, cudaMemcpyDeviceToHost, st));
     if (sigma) CK(cudaMemcpyAsync(sigma, B.sigma3, nb * 4, cudaMemcpyDeviceToHost, st));
-    rc = read_scalars(ctx);
+    rc = read_scalars(ctx, ctx->call);
     if (rc) return rc;
     if (sum) {
         ctx->last_nobj = ctx->last_ns = 0;
@@ -1809,17 +1799,17 @@ int sexgpu_filter(sexgpu_ctx *ctx, const float *sub, int w, int h, const float *
     EN(sub, N * 4);
     EN(cd, N * 4);
     EN(lab, N * 4);
-    EN(sc, sizeof(FrameScalars));
-    EN(rownode, 16);
+    EN(call.sc, sizeof(FrameScalars));
+    EN(call.rownode, 16);
     CK(cudaMemcpyAsync(ctx->img.p, sub, N * 4, cudaMemcpyHostToDevice, st));
     FrameScalars z;
     memset(&z, 0, sizeof(z));
     z.backmean = 0.0f;
     z.dthresh = 1e30f;
-    CK(cudaMemcpyAsync(ctx->sc.p, &z, sizeof(z), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(ctx->call.sc.p, &z, sizeof(z), cudaMemcpyHostToDevice, st));
     BackBufs B;
     memset(&B, 0, sizeof(B));
-    B.rownode = P<float>(ctx->rownode);
+    B.rownode = P<float>(ctx->call.rownode);
     FrameParams Pm;
     memset(&Pm, 0, sizeof(Pm));
     Pm.w = w;
@@ -1829,11 +1819,11 @@ int sexgpu_filter(sexgpu_ctx *ctx, const float *sub, int w, int h, const float *
     Pm.filter_flag = 1;
     Pm.conv_w = mw;
     Pm.conv_h = mh;
-    int rc = load_tables(ctx, Pm, mask, mw, mh, B);
+    int rc = load_tables(ctx, ctx->call, Pm, mask, mw, mh, B);
     if (rc) return rc;
     int nl = 0;
     launch_sub_filter(P<float>(ctx->img), P<float>(ctx->sub), P<float>(ctx->cd), P<int>(ctx->lab), nullptr, B, Pm,
-                      P<FrameScalars>(ctx->sc), nullptr, ctx->cmask, st, nl);
+                      P<FrameScalars>(ctx->call.sc), nullptr, ctx->cmask, st, nl);
     CK(cudaMemcpyAsync(cd, ctx->cd.p, N * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     CK(cudaGetLastError());
@@ -2116,7 +2106,7 @@ static void build_batch_graph(sexgpu_ctx *ctx, const sexgpu_batch_frame *frames,
                                                 wc->rows.p, ((size_t)b->cap[i] + 1) * S,
                                                 cudaMemcpyDeviceToDevice) == cudaSuccess;
             ok = ok && cudaGraphAddMemcpyNode1D(&sc, g, &child, 1, (char *)b->sc_dev + (size_t)i * sizeof(FrameScalars),
-                                                wc->sc.p, sizeof(FrameScalars), cudaMemcpyDeviceToDevice) ==
+                                                wc->bk.sc.p, sizeof(FrameScalars), cudaMemcpyDeviceToDevice) ==
                            cudaSuccess;
             cudaGraphNode_t two[2] = {r, sc};
             ok = ok && cudaGraphAddEmptyNode(&join, g, two, 2) == cudaSuccess;

@@ -177,7 +177,9 @@ int sexgpu_extract_device(sexgpu_ctx *ctx, const float *d_img, const float *d_va
                           const sexgpu_config *cfg, sexgpu_summary *sum);
 
 /* Copy the results of the last extraction to host memory (any pointer may
- * be NULL). */
+ * be NULL).  sub and cd are to be copied before sexgpu_background or
+ * sexgpu_filter is called on the context, which use the same frame buffers;
+ * the background maps below stay those of the extraction. */
 int sexgpu_copy_results(sexgpu_ctx *ctx, sexgpu_object *objs, int max_objects, int *nobj,
                         int32_t *segmap, float *sub, float *cd);
 
