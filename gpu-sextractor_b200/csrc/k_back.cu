@@ -994,14 +994,17 @@ __device__ unsigned select_kth(const float *v, int n, int k, unsigned lowkey, un
     for (int shift = 24; shift >= 0; shift -= 8) {
         for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
         __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            unsigned key = f2ord(v[i]);
-            if (key < lowkey) continue;
-            if ((key & mask) == prefix) {
-                // (mesh values are close together: most of a warp on one bin)
-                const unsigned d = (key >> shift) & 255, same = __match_any_sync(__activemask(), d);
-                if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&hist[d], (unsigned)__popc(same));
+        // (mesh values are close together: most of a warp on one bin, which it
+        // counts once; whole warps, 256 for a lane without a value)
+        for (int i0 = 0; i0 < n; i0 += blockDim.x) {
+            const int i = i0 + threadIdx.x;
+            unsigned d = 256u;
+            if (i < n) {
+                const unsigned key = f2ord(v[i]);
+                if (key >= lowkey && (key & mask) == prefix) d = (key >> shift) & 255u;
             }
+            const unsigned same = __match_any_sync(0xffffffffu, d);
+            if (d < 256u && (int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&hist[d], (unsigned)__popc(same));
         }
         __syncthreads();
         __shared__ unsigned s_digit, s_k;
@@ -1272,21 +1275,25 @@ __global__ void __launch_bounds__(SPL_THREADS) k_row_nodes(const float *__restri
     }
     if (nby <= 1) return;
     __syncthreads();
-    if (threadIdx.x < rows) {
+    const bool walks = threadIdx.x < rows;
+    float *u = su + threadIdx.x * pitch;
+    if (walks) {
         const float *n = spl + threadIdx.x * pitch;
-        float *u = su + threadIdx.x * pitch;
         float temp, dprev = 0.0f, uprev = 0.0f;
-        // (every row's d is the same: written alike by all)
+        // (every row's d is the same: the first row's is kept)
 #pragma unroll 4
         for (int x = 1; x < nbx - 1; x++) {
             temp = -1 / (dprev + 4);
-            sd[x] = dprev = temp;
+            dprev = temp;
+            if (threadIdx.x == 0) sd[x] = temp;
             temp *= uprev - 6 * (n[x + 1] + n[x - 1] - 2 * n[x]);
             u[x] = uprev = temp;
         }
         u[0] = u[nbx - 1] = 0.0;
+    }
+    __syncthreads();
+    if (walks) {
         float dnext = 0.0f;
-        __syncwarp(__activemask());
 #pragma unroll 4
         for (int x = nbx - 2; x >= 1; x--) u[x] = dnext = (sd[x] * dnext + u[x]) / 6.0f;
     }

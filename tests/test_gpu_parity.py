@@ -512,3 +512,20 @@ def test_weight_scale_of_meshes(gpu_ctx, w, h, bs, wtype, spread):
     _, oseg, os_ = O.extract(img, weight=wmap, **kw)
     assert gs.sigfac == os_.sigfac and gs.npix_above == os_.npix_above
     assert np.array_equal(gseg, oseg)
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (2, 1), (31, 1), (1, 33), (32, 32), (41, 25), (255, 3), (64, 64), (241, 17)])
+@pytest.mark.parametrize("flat", [0.0, 0.3, 0.7])
+def test_medians_of_mesh_maps(gpu_ctx, nx, ny, flat):
+    """Medians over mesh counts on either side of whole warps and blocks and of
+    the count up to which they are taken beside the row nodes, with meshes of no
+    scatter (of which more than half send the rms to the positive ones), and
+    rows of nodes of any length: bit for bit."""
+    rng = np.random.default_rng(1000 * nx + ny)
+    img = rng.normal(500.0, 10.0, (8 * ny, 8 * nx)).astype(np.float32)
+    for k in np.flatnonzero(rng.random(nx * ny) < flat):
+        y, x = 8 * (k // nx), 8 * (k % nx)
+        img[y:y + 8, x:x + 8] = rng.integers(480, 520)
+    got, want = gpu_ctx.background(img, back_size=8, back_filtersize=1), O.background(img, back_size=8, back_filtersize=1)
+    assert all(np.array_equal(a, b) for a, b in zip(got[:3], want[:3]))
+    assert (got[3].backmean, got[3].backsig) == (want[3].backmean, want[3].backsig)
