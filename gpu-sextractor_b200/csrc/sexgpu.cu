@@ -2491,7 +2491,11 @@ int sexgpu_autotune(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, in
     };
     int rc = SEXGPU_OK;
     float best_ms = 3.0e38f, ms = 0.f;
-    int best_graph = ctx->graph_mode, best_kron = ctx->kron_warp_max;
+    int best_graph = ctx->graph_mode, best_kron = 0;
+    const int kron_before = ctx->kron_warp_max;
+    // ("graph" is timed with box sizes by the number of objects, the default,
+    // so the faster of the two is that rule's time)
+    ctx->kron_warp_max = 0;
     for (int g = 0; g <= 1 && !rc; g++) {
         rc = trial("graph", g, ms);
         if (!rc && ms < best_ms) {
@@ -2500,7 +2504,6 @@ int sexgpu_autotune(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, in
         }
     }
     if (!rc) rc = sexgpu_set_param(ctx, "graph", best_graph);
-    best_ms = 3.0e38f;
     for (int v = 1024; v <= 32768 && !rc; v *= 2) {
         rc = trial("kron_warp_max", v, ms);
         if (!rc && ms < best_ms) {
@@ -2508,7 +2511,10 @@ int sexgpu_autotune(sexgpu_ctx *ctx, const float *d_img, const float *d_wmap, in
             best_kron = v;
         }
     }
-    if (!rc) rc = sexgpu_set_param(ctx, "kron_warp_max", best_kron);
+    // a size of its own only where it beats the rule (it is also what frames of
+    // other object counts will get), and not the size that the rule gives here
+    if (best_kron == kr_warp_max(ctx->last_nobj)) best_kron = 0;
+    ctx->kron_warp_max = rc ? kron_before : best_kron;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc) return rc;

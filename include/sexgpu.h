@@ -319,7 +319,10 @@ typedef struct {
  * faster, "kron_warp_max" 1024, 2048, ..., 32768: each candidate after its
  * warm-up runs (a graph learns and captures), best of reps runs timed with
  * CUDA events on the context's stream.  The fastest value of each parameter
- * stays set on the context.  Every candidate's catalogue rows are compared
+ * stays set on the context; "graph" is timed with the default of
+ * "kron_warp_max", sizes by the number of objects, and a single size is set
+ * only where it is faster than that and not the size it gives for this frame
+ * (otherwise the default is set again).  Every candidate's catalogue rows are compared
  * with the first candidate's, byte for byte: SEXGPU_ERR_MISMATCH if they
  * differ.  Up to max_entries candidates go to entries (may be NULL); returns
  * the number of candidates timed, or an error code. */
