@@ -66,3 +66,32 @@ def test_exact_sum_out_of_range_reported(gpu_ctx, masks):
         gpu_ctx.extract(img, filter_flag=0, back_type=1, back_value=0.0, thresh_type=1, detect_thresh=1e-30,
                         analysis_thresh=1e-30)
     _check_recovers(gpu_ctx, masks, 75)
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("first", ["frame", "error", "background"])
+def test_first_frames_of_a_context(masks, first, graph):
+    """A context's first reads of the frame scalars go to pageable memory, later
+    ones to a page of its own: counts, thresholds and errors are the same over
+    its first frames, whichever call comes first."""
+    import sexgpu
+    img = synth.frame_c0(seed=76, w=200, h=150, nsrc=60)
+    kw = dict(conv=masks["default"])
+    o, oseg, os_ = O.extract(img, **kw)
+    with sexgpu.Context(0) as ctx:
+        ctx.set_param("graph", graph)
+        if first == "error":
+            with pytest.raises(RuntimeError, match="zero or negative threshold"):
+                ctx.extract(img, thresh_type=1, detect_thresh=0.0, analysis_thresh=0.0, **kw)
+        elif first == "background":
+            for _ in range(5):
+                got, want = ctx.background(img), O.background(img)
+                assert np.array_equal(got[0], want[0]) and got[3].backsig == want[3].backsig
+        for _ in range(4):
+            g, gseg, gs = ctx.extract(img, **kw)
+            assert np.array_equal(gseg, oseg)
+            compare_catalogs(g, o)
+            assert (gs.backmean, gs.dthresh, gs.nobj, gs.nraw, gs.npix_above) == \
+                (os_.backmean, os_.dthresh, os_.nobj, os_.nraw, os_.npix_above)
+        with pytest.raises(RuntimeError, match="zero or negative threshold"):
+            ctx.extract(img, thresh_type=1, detect_thresh=0.0, analysis_thresh=0.0, **kw)
