@@ -95,3 +95,64 @@ def test_first_frames_of_a_context(masks, first, graph):
                 (os_.backmean, os_.dthresh, os_.nobj, os_.nraw, os_.npix_above)
         with pytest.raises(RuntimeError, match="zero or negative threshold"):
             ctx.extract(img, thresh_type=1, detect_thresh=0.0, analysis_thresh=0.0, **kw)
+
+
+def _tile_frame(kind):
+    """Objects each inside one 64 x 32 tile of the labelling (every label is one
+    step from its root) and far apart (nothing to CLEAN).  single: cones, one
+    peak each; ramps: pairs of peaks at the ends of long slopes, so that pixels
+    are many steps from their peak; steps: rows of peaks, each higher than the
+    one before and joined to it at a lower level, all other pixels next to a
+    peak, so that only the walks over the joins are long."""
+    img = np.zeros((96, 192), np.float32)
+    for t in range(9):
+        y, x = 16 + 32 * (t // 3), 64 * (t % 3) + 8
+        if kind == "single":
+            dy, dx = np.mgrid[-8:9, -8:9]
+            img[y - 8:y + 9, x + 12:x + 29] = 400.0 * np.exp(-0.02 * (dx * dx + dy * dy) - 0.001 * dx - 0.002 * dy) + t
+        elif kind == "ramps":
+            slope = 10.0 + 20.0 * np.abs(np.arange(41) - 20.0 - 0.25 * t)
+            img[y, x:x + 41] = slope
+            img[y + 1, x:x + 41] = 0.5 * slope
+        else:
+            img[y - 1:y + 2, x - 1:x + 24] = 6.0 + 0.01 * np.arange(25)
+            for k in range(8):
+                img[y, x + 3 * k] = 100.0 * 2.0 ** k
+                if k < 7:
+                    img[y, x + 3 * k + 1:x + 3 * k + 3] = 90.0 * 0.7 ** k
+    return img
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("cap", [1, 2])
+@pytest.mark.parametrize("kind", ["ramps", "steps"])
+def test_loop_cap_of_the_deblending(kind, cap, graph):
+    """Only the deblending's walks run out: frames of single peaks pass under the
+    cap, frames of joined peaks end with the error, in the plain form and in a
+    replayed graph whose later stages run on zeroed counts, and the context
+    then extracts either as the oracle does."""
+    import sexgpu
+    kw = dict(filter_flag=0, back_type=1, back_value=0.0, thresh_type=1, detect_thresh=5.0, analysis_thresh=5.0,
+              deblend_nthresh=64, deblend_mincont=0.0)
+    single, joined = _tile_frame("single"), _tile_frame(kind)
+
+    def check(img):
+        g, gseg, _ = ctx.extract(img, **kw)
+        o, oseg, _ = O.extract(img, **kw)
+        assert np.array_equal(gseg, oseg) and len(g) >= 9
+        compare_catalogs(g, o)
+
+    with sexgpu.Context(0) as ctx:
+        ctx.set_param("graph", graph)
+        ctx.set_param("loop_cap", cap)
+        for turn in range(2):
+            for _ in range(3):
+                check(single)
+            assert ctx.graph_stats()[0] == graph
+            with pytest.raises(RuntimeError, match="device loop cap reached"):
+                ctx.extract(joined, **kw)
+        check(single)
+        ctx.set_param("loop_cap", 0)
+        for _ in range(3):
+            check(joined)
+        check(single)
