@@ -243,9 +243,6 @@ __device__ __forceinline__ XSum xs_warp_sum(XSum s) {
     return r;
 }
 
-// the same, for callers that read the result in lane 0 only
-__device__ __forceinline__ XSum xs_warp_reduce(XSum s) { return xs_warp_sum(s); }
-
 // ---------------------------------------------------------------------------
 // Exact sums of float terms, binned form: two double bins of W binary orders
 // each, the upper one ending at the order `top` (a hint, for instance the order
@@ -320,59 +317,6 @@ __device__ __forceinline__ void xs_add_double(XSum &s, double d) {
 __device__ __forceinline__ void xs_add_bins(XSum &s, double b0, double b1) {
     xs_add_double(s, b1);
     xs_add_double(s, b0);
-}
-
-// ---------------------------------------------------------------------------
-// Fixed-scale exact accumulators usable with atomics: value =
-// sum_k (int64)w[k] * 2^(32k) in units of 2^(e0-23).  A float term of
-// exponent e >= e0 is split into 32-bit limbs; each limb word stays exact for
-// up to 2^31 terms.
-// ---------------------------------------------------------------------------
-struct Limbs4 {
-    unsigned long long w[4];
-};
-
-__device__ __forceinline__ void limbs_term(float f, int e0, unsigned int lim[4], bool &neg, int &bad) {
-    unsigned int u = __float_as_uint(f);
-    int ef = (int)((u >> 23) & 0xff);
-    lim[0] = lim[1] = lim[2] = lim[3] = 0;
-    neg = (u >> 31) != 0;
-    if (ef == 0) return;
-    int sh = ef - 127 - e0;
-    if (sh < 0 || sh > 100) {
-        bad = 1;
-        return;
-    }
-    unsigned __int128 t = ((unsigned __int128)((u & 0x7fffffu) | 0x800000u)) << sh;
-    lim[0] = (unsigned int)t;
-    lim[1] = (unsigned int)(t >> 32);
-    lim[2] = (unsigned int)(t >> 64);
-    lim[3] = (unsigned int)(t >> 96);
-}
-
-__device__ __forceinline__ void limbs_atomic_add_term(unsigned long long *acc, float f, int e0, int *status) {
-    unsigned int lim[4];
-    bool neg;
-    int bad = 0;
-    limbs_term(f, e0, lim, neg, bad);
-    if (bad) {
-        atomicOr(status, SX_ST_RANGE);
-        return;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-        if (lim[k]) atomicAdd(acc + k, neg ? (unsigned long long)(-(long long)lim[k]) : (unsigned long long)lim[k]);
-}
-
-__device__ __forceinline__ XSum limbs_to_xsum(const unsigned long long *w, int e0) {
-    XSum s;
-    __int128 v = 0;
-#pragma unroll
-    for (int k = 3; k >= 0; k--) v = (v << 32) + (__int128)(long long)w[k];
-    s.v = v;
-    s.e = e0;
-    s.ovf = 0;
-    return s;
 }
 
 // orderable integer image of a float (monotone for all finite floats)

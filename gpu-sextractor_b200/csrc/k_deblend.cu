@@ -54,7 +54,11 @@
 namespace sx {
 
 constexpr int DT_THREADS = 256;
-constexpr int DT_LIMBS = 5;         // flux limbs of DT_RADIX bits: 24-bit mantissas shifted by up to 100
+// Fluxes of buckets: sum_k acc[k] * 2^(DT_RADIX k) in units of 2^(e0cd - 23),
+// exact under atomics in any order.  A value of exponent e >= e0cd is a 24-bit
+// mantissa shifted by e - e0cd <= 100 bits (more sets SX_ST_RANGE), so it falls
+// into two neighbouring limbs; the 64-bit words hold the limbs of any frame.
+constexpr int DT_LIMBS = 5;
 constexpr int DT_RADIX = 27;        // 32 lanes' limbs add up in 32 bits
 constexpr unsigned DT_LIMB_MASK = (1u << DT_RADIX) - 1u;
 

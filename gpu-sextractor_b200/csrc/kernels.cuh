@@ -143,7 +143,6 @@ struct ObjBufs {
     float *sprob;                       // CLASS_STAR
     float *dbkg;                        // LOCAL photometry background per object, or null (GLOBAL)
     MeshStat *lstat;                    // LOCAL annulus statistics
-    unsigned long long *sortkey;
     float4 *aper;                       // every aperture: (flux, error, mag, mag error), naper per object
 };
 

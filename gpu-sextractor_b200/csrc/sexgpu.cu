@@ -140,7 +140,6 @@ struct sexgpu_ctx {
     PipeState ps;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
-    std::vector<DevBuf *> bufs;
     std::string err;
     // frame-size buffers
     DevBuf img, sub, cd, lab, cnt, flag, pos, alloc, seg, pos2idx, var, imgm, wvar, wratio;
@@ -151,7 +150,6 @@ struct sexgpu_ctx {
     int qhead = 0, qcount = 0;
     cudaStream_t qstream = nullptr;
     cudaEvent_t qev[2] = {nullptr, nullptr};
-    // scan / sort scratch
     DevBuf scan_tmp, keys, vals;  // scan scratch; raw object of every element; object pixel lists
     // the current extraction's background (its maps are read after it,
     // sexgpu_background_map / _rms), and that of the calls that are no
