@@ -42,8 +42,9 @@ constexpr int EX_TOP = 4;        // largest filtered values a lane keeps
 constexpr int EX_TOP_AREA = 16;  // DETECT_MINAREA up to which they are tried first
 
 // k-th smallest (0-based) of the cd values of n pixels, as float bits; the
-// values are positive (object pixels lie above the detection threshold), so
-// their bit patterns sort like the values.  Four 8-bit radix passes; in each
+// values are 0 or positive (object pixels lie at or above the detection
+// threshold, which is 0 where the variance is; the filter's sums begin with +0),
+// so their bit patterns sort like the values.  Four 8-bit radix passes; in each
 // pass the digit that holds rank k is found by a warp scan over 256 bins
 // (lane l owns bins 8l..8l+7).
 __device__ unsigned warp_select(const unsigned *opix, int n, const float *cd, int k, unsigned *hist) {
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A
     const float dthresh = A.O.dthr[o], thresh = A.O.athr[o], gthresh = A.sc->thresh, backsig = A.sc->backsig;
     const double mxo = A.O.mx[o], myo = A.O.my[o];
     double dbacknoise2 = backsig * backsig;
-    unsigned pk = 0u, bc = 0u, bp = 0u;
+    unsigned pk = 0u, bc = 0u, bp = 0xffffffffu;
     int area = 0;
     // flux and variance in double bins (hints: the object's peak, the frame's
     // noise), else with XSum
@@ -294,10 +295,10 @@ __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A
             int iy = (int)fdiv(p, A.wdiv), ix = (int)p - iy * w;
             pk = max(pk, f2ord(pv));
             // first maximum of cd in raster order: max cd, then smallest index
-            // (a lane's pixels come in that order); cd is positive, so its bits
-            // sort like its values
+            // (a lane's pixels come in that order); cd is 0 or positive, so its
+            // bits sort like its values (a lane's first pixel counts even at 0)
             unsigned key = __float_as_uint(cdpix);
-            if (key > bc) {
+            if (key > bc || bp == 0xffffffffu) {
                 bc = key;
                 bp = p;
             }

@@ -529,3 +529,22 @@ def test_medians_of_mesh_maps(gpu_ctx, nx, ny, flat):
     got, want = gpu_ctx.background(img, back_size=8, back_filtersize=1), O.background(img, back_size=8, back_filtersize=1)
     assert all(np.array_equal(a, b) for a, b in zip(got[:3], want[:3]))
     assert (got[3].backmean, got[3].backsig) == (want[3].backmean, want[3].backsig)
+
+
+@pytest.mark.parametrize("w,h", [(5, 37), (36, 13), (103, 81), (322, 171)])
+@pytest.mark.parametrize("weight_type", [1, 2, 4])
+@pytest.mark.parametrize("minarea", [1, 5, 30])
+def test_objects_of_zero_variance(gpu_ctx, masks, w, h, weight_type, minarea):
+    """Where the variance is 0 the threshold is, and objects may have filtered
+    values of 0 only: their peak is their first pixel all the same."""
+    rng = np.random.default_rng(w + minarea)
+    img = np.full((h, w), 137.0, np.float32)
+    img[rng.random((h, w)) < 0.02] = -1e30
+    kw = dict(back_size=64, conv=masks["default"], detect_thresh=1.5, analysis_thresh=1.5, detect_minarea=minarea,
+              deblend_nthresh=8, weight_type=weight_type)
+    if weight_type != 4:
+        kw["weight"] = np.where(rng.random((h, w)) < 0.3, 0.0, 25.0).astype(np.float32)
+    g, gseg, gs = gpu_ctx.extract(img, **kw)
+    o, oseg, os_ = O.extract(img, **kw)
+    assert np.array_equal(gseg, oseg) and gs.nraw == os_.nraw
+    compare_catalogs(g, o)
