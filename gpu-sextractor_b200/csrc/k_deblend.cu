@@ -421,14 +421,31 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_fill(const __grid_constant__ 
 }
 
 // ---- 4. the cut
+// a flux from its limbs, rounded once to double and then to float as every
+// exact sum is.  It may have up to 155 bits (values 100 binary orders above the
+// threshold, as blank pixels give under a mask with negative taps): above 127
+// the two lowest limbs only count as "not zero", far below the last bit kept.
 template <class T>
 __device__ __forceinline__ float dt_flux(const T *a, int e0) {
-    XSum s;
-    __int128 v = 0;
+    unsigned l[DT_LIMBS];
+    unsigned long long c = 0ull;
 #pragma unroll
-    for (int k = DT_LIMBS - 1; k >= 0; k--) v = (v << DT_RADIX) + (__int128)(unsigned long long)a[k];
+    for (int k = 0; k < DT_LIMBS; k++) {
+        c += a[k];
+        l[k] = (unsigned)c & DT_LIMB_MASK;
+        c >>= DT_RADIX;
+    }
+    const bool wide = c != 0ull || (l[DT_LIMBS - 1] >> (126 - DT_RADIX * (DT_LIMBS - 1))) != 0u;
+    XSum s;
+    __int128 v = wide ? (__int128)c : 0;
+#pragma unroll
+    for (int k = DT_LIMBS - 1; k >= 2; k--) v = (v << DT_RADIX) + l[k];
+    if (wide)
+        v |= (l[0] | l[1]) != 0u;
+    else
+        v = (((v << DT_RADIX) + l[1]) << DT_RADIX) + l[0];
     s.v = v;
-    s.e = e0;
+    s.e = e0 + (wide ? 2 * DT_RADIX : 0);
     s.ovf = 0;
     return xs_float(s);
 }

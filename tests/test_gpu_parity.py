@@ -548,3 +548,18 @@ def test_objects_of_zero_variance(gpu_ctx, masks, w, h, weight_type, minarea):
     o, oseg, os_ = O.extract(img, **kw)
     assert np.array_equal(gseg, oseg) and gs.nraw == os_.nraw
     compare_catalogs(g, o)
+
+
+@pytest.mark.parametrize("w,h,mask", [(97, 244, "mexhat_4.0_9x9"), (322, 515, "mexhat_5.0_11x11"),
+                                      (720, 198, "mexhat_5.0_11x11")])
+@pytest.mark.parametrize("nthresh,mincont", [(2, 0.1), (8, 0.005), (32, 0.005), (64, 0.0001), (32, 1.0)])
+def test_deblending_far_above_the_threshold(gpu_ctx, masks, w, h, mask, nthresh, mincont):
+    """Under a mask with negative taps blank pixels (-1e30) leave filtered values
+    90 binary orders above the threshold; thousands of them add up to branch
+    fluxes of more than 127 bits in units of the threshold's last bit, which the
+    MINCONT cut has to get right all the same."""
+    rng = np.random.default_rng(w)
+    img = rng.normal(1000.0, 10.0, (h, w)).astype(np.float32)
+    img[rng.random((h, w)) < 0.025] = -1e30
+    g = run_both(gpu_ctx, img, conv=masks[mask], deblend_nthresh=nthresh, deblend_mincont=mincont)
+    assert g["fdpeak"].max() > 1e28
