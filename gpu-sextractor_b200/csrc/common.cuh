@@ -83,8 +83,9 @@ __device__ __forceinline__ int sx_count(int n, const int *n_dev) { return n_dev 
 // The value v * 2^(e-23) is exact; e is the smallest binary exponent of the
 // non-zero terms seen so far.  Adding a smaller-exponent term shifts v left
 // (exactly).  Any order of adds and merges gives the same exact value, which
-// is rounded once when read; denormal terms count as zero; a sum whose
-// dynamic range would exceed 125 bits raises ovf.
+// is rounded once when read; denormal terms count as zero.  A partial sum that
+// would need more than 126 bits raises ovf.  Whether one does depends on the
+// order, so the kernel that reads the sum then takes it again as a WideSum.
 // ---------------------------------------------------------------------------
 #define XS_EMPTY 1000
 
@@ -106,6 +107,12 @@ __device__ __forceinline__ int xs_bits(__int128 v) {
     if (hi) return 128 - __clzll(hi);
     if (lo) return 64 - __clzll(lo);
     return 0;
+}
+
+// |v| at or above 2^126: two of them could wrap
+__device__ __forceinline__ bool xs_full(__int128 v) {
+    const unsigned long long hi = (unsigned long long)((unsigned __int128)v >> 64);
+    return (hi ^ (hi << 1)) >> 63;
 }
 
 __device__ __forceinline__ void xs_rescale(XSum &s, int e) {
@@ -139,6 +146,7 @@ __device__ __forceinline__ void xs_add(XSum &s, float f) {
         s.v -= t;
     else
         s.v += t;
+    if (xs_full(s.v)) s.ovf = 1;
 }
 
 __device__ __forceinline__ void xs_merge(XSum &s, XSum b) {
@@ -155,6 +163,7 @@ __device__ __forceinline__ void xs_merge(XSum &s, XSum b) {
         xs_rescale(b, s.e);
     if (b.ovf) s.ovf = 1;
     s.v += b.v;
+    if (xs_full(s.v)) s.ovf = 1;
 }
 
 // exact value -> nearest double (ties to even)
@@ -231,6 +240,7 @@ __device__ __forceinline__ XSum xs_warp_sum(XSum s) {
             v += (__int128)(((unsigned __int128)hi << 64) | lo);
         }
         r.v = v;
+        r.ovf |= xs_full(v);
         return r;
     }
     s = xs_warp_reduce_tree(s);
@@ -312,11 +322,119 @@ __device__ __forceinline__ void xs_add_double(XSum &s, double d) {
         s.v -= t;
     else
         s.v += t;
+    if (xs_full(s.v)) s.ovf = 1;
 }
 
 __device__ __forceinline__ void xs_add_bins(XSum &s, double b0, double b1) {
     xs_add_double(s, b1);
     xs_add_double(s, b0);
+}
+
+// ---------------------------------------------------------------------------
+// Exact sums in any order, for the few that XSum does not hold: 320-bit integers
+// in units of 2^-149, which hold 2^31 terms of any finite size; denormal terms
+// count as zero, as in xs_add.  bad: a term is not finite, or the terms span
+// more than WS_SPAN binary orders, which XSum holds in no order (one of its
+// mantissas shifted by more than 101 bits needs more than 125).
+// ---------------------------------------------------------------------------
+constexpr unsigned WS_SPAN = 101;
+constexpr int WS_WORDS = 5;
+
+struct WideSum {
+    unsigned long long w[WS_WORDS];
+    unsigned lo, hi;  // smallest and largest exponent field of a term
+    int bad;          // (of a warp's total)
+};
+
+__device__ __forceinline__ void ws_init(WideSum &s) {
+#pragma unroll
+    for (int k = 0; k < WS_WORDS; k++) s.w[k] = 0ull;
+    s.lo = 255u;
+    s.hi = 0u;
+    s.bad = 0;
+}
+
+// w += t, or -= t as adding ~t and 1
+__device__ __forceinline__ void ws_add_words(WideSum &s, const unsigned long long (&t)[WS_WORDS], bool neg) {
+    unsigned long long carry = neg;
+#pragma unroll
+    for (int k = 0; k < WS_WORDS; k++) {
+        const unsigned long long a = s.w[k] + carry, b = a + (neg ? ~t[k] : t[k]);
+        carry = (unsigned long long)(a < carry) | (unsigned long long)(b < a);
+        s.w[k] = b;
+    }
+}
+
+__device__ __forceinline__ void ws_add(WideSum &s, float f) {
+    const unsigned u = __float_as_uint(f), ef = (u >> 23) & 0xff;
+    if (ef == 0u) return;
+    s.lo = min(s.lo, ef);
+    s.hi = max(s.hi, ef);
+    if (ef == 255u) return;
+    const unsigned sh = ef - 1u, o = sh & 63u;
+    const int q = (int)(sh >> 6);
+    const unsigned long long m = (u & 0x7fffffu) | 0x800000u, lo = m << o, hi = o > 40u ? m >> (64u - o) : 0ull;
+    unsigned long long t[WS_WORDS];
+#pragma unroll
+    for (int k = 0; k < WS_WORDS; k++) t[k] = k == q ? lo : k == q + 1 ? hi : 0ull;
+    ws_add_words(s, t, (u >> 31) != 0u);
+}
+
+// the warp's total, in every lane
+__device__ __forceinline__ WideSum ws_warp_sum(WideSum s) {
+    for (int o = 16; o > 0; o >>= 1) {
+        unsigned long long t[WS_WORDS];
+#pragma unroll
+        for (int k = 0; k < WS_WORDS; k++) t[k] = __shfl_xor_sync(0xffffffffu, s.w[k], o);
+        ws_add_words(s, t, false);
+    }
+    s.lo = __reduce_min_sync(0xffffffffu, s.lo);
+    s.hi = __reduce_max_sync(0xffffffffu, s.hi);
+    s.bad = s.hi == 255u || (s.hi > s.lo && s.hi - s.lo > WS_SPAN);
+    return s;
+}
+
+// exact value -> nearest double (ties to even)
+__device__ __forceinline__ double ws_double(WideSum s) {
+    const bool neg = s.w[WS_WORDS - 1] >> 63;
+    if (neg) {
+        WideSum z;
+        ws_init(z);
+        ws_add_words(z, s.w, true);
+        s = z;
+    }
+    // the top word that is not zero, the one below it, and the others
+    int q = -1;
+#pragma unroll
+    for (int k = 0; k < WS_WORDS; k++)
+        if (s.w[k] != 0ull) q = k;
+    if (q < 0) return 0.0;
+    unsigned long long top = 0ull, next = 0ull, rest = 0ull;
+#pragma unroll
+    for (int k = 0; k < WS_WORDS; k++) {
+        top = k == q ? s.w[k] : top;
+        next = k == q - 1 ? s.w[k] : next;
+        rest |= k < q - 1 ? s.w[k] : 0ull;
+    }
+    const int lead = __clzll((long long)top);
+    unsigned long long v = lead ? top << lead | next >> (64 - lead) : top;
+    if ((next << lead | rest) != 0ull) v |= 1ull;
+    const double d = scalbn(__ull2double_rn(v), 64 * q - lead - 149);
+    return neg ? -d : d;
+}
+
+// f(o) by the whole warp, for the o of each lane with need set, one after the
+// other (every lane of the warp calls this); false if there was none.  Callers
+// have loaded what else they need before: the vote waits for need.
+template <class F>
+__device__ __forceinline__ bool warp_each(bool need, int o, F f) {
+    unsigned m = __ballot_sync(0xffffffffu, need);
+    if (!m) return false;
+    for (; m; m &= m - 1u) {
+        f(__shfl_sync(0xffffffffu, o, __ffs(m) - 1));
+        __syncwarp();
+    }
+    return true;
 }
 
 // orderable integer image of a float (monotone for all finite floats)

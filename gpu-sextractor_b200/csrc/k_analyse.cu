@@ -153,15 +153,22 @@ __global__ void __launch_bounds__(AN_WARPS * 32, 2) k_analyse_robust_big(AnaArgs
 __global__ void k_robust_finish(AnaArgs A) {
     sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= sx_count(A.nobj, A.nobj_dev) || A.O.level[o] == 0) return;
-    const MomentRaw R = A.raw[o];
+    const bool live = o < sx_count(A.nobj, A.nobj_dev) && A.O.level[o] != 0;
+    const int oo = live ? o : 0;
+    MomentRaw R = A.raw[oo];
+    int flags = A.O.flags[oo];
+    const double dth = A.O.dthr[oo];
+    const double mxo = A.O.mx[oo], myo = A.O.my[oo];
+    if (warp_each(live && R.ovf, o, [&](int q) {
+            pix_moments_wide(A.cd, A.sub, A.opix + A.O.off[q], A.O.n[q], A.wdiv, A.w, A.raw + q);
+        }))
+        R = A.raw[oo];
+    if (!live) return;
     if (R.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
     const int xmin = R.xmin, ymin = R.ymin, dnpix = R.dnpix, area2 = R.area2;
-    int flags = A.O.flags[o];
     if (xmin == 0 || R.xmax == A.w - 1 || ymin == 0 || R.ymax == A.h - 1) flags |= SX_OBJ_TRUNC;
     const float rv = R.rv, peak = R.peak, cpeak = R.cpeak;
-    const double dth = A.O.dthr[o], dthresh2 = (dth + peak) / 2.0;
-    double mxo = A.O.mx[o], myo = A.O.my[o];
+    const double dthresh2 = (dth + peak) / 2.0;
     double rvd = rv, mx = R.mx, my = R.my;
     double mx2 = R.mx2, my2 = R.my2, mxy = R.mxy;
     double xm = mx / rvd, ym = my / rvd, xm2, ym2, xym;
@@ -433,24 +440,51 @@ __global__ void __launch_bounds__(AN_WARPS * 32, AN_MINB) k_examineiso(AnaArgs A
     }
 }
 
+// an object's flux and variance by one warp where XSum did not hold one of them
+// (ovf), into its state; ovf: WideSum::bad
+__device__ __noinline__ void exam_wide(const AnaArgs &A, int o) {
+    ExamRaw &X = A.xraw[o];
+    const unsigned *pix = A.opix + A.O.off[o];
+    const int n = A.O.n[o];
+    WideSum s, v;
+    ws_init(s);
+    ws_init(v);
+    for (int i = threadIdx.x & 31; i < n; i += 32) {
+        const unsigned p = pix[i];
+        ws_add(s, A.sub[p]);
+        if (A.wvar) ws_add(v, A.wvar[p]);
+    }
+    s = ws_warp_sum(s);
+    v = ws_warp_sum(v);
+    if ((threadIdx.x & 31) == 0) {
+        X.tv = ws_double(s);
+        X.svar = ws_double(v);
+        X.ovf = s.bad | v.bad;
+    }
+}
+
 // examineiso, per object: position errors, fluxes, FWHM fit, background
 // (one thread per object, so that this double-precision tail does not run on
 // one lane of a warp)
-__global__ void k_examine_finish(AnaArgs A) {
+__global__ void k_examine_finish(const __grid_constant__ AnaArgs A) {
     sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= sx_count(A.nobj, A.nobj_dev)) return;
-    const ExamRaw X = A.xraw[o];
+    const bool live = o < sx_count(A.nobj, A.nobj_dev);
+    const int oo = live ? o : 0;
+    ExamRaw X = A.xraw[oo];
+    const int n = A.O.n[oo], w = A.w;
+    const double mxo = A.O.mx[oo], myo = A.O.my[oo];
+    const float backsig = A.sc->backsig;
+    const double var = backsig * backsig;
+    const float dbkg = A.O.dbkg ? A.O.dbkg[oo] : 0.0f;
+    const int singu = A.O.singu[oo];
+    const float fdflux = A.O.fdflux[oo], a = A.O.a[oo], b = A.O.b[oo];
+    if (warp_each(live && X.ovf, o, [&](int q) { exam_wide(A, q); })) X = A.xraw[oo];
+    if (!live) return;
     double esum = X.err[0], emx2 = X.err[1], emy2 = X.err[2], emxy = X.err[3];
     const double s = X.fit[0], sx = X.fit[1], sy = X.fit[2], sxx = X.fit[3], sxy = X.fit[4];
     const float opeak = X.opeak, thresh0 = X.thresh0, mthresh = X.mthresh;
-    const int peakpix = X.peakpix, area = X.area, n = A.O.n[o], w = A.w;
-    const double mxo = A.O.mx[o], myo = A.O.my[o];
-    const float backsig = A.sc->backsig;
-    const double var = backsig * backsig;
-    const float dbkg = A.O.dbkg ? A.O.dbkg[o] : 0.0f;
-    const int singu = A.O.singu[o];
-    const float fdflux = A.O.fdflux[o], a = A.O.a[o], b = A.O.b[o];
+    const int peakpix = X.peakpix, area = X.area;
     float bkg = back_at(A.back, A.nbx, A.nby, A.bw, A.bh, (int)(mxo + 0.5), (int)(myo + 0.5));
     {
         double flux2 = fdflux * fdflux;

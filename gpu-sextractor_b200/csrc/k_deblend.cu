@@ -1079,16 +1079,24 @@ __global__ void __launch_bounds__(DT_THREADS, 2) k_da_moments_big(const __grid_c
 __global__ void k_da_finish(const __grid_constant__ DebArgs A) {
     sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= sx_count(A.nobj, A.nobj_dev)) return;
-    const MomentRaw R = A.raw[o];
+    const bool live = o < sx_count(A.nobj, A.nobj_dev);
+    const int oo = live ? o : 0;
+    MomentRaw R = A.raw[oo];
+    const int L = A.O.level[oo];
+    const double dthresh = A.O.node_dthresh[oo];
+    if (warp_each(live && R.ovf, o, [&](int q) {
+            pix_moments_wide(A.cd, A.sub, A.D.ownpix + A.O.off[q], A.O.n[q], A.wdiv, A.w, A.raw + q);
+        }))
+        R = A.raw[oo];
+    if (!live) return;
     if (R.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
-    const int L = A.O.level[o], xmin = R.xmin, xmax = R.xmax, ymin = R.ymin, ymax = R.ymax;
+    const int xmin = R.xmin, xmax = R.xmax, ymin = R.ymin, ymax = R.ymax;
     int flag = 0;
     if (L > 0) flag |= SX_OBJ_MERGED;
     if (xmin == 0 || xmax == A.w - 1 || ymin == 0 || ymax == A.h - 1) flag |= SX_OBJ_TRUNC;
     const float rv = R.rv, peak = R.peak;
     const double rvd = rv, mx = R.mx, my = R.my, mx2 = R.mx2, my2 = R.my2, mxy = R.mxy;
-    const double dthresh = A.O.node_dthresh[o], dthresh2 = (dthresh + peak) / 2.0;
+    const double dthresh2 = (dthresh + peak) / 2.0;
     const double xm = mx / rvd, ym = my / rvd;
     double xm2 = mx2 / rvd - xm * xm, ym2 = my2 / rvd - ym * ym, xym = mxy / rvd - xm * ym;
     double temp, temp2, theta, pmx2, pmy2, darea, t1t2;

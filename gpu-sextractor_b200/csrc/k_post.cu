@@ -390,18 +390,22 @@ struct KronLane {
 // a warp's sums over rows y0 .. y1 - 1 and strips c0, c0 + cstep, ... of the
 // box; area, areab in every lane.  BIN: in double bins (hints: the object's peak
 // and, for r*pix, the ellipse's largest r, for the variances the frame's);
-// false when a term did not fit.  Otherwise with XSum.
-template <int PASS, bool WVAR, bool BIN>
+// false when a term did not fit.  XS: with XSum.  WIDE: with WideSum (t0: the
+// sum of the lane's parity; x.ovf: WideSum::bad).
+enum { KS_BIN, KS_XS, KS_WIDE };
+
+template <int PASS, bool WVAR, int MODE>
 __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, double my, const KronGeo &g, int y0,
                                             int y1, int c0, int cstep, KronLane &out, int &area_out, int &areab_out) {
     const int lane = threadIdx.x & 31, w = A.w, h = A.h;
     const int cl = lane & 7, rl = lane >> 3;
     const int corrflag = (A.mask_type == 2);
-    constexpr bool TWO = PASS == 1 || WVAR;
+    constexpr bool TWO = PASS == 1 || WVAR, BIN = MODE == KS_BIN;
     const int W = bin_width(min((y1 - y0) * (g.xmax - g.xmin), BIN_MAX_TERMS));
     unsigned low0 = 0u, low1 = 0u;
     Bin2 b0, b1;
     XSum x0, x1;
+    WideSum w0, w1;
     if (BIN) {
         const int peak = bs_order(A.O.peak[o]);
         low0 = bin_low(PASS == 1 ? peak + bs_order(sqrtf(g.klim2)) + 1 : peak, W);
@@ -409,9 +413,12 @@ __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, 
         low1 = bin_low(WVAR ? bs_order(bsig * bsig) + 8 : peak, W);
         bin_init(b0);
         bin_init(b1);
-    } else {
+    } else if (MODE == KS_XS) {
         xs_init(x0);
         xs_init(x1);
+    } else {
+        ws_init(w0);
+        ws_init(w1);
     }
     int area = 0, areab = 0;
     bool ok = true;
@@ -475,9 +482,12 @@ __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, 
                         if (BIN) {
                             ok &= bin_add(b0, rp, low0, W);
                             ok &= bin_add(b1, pix, low1, W);
-                        } else {
+                        } else if (MODE == KS_XS) {
                             xs_add(x0, rp);
                             xs_add(x1, pix);
+                        } else {
+                            ws_add(w0, rp);
+                            ws_add(w1, pix);
                         }
                     } else
                         areab++;
@@ -502,9 +512,12 @@ __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, 
                     if (BIN) {
                         ok &= bin_add(b0, pix, low0, W);
                         if (WVAR) ok &= bin_add(b1, pv, low1, W);
-                    } else {
+                    } else if (MODE == KS_XS) {
                         xs_add(x0, pix);
                         if (WVAR) xs_add(x1, pv);
+                    } else {
+                        ws_add(w0, pix);
+                        if (WVAR) ws_add(w1, pv);
                     }
                 }
             }
@@ -519,10 +532,15 @@ __device__ __forceinline__ bool kron_strips(const EndArgs &A, int o, double mx, 
         const int src = 16 * (lane & 1);
         out.t0 = __shfl_sync(0xffffffffu, r, src);
         out.t1 = __shfl_sync(0xffffffffu, r, src + 8);
-    } else {
+    } else if (MODE == KS_XS) {
         x0 = xs_warp_sum(x0);
         x1 = xs_warp_sum(x1);
         out.x = lane & 1 ? x1 : x0;
+    } else {
+        w0 = ws_warp_sum(w0);
+        w1 = ws_warp_sum(w1);
+        out.t0 = ws_double(lane & 1 ? w1 : w0);
+        out.x.ovf = w0.bad | w1.bad;
     }
     area_out = __reduce_add_sync(0xffffffffu, area);
     areab_out = __reduce_add_sync(0xffffffffu, areab);
@@ -535,7 +553,7 @@ __device__ __noinline__ void kron_strips_xsum(const EndArgs &A, int o, double mx
                                               int y1, int c0, int cstep, KronPart *out) {
     KronLane l;
     int area, areab;
-    kron_strips<PASS, WVAR, false>(A, o, mx, my, g, y0, y1, c0, cstep, l, area, areab);
+    kron_strips<PASS, WVAR, KS_XS>(A, o, mx, my, g, y0, y1, c0, cstep, l, area, areab);
     out->s0 = l.x;
     out->area = area;
     out->areab = areab;
@@ -546,7 +564,7 @@ __device__ __forceinline__ void kron_warp(const EndArgs &A, int o, double mx, do
                                           int y1, int c0, int cstep, KronLane &l, int &area, int &areab) {
     // at most BIN_MAX_TERMS terms of the warp per bin
     l.binned = (long long)(y1 - y0) * (g.xmax - g.xmin) <= BIN_MAX_TERMS &&
-               kron_strips<PASS, WVAR, true>(A, o, mx, my, g, y0, y1, c0, cstep, l, area, areab);
+               kron_strips<PASS, WVAR, KS_BIN>(A, o, mx, my, g, y0, y1, c0, cstep, l, area, areab);
     if (l.binned) return;
     KronPart p;
     kron_strips_xsum<PASS, WVAR>(A, o, mx, my, g, y0, y1, c0, cstep, &p);
@@ -568,6 +586,24 @@ __device__ __forceinline__ void kron_store(const EndArgs &A, int o, const KronLa
         R.ovf = ovf;
     } else if (lane == 1)
         R.s1 = d;
+}
+
+// an object's sums over its whole box by one warp, where XSum did not hold one of
+// them (R.ovf), into its state; R.ovf: WideSum::bad.  Called by the kernels
+// that read the sums, so that the passes keep their registers.
+template <int PASS, bool WVAR>
+__device__ __noinline__ void kron_box_wide(const EndArgs &A, int o) {
+    const int lane = threadIdx.x & 31;
+    const KronGeo g = A.geo[o];
+    KronLane l;
+    int area, areab;
+    kron_strips<PASS, WVAR, KS_WIDE>(A, o, A.O.mx[o], A.O.my[o], g, g.ymin, g.ymax, 0, 1, l, area, areab);
+    EndRaw &R = A.raw[o];
+    if (lane == 0) {
+        R.s0 = l.t0;
+        R.ovf = l.x.ovf;
+    } else if (lane == 1)
+        R.s1 = l.t0;
 }
 
 // Queue object o's pass-`pass` box (one thread).  False when the queue is
@@ -735,16 +771,23 @@ __global__ void __launch_bounds__(EO_WARPS * 32, 8) k_end_pass(const __grid_cons
 __global__ void k_kron_mid(const __grid_constant__ EndArgs A) {
     sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= sx_count(A.n, A.n_dev) || A.O.fmaster[o] >= 0) return;
-    EndRaw &R = A.raw[o];
-    if (R.ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
+    const bool live = o < sx_count(A.n, A.n_dev) && A.O.fmaster[o] < 0;
+    EndRaw &R = A.raw[live ? o : 0];
     const int areab = R.areab, area = R.area + R.areab;
+    double r1 = R.s0, v1 = R.s1;
+    int ovf = R.ovf;
+    if (warp_each(live && ovf, o, [&](int q) { kron_box_wide<1, false>(A, q); })) {
+        r1 = R.s0;
+        v1 = R.s1;
+        ovf = R.ovf;
+    }
+    if (!live) return;
+    if (ovf) atomicOr(&A.sc->status, SX_ST_RANGE);
     R.kron = 0.0f;
     R.have2 = 0;
     KronGeo g;
     if (!area) return;
     float kron;
-    const double r1 = R.s0, v1 = R.s1;
     if (r1 > 0.0 && v1 > 0.0) {
         kron = A.autoparam0 * r1 / v1;
         if (kron < A.autoparam1) kron = A.autoparam1;
@@ -767,11 +810,10 @@ __global__ void k_kron_mid(const __grid_constant__ EndArgs A) {
 __global__ void k_end_finish(const __grid_constant__ EndArgs A) {
     sx_pdl();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= sx_count(A.n, A.n_dev)) return;
-    const bool victim = A.O.fmaster[o] >= 0;
-    A.surv[o] = victim ? 0 : 1;
-    if (victim) return;
-    for (int k = 0; k < A.naper; k++) {
+    const bool live = o < sx_count(A.n, A.n_dev), victim = live && A.O.fmaster[o] >= 0;
+    if (live) A.surv[o] = victim ? 0 : 1;
+    const bool mine = live && !victim;
+    for (int k = 0; mine && k < A.naper; k++) {
         const double2 ap = A.aper[(size_t)o * A.naper + k];
         const double tv = ap.x;
         double sigtv = ap.y;
@@ -788,7 +830,15 @@ __global__ void k_end_finish(const __grid_constant__ EndArgs A) {
         }
         if (A.naper > 1) A.O.aper[(size_t)o * A.naper + k] = make_float4(f, fe, mg, me);
     }
-    const EndRaw R = A.raw[o];
+    EndRaw R = A.raw[mine ? o : 0];
+    if (warp_each(mine && R.have2 && R.ovf, o, [&](int q) {
+            if (A.wvar)
+                kron_box_wide<2, true>(A, q);
+            else
+                kron_box_wide<2, false>(A, q);
+        }))
+        R = A.raw[mine ? o : 0];
+    if (!mine) return;
     const bool have2 = R.have2 != 0;
     int flags = R.flags;
     float kron = R.kron;

@@ -198,6 +198,44 @@ __device__ __forceinline__ void pix_moments_warp(const float *cd, const float *s
     pix_moments_store(v, ovf, dn, a2, b, R);
 }
 
+// The sums of a list by one warp where XSum did not hold one of them (R->ovf),
+// one pass over the list each, into R; R->ovf: WideSum::bad.  Called by
+// the finishing kernels, so that the kernels that sum keep their registers.
+__device__ __noinline__ void pix_moments_wide(const float *cd, const float *sub, const unsigned *pix, int n,
+                                              FastDiv wdiv, int w, MomentRaw *R) {
+    const int lane = threadIdx.x & 31, x0 = R->xmin, y0 = R->ymin;
+    double mine = 0.0;
+    int bad = 0;
+    for (int k = 0; k < PM_SUMS; k++) {
+        WideSum s;
+        ws_init(s);
+        for (int i = lane; i < n; i += 32) {
+            const unsigned p = pix[i];
+            const int yy = (int)fdiv(p, wdiv), x = (int)p - yy * w - x0, y = yy - y0;
+            const float cval = cd[p];
+            ws_add(s, k == 0   ? cval
+                      : k == 1 ? sub[p]
+                      : k == 2 ? cval * x
+                      : k == 3 ? cval * y
+                      : k == 4 ? cval * x * x
+                      : k == 5 ? cval * y * y
+                               : cval * x * y);
+        }
+        s = ws_warp_sum(s);
+        bad |= s.bad;
+        const double d = ws_double(s);
+        if (lane == k) mine = d;
+    }
+    if (lane == 0)
+        R->rv = (float)mine;
+    else if (lane == 1)
+        R->tv = (float)mine;
+    else if (lane < PM_SUMS)
+        (&R->mx)[lane - 2] = mine;
+    else if (lane == PM_SUMS)
+        R->ovf = bad;
+}
+
 // a whole block over one list (at most 32 warps)
 struct PixBlock {
     PixBox box[32];

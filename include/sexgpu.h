@@ -35,7 +35,8 @@ extern "C" {
 #define SEXGPU_ERR_ARG        -1   /* bad argument (sizes, config values) */
 #define SEXGPU_ERR_CUDA       -2   /* CUDA runtime error */
 #define SEXGPU_ERR_NOMEM      -3   /* device allocation failed */
-#define SEXGPU_ERR_RANGE      -4   /* an exact sum exceeded its dynamic range */
+#define SEXGPU_ERR_RANGE      -4   /* a filtered value more than 100 binary orders above the smallest threshold,
+                                      or an exact sum whose terms are further apart or not finite */
 #define SEXGPU_ERR_CAPACITY   -5   /* caller buffer too small (count returned) */
 #define SEXGPU_ERR_NODEVICE   -6   /* no usable CUDA device */
 #define SEXGPU_ERR_THRESH     -7   /* zero or negative threshold (src/back.c:196) */

@@ -563,3 +563,39 @@ def test_deblending_far_above_the_threshold(gpu_ctx, masks, w, h, mask, nthresh,
     img[rng.random((h, w)) < 0.025] = -1e30
     g = run_both(gpu_ctx, img, conv=masks[mask], deblend_nthresh=nthresh, deblend_mincont=mincont)
     assert g["fdpeak"].max() > 1e28
+
+
+@pytest.mark.parametrize("length,bits,bright", [(60, 84, 12), (60, 88, 3), (60, 86, 25), (60, 94, 2), (200, 80, 12),
+                                                (200, 80, 40), (200, 82, 60), (200, 88, 40), (700, 76, 40), (700, 78, 200),
+                                                (700, 84, 3)])
+def test_sums_far_above_the_threshold(gpu_ctx, length, bits, bright):
+    """A bar with some pixels 2^bits above the others.  Its moments are exact sums
+    (math.fsum) where no term lies more than 101 binary orders above another,
+    though all together need more than the 126 bits that partial sums have and
+    would fit or not with the order of the pixels; where the oracle's 127 bits
+    hold them, every column is the oracle's.  Terms further apart are reported."""
+    import math
+    rng = np.random.default_rng(length + bits + bright)
+    img = np.zeros((64, length + 60), np.float32)
+    img[30:33, 30:30 + length] = rng.uniform(6, 20, (3, length))
+    img[24:30, 40:46] = rng.uniform(6, 20, (6, 6))
+    img[31, 30 + length - 1 - 2 * np.arange(bright)] = 2.0 ** bits * rng.uniform(6, 20, bright)
+    kw = dict(filter_flag=0, back_type=1, back_value=0.0, thresh_type=1, detect_thresh=5.0, analysis_thresh=5.0)
+    yy, xx = np.nonzero(img)
+    v, x, y = img[yy, xx], (xx - 30).astype(np.float32), (yy - 24).astype(np.float32)
+    terms = [t[t > 0].astype(np.float64) for t in (v, v * x, v * y, v * x * x, v * y * y, v * x * y)]
+    total, mx, my = (math.fsum(t) for t in terms[:3])
+    rv = float(np.float32(total))
+    span = max(int(np.ptp(np.frexp(t)[1])) for t in terms)
+    need = max(math.fsum(t) / 2.0 ** (np.frexp(t)[1].min() - 24) for t in terms)
+    for _ in range(3):
+        if span > 101:
+            with pytest.raises(RuntimeError, match="exact sum out of range"):
+                gpu_ctx.extract(img, **kw)
+            continue
+        g, _, _ = gpu_ctx.extract(img, **kw)
+        assert len(g) == 1
+        assert (g["fdflux"][0], g["dflux"][0], g["flux"][0]) == (np.float32(total),) * 3
+        assert (g["mx"][0], g["my"][0]) == (mx / rv + 30, my / rv + 24)
+        if need < 2.0 ** 126:
+            compare_catalogs(g, O.extract(img, **kw)[0])
