@@ -83,9 +83,12 @@ __device__ __forceinline__ int sx_count(int n, const int *n_dev) { return n_dev 
 // The value v * 2^(e-23) is exact; e is the smallest binary exponent of the
 // non-zero terms seen so far.  Adding a smaller-exponent term shifts v left
 // (exactly).  Any order of adds and merges gives the same exact value, which
-// is rounded once when read; denormal terms count as zero.  A partial sum that
-// would need more than 126 bits raises ovf.  Whether one does depends on the
-// order, so the kernel that reads the sum then takes it again as a WideSum.
+// is rounded once when read; denormal terms count as zero.  A term or a partial
+// sum that does not fit when it is brought to the smallest exponent raises ovf.
+// Whether one does depends on the order, so the kernel that reads the sum then
+// takes it again as a WideSum.  (Terms that fit one by one may still add up to
+// more than 127 bits: with FULL, for terms in no fixed order, that raises ovf
+// too.)
 // ---------------------------------------------------------------------------
 #define XS_EMPTY 1000
 
@@ -129,6 +132,7 @@ __device__ __forceinline__ void xs_rescale(XSum &s, int e) {
     s.e = e;
 }
 
+template <bool FULL = false>
 __device__ __forceinline__ void xs_add(XSum &s, float f) {
     unsigned int u = __float_as_uint(f);
     int ef = (int)((u >> 23) & 0xff);
@@ -146,9 +150,10 @@ __device__ __forceinline__ void xs_add(XSum &s, float f) {
         s.v -= t;
     else
         s.v += t;
-    if (xs_full(s.v)) s.ovf = 1;
+    if (FULL && xs_full(s.v)) s.ovf = 1;
 }
 
+template <bool FULL = false>
 __device__ __forceinline__ void xs_merge(XSum &s, XSum b) {
     if (b.ovf) s.ovf = 1;
     if (b.e == XS_EMPTY) return;
@@ -163,7 +168,7 @@ __device__ __forceinline__ void xs_merge(XSum &s, XSum b) {
         xs_rescale(b, s.e);
     if (b.ovf) s.ovf = 1;
     s.v += b.v;
-    if (xs_full(s.v)) s.ovf = 1;
+    if (FULL && xs_full(s.v)) s.ovf = 1;
 }
 
 // exact value -> nearest double (ties to even)
@@ -204,8 +209,9 @@ __device__ __forceinline__ XSum xs_shfl_down(const XSum &s, int off) {
 }
 
 // full-warp reduction by a merge tree; the result is valid in lane 0
+template <bool FULL>
 __device__ __noinline__ XSum xs_warp_reduce_tree(XSum s) {
-    for (int off = 16; off > 0; off >>= 1) xs_merge(s, xs_shfl_down(s, off));
+    for (int off = 16; off > 0; off >>= 1) xs_merge<FULL>(s, xs_shfl_down(s, off));
     return s;
 }
 
@@ -214,6 +220,7 @@ __device__ __noinline__ XSum xs_warp_reduce_tree(XSum s) {
 // add in an int128 without overflow (a butterfly of plain integer adds).
 // Otherwise the merge tree above decides, with its range check.  The exact
 // value, and so every rounding of it, is the same either way.
+template <bool FULL = false>
 __device__ __forceinline__ XSum xs_warp_sum(XSum s) {
     int emin = s.e;
     for (int o = 16; o > 0; o >>= 1) emin = min(emin, __shfl_xor_sync(0xffffffffu, emin, o));
@@ -240,10 +247,10 @@ __device__ __forceinline__ XSum xs_warp_sum(XSum s) {
             v += (__int128)(((unsigned __int128)hi << 64) | lo);
         }
         r.v = v;
-        r.ovf |= xs_full(v);
+        if (FULL) r.ovf |= xs_full(v);
         return r;
     }
-    s = xs_warp_reduce_tree(s);
+    s = xs_warp_reduce_tree<FULL>(s);
     unsigned long long lo = (unsigned long long)s.v, hi = (unsigned long long)(s.v >> 64);
     lo = __shfl_sync(0xffffffffu, lo, 0);
     hi = __shfl_sync(0xffffffffu, hi, 0);
@@ -301,6 +308,7 @@ __device__ __forceinline__ int bs_order(float f) { return (int)((__float_as_uint
 
 // s += d exactly, for a double d that is a multiple of a power of two no
 // smaller than 2^-1074 (every bin sum is)
+template <bool FULL = false>
 __device__ __forceinline__ void xs_add_double(XSum &s, double d) {
     if (d == 0.0) return;
     const unsigned long long u = (unsigned long long)__double_as_longlong(d);
@@ -322,12 +330,13 @@ __device__ __forceinline__ void xs_add_double(XSum &s, double d) {
         s.v -= t;
     else
         s.v += t;
-    if (xs_full(s.v)) s.ovf = 1;
+    if (FULL && xs_full(s.v)) s.ovf = 1;
 }
 
+template <bool FULL = false>
 __device__ __forceinline__ void xs_add_bins(XSum &s, double b0, double b1) {
-    xs_add_double(s, b1);
-    xs_add_double(s, b0);
+    xs_add_double<FULL>(s, b1);
+    xs_add_double<FULL>(s, b0);
 }
 
 // ---------------------------------------------------------------------------

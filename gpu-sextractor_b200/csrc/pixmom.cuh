@@ -77,7 +77,8 @@ __device__ __forceinline__ double warp_sum8(const double v[8], int lane) {
 }
 
 // the sums with XSum, for a term the bins do not hold (out of line: the rare
-// path, kept out of the callers' registers); lane k < PM_SUMS gets sum k
+// path, kept out of the callers' registers); lane k < PM_SUMS gets sum k (FULL:
+// a branch's own pixels come in any order)
 __device__ __noinline__ void pix_moments_xsum(const float *cd, const float *sub, const unsigned *pix, int i0, int i1,
                                               FastDiv wdiv, int w, int x0, int y0, XSum *out) {
     const int lane = threadIdx.x & 31;
@@ -87,18 +88,18 @@ __device__ __noinline__ void pix_moments_xsum(const float *cd, const float *sub,
         const unsigned p = pix[i];
         const int yy = (int)fdiv(p, wdiv), x = (int)p - yy * w - x0, y = yy - y0;
         const float cval = cd[p], val = sub[p];
-        xs_add(s[0], cval);
-        xs_add(s[1], val);
-        xs_add(s[2], cval * x);
-        xs_add(s[3], cval * y);
-        xs_add(s[4], cval * x * x);
-        xs_add(s[5], cval * y * y);
-        xs_add(s[6], cval * x * y);
+        xs_add<true>(s[0], cval);
+        xs_add<true>(s[1], val);
+        xs_add<true>(s[2], cval * x);
+        xs_add<true>(s[3], cval * y);
+        xs_add<true>(s[4], cval * x * x);
+        xs_add<true>(s[5], cval * y * y);
+        xs_add<true>(s[6], cval * x * y);
     }
     XSum mine;
     xs_init(mine);
     for (int k = 0; k < PM_SUMS; k++) {
-        const XSum t = xs_warp_sum(s[k]);
+        const XSum t = xs_warp_sum<true>(s[k]);
         if (lane == k) mine = t;
     }
     *out = mine;
@@ -259,11 +260,11 @@ __device__ __forceinline__ void pix_moments_block(const float *cd, const float *
         const int i1 = min(n, i0 + DA_WARP_MAX);
         double t0, t1;
         if (pix_moments(cd, sub, pix, i0, i1, wdiv, w, b, dth, t0, t1, dn, a2)) {
-            xs_add_bins(x, t0, t1);
+            xs_add_bins<true>(x, t0, t1);
         } else {
             XSum t;
             pix_moments_xsum(cd, sub, pix, i0, i1, wdiv, w, b.xmin, b.ymin, &t);
-            xs_merge(x, t);
+            xs_merge<true>(x, t);
         }
     }
     dn = __reduce_add_sync(0xffffffffu, dn);
@@ -278,7 +279,7 @@ __device__ __forceinline__ void pix_moments_block(const float *cd, const float *
         xs_init(x);
         dn = a2 = 0;
         for (int k = 0; k < nw; k++) {
-            if (lane < PM_SUMS) xs_merge(x, sh.x[k][lane]);
+            if (lane < PM_SUMS) xs_merge<true>(x, sh.x[k][lane]);
             dn += sh.dnpix[k];
             a2 += sh.area2[k];
         }
