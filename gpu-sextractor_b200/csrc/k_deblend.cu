@@ -1180,8 +1180,9 @@ __global__ void k_da_finish(const __grid_constant__ DebArgs A) {
 // less than 2^-23 of 1 + |offset|, so the quadratic form, of terms that add up
 // to T, by less than 2e-6 (T + the coefficients' sum).  In a raw object of many
 // branches most are far away: a bound by the offset alone passes those over
-// first (deblending of a cluster with one raw object of 2 M pixels 2.72 -> 2.55
-// ms; with few branches it only costs).
+// first: deblending of a cluster with one raw object of 2 M pixels 2.80 -> 2.51
+// ms, the same from 8, 16, 32 or 64 branches on; of a crowded field 1.360, 1.352,
+// 1.340 and 1.341 ms, 1.341 without.
 constexpr int GATHER_MANY = 32;  // branches
 
 __global__ void __launch_bounds__(DT_THREADS) k_da_gather(const __grid_constant__ DebArgs A) {

@@ -97,9 +97,20 @@ struct DevCache {
 constexpr int KR_CHUNK = 4096;     // box pixels per CTA work item (whole rows, at least one)
 // Larger boxes than this are queued, unless the caller has set a size: the fewer
 // objects there are, the sooner the longest box of a warp is what a pass waits
-// for.  Photometry of 3900 objects on 1024 x 1024 pixels: 0.086 ms at 1024, 0.105
-// at 2048, 0.19 at 8192; 19,500 (cluster): 0.37, 0.34, 0.34; 68,000: 1.40 (the
-// queue overflows), 0.62, 0.65; 780,000: 13.7, 11.4, 10.5 (10.46 at 6144).
+// for.  Photometry in ms by objects and size (fields of 0.006 sources a pixel up
+// to 20,800 objects, of 0.0119 above; 780,000 are a mosaic of its own):
+//              1024    2048    6144    8192 pixels
+//     3,900   0.088   0.107   0.172   0.170
+//     7,100   0.117   0.125   0.201   0.197
+//    10,500   0.131   0.153   0.204   0.206
+//    20,800   0.195   0.198   0.235   0.255
+//    77,900   0.971   0.633   0.656   0.672   (the queue overflows at 1024)
+//   116,000   1.305   0.906   0.914   0.924
+//   146,000   1.497   1.099   1.113   1.113
+//   190,000   1.762   1.414   1.386   1.399
+//   780,000   13.7    11.4    10.46   10.5
+// Neither line costs much where it lies: 1024 would be as good or better up to some
+// 20,000 objects, and 2048 up to some 150,000.
 inline int kr_warp_max(int nobj) { return nobj <= 8192 ? 1024 : nobj <= 131072 ? 2048 : 6144; }
 // queued boxes and work items per pass: an eighth of the objects and 8 items
 // each, at least 8192 boxes (a crowded mosaic queues 2% of its objects; with
